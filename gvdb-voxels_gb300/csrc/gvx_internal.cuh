@@ -172,10 +172,7 @@ struct GvxNoAllocScope {
 
 // ---- onesweep radix sort (gvx_sort.cu) -----------------------------------
 struct SortScratch {
-    DevBuf hist;      // passes * 256 counts
-    DevBuf base;      // passes * 256 exclusive bases
-    DevBuf lookback;  // tiles * 256 status words
-    DevBuf counter;   // tile counters, one per pass
+    DevBuf buf;  // digit histograms, tile counters and look-back words (gvx_sort.cu)
 };
 // one sort pass with its first tile withheld: the bounded look-back times out (a test hook)
 gvx_status gvx_sort_pass_withheld_tile(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
@@ -183,13 +180,23 @@ gvx_status gvx_sort_pass_withheld_tile(const uint32_t* kin, const uint32_t* vin,
                                        int64_t* launches);
 // Sorts (keys, vals) by the low `bits` bits of the keys, stable.  The keys
 // must already be in keys[0]/vals[0]; the result ends in buffer index *result
-// (0 or 1).  If the histogram of the pass digits was accumulated by the
-// producer of the keys (hist_ready), it is used as is.
+// (0 or 1).  `prepared`: gvx_sort_prepare(s, n, bits) was queued and the producer of the
+// keys has counted their digits into gvx_sort_hist_ptr(s) since.
 gvx_status gvx_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], uint32_t n, int bits, SortScratch& s,
-                          bool hist_ready, cudaStream_t st, uint32_t* d_err, int* result, int64_t* launches);
+                          bool prepared, cudaStream_t st, uint32_t* d_err, int* result, int64_t* launches);
+// the same from (kin, vin), left as they are, into (kout, vout), by way of (ktmp, vtmp) when
+// more than one pass is needed; no two of the six overlap; n > 1, bits > 0
+gvx_status gvx_sort_pairs_to(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout,
+                             uint32_t* ktmp, uint32_t* vtmp, uint32_t n, int bits, SortScratch& s, cudaStream_t st,
+                             uint32_t* d_err, int64_t* launches);
+// one pass over `tiles` tiles of `tile` pairs (1024, 4096 or 8192) by the digit (key >> shift) & 255,
+// hist: how often each digit occurs in the whole input
+gvx_status gvx_onesweep_pass(uint32_t tile, uint32_t tiles, const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
+                             uint32_t* vout, uint32_t n, int shift, const uint32_t* hist, uint32_t* lookback,
+                             uint32_t* counter, uint32_t* err, cudaStream_t st);
 int gvx_sort_passes(int bits);
-// zero the global histogram before a fused key producer accumulates into it
-gvx_status gvx_sort_prepare_hist(SortScratch& s, int bits, cudaStream_t st);
+// the scratch of a sort of n keys, zeroed, before its key producer counts digits into the histograms
+gvx_status gvx_sort_prepare(SortScratch& s, uint32_t n, int bits, cudaStream_t st);
 uint32_t* gvx_sort_hist_ptr(SortScratch& s);
 
 // device helper used by key producers: accumulate digit histograms of a key

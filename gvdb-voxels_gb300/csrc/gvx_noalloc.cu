@@ -34,17 +34,13 @@
 
 // the onesweep kernels of gvx_sort.cu
 __global__ void k_sort_hist(const uint32_t* keys, uint32_t n, int passes, uint32_t* hist);
-__global__ void k_sort_bases(const uint32_t* hist, uint32_t* base);
-__global__ void k_onesweep(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint32_t n,
-                           int shift, const uint32_t* base, uint32_t* lookback, uint32_t* counter, uint32_t* err);
 
 namespace {
 constexpr uint32_t kMaxKeys = GVX_NOALLOC_SORT_MAX_KEYS;
-constexpr uint32_t kTile = 4096;  // keys per onesweep tile (gvx_sort.cu)
+constexpr uint32_t kTile = 4096;  // pairs per onesweep tile (gvx_sort.cu)
 constexpr uint32_t kMaxTiles = (kMaxKeys + kTile - 1) / kTile;
 constexpr size_t kHistOff = 0;                                       // 4 passes * 256 counts
-constexpr size_t kBaseOff = kHistOff + 4 * 256 * 4;                  // 4 passes * 256 bases
-constexpr size_t kCounterOff = kBaseOff + 4 * 256 * 4;               // 4 tile counters
+constexpr size_t kCounterOff = kHistOff + 4 * 256 * 4;               // 4 tile counters
 constexpr size_t kErrOff = kCounterOff + 256;                        // device error word (sticky)
 constexpr size_t kLookbackOff = kErrOff + 256;                       // 4 passes * tiles * 256 words
 constexpr size_t kKeysOff = kLookbackOff + (size_t)4 * kMaxTiles * 256 * 4;
@@ -159,7 +155,6 @@ extern "C" gvx_status gvx_radix_sort_noalloc(const uint32_t* keys_in, const uint
     const int passes = (bits + 7) / 8;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     uint32_t* hist = (uint32_t*)(base + kHistOff);
-    uint32_t* bases = (uint32_t*)(base + kBaseOff);
     uint32_t* counter = (uint32_t*)(base + kCounterOff);
     uint32_t* err = (uint32_t*)(base + kErrOff);
     uint32_t* lookback = (uint32_t*)(base + kLookbackOff);
@@ -172,7 +167,6 @@ extern "C" gvx_status gvx_radix_sort_noalloc(const uint32_t* keys_in, const uint
     GVX_CK(cudaMemsetAsync(counter, 0, 4 * 4, st));
     GVX_CK(cudaMemsetAsync(lookback, 0, (size_t)passes * tiles * 256 * 4, st));
     k_sort_hist<<<tiles < 1024 ? tiles : 1024, 256, 0, st>>>(keys_in, n, passes, hist);
-    k_sort_bases<<<passes, 256, 0, st>>>(hist, bases);
     // the last pass lands in the caller's output; earlier passes alternate with
     // the scratch copy.  With an odd pass count the first pass writes the
     // output, so an input that overlaps an output is first copied to the
@@ -191,8 +185,8 @@ extern "C" gvx_status gvx_radix_sort_noalloc(const uint32_t* keys_in, const uint
         const bool to_out = ((passes - 1 - p) & 1) == 0;
         uint32_t* kdst = to_out ? keys_out : ktmp;
         uint32_t* vdst = to_out ? vals_out : vtmp;
-        k_onesweep<<<tiles, 256, 0, st>>>(ksrc, vsrc, kdst, vdst, n, 8 * p, bases + p * 256,
-                                          lookback + (size_t)p * tiles * 256, counter + p, err);
+        GVX_CK_STATUS(gvx_onesweep_pass(kTile, tiles, ksrc, vsrc, kdst, vdst, n, 8 * p, hist + p * 256,
+                                        lookback + (size_t)p * tiles * 256, counter + p, err, st));
         ksrc = kdst;
         vsrc = vdst;
     }
@@ -238,7 +232,6 @@ extern "C" gvx_status gvx_test_sort_noalloc_withheld_tile(const uint32_t* keys_i
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t* hist = (uint32_t*)(base + kHistOff);
-    uint32_t* bases = (uint32_t*)(base + kBaseOff);
     uint32_t* counter = (uint32_t*)(base + kCounterOff);
     uint32_t* err = (uint32_t*)(base + kErrOff);
     uint32_t* lookback = (uint32_t*)(base + kLookbackOff);
@@ -247,8 +240,8 @@ extern "C" gvx_status gvx_test_sort_noalloc_withheld_tile(const uint32_t* keys_i
     GVX_CK(cudaMemsetAsync(lookback, 0, (size_t)tiles * 256 * 4, st));
     GVX_CK(cudaMemcpyAsync(counter, &one, 4, cudaMemcpyHostToDevice, st));
     k_sort_hist<<<tiles < 1024 ? tiles : 1024, 256, 0, st>>>(keys_in, n, 1, hist);
-    k_sort_bases<<<1, 256, 0, st>>>(hist, bases);
-    k_onesweep<<<tiles - 1, 256, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n, 0, bases, lookback, counter, err);
+    GVX_CK_STATUS(gvx_onesweep_pass(kTile, tiles - 1, keys_in, vals_in, keys_out, vals_out, n, 0, hist, lookback,
+                                    counter, err, st));
     GVX_CK(cudaGetLastError());
     return GVX_OK;
 }

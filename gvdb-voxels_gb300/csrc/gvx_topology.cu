@@ -1201,7 +1201,7 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
     const uint32_t invalid_key = 1u << (ks.total_bits + kshift);
     const int bits = ks.total_bits + kshift + 1;
     const int passes = gvx_sort_passes(bits);
-    gvx_status rc = gvx_sort_prepare_hist(g->sort, bits, g->stream);
+    gvx_status rc = gvx_sort_prepare(g->sort, (uint32_t)n, bits, g->stream);
     if (rc) return rc;
     const unsigned kb = std::min(blocks_for(n, 256), 152u * 8u);
     k_keys<<<kb, 256, 0, g->stream>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, t[0], t[1], t[2],
