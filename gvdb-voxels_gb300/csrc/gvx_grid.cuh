@@ -119,6 +119,10 @@ struct gvx_grid {
     bool oct_valid = false;  // the sorted points are in octant order inside every leaf, leaf_oct filled
     uint32_t oct_leaves = 0;
     DevCount oct_count{};  // leaves to partition, read on the device (a planned build); else oct_leaves
+    // leaves of many points (kDenseLeaf), bricks of 8: their points in cell order inside every octant
+    int* leaf_dense = nullptr;      // per leaf 0, or 1 + its number among them (in leaf_oct's buffer); null: none are made
+    uint32_t* dense_count = nullptr;
+    DevBuf cell_tab;                // per dense leaf the first sorted index of its 512 cells; the list of the dense leaves
     DevBuf leaf_slot;    // atlas slot per leaf, -1 if inactive
     DevBuf slot_leaf;    // leaf per atlas slot (active slots only)
     DevBuf nbr;          // 27 leaf indices per leaf
@@ -172,8 +176,9 @@ struct gvx_grid {
     DevBuf inc0, inc_remap;  // incremental build: linked + new level-0 bitmaps, linked rank -> pool index
     DevBuf d_err, d_bbox;
     DevBuf d_rmax;  // float bits of the largest per-point radius of the last point permute
-    DevBuf d_next;  // work-unit counter of the splat launch (+ the count of touched slots)
+    DevBuf d_next;  // work-unit counters of the splat launch
     DevBuf touched; // slots an accumulating splat visits
+    DevBuf dense_units;  // units the trilinear density splat lists for k_tri_dense
     void* h_pin = nullptr;  // pinned staging of the topology's small readbacks
     struct gvx_topo_staged* staged = nullptr;  // a staged RebuildTopology between its stages (batches)
     struct gvx_topo_plan* plan = nullptr;      // fixed key space and capacities of planned builds

@@ -133,6 +133,12 @@ struct SplatArgs {
     // reach (unit_slots[0 .. *unit_count), in no particular order); null: every slot
     const uint32_t* unit_slots;
     const uint32_t* unit_count;
+    // k_splat_tri, bricks of 8: per leaf 0 or 1 + its number among the dense leaves, whose points are in
+    // cell order, and per dense leaf the first sorted index of each of its 512 cells; null: no such order
+    const int* leaf_dense;
+    const int* cell_tab;
+    uint32_t* dense_units;  // units listed for k_tri_dense, and the list (grid, slot, z0, layers); null: none are
+    uint4* dense_list;
 };
 
 // Shared-memory tile of one padded brick.  Density only: float per voxel.
@@ -494,6 +500,30 @@ __device__ __forceinline__ void push_out(const SplatArgs& a, const unsigned char
     }
 }
 
+// the apron regions `reset` (bit (dx+1)*9 + (dy+1)*3 + (dz+1)) of a slab's tile to the boundary value
+template <bool HAS_DEN, bool HAS_VEL>
+__device__ __forceinline__ void reset_regions(const SplatArgs& a, unsigned char* tile, uint32_t reset, int z0, int nl,
+                                              int TY, int yoff, int lane)
+{
+    const int P = a.P;
+#pragma unroll 1
+    for (int k = 0; k < 27; k++) {
+        if (!((reset >> k) & 1u)) continue;
+        const int dx = k / 9 - 1, dy = (k / 3) % 3 - 1, dz = k % 3 - 1;
+        const int xb = dx < 0 ? 0 : (dx > 0 ? P - 1 : 1), yb = dy < 0 ? 0 : (dy > 0 ? P - 1 : 1);
+        const int bx = dx == 0 ? a.lb : 0, by = dy == 0 ? a.lb : 0;  // log2 of the region's x, y extents
+        const int zlo = max(dz < 0 ? 0 : (dz > 0 ? P - 1 : 1), z0);
+        const int zhi = min(dz < 0 ? 0 : (dz > 0 ? P - 1 : P - 2), z0 + nl - 1);
+        const int cnt = zhi >= zlo ? (zhi - zlo + 1) << (bx + by) : 0;
+        for (int c = lane; c < cnt; c += 32) {
+            const int x = xb + (c & ((1 << bx) - 1)), y = yb + ((c >> bx) & ((1 << by) - 1));
+            const int z = zlo + (c >> (bx + by));
+            Tile<HAS_DEN, HAS_VEL>::set(tile, ((z - z0) * TY + (y - yoff)) * P + x, a.boundval);
+        }
+    }
+    __syncwarp();
+}
+
 // One warp per (brick, z-slab): the padded brick's layers are split into
 // slabs of a.slab_layers layers, each with its own shared tile, so a warp's
 // tile is a fraction of the brick and more warps stay resident.  Every slab
@@ -776,24 +806,7 @@ __device__ __forceinline__ void splat_unit(const SplatArgs& a, const uint32_t u,
     uint32_t reset = ~nbmask & 0x7FFFFFFu & ~(1u << 13);
     if (a.boundval == 0.0f) reset &= __reduce_or_sync(kFull, touched);
     if (push) reset &= (1u << 4) | (1u << 22);  // the tile's only apron voxels: the two x faces
-    if (ap && reset && !a.accum) {
-#pragma unroll 1
-        for (int k = 0; k < 27; k++) {
-            if (!((reset >> k) & 1u)) continue;
-            const int dx = k / 9 - 1, dy = (k / 3) % 3 - 1, dz = k % 3 - 1;
-            const int xb = dx < 0 ? 0 : (dx > 0 ? P - 1 : 1), yb = dy < 0 ? 0 : (dy > 0 ? P - 1 : 1);
-            const int bx = dx == 0 ? a.lb : 0, by = dy == 0 ? a.lb : 0;  // log2 of the region's x, y extents
-            const int zlo = max(dz < 0 ? 0 : (dz > 0 ? P - 1 : 1), z0);
-            const int zhi = min(dz < 0 ? 0 : (dz > 0 ? P - 1 : P - 2), z0 + nl - 1);
-            const int cnt = zhi >= zlo ? (zhi - zlo + 1) << (bx + by) : 0;
-            for (int c = lane; c < cnt; c += 32) {
-                const int x = xb + (c & ((1 << bx) - 1)), y = yb + ((c >> bx) & ((1 << by) - 1));
-                const int z = zlo + (c >> (bx + by));
-                T::set(tile, ((z - z0) * TY + (y - yoff)) * P + x, a.boundval);
-            }
-        }
-        __syncwarp();
-    }
+    if (ap && reset && !a.accum) reset_regions<HAS_DEN, HAS_VEL>(a, tile, reset, z0, nl, TY, yoff, lane);
 
     // ---- out to HBM
     if (push) {
@@ -819,18 +832,8 @@ __device__ __forceinline__ void splat_unit(const SplatArgs& a, const uint32_t u,
     }
 }
 
-// resident blocks per SM the registers are budgeted for: 8 for the trilinear splats without
-// velocity (a few bytes of spill; sparse batched clouds, 2 points a brick: 2.30 -> 2.02 ms on
-// 800k bricks, the memory latency of a brick's short candidate chain hidden by more warps), 6 for
-// the others, whose registers would spill tens of bytes at 8
-template <bool HAS_DEN, bool HAS_VEL, int MODE>
-constexpr int splat_min_blocks()
-{
-    return !HAS_VEL && MODE == GVX_SPLAT_TRILINEAR ? 8 : kSlabMinBlocks;
-}
-
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kSlabWarps * 32, splat_min_blocks<HAS_DEN, HAS_VEL, MODE>()) k_splat_slab(SplatArgs a)
+__global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks) k_splat_slab(SplatArgs a)
 {
     using T = Tile<HAS_DEN, HAS_VEL>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -865,7 +868,7 @@ __global__ void __launch_bounds__(kSlabWarps * 32, splat_min_blocks<HAS_DEN, HAS
 // k are [ustart[k], ustart[k+1]) of one global range, taken by the warps from
 // a counter; every grid has the same brick and tile shape (slab_layers, P).
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kSlabWarps * 32, splat_min_blocks<HAS_DEN, HAS_VEL, MODE>())
+__global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks)
     k_splat_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
     using T = Tile<HAS_DEN, HAS_VEL>;
@@ -906,6 +909,479 @@ __global__ void __launch_bounds__(kSlabWarps * 32, splat_min_blocks<HAS_DEN, HAS
                                                        s_ro[wid], phase, lane);
     }
     if (!(HAS_DEN && HAS_VEL) && lane == 0) bulk_wait_all();
+}
+
+// ---------------------------------------------------------------------------
+// TRILINEAR density alone: the splat of sparse clouds (batches of point clouds, depth frames, small
+// live clouds), 1-10 points a brick, where a brick's fixed work is most of it.
+//
+// What bounds it: instruction issue (the general slab kernel spends 2 x 1,080 warp instructions on a
+// brick of two points, 75% of the issue slots) ahead of the HBM writes of the bricks.  So, unlike
+// splat_unit:
+//  - a lane's candidates are ONE range per neighbour, from its first needed octant to its last one
+//    (a superset of the needed octants, two loads instead of nine and no list of runs; the footprint
+//    test drops the others), found from a candidate's number with one warp-wide OR of the ranges'
+//    starts and a popcount, without a search;
+//  - the hits of a round of candidates go to shared memory in order, and four of them are added at a
+//    time, eight lanes (the corners of the footprint) each; lanes that meet on a voxel add one after
+//    another in the points' order.  Every voxel's sum is that of the slab kernel, term by term;
+//  - one unit is the whole padded brick where that leaves enough units for the chip (kTriWholeBricks);
+//  - the next unit's brick is known, and its neighbour list, ranges and origin are asked for, while
+//    the current one is summed.
+// 24 batched clouds, 5M points, 2.07M bricks: 7.10 -> 2.37 ms (8.3 GB written: 3.5 TB/s), 100k points
+// in 36k bricks 92 -> 43 us, a fusion frame's splat 108 -> 84 us.
+struct TriLane {
+    int dx, dy, dz;   // the lane's neighbour, lanes 27-31 none
+    int lox, hix, loy, hiy;  // first and last half of the neighbour that can reach the tile, along x and y
+    bool need;        // some half can, along both
+};
+
+// halves of a neighbour at offset d (bricks) whose points reach voxels [v0, v1] of the brick: points of
+// floor coordinate f touch f and f + 1
+__device__ __forceinline__ bool tri_halves(int d, int b, int v0, int v1, int& lo, int& hi)
+{
+    const int hb = b >> 1, c = d * b;
+    const bool n0 = c <= v1 && c + hb - 1 >= v0 - 1, n1 = c + hb <= v1 && c + b - 1 >= v0 - 1;
+    lo = n0 ? 0 : 1;
+    hi = n1 ? 1 : 0;
+    return n0 || n1;
+}
+
+// the unit's brick and slab, and what the lane needs of them
+struct TriUnit {
+    uint32_t s;      // atlas slot
+    int z0, nl;      // padded layers of the unit
+    int leaf;
+    int nl27;        // the lane's neighbour (leaf index, -1: none)
+    int4 org;        // the node's first 16 bytes: (lev.., x, y, z)
+    int start, end;  // the lane's candidates in the sorted points
+};
+
+__device__ __forceinline__ void tri_slot(const SplatArgs& a, uint32_t u, TriUnit& t)
+{
+    const uint32_t S = (uint32_t)a.slabs;
+    const uint32_t ui = S == 1u ? u : u / S;
+    t.s = a.unit_slots ? a.unit_slots[ui] : ui;
+    t.z0 = (int)(u - ui * S) * a.slab_layers;
+    t.nl = min(a.slab_layers, a.P - t.z0);
+    t.leaf = a.slot_leaf[t.s];
+}
+__device__ __forceinline__ void tri_neighbour(const SplatArgs& a, TriUnit& t, int nbi)
+{
+    t.nl27 = nbi >= 0 ? a.nbr[(size_t)t.leaf * 27 + nbi] : -1;
+    t.org = *(const int4*)(a.nodes0 + t.leaf);
+}
+__device__ __forceinline__ void tri_range(const SplatArgs& a, TriUnit& t, const TriLane& L)
+{
+    t.start = t.end = 0;
+    int loz, hiz;
+    if (t.nl27 >= 0 && L.need && tri_halves(L.dz, a.brick, t.z0 - a.apron, t.z0 - a.apron + t.nl - 1, loz, hiz)) {
+        const int o0 = 4 * L.lox + 2 * L.loy + loz, o1 = 4 * L.hix + 2 * L.hiy + hiz + 1;
+        const int* oc = a.leaf_oct + (size_t)t.nl27 * 8;
+        t.start = oc[o0];
+        t.end = o1 == 8 ? a.leaf_range[t.nl27].y : oc[o1];
+    }
+}
+
+// A unit with more than kDenseCandidates candidates in dense leaves (the core of a dense cloud:
+// thousands of points a brick) is summed voxel by voxel, a lane each, from the cells around the voxel:
+// the points of dense leaves are in cell order (k_cell_sort), so the terms of a voxel are eight runs of
+// points, without a test of the others.  Terms are added in the sorted order of the points, as
+// everywhere: leaf by leaf in key order, octant by octant, cell by cell; the two cells along an axis lie
+// in different leaves, octants or cells of an octant, and an axis counts for the order the more the
+// higher that level is.  The points of a leaf that is not dense are in index order inside an octant:
+// its octants are scanned.
+// Each voxel's lookups are a chain of loads: a brick of 3,000 points takes one warp half a millisecond,
+// and every one below the bound loses against the pulled sum (fusion frames of 100-190 points a leaf:
+// 84 us with the bound at 1500, 153 at 768 in whole bricks).  So the unit is put on a list, and
+// k_tri_dense spreads its voxels over the chip (24 clouds of up to 10,600 points a leaf: the pulled
+// sums of the densest brick alone take 3 of 6.8 ms; listed 4.07 + 0.24, before the claims of two).
+constexpr int kDenseCandidates = 1500;
+constexpr uint32_t kDenseCap = 65536;  // listed units at most; more are summed where they were met
+
+// a point's weight at a voxel: every product rounded on its own, so that a voxel's sum has the same bits
+// whichever way it is formed (left to the compiler, one copy of the code may fuse what another does not)
+__device__ __forceinline__ float tri_weight(float w, float wx, float wy, float wz)
+{
+    return __fmul_rn(__fmul_rn(w, wx), __fmul_rn(wy, wz));
+}
+
+// the sums of voxels e0 + lane of the unit
+__device__ __forceinline__ void tri_dense(const SplatArgs& a, const TriUnit& t, int e0, int lane)
+{
+    const int P = a.P, P2 = P * P, ap = a.apron;
+    const int nvox = t.nl * P2;
+    float* out = a.den + (size_t)t.s * (P2 * P) + (size_t)t.z0 * P2;
+    {
+        const int e = e0 + lane;
+        const bool live = e < nvox;
+        const int lz = (live ? e : 0) / P2, r = (live ? e : 0) - lz * P2, ly = r / P, lx = r - ly * P;
+        const int v[3] = {lx - ap, ly - ap, lz + t.z0 - ap};  // in the brick's voxels, -ap .. 7 + ap
+        // an apron voxel of a missing neighbour takes the boundary value
+        const int home = __shfl_sync(kFull, t.nl27, ((v[0] >> 3) + 1) * 9 + ((v[1] >> 3) + 1) * 3 + (v[2] >> 3) + 1);
+        const bool bound = home < 0 && !a.accum;
+        float sum = live && a.accum ? out[e] : 0.0f;
+        // the axes in the order their two cells count: different leaves, then octants, then cells
+        int lev[3], ax[3] = {0, 1, 2};
+#pragma unroll
+        for (int k = 0; k < 3; k++) lev[k] = (v[k] & 7) == 0 ? 2 : (v[k] & 7) == 4 ? 1 : 0;
+        if (lev[1] > lev[0]) {
+            ax[0] = 1;
+            ax[1] = 0;
+        }
+        {
+            const int la = max(lev[0], lev[1]), lb = min(lev[0], lev[1]);
+            if (lev[2] > la) {
+                ax[2] = ax[1];
+                ax[1] = ax[0];
+                ax[0] = 2;
+            } else if (lev[2] > lb) {
+                ax[2] = ax[1];
+                ax[1] = 2;
+            }
+        }
+        const float wv[3] = {(float)(t.org.y + v[0]), (float)(t.org.z + v[1]), (float)(t.org.w + v[2])};
+#pragma unroll 1
+        for (int c = 0; c < 8; c++) {
+            int f[3], near[3];  // the cell along each axis; near: it is the voxel's own (else the one before)
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                near[k] = ax[0] == k ? (c >> 2) & 1 : ax[1] == k ? (c >> 1) & 1 : c & 1;
+                f[k] = v[k] - 1 + near[k];
+            }
+            const int leaf = __shfl_sync(kFull, t.nl27, min(max(((f[0] >> 3) + 1) * 9 + ((f[1] >> 3) + 1) * 3 + (f[2] >> 3) + 1, 0), 31));
+            if (!live || bound || leaf < 0 || f[0] < -8 || f[1] < -8 || f[2] < -8) continue;
+            const int oct = ((f[0] >> 2) & 1) * 4 + ((f[1] >> 2) & 1) * 2 + ((f[2] >> 2) & 1);
+            const int dense = a.leaf_dense[leaf];
+            if (dense) {
+                const int cell = oct * 64 + (f[0] & 3) * 16 + (f[1] & 3) * 4 + (f[2] & 3);
+                const int* ct = a.cell_tab + (size_t)(dense - 1) * 512 + cell;
+                const int i0 = ct[0], i1 = cell == 511 ? a.leaf_range[leaf].y : ct[1];
+                for (int i = i0; i < i1; i += 4) {
+                    float4 p[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) p[q] = a.spos[min(i + q, i1 - 1)];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const float fx = p[q].x - (wv[0] - (float)(1 - near[0])), fy = p[q].y - (wv[1] - (float)(1 - near[1])),
+                                    fz = p[q].z - (wv[2] - (float)(1 - near[2]));
+                        const float w = tri_weight(p[q].w, near[0] ? 1.f - fx : fx, near[1] ? 1.f - fy : fy,
+                                                   near[2] ? 1.f - fz : fz);
+                        if (i + q < i1) sum = __fadd_rn(sum, w);
+                    }
+                }
+            } else {
+                // once per octant: where the axes whose two cells share it take the first
+                if ((lev[0] == 0 && near[0]) || (lev[1] == 0 && near[1]) || (lev[2] == 0 && near[2])) continue;
+                const int* oc = a.leaf_oct + (size_t)leaf * 8 + oct;
+                const int i0 = oc[0], i1 = oct == 7 ? a.leaf_range[leaf].y : oc[1];
+                for (int i = i0; i < i1; i += 4) {
+                    float4 p[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) p[q] = a.spos[min(i + q, i1 - 1)];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const float gx = floorf(p[q].x), gy = floorf(p[q].y), gz = floorf(p[q].z);
+                        const float dx = wv[0] - gx, dy = wv[1] - gy, dz = wv[2] - gz;  // 0 or 1 where it reaches
+                        const float fx = p[q].x - gx, fy = p[q].y - gy, fz = p[q].z - gz;
+                        const float w = tri_weight(p[q].w, dx == 0.f ? 1.f - fx : fx, dy == 0.f ? 1.f - fy : fy,
+                                                   dz == 0.f ? 1.f - fz : fz);
+                        const bool in = (dx == 0.f || dx == 1.f) && (dy == 0.f || dy == 1.f) && (dz == 0.f || dz == 1.f);
+                        if (i + q < i1 && in) sum = __fadd_rn(sum, w);
+                    }
+                }
+            }
+        }
+        if (live) out[e] = bound ? a.boundval : sum;
+    }
+}
+
+struct TriShared {
+    int rs[kSlabWarps][32];      // per range with points: its first sorted index, less its first candidate number
+    float4 hit[kSlabWarps][32];  // the hits of a round of candidates, in order
+    uint64_t bar[kSlabWarps];
+};
+
+// the sums of one unit into `tile` and out to HBM; mid(): called once, before the candidates
+template <class Mid>
+__device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, float* tile, TriShared& sh, int wid,
+                                         int lane, uint32_t& phase, uint32_t grid, Mid mid)
+{
+    const int P = a.P, P2 = P * P, ap = a.apron;
+    const int Ox = t.org.y - ap, Oy = t.org.z - ap, Zlo = t.org.w - ap + t.z0;
+    const int nvox = t.nl * P2;
+    const size_t gofs = (size_t)t.s * (P2 * P) + (size_t)t.z0 * P2;
+    const uint32_t lt = (1u << lane) - 1u;
+    // ---- the lanes' ranges: places among the candidates
+    const int len = t.end - t.start;
+    int off = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, off, o);
+        if (lane >= o) off += v;
+    }
+    const int total = __shfl_sync(kFull, off, 31);
+    off -= len;
+    if (a.accum && total == 0) {  // no point reaches the slab: left as it is
+        mid();
+        return;
+    }
+    if (a.cell_tab && total > kDenseCandidates) {
+        const bool dn = len > 0 && a.leaf_dense[t.nl27] != 0;
+        if (__reduce_add_sync(kFull, dn ? len : 0) > kDenseCandidates) {
+            mid();
+            uint32_t at = kDenseCap;
+            if (a.dense_units && lane == 0) at = atomicAdd(a.dense_units, 1u);
+            at = __shfl_sync(kFull, at, 0);
+            if (at < kDenseCap) {
+                if (lane == 0) a.dense_list[at] = make_uint4(grid, t.s, (uint32_t)t.z0, (uint32_t)t.nl);
+            } else {
+                for (int e0 = 0; e0 < nvox; e0 += 32) tri_dense(a, t, e0, lane);
+            }
+            return;
+        }
+    }
+    const uint32_t some = __ballot_sync(kFull, len > 0);
+    // (active neighbours: those in the lookup the table was made from, which are those with a slot)
+    const uint32_t nbmask = __ballot_sync(kFull, t.nl27 >= 0);
+    if (len > 0) sh.rs[wid][__popc(some & lt)] = t.start - off;
+
+    // ---- the tile, once the last unit's bulk store has read it
+    if (lane == 0) bulk_wait_read_all();
+    __syncwarp();
+    if (a.accum) {
+        if (lane == 0) {
+            mbar_expect_tx(&sh.bar[wid], (uint32_t)nvox * 4u);
+            bulk_g2s(tile, a.den + gofs, (uint32_t)nvox * 4u, &sh.bar[wid]);
+        }
+    } else {
+        for (int i = lane; i < nvox / 4; i += 32) ((float4*)tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    bool loaded = !a.accum;
+    mid();
+
+    uint32_t touched = 0u;
+    const int cx = lane & 1, cy = (lane >> 1) & 1, cz = (lane >> 2) & 1, hq = lane >> 3;
+    for (int base = 0; base < total; base += 32) {
+        const int v = base + lane;
+        // the range of candidate v: the ranges with points that start at or before it, less one
+        const uint32_t starts = __reduce_or_sync(kFull, len > 0 && off >= base && off < base + 32 ? 1u << (off - base) : 0u);
+        const int before = __popc(__ballot_sync(kFull, len > 0 && off < base));
+        bool hit = false;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v < total) {
+            p = a.spos[sh.rs[wid][before - 1 + __popc(starts & (kFull >> (31 - lane)))] + v];
+            const int x = (int)floorf(p.x) - Ox, y = (int)floorf(p.y) - Oy, z = (int)floorf(p.z) - Zlo;
+            // the footprint is x, x + 1 and so on
+            hit = (unsigned)(x + 1) <= (unsigned)P && (unsigned)(y + 1) <= (unsigned)P &&
+                  (unsigned)(z + 1) <= (unsigned)t.nl;
+            if (hit && nbmask != 0x7FFFFFFu && ap) {
+                // the regions of the padded brick reached (see splat_unit): per axis 1 below the
+                // interior, 2 inside, 4 above
+                const int zp = t.z0 + z;
+                const uint32_t tx = (uint32_t)(x < ap) | (uint32_t)(x + 1 >= ap && x <= P - 1 - ap) << 1 |
+                                    (uint32_t)(x + 1 > P - 1 - ap) << 2;
+                const uint32_t ty = (uint32_t)(y < ap) | (uint32_t)(y + 1 >= ap && y <= P - 1 - ap) << 1 |
+                                    (uint32_t)(y + 1 > P - 1 - ap) << 2;
+                const uint32_t tz = (uint32_t)(zp < ap) | (uint32_t)(zp + 1 >= ap && zp <= P - 1 - ap) << 1 |
+                                    (uint32_t)(zp + 1 > P - 1 - ap) << 2;
+                touched |= ((tx & 1u) | (tx & 2u) << 8 | (tx & 4u) << 16) *
+                           ((ty & 1u) | (ty & 2u) << 2 | (ty & 4u) << 4) * tz;
+            }
+        }
+        const uint32_t hm = __ballot_sync(kFull, hit);
+        if (hm == 0u) continue;
+        if (hit) sh.hit[wid][__popc(hm & lt)] = p;
+        if (!loaded) {
+            if (!mbar_wait_bounded(&sh.bar[wid], phase)) atomicOr(a.err, GVX_DERR_TIMEOUT);
+            phase ^= 1u;
+            loaded = true;
+        }
+        __syncwarp();
+        const int nh = __popc(hm);
+        for (int h0 = 0; h0 < nh; h0 += 4) {
+            const bool act = h0 + hq < nh;
+            const float4 q = sh.hit[wid][act ? h0 + hq : 0];
+            const float fx0 = floorf(q.x), fy0 = floorf(q.y), fz0 = floorf(q.z);
+            const int x = (int)fx0 - Ox + cx, y = (int)fy0 - Oy + cy, z = (int)fz0 - Zlo + cz;
+            const bool in = act && (unsigned)x < (unsigned)P && (unsigned)y < (unsigned)P && (unsigned)z < (unsigned)t.nl;
+            const float fx = q.x - fx0, fy = q.y - fy0, fz = q.z - fz0;
+            const float w = tri_weight(q.w, cx ? fx : 1.f - fx, cy ? fy : 1.f - fy, cz ? fz : 1.f - fz);
+            const int i = (z * P + y) * P + x;
+            // how many of the three earlier hits reach this voxel: its offset from their first cell is
+            // 0 or 1 along every axis.  (Bytes x, y, z, all at least 1 here, compared at once; match_any
+            // and a warp maximum held the unit they share 64% busy.)
+            const uint32_t vb = (uint32_t)(x + 1) | (uint32_t)(y + 1) << 8 | (uint32_t)(z + 1) << 16;
+            const uint32_t base = vb - (uint32_t)(cx | cy << 8 | cz << 16);
+            int rank = 0;
+#pragma unroll
+            for (int o = 8; o <= 24; o += 8) {
+                const uint32_t other = __shfl_up_sync(kFull, act ? base : 0u, o);
+                rank += lane >= o && (((vb | 0x808080u) - other) & 0xFEFEFEu) == 0x808080u;
+            }
+            // (an inactive hit comes after the active ones: its base is never an earlier one)
+            if (in && rank == 0) tile[i] = __fadd_rn(tile[i], w);
+            __syncwarp();
+            for (int ph = 1; __any_sync(kFull, in && rank >= ph); ph++) {
+                if (in && rank == ph) tile[i] = __fadd_rn(tile[i], w);
+                __syncwarp();
+            }
+        }
+    }
+    if (!loaded) {  // (candidates, but no hit: the slab as it was)
+        if (!mbar_wait_bounded(&sh.bar[wid], phase)) atomicOr(a.err, GVX_DERR_TIMEOUT);
+        phase ^= 1u;
+        return;
+    }
+    __syncwarp();
+
+    // ---- apron voxels with no neighbouring brick take the boundary value: regions that hits reached
+    uint32_t reset = ~nbmask & 0x7FFFFFFu & ~(1u << 13);
+    if (a.boundval == 0.0f && reset) reset &= __reduce_or_sync(kFull, touched);
+    if (ap && reset && !a.accum) reset_regions<true, false>(a, (unsigned char*)tile, reset, t.z0, t.nl, P, 0, lane);
+
+    // ---- out to HBM (the bulk store's read of the tile is waited for before the tile's next write)
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+        bulk_s2g(a.den + gofs, tile, (uint32_t)nvox * 4u);
+        bulk_commit();
+    }
+}
+
+// Units are claimed two at a time where there are many for every warp: the counter is one address, which
+// takes an atomic every two nanoseconds (24 clouds, 2.07M bricks: 3.24 ms one at a time, 2.37 two, 2.44
+// four, 2.53 eight); costly units do not pile up in a claim, the dense ones being listed elsewhere.
+constexpr uint32_t kTriClaim = 2, kTriClaimUnits = 16;
+
+// Units [0, total) of all grids from the counter `next`; of(u, local) -> the number of u's grid and its
+// unit there, args(k) -> that grid's arguments
+template <class Of, class Args>
+__device__ __forceinline__ void tri_loop(const SplatArgs& a0, uint32_t total, uint32_t* next, unsigned char* smem, Of of,
+                                         Args args)
+{
+    __shared__ __align__(16) TriShared sh;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* tile = (float*)smem + (size_t)wid * (a0.slab_layers * a0.P * a0.P);
+    if (lane == 0) {
+        mbar_init(&sh.bar[wid], 1);
+        mbar_fence_init();
+    }
+    __syncwarp();
+    uint32_t phase = 0;
+    TriLane L;
+    L.dx = lane / 9 - 1, L.dy = (lane / 3) % 3 - 1, L.dz = lane % 3 - 1;
+    const bool nx = tri_halves(L.dx, a0.brick, -a0.apron, a0.P - 1 - a0.apron, L.lox, L.hix);
+    const bool ny = tri_halves(L.dy, a0.brick, -a0.apron, a0.P - 1 - a0.apron, L.loy, L.hiy);
+    L.need = lane < 27 && nx && ny;
+    const int nbi = lane < 27 ? (L.dz + 1) * 9 + (L.dy + 1) * 3 + (L.dx + 1) : -1;
+    // Units from the counter, in three steps ahead of each other: while unit t is summed, the neighbours
+    // (asked for as it starts) and then the candidate ranges of t1 arrive, and the brick of t2.
+    const uint32_t claim = total >= kTriClaimUnits * gridDim.x * kSlabWarps ? kTriClaim : 1u;
+    uint32_t cur = 0u, lim = 0u, pre = lane == 0 ? atomicAdd(next, claim) : 0u, lu;
+    auto take = [&]() {  // the next unit's number (total and above: none)
+        if (cur == lim) {
+            cur = __shfl_sync(kFull, pre, 0);
+            lim = cur + claim;
+            if (lane == 0 && cur < total) pre = atomicAdd(next, claim);
+        }
+        return cur++;
+    };
+    uint32_t u = take();
+    if (u < total) {
+        TriUnit t, t1;
+        uint32_t k = of(u, lu), k1;
+        tri_slot(args(k), lu, t);
+        u = take();
+        bool more = u < total;
+        k1 = k;
+        t1 = t;
+        if (more) {
+            k1 = of(u, lu);
+            tri_slot(args(k1), lu, t1);
+        }
+        tri_neighbour(args(k), t, nbi);
+        tri_range(args(k), t, L);
+        for (;;) {
+            TriUnit t2 = t1;
+            uint32_t k2 = k1;
+            bool more2 = false;
+            if (more) {
+                tri_neighbour(args(k1), t1, nbi);
+                u = take();
+                more2 = u < total;
+                if (more2) {
+                    k2 = of(u, lu);
+                    tri_slot(args(k2), lu, t2);
+                }
+            }
+            tri_unit(args(k), t, tile, sh, wid, lane, phase, k, [&]() {
+                if (more) tri_range(args(k1), t1, L);
+            });
+            if (!more) break;
+            k = k1;
+            t = t1;
+            k1 = k2;
+            t1 = t2;
+            more = more2;
+        }
+    }
+    if (lane == 0) bulk_wait_all();
+}
+
+__global__ void __launch_bounds__(kSlabWarps * 32, 8) k_splat_tri(SplatArgs a)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
+    tri_loop(
+        a, units, a.next, smem,
+        [&](uint32_t u, uint32_t& lu) {
+            lu = u;
+            return 0u;
+        },
+        [&](uint32_t) -> const SplatArgs& { return a; });
+}
+
+// the same over many grids: ustart as in k_splat_batch, the counters after it
+__global__ void __launch_bounds__(kSlabWarps * 32, 8)
+    k_splat_tri_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint32_t s_us[kBatchMaxGrids + 1];
+    for (int i = threadIdx.x; i <= ngrids; i += blockDim.x) s_us[i] = ustart[i];
+    __syncthreads();
+    uint32_t k = 0u;  // the last unit's grid: a warp's units come in rising order, so its search starts there
+    tri_loop(
+        args[0], s_us[ngrids], ustart + ngrids + 1, smem,
+        [&](uint32_t u, uint32_t& lu) {
+            while (s_us[k + 1] <= u) k++;
+            lu = u - s_us[k];
+            return k;
+        },
+        [&](uint32_t g) -> const SplatArgs& { return args[g]; });
+}
+
+// the listed units of k_splat_tri (args: one grid's) or k_splat_tri_batch, 32 voxels a warp
+__global__ void __launch_bounds__(kSlabWarps * 32, 8)
+    k_tri_dense(const SplatArgs* __restrict__ args, SplatArgs one, const uint32_t* __restrict__ units,
+                const uint4* __restrict__ list, int chunks)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = min(*units, kDenseCap) * (uint32_t)chunks, nw = gridDim.x * kSlabWarps;
+    const int dx = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dz = lane % 3 - 1;
+    const int nbi = lane < 27 ? (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1) : -1;
+    for (uint32_t u = blockIdx.x * kSlabWarps + (threadIdx.x >> 5); u < total; u += nw) {
+        const uint4 e = list[u / (uint32_t)chunks];
+        const SplatArgs& a = args ? args[e.x] : one;
+        TriUnit t;
+        t.s = e.y;
+        t.z0 = (int)e.z;
+        t.nl = (int)e.w;
+        t.leaf = a.slot_leaf[t.s];
+        tri_neighbour(a, t, nbi);
+        const int e0 = (int)(u % (uint32_t)chunks) * 32;
+        if (e0 < t.nl * a.P * a.P) tri_dense(a, t, e0, lane);
+    }
 }
 
 // ScatterDensity, race-free: own points only, into the own padded tile.  With
@@ -1129,12 +1605,23 @@ struct SplatKind {
     }
 };
 
+// points from which a splat lists its dense units for a launch of their own: below, the launch would
+// cost more than one warp's half a millisecond on the densest brick that so few points can make
+constexpr int kListDensePoints = 32768;
+
+// the splats of k_splat_tri
+static bool tri_kind(const SplatKind& k) { return k.mode == GVX_SPLAT_TRILINEAR && k.has_d && !k.has_v; }
+
 template <bool D, bool V>
 static void* pick_kernel(const SplatKind& k, bool batch)
 {
-    if (k.mode == GVX_SPLAT_TRILINEAR)
-        return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_TRILINEAR, false, true>
-                     : (void*)k_splat_slab<D, V, GVX_SPLAT_TRILINEAR, false, true>;
+    if (k.mode == GVX_SPLAT_TRILINEAR) {
+        if constexpr (D && !V)
+            return batch ? (void*)k_splat_tri_batch : (void*)k_splat_tri;
+        else
+            return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_TRILINEAR, false, true>
+                         : (void*)k_splat_slab<D, V, GVX_SPLAT_TRILINEAR, false, true>;
+    }
     if (k.ppr)
         return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_CUBIC, true, false>
                      : (void*)k_splat_slab<D, V, GVX_SPLAT_CUBIC, true, false>;
@@ -1182,10 +1669,17 @@ static int clamp_layers(const SlabShape& sh, int P, size_t eb, int want)
     return std::min(std::min(want, sh.span), fit);
 }
 
-// validation of one grid's splat and its kernel kind; *layers in: the wanted slab height (<= 0:
-// half the padded brick), out: clamped to the tile budget
+// The trilinear density splat takes a whole padded brick a unit where the launch has a unit for every
+// resident warp (152 SMs x 32) and the tile is small (4 KB for bricks of 8), else half of it: 100k
+// points in 36k bricks 43 us whole, 65 in halves; fusion frames 84 / 88; 24 clouds 2.4 / 3.3 ms; 6k
+// points in 720 bricks 14 / 11 us
+constexpr int kTriWholeP = 10;
+constexpr uint64_t kTriWholeBricks = 152 * 32;
+
+// validation of one grid's splat and its kernel kind (bricks: how many the launch covers); *layers in:
+// the wanted slab height (<= 0: the default), out: clamped to the tile budget
 static gvx_status splat_check(gvx_grid* g, int mode, float radius, int chan_d, int chan_v, int accum,
-                              bool dense, int* layers, SplatKind* kind)
+                              bool dense, uint64_t bricks, int* layers, SplatKind* kind)
 {
     if (mode != GVX_SPLAT_TRILINEAR && mode != GVX_SPLAT_CUBIC) {
         gvx_set_error("Splat: unknown mode %d", mode);
@@ -1221,7 +1715,8 @@ static gvx_status splat_check(gvx_grid* g, int mode, float radius, int chan_d, i
     const SlabShape sh = slab_shape(g, accum, dense, has_d && has_v);
     // a push tile takes the brick's whole interior (one unit a brick: the candidate ranges and the z
     // pushes once; 4M frame 2.80 -> 2.54 ms against two 4-layer slabs), else half the padded brick
-    *layers = clamp_layers(sh, P, has_v ? 16 : 4, *layers > 0 ? *layers : (sh.push ? sh.span : (sh.span + 1) / 2));
+    const bool whole = sh.push || (mode == GVX_SPLAT_TRILINEAR && !has_v && P <= kTriWholeP && bricks >= kTriWholeBricks);
+    *layers = clamp_layers(sh, P, has_v ? 16 : 4, *layers > 0 ? *layers : (whole ? sh.span : (sh.span + 1) / 2));
     if (*layers < 1) {
         gvx_set_error("Splat: a %d^2 layer of the padded brick exceeds the shared tile budget", P);
         return GVX_ERR_UNSUPPORTED;
@@ -1252,6 +1747,8 @@ static void splat_fill(gvx_grid* g, const SplatKind& k, float radius, int chan_d
     a.nbr = g->nbr.as<int>();
     a.leaf_range = g->leaf_range.as<int2>();
     a.leaf_oct = g->leaf_oct.as<int>();
+    a.leaf_dense = g->leaf_dense;
+    a.cell_tab = g->leaf_dense ? g->cell_tab.as<int>() : nullptr;
     a.spos = g->spos.as<float4>();
     a.svel = need_svel ? g->svel.as<float4>() : nullptr;
     a.per_point_radius = k.ppr;
@@ -1277,12 +1774,13 @@ static void splat_fill(gvx_grid* g, const SplatKind& k, float radius, int chan_d
 // layers <= 0 picks the default slab height (see splat_check); dense < 0: the tile shape from the
 // grid's own points per brick, else as given (a batch decides for all its grids)
 static gvx_status splat_prepare(gvx_grid* g, int mode, int n, float radius, const float trans[3], int chan_d,
-                                int chan_v, int accum, int layers, int dense, SplatArgs* out, SplatKind* kind)
+                                int chan_v, int accum, int layers, int dense, uint64_t bricks, SplatArgs* out,
+                                SplatKind* kind)
 {
     gvx_status rc = check_splat_state(g, "Splat");
     if (rc) return rc;
     const bool dn = dense < 0 ? dense_cloud((uint64_t)n, (uint64_t)g->atlas_used) : dense != 0;
-    rc = splat_check(g, mode, radius, chan_d, chan_v, accum, dn, &layers, kind);
+    rc = splat_check(g, mode, radius, chan_d, chan_v, accum, dn, bricks ? bricks : (uint64_t)g->atlas_used, &layers, kind);
     if (rc) return rc;
     rc = gvx_prepare_points(g, n, trans, kind->has_v || kind->ppr);
     if (rc) return rc;
@@ -1345,7 +1843,7 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
 {
     SplatArgs a;
     SplatKind kind;
-    gvx_status rc = splat_prepare(g, mode, n, radius, trans, chan_d, chan_v, accum, 0, -1, &a, &kind);
+    gvx_status rc = splat_prepare(g, mode, n, radius, trans, chan_d, chan_v, accum, 0, -1, 0, &a, &kind);
     if (rc) return rc;
     if (a.nslots) {
         const size_t smem = splat_smem(a, kind);
@@ -1357,9 +1855,15 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
         const uint64_t ctas_needed = (units + kSlabWarps - 1) / kSlabWarps;
         const uint32_t grid =
             (uint32_t)std::min<uint64_t>(ctas_needed, (uint64_t)sm_count(g->device) * std::max(per_sm, 1));
-        GVX_CK(gvx_ensure(g->d_next, 2 * sizeof(uint32_t)));
-        GVX_CK(cudaMemsetAsync(g->d_next.p, 0, 2 * sizeof(uint32_t), g->stream));
+        GVX_CK(gvx_ensure(g->d_next, 3 * sizeof(uint32_t)));  // units taken, slots touched, units listed
+        GVX_CK(cudaMemsetAsync(g->d_next.p, 0, 3 * sizeof(uint32_t), g->stream));
         a.next = g->d_next.as<uint32_t>();
+        const bool list_dense = tri_kind(kind) && a.cell_tab && n >= kListDensePoints;
+        if (list_dense) {
+            GVX_CK(gvx_ensure(g->dense_units, kDenseCap * sizeof(uint4)));
+            a.dense_units = g->d_next.as<uint32_t>() + 2;
+            a.dense_list = g->dense_units.as<uint4>();
+        }
         if (accum) {
             // only the bricks that this grouping's points can reach (accumulating frames of a growing
             // scene touch a small part of it: the fusion frames, about a tenth of 129k bricks)
@@ -1373,6 +1877,12 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
         void* args[] = {&a};
         GVX_CK(cudaLaunchKernel(kern, dim3(grid), dim3(kSlabWarps * 32), args, smem, g->stream));
         g->launches++;
+        if (list_dense) {
+            k_tri_dense<<<sm_count(g->device) * 8, kSlabWarps * 32, 0, g->stream>>>(
+                nullptr, a, a.dense_units, a.dense_list, (a.slab_layers * a.P * a.P + 31) / 32);
+            g->launches++;
+            GVX_CK(cudaGetLastError());
+        }
     }
     splat_finish(g, chan_d, chan_v, accum);
     return GVX_OK;
@@ -1409,6 +1919,7 @@ struct gvx_batch {
     int64_t launches = 0;
     // gvx_batch_frame: the grids' planned builds and the splat, captured in one graph
     DevBuf f_args, f_ustart, f_cnt, f_caps;
+    DevBuf dense_units;  // the units k_splat_tri_batch lists for k_tri_dense
     cudaEvent_t f_fork = nullptr;
     std::vector<cudaEvent_t> f_join;     // one per grid
     cudaGraph_t f_graph = nullptr;
@@ -1429,6 +1940,13 @@ static bool batch_dense(const gvx_batch* b)
         bricks += (uint64_t)g->atlas_used;
     }
     return dense_cloud(pts, bricks);
+}
+
+static uint64_t batch_bricks(const gvx_batch* b)
+{
+    uint64_t bricks = 0;
+    for (const gvx_grid* g : b->grids) bricks += (uint64_t)g->atlas_used;
+    return bricks;
 }
 
 static void frame_drop_graph(gvx_batch* b)
@@ -1460,6 +1978,27 @@ static std::string tune_key(int device, const SplatArgs& a, const SplatKind& k)
     return buf;
 }
 
+// the listed units of a trilinear density batch (their count at `units`)
+static gvx_status batch_dense_units(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, const SplatArgs* dargs,
+                                    const uint32_t* units)
+{
+    if (!tri_kind(k)) return GVX_OK;
+    SplatArgs none;
+    memset(&none, 0, sizeof(none));
+    k_tri_dense<<<sm_count(b->device) * 8, kSlabWarps * 32, 0, b->stream>>>(
+        dargs, none, units, b->dense_units.as<uint4>(), (a0.slab_layers * a0.P * a0.P + 31) / 32);
+    b->launches++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
+}
+
+// where a batch's dense units are listed: the counter after the unit counter of `ustart`
+static void batch_set_dense(gvx_batch* b, SplatArgs& a, DevBuf& ustart, size_t ngrids)
+{
+    a.dense_units = ustart.as<uint32_t>() + ngrids + 2;
+    a.dense_list = b->dense_units.as<uint4>();
+}
+
 // one launch of the batch kernel over args/ustart already on the device
 static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, int ngrids, int blocks)
 {
@@ -1467,11 +2006,11 @@ static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs
     void* kern = splat_kernel(k, true);
     const SplatArgs* dargs = b->d_args.as<SplatArgs>();
     uint32_t* dus = b->d_ustart.as<uint32_t>();
-    GVX_CK(cudaMemsetAsync(dus + ngrids + 1, 0, sizeof(uint32_t), b->stream));  // the unit counter
+    GVX_CK(cudaMemsetAsync(dus + ngrids + 1, 0, 2 * sizeof(uint32_t), b->stream));  // units taken, units listed
     void* args[] = {(void*)&dargs, (void*)&dus, (void*)&ngrids};
     GVX_CK(cudaLaunchKernel(kern, dim3(blocks), dim3(kSlabWarps * 32), args, smem, b->stream));
     b->launches++;
-    return GVX_OK;
+    return batch_dense_units(b, k, a0, dargs, dus + ngrids + 2);
 }
 
 // argument table of every grid for a slab height, and the unit ranges
@@ -1480,14 +2019,16 @@ static gvx_status batch_tables(gvx_batch* b, int mode, float radius, int chan_d,
 {
     args.resize(b->grids.size());
     ustart.assign(b->grids.size() + 1, 0u);
+    GVX_CK(gvx_ensure(b->d_ustart, (ustart.size() + 2) * sizeof(uint32_t)));  // + units taken, units listed
     uint64_t tot = 0;
     const int dense = batch_dense(b) ? 1 : 0;
+    const uint64_t bricks = std::max<uint64_t>(batch_bricks(b), 1);
     for (size_t i = 0; i < b->grids.size(); i++) {
         gvx_grid* g = b->grids[i];
         const int n = g->group_valid ? g->group_n : g->pts.n;
         const float* t = g->group_valid ? g->group_trans : nullptr;
         SplatKind k;
-        gvx_status rc = splat_prepare(g, mode, n, radius, t, chan_d, chan_v, accum, layers, dense, &args[i], &k);
+        gvx_status rc = splat_prepare(g, mode, n, radius, t, chan_d, chan_v, accum, layers, dense, bricks, &args[i], &k);
         if (rc) return rc;
         if (i == 0) {
             kind = k;
@@ -1495,6 +2036,10 @@ static gvx_status batch_tables(gvx_batch* b, int mode, float radius, int chan_d,
                    args[i].push != args[0].push) {
             gvx_set_error("BatchSplat: grid %zu differs from grid 0 in brick shape, channels or radius kind", i);
             return GVX_ERR_INVALID_ARG;
+        }
+        if (tri_kind(kind)) {
+            GVX_CK(gvx_ensure(b->dense_units, kDenseCap * sizeof(uint4)));
+            batch_set_dense(b, args[i], b->d_ustart, b->grids.size());
         }
         ustart[i] = (uint32_t)tot;
         tot += (uint64_t)args[i].nslots * args[i].slabs;
@@ -1510,7 +2055,6 @@ static gvx_status batch_tables(gvx_batch* b, int mode, float radius, int chan_d,
 static gvx_status batch_upload(gvx_batch* b, const std::vector<SplatArgs>& args, const std::vector<uint32_t>& ustart)
 {
     GVX_CK(gvx_ensure(b->d_args, args.size() * sizeof(SplatArgs)));
-    GVX_CK(gvx_ensure(b->d_ustart, (ustart.size() + 1) * sizeof(uint32_t)));  // + the unit counter
     GVX_CK(cudaMemcpyAsync(b->d_args.p, args.data(), args.size() * sizeof(SplatArgs), cudaMemcpyHostToDevice,
                            b->stream));
     GVX_CK(cudaMemcpyAsync(b->d_ustart.p, ustart.data(), ustart.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
@@ -1591,8 +2135,8 @@ static gvx_status batch_tune(gvx_batch* b, int mode, float radius, int chan_d, i
 // from the builds' slot counts on the device (k_batch_ustart).
 
 // unit ranges of a batch whose slot counts are in device memory: ustart[k] = slabs * the sum
-// of the slot counts of grids < k (each clamped to its capacity); the unit counter
-// ustart[ngrids + 1] zeroed
+// of the slot counts of grids < k (each clamped to its capacity); the counters of units
+// taken and units listed, ustart[ngrids + 1] and [ngrids + 2], zeroed
 __global__ void k_batch_ustart(const uint32_t* const* __restrict__ counts, const uint32_t* __restrict__ caps,
                                int ngrids, int slabs, uint32_t* __restrict__ ustart)
 {
@@ -1603,7 +2147,7 @@ __global__ void k_batch_ustart(const uint32_t* const* __restrict__ counts, const
         t += min(*counts[k], caps[k]) * (uint32_t)slabs;
     }
     ustart[ngrids] = t;
-    ustart[ngrids + 1] = 0u;
+    ustart[ngrids + 1] = ustart[ngrids + 2] = 0u;
 }
 
 // the sorted attributes InsertPoints writes, then the planned build (whose octant pass writes them)
@@ -1665,6 +2209,7 @@ static gvx_status frame_upload(gvx_batch* b, const SplatKind& kind, float radius
     std::vector<uint32_t> caps(ng);
     for (size_t i = 0; i < ng; i++) {
         splat_fill(b->grids[i], kind, radius, chan_d, chan_v, 0, batch_dense(b), layers, &args[i]);
+        if (tri_kind(kind)) batch_set_dense(b, args[i], b->f_ustart, ng);
         cnt[i] = gvx_topo_plan_slots(b->grids[i], &caps[i]);
     }
     GVX_CK(cudaMemcpyAsync(b->f_args.p, args.data(), ng * sizeof(SplatArgs), cudaMemcpyHostToDevice, b->stream));
@@ -1687,6 +2232,7 @@ static gvx_status frame_splat(gvx_batch* b, const SplatKind& kind, const SplatAr
     void* kargs[] = {(void*)&dargs, (void*)&dus, (void*)&n};
     GVX_CK(cudaLaunchKernel(kern, dim3(blocks), dim3(kSlabWarps * 32), kargs, smem, b->stream));
     b->launches += 2;
+    GVX_CK_STATUS(batch_dense_units(b, kind, a0, dargs, dus + ng + 2));
     // every grid's device error word (topology and splat) into its plan's record
     for (gvx_grid* g : b->grids) GVX_CK_STATUS(gvx_topo_plan_record_error(g, b->stream));
     return GVX_OK;
@@ -1823,6 +2369,7 @@ gvx_status gvx_batch_destroy(gvx_batch* b)
     frame_drop_graph(b);
     gvx_free(b->d_args);
     gvx_free(b->d_ustart);
+    gvx_free(b->dense_units);
     for (DevBuf* d : {&b->f_args, &b->f_ustart, &b->f_cnt, &b->f_caps}) gvx_free(*d);
     if (b->f_fork) cudaEventDestroy(b->f_fork);
     for (cudaEvent_t e : b->f_join) cudaEventDestroy(e);
@@ -2091,7 +2638,7 @@ gvx_status gvx_batch_frame(gvx_batch* b, float topo_radius, int mode, float radi
         gvx_grid* g = b->grids[i];
         int l = b->tuning.layers;
         SplatKind k;
-        gvx_status rc = splat_check(g, mode, radius, chan_density, chan_vel, 0, batch_dense(b), &l, &k);
+        gvx_status rc = splat_check(g, mode, radius, chan_density, chan_vel, 0, batch_dense(b), batch_bricks(b), &l, &k);
         if (rc) return rc;
         if (i == 0) {
             kind = k;
@@ -2145,7 +2692,8 @@ gvx_status gvx_batch_frame(gvx_batch* b, float topo_radius, int mode, float radi
         }
     }
     GVX_CK(gvx_ensure(b->f_args, ng * sizeof(SplatArgs)));
-    GVX_CK(gvx_ensure(b->f_ustart, (ng + 2) * sizeof(uint32_t)));
+    GVX_CK(gvx_ensure(b->f_ustart, (ng + 3) * sizeof(uint32_t)));
+    if (tri_kind(kind)) GVX_CK(gvx_ensure(b->dense_units, kDenseCap * sizeof(uint4)));
     GVX_CK(gvx_ensure(b->f_cnt, ng * sizeof(void*)));
     GVX_CK(gvx_ensure(b->f_caps, ng * sizeof(uint32_t)));
 

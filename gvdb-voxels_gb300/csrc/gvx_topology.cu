@@ -628,8 +628,11 @@ __global__ void k_write_root(GvxNode* root, int lev, int px, int py, int pz)
 // run of equal leaf keys in sorted order -> [start, end) of its leaf.  With octants in the keys
 // (kshift 3) also the first sorted index of every octant of the leaf's points (leaf_oct[8 l + o] =
 // start + the points of octants < o), written at the starts of the octant runs and at the leaf's end
+// dense_list (optional): the leaves of kDenseLeaf points and more, in no order -- the keys are sorted, so
+// such a run reaches kDenseLeaf - 1 entries back from its last one
+constexpr int kDenseLeaf = 128;
 __global__ void k_group_runs(const uint32_t* __restrict__ skeys, uint32_t n, int kshift, uint32_t invalid_key,
-                             LeafLookup L, int2* leaf_range, int* leaf_oct)
+                             LeafLookup L, int2* leaf_range, int* leaf_oct, uint32_t* dense_list, uint32_t* dense_count)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -645,7 +648,11 @@ __global__ void k_group_runs(const uint32_t* __restrict__ skeys, uint32_t n, int
     const int leaf = ll_find(L, c[0], c[1], c[2]);
     if (leaf < 0) return;
     if (first) leaf_range[leaf].x = (int)i;
-    if (last) leaf_range[leaf].y = (int)(i + 1);
+    if (last) {
+        leaf_range[leaf].y = (int)(i + 1);
+        if (dense_list && i + 1 >= (uint32_t)kDenseLeaf && (skeys[i + 1 - kDenseLeaf] >> kshift) == k)
+            dense_list[atomicAdd(dense_count, 1u)] = (uint32_t)leaf;
+    }
     if (kshift) {
         int* lo = leaf_oct + (size_t)leaf * 8;
         const int o = (int)(sk & 7u);
@@ -653,6 +660,94 @@ __global__ void k_group_runs(const uint32_t* __restrict__ skeys, uint32_t n, int
             for (int q = first ? 0 : (int)(prev & 7u) + 1; q <= o; q++) lo[q] = (int)i;
         if (last)
             for (int q = o + 1; q < 8; q++) lo[q] = (int)(i + 1);
+    }
+}
+
+// Points of the dense leaves (bricks of 8, octants in the sort keys) in cell order: a stable counting
+// sort of each leaf's range of sorted point indices by the cell of the point's voxel, octant first (the
+// order the keys already give), then (x, y, z) inside the octant; cell_tab gets the first sorted index
+// of every cell.  One block a leaf, every warp a contiguous part of its points, so that equal cells keep
+// their order; the leaves differ in size by factors of a hundred, the blocks take them in turn.
+constexpr int kCellThreads = 512, kCellWarps = kCellThreads / 32;
+__global__ void __launch_bounds__(kCellThreads)
+    k_cell_sort(const uint32_t* __restrict__ dense_list, const uint32_t* __restrict__ dense_count,
+                const int2* __restrict__ leaf_range, const char* pos, int off, int stride, float ox, float oy, float oz,
+                uint32_t* vals, uint32_t* vtmp, int* __restrict__ cell_tab, int* __restrict__ leaf_dense)
+{
+    __shared__ int s_cnt[kCellWarps][512];
+    __shared__ int s_sum[kCellWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto cell_of = [&](uint32_t v) {
+        float w[3];
+        load_pos(pos, off, stride, v, w);
+        const int x = (int)(w[0] + ox), y = (int)(w[1] + oy), z = (int)(w[2] + oz);
+        return ((x >> 2) & 1) << 8 | ((y >> 2) & 1) << 7 | ((z >> 2) & 1) << 6 | (x & 3) << 4 | (y & 3) << 2 | (z & 3);
+    };
+    const uint32_t count = *dense_count;
+    for (uint32_t d = blockIdx.x; d < count; d += gridDim.x) {
+        const uint32_t leaf = dense_list[d];
+        const int2 r = leaf_range[leaf];
+        const int per = (r.y - r.x + kCellThreads - 1) / kCellThreads * 32;  // points a warp
+        const int b0 = min(r.x + warp * per, r.y), b1 = min(b0 + per, r.y);
+#pragma unroll
+        for (int w = 0; w < kCellWarps; w++) s_cnt[w][tid] = 0;
+        __syncthreads();
+        for (int i0 = b0 + lane; i0 < b1; i0 += 128) {
+            int c[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) c[q] = i0 + 32 * q < b1 ? cell_of(vals[i0 + 32 * q]) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (c[q] >= 0) atomicAdd(&s_cnt[warp][c[q]], 1);
+        }
+        __syncthreads();
+        int run = 0;  // thread c: the places of cell c's points, warp after warp
+#pragma unroll
+        for (int w = 0; w < kCellWarps; w++) {
+            const int n = s_cnt[w][tid];
+            s_cnt[w][tid] = run;
+            run += n;
+        }
+        int x = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_sum[warp] = x;
+        __syncthreads();
+        int start = r.x + x - run;
+        for (int w = 0; w < warp; w++) start += s_sum[w];
+#pragma unroll
+        for (int w = 0; w < kCellWarps; w++) s_cnt[w][tid] += start;
+        cell_tab[(size_t)d * 512 + tid] = start;
+        if (tid == 0) leaf_dense[leaf] = (int)d + 1;
+        __syncthreads();
+        for (int i0 = b0; i0 < b1; i0 += 128) {
+            uint32_t v[4];
+            int c[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int i = i0 + 32 * q + lane;
+                v[q] = i < b1 ? vals[i] : 0u;
+                c[q] = i < b1 ? cell_of(v[q]) : -1 - lane;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const uint32_t same = __match_any_sync(0xFFFFFFFFu, c[q]);
+                int at = 0;
+                if (c[q] >= 0) {
+                    at = s_cnt[warp][c[q]];
+                    vtmp[at + __popc(same & ((1u << lane) - 1u))] = v[q];
+                }
+                __syncwarp();
+                if (c[q] >= 0 && lane == __ffs(same) - 1) s_cnt[warp][c[q]] = at + __popc(same);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        for (int i = r.x + tid; i < r.y; i += kCellThreads) vals[i] = vtmp[i];
+        __syncthreads();
     }
 }
 
@@ -1227,13 +1322,25 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
 static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves)
 {
     GVX_CK(gvx_ensure(g->leaf_range, (size_t)(nleaves + 1) * sizeof(int2)));
-    GVX_CK(gvx_ensure(g->leaf_oct, (size_t)(nleaves + 1) * 8 * sizeof(int)));
+    // (after the octants, and cleared with them: the dense numbers of the leaves, the dense leaves' count)
+    const size_t oct_words = (size_t)(nleaves + 1) * 9 + 1;
+    GVX_CK(gvx_ensure(g->leaf_oct, oct_words * sizeof(int)));
     GVX_CK(cudaMemsetAsync(g->leaf_range.p, 0, (size_t)(nleaves + 1) * sizeof(int2), g->stream));
-    GVX_CK(cudaMemsetAsync(g->leaf_oct.p, 0, (size_t)(nleaves + 1) * 8 * sizeof(int), g->stream));
+    GVX_CK(cudaMemsetAsync(g->leaf_oct.p, 0, oct_words * sizeof(int), g->stream));
+    const bool dense = g->key_shift && g->brick == 8;
+    uint32_t* dense_list = nullptr;
+    g->leaf_dense = dense ? g->leaf_oct.as<int>() + (size_t)(nleaves + 1) * 8 : nullptr;
+    g->dense_count = dense ? (uint32_t*)(g->leaf_dense + nleaves + 1) : nullptr;
+    if (dense) {
+        const size_t most = g->n_sorted / kDenseLeaf + 1;
+        GVX_CK(gvx_ensure(g->cell_tab, most * 513 * sizeof(int)));  // 512 cells a leaf, then the list of the leaves
+        dense_list = g->cell_tab.as<uint32_t>() + most * 512;
+    }
     if (g->n_sorted) {
         k_group_runs<<<blocks_for(g->n_sorted, 256), 256, 0, g->stream>>>(
             g->keys[g->sorted_buf].as<uint32_t>(), g->n_sorted, g->key_shift, 1u << g->lookup.ks.total_bits,
-            g->lookup, g->leaf_range.as<int2>(), g->leaf_oct.as<int>());
+            g->lookup, g->leaf_range.as<int2>(), g->leaf_oct.as<int>(),
+            dense_list, g->dense_count);
         g->launches++;
     }
     g->oct_leaves = nleaves;
@@ -1286,6 +1393,15 @@ gvx_status gvx_topo_octants(gvx_grid* g, const GvxSortedAttr* attr)
     memset(&none, 0, sizeof(none));
     const uint32_t nleaves = g->oct_leaves;
     if (g->key_shift) {
+        if (g->leaf_dense && g->n_sorted >= (uint32_t)kDenseLeaf) {
+            k_cell_sort<<<std::min(g->n_sorted / kDenseLeaf, 152u * 4u), kCellThreads, 0, g->stream>>>(
+                g->cell_tab.as<uint32_t>() + ((size_t)g->n_sorted / kDenseLeaf + 1) * 512, g->dense_count, g->leaf_range.as<int2>(), g->pts.pos, g->pts.pos_off,
+                g->pts.pos_stride, g->sort_trans[0], g->sort_trans[1], g->sort_trans[2],
+                g->vals[g->sorted_buf].as<uint32_t>(), g->vals[1 - g->sorted_buf].as<uint32_t>(),
+                g->cell_tab.as<int>(), g->leaf_dense);
+            g->launches++;
+            GVX_CK(cudaGetLastError());
+        }
         if (g->n_sorted && attr && attr->spos) {
             k_attr_permute<<<blocks_for(g->n_sorted, 256), 256, 0, g->stream>>>(
                 g->vals[g->sorted_buf].as<uint32_t>(), g->n_sorted, g->pts.pos, g->pts.pos_off, g->pts.pos_stride,
