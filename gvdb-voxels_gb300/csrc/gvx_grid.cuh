@@ -177,6 +177,8 @@ struct gvx_grid {
     DevBuf d_err, d_bbox;
     DevBuf d_rmax;  // float bits of the largest per-point radius of the last point permute
     DevBuf d_next;  // work-unit counters of the splat launch
+    DevBuf push_tab;  // places of the push tiles' boundary voxels, for bricks of padded side push_tab_P
+    int push_tab_P = 0, push_count = 0;
     DevBuf touched; // slots an accumulating splat visits
     DevBuf dense_units;  // units the trilinear density splat lists for k_tri_dense
     void* h_pin = nullptr;  // pinned staging of the topology's small readbacks

@@ -35,40 +35,15 @@
 
 namespace {
 constexpr int kSplatThreads = 256;
-constexpr int kSlabWarps = 4;        // warps (brick slabs) per block of the splat
-constexpr int kSlabMinBlocks = 6;    // resident blocks per SM the register budget is sized for
+constexpr int kTriWarps = 4;                // warps (brick slabs) per block of k_splat_tri
+// resident blocks per SM its registers are budgeted for: 24 clouds' splat 2.63 ms at 8 (64 registers, 200
+// bytes of spill), 2.37 at 7, 1.97 at 6, 2.12 at 5
+constexpr int kTriMinBlocks = 6;
 constexpr size_t kSlabTileMax = 48 * 1024;  // shared tile bytes of one warp at most
 constexpr int kBatchMaxGrids = 256;         // grids of one batched launch
-constexpr int kMaxRanges = 27 * 4;          // candidate ranges of a slab: at most 4 octant runs per neighbour
 constexpr float kInvPi = 0.318309886183790671538f;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 }  // namespace
-
-// apron voxel number e of a padded brick (apron 1) -> padded coordinates:
-// the two z faces, then per inner z layer the two y rows and the two x ends
-__device__ __forceinline__ void apron_voxel_coords(int e, int P, int& x, int& y, int& z)
-{
-    const int P2 = P * P;
-    if (e < 2 * P2) {
-        z = e < P2 ? 0 : P - 1;
-        const int r = e % P2;
-        y = r / P;
-        x = r % P;
-        return;
-    }
-    const int ring = 4 * P - 4;
-    const int j = e - 2 * P2;
-    z = 1 + j / ring;
-    const int r = j % ring;
-    if (r < 2 * P) {
-        y = r < P ? 0 : P - 1;
-        x = r % P;
-    } else {
-        const int r2 = r - 2 * P;
-        y = 1 + r2 / 2;
-        x = (r2 & 1) ? P - 1 : 0;
-    }
-}
 
 // sorted point attributes: (x, y, z, weight) and (vx, vy, vz, radius); with
 // per-point radii also the largest radius (float bits, NaN counted as huge)
@@ -120,6 +95,8 @@ struct SplatArgs {
     // its apron), and the slab's boundary rows go to the neighbours' y/z aprons; else the whole
     // padded brick.  tile_rows: rows of a tile layer (the brick, or the padded brick)
     bool push;
+    const uint32_t* push_tab;  // one unit a brick: the boundary voxels' places (push_table), or null
+    int push_count;
     int tile_rows;
     int lb;              // log2(brick)
     int reach;           // voxels a point's footprint reaches beyond its own voxel (neighbour pruning)
@@ -159,11 +136,16 @@ struct Tile {
             o.x = __fmaf_rn(wgt, ux, o.x);
             o.y = __fmaf_rn(wgt, uy, o.y);
             o.z = __fmaf_rn(wgt, uz, o.z);
-            if (HAS_DEN) o.w += wgt;
+            if (HAS_DEN) o.w = __fadd_rn(o.w, wgt);
             v[i] = o;
         } else {
-            ((float*)t)[i] += wgt;
+            ((float*)t)[i] = __fadd_rn(((float*)t)[i], wgt);
         }
+    }
+    // density alone: norm * shape joins the sum in one rounding
+    __device__ static void add_product(unsigned char* t, int i, float norm, float shape)
+    {
+        ((float*)t)[i] = __fmaf_rn(norm, shape, ((float*)t)[i]);
     }
     __device__ static void set(unsigned char* t, int i, float val)
     {
@@ -173,208 +155,6 @@ struct Tile {
             ((float*)t)[i] = val;
     }
 };
-
-// The footprint cells of a batch of hit points (lane i holds the i-th point of
-// the batch in sorted order; lanes without a point have ncell 0), dealt to the
-// lanes 32 at a time.  Lanes whose cells share a row apply their updates one
-// after another in lane order, which is the points' sorted order (the cells of
-// one point lie in distinct rows or distinct chunks of a row); rows apart apply
-// together.  So every voxel sums its contributions in the same order in every
-// brick that holds it.
-//
-// SMALL footprints (trilinear, and cubic of a uniform radius <= 2) span at most
-// 4 voxels on every axis: a cell is one row of the box, and of a cubic box
-// only the rows that can reach the sphere are dealt.  Their decode is a table
-// of 5 bits per layer k of the box, at bit 5k: the first row (2 bits, counted
-// from yl) and the number of rows (3 bits).  Other footprints deal every row
-// of the box in chunks of up to 4 voxels, decoded by division with multipliers
-// m = ceil(2^32 / n) (umulhi(c, m) == c / n for every c < 2^32 / n; 0 stands
-// for n = 1).
-template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__device__ __forceinline__ void deal_cells(unsigned char* tile, const float4 p, const float4 uv, uint32_t box0,
-                                           const uint32_t box1, int ncell, const int P, const int TY, const int yoff,
-                                           const int Ox, const int Oy, const int Zlo, const float R0,
-                                           const float h0, const float inv_h0, const float norm0, const float r2h0,
-                                           const float r2l0, const int lane)
-{
-    using T = Tile<HAS_DEN, HAS_VEL>;
-    constexpr bool CUBIC = MODE == GVX_SPLAT_CUBIC;
-    uint32_t aux1 = 0u, aux2 = 0u;  // SMALL: the row table; else the multipliers of the chunk and row counts
-    if (ncell > 0) {
-        const int yl = (int)((box0 >> 16) & 255u), yh = (int)(box0 >> 24);
-        if (SMALL) {
-            const int zl = (int)(box1 & 255u), zh = (int)((box1 >> 8) & 255u);
-            // A row whose float dy, dz give dy^2 + dz^2 < R^2 (1 + 1e-6) in float holds every row
-            // with R^2 - dy^2 - dz^2 > 0 exactly (the rows the weights below can reach), with a
-            // margin of several roundings; the rows of one layer that pass form one run.
-            const float lim = r2h0 * 1.000001f;
-            int cnt = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                if (zl + k > zh) break;
-                int first = 0, n = yh - yl + 1;
-                if (CUBIC) {
-                    const float dz = (float)(zl + k + Zlo) - p.z;
-                    const float dz2 = dz * dz;
-                    first = -1;
-                    n = 0;
-#pragma unroll
-                    for (int yy = 0; yy < 4; yy++) {
-                        if (yl + yy > yh) break;
-                        const float dy = (float)(yl + yy + Oy) - p.y;
-                        if (dy * dy + dz2 < lim) {
-                            if (first < 0) first = yy;
-                            n++;
-                        }
-                    }
-                    first = max(first, 0);
-                }
-                aux1 |= (uint32_t)(first | (n << 2)) << (5 * k);
-                cnt += n;
-            }
-            // a point whose box reaches the slab but whose sphere does not keeps one (empty) row,
-            // so that every point of the batch owns a cell
-            if (cnt == 0) {
-                aux1 = 1u << 2;
-                cnt = 1;
-            }
-            ncell = cnt;
-            box0 = (box0 & 0x00FFFFFFu) | ((uint32_t)zl << 24);  // xl, xh, yl, zl
-        } else {
-            const uint32_t nch = (((box0 >> 8) & 255u) - (box0 & 255u) + 4u) >> 2;
-            const uint32_t ny = (uint32_t)(yh - yl + 1);
-            aux1 = nch > 1u ? 0xFFFFFFFFu / nch + 1u : 0u;
-            aux2 = ny > 1u ? 0xFFFFFFFFu / ny + 1u : 0u;
-        }
-    }
-    // inclusive scan of the cell counts over the lanes
-    int cend = ncell;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kFull, cend, o);
-        if (lane >= o) cend += t;
-    }
-    const int ctot = __shfl_sync(kFull, cend, 31);
-    const int cstart = cend - ncell;
-    for (int g0 = 0; g0 < ctot; g0 += 32) {
-        const int g = g0 + lane;
-        const bool act = g < ctot;
-        // the point dealing this cell: the points are lanes 0 .. nb-1, each with a cell at least,
-        // so it is the number of points that start at or before g, less one
-        const bool own = ncell > 0;
-        const uint32_t starts =
-            __reduce_or_sync(kFull, own && cstart >= g0 && cstart < g0 + 32 ? 1u << (cstart - g0) : 0u);
-        const int before = __popc(__ballot_sync(kFull, own && cstart < g0));
-        const int j = before - 1 + __popc(starts & (kFull >> (31 - lane)));
-        const float px = __shfl_sync(kFull, p.x, j), py = __shfl_sync(kFull, p.y, j);
-        const float pz = __shfl_sync(kFull, p.z, j), pw = __shfl_sync(kFull, p.w, j);
-        float ux = 0.f, uy = 0.f, uz = 0.f;
-        if (HAS_VEL) {
-            ux = __shfl_sync(kFull, uv.x, j);
-            uy = __shfl_sync(kFull, uv.y, j);
-            uz = __shfl_sync(kFull, uv.z, j);
-        }
-        const uint32_t b0 = __shfl_sync(kFull, box0, j);
-        const uint32_t a1 = __shfl_sync(kFull, aux1, j);
-        const int cell = g - __shfl_sync(kFull, cstart, j);
-        const float pR = PPR ? __shfl_sync(kFull, uv.w, j) : 0.0f;
-        const int xl = (int)(b0 & 255u), xh = (int)((b0 >> 8) & 255u), yl = (int)((b0 >> 16) & 255u);
-        int lx, ly, lz;
-        if (SMALL) {
-            const int s1 = (int)((a1 >> 2) & 7u), s2 = s1 + (int)((a1 >> 7) & 7u), s3 = s2 + (int)((a1 >> 12) & 7u);
-            const int k = (cell >= s1) + (cell >= s2) + (cell >= s3);
-            const int pre = k == 0 ? 0 : (k == 1 ? s1 : (k == 2 ? s2 : s3));
-            lx = xl;
-            ly = yl + (int)((a1 >> (5 * k)) & 3u) + (cell - pre);
-            lz = (int)(b0 >> 24) + k;
-        } else {
-            const uint32_t b1 = __shfl_sync(kFull, box1, j), m2 = __shfl_sync(kFull, aux2, j);
-            const int zl = (int)(b1 & 255u);
-            const int nch = (xh - xl + 4) >> 2, ny = (int)(b0 >> 24) - yl + 1;
-            const int r = a1 ? (int)__umulhi((uint32_t)cell, a1) : cell;  // cell / nch
-            const int zz = m2 ? (int)__umulhi((uint32_t)r, m2) : r;       // r / ny
-            lx = xl + 4 * (cell - r * nch);
-            ly = yl + (r - zz * ny);
-            lz = zl + zz;
-        }
-        // the lane's voxels lx .. min(lx + 3, xh) of row (ly, lz): values, and a bit per voxel touched
-        float w[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t vm = 0u;
-        const int t0 = (lz * TY + (ly - yoff)) * P + lx;  // (the tile's rows start at padded y = yoff)
-        if (act) {
-            if (!CUBIC) {
-                const float fx0 = floorf(px), fy0 = floorf(py), fz0 = floorf(pz);
-                const float fx = px - fx0, fy = py - fy0, fz = pz - fz0;
-                const float wyz = ((float)(ly + Oy) == fy0 ? 1.f - fy : fy) * ((float)(lz + Zlo) == fz0 ? 1.f - fz : fz);
-                const float wxa = (float)(lx + Ox) == fx0 ? 1.f - fx : fx;
-                w[0] = pw * wxa * wyz;
-                vm = 1u;
-                if (lx + 1 <= xh) {
-                    w[1] = pw * fx * wyz;  // lx + 1 is floor(px) + 1 here
-                    vm |= 2u;
-                }
-            } else {
-                // M4 cubic spline (Monaghan & Lattanzio 1985), 3D normalisation 1/(pi h^3),
-                // support R = 2h.  Along the row R^2 - d^2 is formed from an error-free
-                // c = R^2 - dy^2 - dz^2 (two-product, two-sum) so that the outer branch
-                // 0.25 (2-q)^3 = 0.25 ((R^2-d^2) / (h (R+d)))^3 keeps FP32 relative
-                // accuracy up to the edge of the support.
-                float R = R0, h = h0, inv_h = inv_h0, norm = norm0, r2h = r2h0, r2l = r2l0;
-                if (PPR) {
-                    R = pR;
-                    h = 0.5f * R;
-                    inv_h = 1.0f / h;
-                    norm = kInvPi * inv_h * inv_h * inv_h;
-                    r2h = R * R;
-                    r2l = fmaf(R, R, -r2h);
-                }
-                norm *= pw;
-                const float dy = (float)(ly + Oy) - py, dz = (float)(lz + Zlo) - pz;
-                const float qy = dy * dy, ey = fmaf(dy, dy, -qy);
-                const float qz = dz * dz, ez = fmaf(dz, dz, -qz);
-                const float syz = qy + qz;
-                float bv = syz - qy;
-                const float e1 = (qy - (syz - bv)) + (qz - bv);
-                const float c1 = r2h - syz;
-                bv = c1 - r2h;
-                const float e2 = (r2h - (c1 - bv)) + (-syz - bv);
-                const float cl = e2 + r2l - ((ey + ez) + e1);
-                if (c1 + cl > 0.0f) {
-                    // the four voxels without branches (a slot outside the row or the support
-                    // is computed and masked), so that their independent chains interleave
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const float dx = (float)(lx + k + Ox) - px;
-                        const float t = fmaf(-dx, dx, c1) + cl;  // R^2 - d^2
-                        const float d2 = fmaf(dx, dx, syz);
-                        const float d = d2 > 0.0f ? d2 * rsqrtf(d2) : 0.0f;
-                        const float q = d * inv_h;
-                        const float wi = fmaf(q * q, fmaf(0.75f, q, -1.5f), 1.0f);  // q < 1
-                        const float uu = __fdividef(t, h * (R + d));               // 2 - q
-                        const float wk = norm * (q < 1.0f ? wi : 0.25f * uu * uu * uu);
-                        const bool ok = lx + k <= xh && t > 0.0f;
-                        w[k] = ok ? wk : 0.0f;
-                        vm |= ok ? 1u << k : 0u;
-                    }
-                }
-            }
-        }
-        // lanes sharing a row apply in lane order (the cells of one point lie in distinct rows
-        // or distinct chunks of a row); rows apart apply together
-        const int key = act ? (lz * P + ly) : -1 - lane;
-        const uint32_t grp = __match_any_sync(kFull, key);
-        const int rank = __popc(grp & ((1u << lane) - 1u));
-        const int nph = (int)__reduce_max_sync(kFull, (uint32_t)rank) + 1;
-        for (int ph = 0; ph < nph; ph++) {
-            if (rank == ph && vm) {
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if ((vm >> k) & 1u) T::add(tile, t0 + k, w[k], ux, uy, uz);
-            }
-            __syncwarp();
-        }
-    }
-}
 
 // one voxel out: the tile's (density in .w with velocity), or the boundary value
 template <bool HAS_DEN, bool HAS_VEL>
@@ -424,6 +204,30 @@ __device__ __forceinline__ void push_out(const SplatArgs& a, const unsigned char
                                          int nbs, int lane)
 {
     const int P = a.P, P3 = P * P * P, b = a.brick, lb = a.lb, TY = b;
+    // a brick with all the neighbours that its rows may go to, one unit: the boundary voxels' places come
+    // from a table, 32 a step (the general code below: 1,490 instructions a brick)
+    if (a.push_tab && (__ballot_sync(kFull, nbs >= 0) & 0x0043FE10u) == 0x0043FE10u) {
+        float4* const tv = (float4*)tile;
+        const size_t own = (size_t)s * P3;
+        const int lay = TY * P;
+        for (int z = 0; z < nl; z++) {
+            const size_t at = own + (uint32_t)((z0 + z) * P * P + P);
+            for (int e = lane; e < lay; e += 32) {
+                const float4 o = tv[z * lay + e];
+                a.den[at + e] = o.w;
+                a.vel[at + e] = make_float4(o.x, o.y, o.z, 0.0f);
+            }
+        }
+        for (int e = lane; e < a.push_count; e += 32) {  // (a multiple of 32, the last entries repeated)
+            const uint32_t c = a.push_tab[e];
+            const int r = __shfl_sync(kFull, nbs, (int)(c >> 24));
+            const float4 o = tv[c & 0xFFFu];
+            const size_t at = (size_t)r * P3 + ((c >> 12) & 0xFFFu);
+            a.den[at] = o.w;
+            a.vel[at] = make_float4(o.x, o.y, o.z, 0.0f);
+        }
+        return;
+    }
     const uint32_t mP = 0xFFFFFFFFu / (uint32_t)P + 1u;  // e / P == umulhi(e, mP) for e < 2^16
     // the brick's own rows: a tile layer is contiguous in the slot from padded (y 1, z)
     const size_t own = (size_t)s * P3;
@@ -524,146 +328,485 @@ __device__ __forceinline__ void reset_regions(const SplatArgs& a, unsigned char*
     __syncwarp();
 }
 
-// One warp per (brick, z-slab): the padded brick's layers are split into
-// slabs of a.slab_layers layers, each with its own shared tile, so a warp's
-// tile is a fraction of the brick and more warps stay resident.  Every slab
-// sees the same candidate points in the same order, so a voxel's sum does not
-// depend on the split.  splat_unit processes work unit u = slot * slabs + slab.
+// ---------------------------------------------------------------------------
+// Work units: one warp per (brick, z-slab).  The layers of a brick's tile (the padded brick, or its
+// interior for push tiles) are split into slabs of a.slab_layers layers, each with its own shared tile,
+// so a warp's tile is a fraction of the brick and more warps stay resident.  Every slab sees the same
+// candidate points in the same order, so a voxel's sum does not depend on the split.
+
+// the unit's brick and slab, and what the lane needs of them
+struct SplatUnit {
+    uint32_t s;      // atlas slot
+    int z0, nl;      // padded layers of the unit
+    int leaf;
+    int nl27;        // the lane's neighbour (leaf index, -1: none): lane r is neighbour (r/9, r/3%3, r%3) - 1
+    int4 org;        // the node's first 16 bytes: (lev.., x, y, z)
+    int start, end;  // the lane's candidates in the sorted points
+};
+
+// halves of a neighbour at offset d (bricks) whose points reach voxels [v0, v1] of the brick along an
+// axis: points of floor coordinate f touch [f - below, f + above]
+__device__ __forceinline__ bool unit_halves(int d, int b, int v0, int v1, int below, int above, int& lo, int& hi)
+{
+    const int hb = b >> 1, c = d * b;
+    const bool n0 = c - below <= v1 && c + hb - 1 + above >= v0, n1 = c + hb - below <= v1 && c + b - 1 + above >= v0;
+    lo = n0 ? 0 : 1;
+    hi = n1 ? 1 : 0;
+    return n0 || n1;
+}
+
+__device__ __forceinline__ void unit_slot(const SplatArgs& a, uint32_t u, bool push, SplatUnit& t)
+{
+    const uint32_t S = (uint32_t)a.slabs;
+    const uint32_t ui = S == 1u ? u : u / S;
+    const int y0 = push ? a.apron : 0;
+    t.s = a.unit_slots ? a.unit_slots[ui] : ui;
+    t.z0 = y0 + (int)(u - ui * S) * a.slab_layers;
+    t.nl = min(a.slab_layers, a.P - y0 - t.z0);
+    t.leaf = a.slot_leaf[t.s];
+}
+__device__ __forceinline__ void unit_neighbour(const SplatArgs& a, SplatUnit& t, int nbi)
+{
+    t.nl27 = nbi >= 0 ? a.nbr[(size_t)t.leaf * 27 + nbi] : -1;
+    t.org = *(const int4*)(a.nodes0 + t.leaf);
+}
+// one range of candidates per neighbour: from its first octant that can reach the tile to its last one
+// (a superset of the octants that can: two loads, and no list of runs; the footprint test drops the rest)
+__device__ __forceinline__ void unit_octants(const SplatArgs& a, SplatUnit& t, int o0, int o1)
+{
+    const int* oc = a.leaf_oct + (size_t)t.nl27 * 8;
+    t.start = oc[o0];
+    t.end = o1 == 7 ? a.leaf_range[t.nl27].y : oc[o1 + 1];
+}
+
+// Units are claimed two at a time where there are many for every warp: the counter is one address, which
+// takes an atomic every two nanoseconds (trilinear splat of 24 clouds, 2.07M bricks: 3.24 ms one at a
+// time, 2.37 two, 2.44 four, 2.53 eight).  Where units are fewer, their costs differ by more than the
+// claims cost: one at a time.
+constexpr uint32_t kClaim = 2, kClaimUnits = 16;
+
+// Units [0, total) of all grids from the counter `next`: of(u, local) -> the number of u's grid and its
+// unit there, args(k) -> that grid's arguments, range(a, t): the lane's candidates, run(a, t, k, mid): the
+// unit, which calls mid() once.  Three steps ahead of each other: while unit t is summed, the neighbours
+// (asked for as it starts) and then the candidate ranges of t1 arrive, and the brick of t2.
+template <class Of, class Args, class Range, class Run>
+__device__ __forceinline__ void unit_loop(uint32_t total, uint32_t* next, bool push, int lane, Of of, Args args,
+                                          Range range, Run run)
+{
+    const int nbi = lane < 27 ? (lane % 3) * 9 + (lane / 3 % 3) * 3 + lane / 9 : -1;
+    const uint32_t claim = total >= kClaimUnits * gridDim.x * (blockDim.x >> 5) ? kClaim : 1u;
+    uint32_t cur = 0u, lim = 0u, pre = lane == 0 ? atomicAdd(next, claim) : 0u, lu;
+    auto take = [&]() {  // the next unit's number (total and above: none)
+        if (cur == lim) {
+            cur = __shfl_sync(kFull, pre, 0);
+            lim = cur + claim;
+            if (lane == 0 && cur < total) pre = atomicAdd(next, claim);
+        }
+        return cur++;
+    };
+    uint32_t u = take();
+    if (u >= total) return;
+    SplatUnit t, t1;
+    uint32_t k = of(u, lu), k1;
+    unit_slot(args(k), lu, push, t);
+    u = take();
+    bool more = u < total;
+    k1 = k;
+    t1 = t;
+    if (more) {
+        k1 = of(u, lu);
+        unit_slot(args(k1), lu, push, t1);
+    }
+    unit_neighbour(args(k), t, nbi);
+    range(args(k), t);
+    for (;;) {
+        SplatUnit t2 = t1;
+        uint32_t k2 = k1;
+        bool more2 = false;
+        if (more) {
+            unit_neighbour(args(k1), t1, nbi);
+            u = take();
+            more2 = u < total;
+            if (more2) {
+                k2 = of(u, lu);
+                unit_slot(args(k2), lu, push, t2);
+            }
+        }
+        run(args(k), t, k, [&]() {
+            if (more) range(args(k1), t1);
+        });
+        if (!more) break;
+        k = k1;
+        t = t1;
+        k1 = k2;
+        t1 = t2;
+        more = more2;
+    }
+}
+
+// the lanes' ranges in a row: a lane's first candidate number `off`, the candidates' count; the ranges
+// with points leave in rs, in order, their first sorted index less their first candidate number
+__device__ __forceinline__ int unit_candidates(const SplatUnit& t, int lane, int& off)
+{
+    const int len = t.end - t.start;
+    off = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, off, o);
+        if (lane >= o) off += v;
+    }
+    const int total = __shfl_sync(kFull, off, 31);
+    off -= len;
+    return total;
+}
+__device__ __forceinline__ void unit_ranges(const SplatUnit& t, int lane, int off, int* rs)
+{
+    const uint32_t some = __ballot_sync(kFull, t.end > t.start);
+    if (t.end > t.start) rs[__popc(some & ((1u << lane) - 1u))] = t.start - off;
+}
+// sorted index of candidate base + lane: its range is the number of ranges with points that start at or
+// before it, less one
+__device__ __forceinline__ int unit_candidate(const SplatUnit& t, int lane, int off, int base, const int* rs)
+{
+    const bool some = t.end > t.start;
+    const uint32_t starts = __reduce_or_sync(kFull, some && off >= base && off < base + 32 ? 1u << (off - base) : 0u);
+    const int before = __popc(__ballot_sync(kFull, some && off < base));
+    return rs[before - 1 + __popc(starts & (kFull >> (31 - lane)))] + base + lane;
+}
+
+// the regions of the padded brick that voxels [xl, xh] x [yl, yh] x [zl, zh] (padded) reach, bit
+// (dx+1)*9 + (dy+1)*3 + (dz+1): per axis 1 = below the interior, 2 = inside, 4 = above it; the product
+// of the three spread sets has one bit per region reached (no carries)
+__device__ __forceinline__ uint32_t box_regions(int xl, int xh, int yl, int yh, int zl, int zh, int P, int ap)
+{
+    const int hi = P - 1 - ap;
+    const uint32_t tx = (uint32_t)(xl < ap) | (uint32_t)(xl <= hi && xh >= ap) << 1 | (uint32_t)(xh > hi) << 2;
+    const uint32_t ty = (uint32_t)(yl < ap) | (uint32_t)(yl <= hi && yh >= ap) << 1 | (uint32_t)(yh > hi) << 2;
+    const uint32_t tz = (uint32_t)(zl < ap) | (uint32_t)(zl <= hi && zh >= ap) << 1 | (uint32_t)(zh > hi) << 2;
+    return ((tx & 1u) | (tx & 2u) << 8 | (tx & 4u) << 16) * ((ty & 1u) | (ty & 2u) << 2 | (ty & 4u) << 4) * tz;
+}
+
+// ---------------------------------------------------------------------------
+// CUBIC splats, and TRILINEAR ones with velocity: the hits of a unit -- the candidates whose footprint
+// box meets the tile -- are gathered, in the points' order, in shared memory, and their footprints' rows
+// are dealt to the lanes.
+//
+// What bounds it: instruction issue (4M SPH frame, a launch of the same density: 63% of the issue slots,
+// 5,700 warp instructions a brick, 25.7 lanes active; of the 7,000 that a unit of the kernel before took,
+// 3,000 were the voxels' weights and their first turn at the tile, 1,490 the pushes, 1,090 candidates and
+// zeroing, 760 the lookups of a cell's point, 670 the further turns of lanes that share a row).  So:
+//  - candidates come as one range per neighbour and are located without a search (unit_candidate);
+//  - hits are stored where the dealing reads them, instead of being passed from lane to lane into a batch
+//    and again to the lanes that deal them;
+//  - deal_cells is in the code once: a second copy for the last hits cost more in instruction fetches
+//    (1.3 of 8 stalled cycles) than the loop around it;
+//  - a push tile's boundary voxels find their places in a table (push_table).
+// 4M points 2.53 -> 2.22 ms, 778k 461 -> 417 us, a million points of radii 1-3 without velocity 1.35 ->
+// 0.86 ms (with whole bricks a unit).  Tried and dropped: lanes that own rows of the tile and take their
+// hits from a mask per row (3.41 ms: half the lanes idle), cells queued row by row so that lanes rarely
+// share one (3.95 ms: the queue costs more than the turns it saves), predicated stores instead of
+// branches in a turn (2.64 against 2.53).
+constexpr int kCellWarps = 4;
+
+// hits gathered before they are dealt: 24 with density and velocity, so that five blocks of four 10 KB
+// tiles and their hits fit an SM (a 8^3 brick's interior, x with its apron)
+template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR>
+struct Hits {
+    static constexpr int most = HAS_DEN && HAS_VEL ? 24 : 32;
+    // beside (x, y, z, weight): with velocity (vx, vy, vz, R), else with per-point radii (1/h, norm, low
+    // part of R^2, R)
+    static constexpr bool Q = HAS_VEL || PPR;
+    static __host__ __device__ size_t bytes() { return most * sizeof(float4) * (Q ? 2 : 1); }
+};
+
+// M4 cubic spline (Monaghan & Lattanzio 1985), 3D normalisation 1/(pi h^3), support R = 2h
+struct CubicRadius {
+    float R, h, inv_h, norm, r2l, r2h;
+    __device__ explicit CubicRadius(float R_) : R(R_), h(0.5f * R_), inv_h(1.0f / h)
+    {
+        norm = kInvPi * inv_h * inv_h * inv_h;
+        r2h = __fmul_rn(R, R);
+        r2l = fmaf(R, R, -r2h);
+    }
+    __device__ CubicRadius(float R_, float inv_h_, float norm_, float r2l_)
+        : R(R_), h(0.5f * R_), inv_h(inv_h_), norm(norm_), r2l(r2l_)
+    {
+        r2h = __fmul_rn(R, R);
+    }
+};
+
+// approximate reciprocal square root and quotient without the scaling of denormal arguments (none here:
+// the callers' arguments are at least 1e-36, or their result is not used)
+__device__ __forceinline__ float rsqrt_fast(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float div_fast(float x, float y)
+{
+    float q;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(q) : "f"(x), "f"(y));
+    return q;
+}
+
+// The footprint cells of the hits 0 .. nb-1 (sp, sq: in shared memory, in sorted order), dealt to the
+// lanes 32 at a time.  Lanes whose cells share a row apply their updates one
+// after another in lane order, which is the points' sorted order (the cells of
+// one point lie in distinct rows or distinct chunks of a row); rows apart apply
+// together.  So every voxel sums its contributions in the same order in every
+// brick that holds it.
+//
+// SMALL footprints (trilinear, and cubic of a uniform radius <= 2) span at most
+// 4 voxels on every axis: a cell is one row of the box, and of a cubic box
+// only the rows that can reach the sphere are dealt.  Their decode is a table
+// of 5 bits per layer k of the box, at bit 5k: the first row (2 bits, counted
+// from yl) and the number of rows (3 bits).  Other footprints deal every row
+// of the box in chunks of up to 4 voxels, decoded by division with multipliers
+// m = ceil(2^32 / n) (umulhi(c, m) == c / n for every c < 2^32 / n; 0 stands
+// for n = 1).
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__device__ __forceinline__ void splat_unit(const SplatArgs& a, const uint32_t u, unsigned char* tile, uint64_t* bar,
-                                           int* s_rs_w, int* s_ro_w, uint32_t& phase,
-                                           const int lane)
+__device__ __forceinline__ void deal_cells(unsigned char* tile, const float4* sp, const float4* sq, const int nb,
+                                           const int P, const int TY, const int yoff, const int nl, const int Ox,
+                                           const int Oy, const int Zlo, const CubicRadius& uni, const int lane)
+{
+    using T = Tile<HAS_DEN, HAS_VEL>;
+    constexpr bool CUBIC = MODE == GVX_SPLAT_CUBIC;
+    // the lane's hit: its box in the tile (8 bits a bound), its cells; aux1, aux2: SMALL the row table,
+    // else the multipliers of the chunk and row counts
+    uint32_t box0 = 0u, box1 = 0u, aux1 = 0u, aux2 = 0u;
+    int ncell = 0;
+    if (lane < nb) {
+        const float4 p = sp[lane];
+        int xl, xh, yl, yh, zl, zh;
+        if (!CUBIC) {
+            xl = (int)floorf(p.x) - Ox, yl = (int)floorf(p.y) - Oy, zl = (int)floorf(p.z) - Zlo;
+            xh = xl + 1, yh = yl + 1, zh = zl + 1;
+        } else {
+            const float R = PPR ? sq[lane].w : uni.R;
+            xl = (int)floorf(p.x - R) + 1 - Ox, xh = (int)ceilf(p.x + R) - 1 - Ox;
+            yl = (int)floorf(p.y - R) + 1 - Oy, yh = (int)ceilf(p.y + R) - 1 - Oy;
+            zl = (int)floorf(p.z - R) + 1 - Zlo, zh = (int)ceilf(p.z + R) - 1 - Zlo;
+        }
+        xl = max(xl, 0), xh = min(xh, P - 1);
+        yl = max(yl, yoff), yh = min(yh, yoff + TY - 1);
+        zl = max(zl, 0), zh = min(zh, nl - 1);
+        const int ny = yh - yl + 1;
+        if (SMALL) {
+            // A row whose float dy, dz give dy^2 + dz^2 < R^2 (1 + 1e-6) in float holds every row
+            // with R^2 - dy^2 - dz^2 > 0 exactly (the rows the weights below can reach), with a
+            // margin of several roundings; the rows of one layer that pass form one run.
+            const float lim = uni.r2h * 1.000001f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (zl + k > zh) break;
+                int first = 0, n = ny;
+                if (CUBIC) {
+                    const float dz = (float)(zl + k + Zlo) - p.z;
+                    const float dz2 = dz * dz;
+                    first = -1;
+                    n = 0;
+#pragma unroll
+                    for (int yy = 0; yy < 4; yy++) {
+                        if (yl + yy > yh) break;
+                        const float dy = (float)(yl + yy + Oy) - p.y;
+                        if (dy * dy + dz2 < lim) {
+                            if (first < 0) first = yy;
+                            n++;
+                        }
+                    }
+                    first = max(first, 0);
+                }
+                aux1 |= (uint32_t)(first | (n << 2)) << (5 * k);
+                ncell += n;
+            }
+            // a point whose box reaches the slab but whose sphere does not keeps one (empty) row,
+            // so that every point of the batch owns a cell
+            if (ncell == 0) {
+                aux1 = 1u << 2;
+                ncell = 1;
+            }
+            box0 = (uint32_t)xl | (uint32_t)xh << 8 | (uint32_t)yl << 16 | (uint32_t)zl << 24;
+        } else {
+            const uint32_t nch = (uint32_t)(xh - xl + 4) >> 2;
+            aux1 = nch > 1u ? 0xFFFFFFFFu / nch + 1u : 0u;
+            aux2 = ny > 1 ? 0xFFFFFFFFu / (uint32_t)ny + 1u : 0u;
+            ncell = (int)nch * ny * (zh - zl + 1);
+            box0 = (uint32_t)xl | (uint32_t)xh << 8 | (uint32_t)yl << 16 | (uint32_t)yh << 24;
+            box1 = (uint32_t)zl;
+        }
+    }
+    // inclusive scan of the cell counts over the lanes
+    int cend = ncell;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, cend, o);
+        if (lane >= o) cend += t;
+    }
+    const int ctot = __shfl_sync(kFull, cend, 31);
+    const int cstart = cend - ncell;
+    for (int g0 = 0; g0 < ctot; g0 += 32) {
+        const int g = g0 + lane;
+        const bool act = g < ctot;
+        // the hit dealing this cell: each hit has a cell at least, so it is the number of hits that
+        // start at or before g, less one
+        const bool own = ncell > 0;
+        const uint32_t starts =
+            __reduce_or_sync(kFull, own && cstart >= g0 && cstart < g0 + 32 ? 1u << (cstart - g0) : 0u);
+        const int before = __popc(__ballot_sync(kFull, own && cstart < g0));
+        const int j = before - 1 + __popc(starts & (kFull >> (31 - lane)));
+        const float4 p = sp[j];
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (HAS_VEL || PPR) q = sq[j];
+        const uint32_t b0 = __shfl_sync(kFull, box0, j);
+        const uint32_t a1 = __shfl_sync(kFull, aux1, j);
+        const int cell = g - __shfl_sync(kFull, cstart, j);
+        const int xl = (int)(b0 & 255u), xh = (int)((b0 >> 8) & 255u), yl = (int)((b0 >> 16) & 255u);
+        int lx, ly, lz;
+        if (SMALL) {
+            const int s1 = (int)((a1 >> 2) & 7u), s2 = s1 + (int)((a1 >> 7) & 7u), s3 = s2 + (int)((a1 >> 12) & 7u);
+            const int k = (cell >= s1) + (cell >= s2) + (cell >= s3);
+            const int pre = k == 0 ? 0 : (k == 1 ? s1 : (k == 2 ? s2 : s3));
+            lx = xl;
+            ly = yl + (int)((a1 >> (5 * k)) & 3u) + (cell - pre);
+            lz = (int)(b0 >> 24) + k;
+        } else {
+            const uint32_t b1 = __shfl_sync(kFull, box1, j), m2 = __shfl_sync(kFull, aux2, j);
+            const int nch = (xh - xl + 4) >> 2, ny = (int)(b0 >> 24) - yl + 1;
+            const int r = a1 ? (int)__umulhi((uint32_t)cell, a1) : cell;  // cell / nch
+            const int zz = m2 ? (int)__umulhi((uint32_t)r, m2) : r;       // r / ny
+            lx = xl + 4 * (cell - r * nch);
+            ly = yl + (r - zz * ny);
+            lz = (int)b1 + zz;
+        }
+        // the lane's voxels lx .. min(lx + 3, xh) of row (ly, lz): values, and a bit per voxel touched
+        float w[4] = {0.f, 0.f, 0.f, 0.f}, norm = 0.f;
+        uint32_t vm = 0u;
+        const int t0 = (lz * TY + (ly - yoff)) * P + lx;  // (the tile's rows start at padded y = yoff)
+        if (act) {
+            if (!CUBIC) {
+                const float fx0 = floorf(p.x), fy0 = floorf(p.y), fz0 = floorf(p.z);
+                const float fx = p.x - fx0, fy = p.y - fy0, fz = p.z - fz0;
+                const float wyz = __fmul_rn((float)(ly + Oy) == fy0 ? 1.f - fy : fy,
+                                            (float)(lz + Zlo) == fz0 ? 1.f - fz : fz);
+                const float wxa = (float)(lx + Ox) == fx0 ? 1.f - fx : fx;
+                w[0] = __fmul_rn(__fmul_rn(p.w, wxa), wyz);
+                vm = 1u;
+                if (lx + 1 <= xh) {
+                    w[1] = __fmul_rn(__fmul_rn(p.w, fx), wyz);  // lx + 1 is floor(px) + 1 here
+                    vm |= 2u;
+                }
+            } else {
+                // Along the row R^2 - d^2 is formed from an error-free
+                // c = R^2 - dy^2 - dz^2 (two-product, two-sum) so that the outer branch
+                // 0.25 (2-q)^3 = 0.25 ((R^2-d^2) / (h (R+d)))^3 keeps FP32 relative
+                // accuracy up to the edge of the support.
+                const CubicRadius c = !PPR ? uni : HAS_VEL ? CubicRadius(q.w) : CubicRadius(q.w, q.x, q.y, q.z);
+                norm = c.norm * p.w;
+                const float dy = (float)(ly + Oy) - p.y, dz = (float)(lz + Zlo) - p.z;
+                // (each step rounded on its own: a fused one would not have the error it is assumed to have)
+                const float qy = __fmul_rn(dy, dy), ey = fmaf(dy, dy, -qy);
+                const float qz = __fmul_rn(dz, dz), ez = fmaf(dz, dz, -qz);
+                const float syz = __fadd_rn(qy, qz);
+                float bv = __fsub_rn(syz, qy);
+                const float e1 = __fadd_rn(__fsub_rn(qy, __fsub_rn(syz, bv)), __fsub_rn(qz, bv));
+                const float c1 = __fsub_rn(c.r2h, syz);
+                bv = __fsub_rn(c1, c.r2h);
+                const float e2 = __fadd_rn(__fsub_rn(c.r2h, __fsub_rn(c1, bv)), __fsub_rn(-syz, bv));
+                const float cl = e2 + c.r2l - ((ey + ez) + e1);
+                if (c1 + cl > 0.0f) {
+                    // the four voxels without branches (a slot outside the row or the support
+                    // is computed and masked), so that their independent chains interleave
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float dx = (float)(lx + k + Ox) - p.x;
+                        const float t = fmaf(-dx, dx, c1) + cl;  // R^2 - d^2
+                        const float d2 = fmaf(dx, dx, syz);
+                        const float d = d2 > 1.0e-36f ? d2 * rsqrt_fast(d2) : 0.0f;
+                        const float qq = d * c.inv_h;
+                        const float wi = fmaf(qq * qq, fmaf(0.75f, qq, -1.5f), 1.0f);  // q < 1
+                        const float uu = div_fast(t, c.h * (c.R + d));                 // 2 - q
+                        const float shape = qq < 1.0f ? wi : 0.25f * uu * uu * uu;
+                        const bool ok = lx + k <= xh && t > 0.0f;
+                        w[k] = HAS_VEL ? __fmul_rn(norm, shape) : shape;
+                        vm |= ok ? 1u << k : 0u;
+                    }
+                }
+            }
+        }
+        // lanes sharing a row apply in lane order (the cells of one point lie in distinct rows
+        // or distinct chunks of a row); rows apart apply together
+        const int key = act ? (lz * P + ly) : -1 - lane;
+        const uint32_t grp = __match_any_sync(kFull, key);
+        const int rank = __popc(grp & ((1u << lane) - 1u));
+        const int nph = (int)__reduce_max_sync(kFull, (uint32_t)rank) + 1;
+        for (int ph = 0; ph < nph; ph++) {
+            if (rank == ph && vm) {
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if ((vm >> k) & 1u) {
+                        if (CUBIC && !HAS_VEL)
+                            T::add_product(tile, t0 + k, norm, w[k]);
+                        else
+                            T::add(tile, t0 + k, w[k], q.x, q.y, q.z);
+                    }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// shared memory of one warp: the tile, the hits
+template <bool HAS_DEN, bool HAS_VEL>
+__host__ __device__ inline size_t cell_tile_bytes(int layers, int rows, int P)
+{
+    return (Tile<HAS_DEN, HAS_VEL>::bytes(layers * rows * P) + 15) & ~(size_t)15;
+}
+template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR>
+__host__ __device__ inline size_t cell_warp_bytes(int layers, int rows, int P)
+{
+    return cell_tile_bytes<HAS_DEN, HAS_VEL>(layers, rows, P) + Hits<HAS_DEN, HAS_VEL, MODE, PPR>::bytes();
+}
+
+template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL, class Mid>
+__device__ __forceinline__ void cell_unit(const SplatArgs& a, const SplatUnit& t, unsigned char* mem, uint64_t* bar,
+                                         int* rs, uint32_t& phase, const int lane, Mid mid)
 {
     using T = Tile<HAS_DEN, HAS_VEL>;
     constexpr bool CUBIC = MODE == GVX_SPLAT_CUBIC;
     // single-channel tiles go to HBM in one bulk (TMA) copy; the combined
     // density+velocity tile is split into the two channels by vector stores
     constexpr bool BULK = !(HAS_DEN && HAS_VEL);
-    // cubic constants of a uniform radius (per point with PPR)
-    const float R0 = a.radius, h0 = 0.5f * R0, inv_h0 = CUBIC && !PPR ? 1.0f / h0 : 0.0f;
-    const float norm0 = kInvPi * inv_h0 * inv_h0 * inv_h0, r2h0 = R0 * R0, r2l0 = fmaf(R0, R0, -r2h0);
-    const int P = a.P, P2 = P * P, P3 = P2 * P, ap = a.apron, b = a.brick;
-    const int L = a.slab_layers, S = a.slabs;
-    // the tile: rows [yoff, yoff + TY) of layers [z0, z0 + nl) of the padded brick, x whole
     constexpr bool PUSHABLE = HAS_DEN && HAS_VEL;  // the host sets push for these kernels only
     const bool push = PUSHABLE && a.push;
-    const int TY = push ? a.tile_rows : P, yoff = push ? ap : 0, zend = push ? P - ap : P;
-    const uint32_t ui = u / (uint32_t)S;  // the unit's brick in the unit order, its slab u - ui * S
-    const uint32_t s = a.unit_slots ? a.unit_slots[ui] : ui;
-    const int z0 = yoff + (int)(u - ui * (uint32_t)S) * L;  // first padded layer of the slab
-    const int nl = min(L, zend - z0);
-    const int nvox = nl * TY * P;
-    const size_t gofs = (size_t)s * P3 + (size_t)z0 * P2;  // slab start in the channel (no push)
-    const int leaf = a.slot_leaf[s];
-    const GvxNode* nd = a.nodes0 + leaf;
-    const int Ox = nd->pos[0] - ap, Oy = nd->pos[1] - ap, Oz = nd->pos[2] - ap;  // padded origin
-    const int Zlo = Oz + z0, Zhi = Oz + z0 + nl - 1;                          // world z of the slab
+    const CubicRadius uni(CUBIC && !PPR ? a.radius : 2.0f);
+    const int P = a.P, P2 = P * P, ap = a.apron;
+    const int TY = push ? a.tile_rows : P, yoff = push ? ap : 0;
+    const int z0 = t.z0, nl = t.nl, nvox = nl * TY * P;
+    const size_t gofs = (size_t)t.s * (P2 * P) + (size_t)z0 * P2;  // slab start in the channel (no push)
+    const int Ox = t.org.y - ap, Oy = t.org.z - ap, Zlo = t.org.w - ap + z0;
+    unsigned char* tile = mem;
+    using H = Hits<HAS_DEN, HAS_VEL, MODE, PPR>;
+    float4* sp = (float4*)(mem + cell_tile_bytes<HAS_DEN, HAS_VEL>(a.slab_layers, TY, P));
+    float4* sq = sp + H::most;
+    const uint32_t lt = (1u << lane) - 1u;
 
-    // ---- candidate ranges: the octants of the 27 neighbours (the brick itself included) whose
-    // points can reach the slab, in the sorted order of the points -- neighbours by key, i.e. by
-    // (dx, dy, dz), and inside a brick by octant 4 hx + 2 hy + hz.  Lane r < 27 takes the
-    // neighbour (dx, dy, dz) = (r / 9, r / 3 % 3, r % 3) - 1.  Along each axis a half of a brick
-    // (floor coordinates [c, c + b/2)) is read when its points, whose footprints reach `reach`
-    // voxels from their own, can touch the tile's extent.  A lane's octants are merged
-    // into runs of adjacent octants: at most 4 ranges a lane.
-    // with per-point radii the reach is that of the largest radius (ceil R voxels, at most brick - 1)
-    const int reach = PPR && a.rmax ? min(a.reach, (int)ceilf(__uint_as_float(*a.rmax))) : a.reach;
-    bool has_nb = false;
-    int nbs = -1;        // lane r < 27: the atlas slot of neighbour r (-1: none)
-    uint32_t need = 0u;  // octants to read
-    int oc[9];           // first index of each octant, and the end of the brick's points
-#pragma unroll
-    for (int o = 0; o < 9; o++) oc[o] = 0;
-    if (lane < 27) {
-        const int dx = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dz = lane % 3 - 1;
-        const int nl_ = a.nbr[(size_t)leaf * 27 + (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)];
-        if (nl_ >= 0) {
-            nbs = a.leaf_slot[nl_];
-            has_nb = nbs >= 0;
-            const int hb = b >> 1;
-            const int cx = nd->pos[0] + dx * b, cy = nd->pos[1] + dy * b, cz = nd->pos[2] + dz * b;
-            uint32_t mx = 0u, my = 0u, mz = 0u;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int x0 = cx + h * hb, y0 = cy + h * hb, z0h = cz + h * hb;
-                mx |= (uint32_t)(x0 - reach <= Ox + P - 1 && x0 + hb - 1 + reach >= Ox) << h;
-                my |= (uint32_t)(y0 - reach <= Oy + yoff + TY - 1 && y0 + hb - 1 + reach >= Oy + yoff) << h;
-                mz |= (uint32_t)(z0h - reach <= Zhi && z0h + hb - 1 + reach >= Zlo) << h;
-            }
-#pragma unroll
-            for (int o = 0; o < 8; o++) need |= ((mx >> (o >> 2)) & (my >> ((o >> 1) & 1)) & (mz >> (o & 1)) & 1u) << o;
-            if (need) {
-                const int4* q = (const int4*)(a.leaf_oct + (size_t)nl_ * 8);
-                const int4 q0 = q[0], q1 = q[1];
-                oc[0] = q0.x, oc[1] = q0.y, oc[2] = q0.z, oc[3] = q0.w;
-                oc[4] = q1.x, oc[5] = q1.y, oc[6] = q1.z, oc[7] = q1.w;
-                oc[8] = a.leaf_range[nl_].y;
-            }
-        }
-    }
-    const uint32_t nbmask = __ballot_sync(kFull, has_nb);  // bit r: neighbour r (key order) is active
-    // runs of needed octants: their count and points
-    int nr = 0, len = 0;
-    {
-        bool in = false;
-        int rs0 = 0;
-#pragma unroll
-        for (int o = 0; o <= 8; o++) {
-            const bool nd_o = o < 8 && ((need >> o) & 1u);
-            if (nd_o && !in) {
-                rs0 = oc[o];
-                in = true;
-            } else if (!nd_o && in) {
-                if (oc[o] > rs0) {
-                    nr++;
-                    len += oc[o] - rs0;
-                }
-                in = false;
-            }
-        }
-    }
-    int incl = len, rincl = nr;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kFull, incl, o), u = __shfl_up_sync(kFull, rincl, o);
-        if (lane >= o) {
-            incl += t;
-            rincl += u;
-        }
-    }
-    const int total = __shfl_sync(kFull, incl, 31);
-    const int m = __shfl_sync(kFull, rincl, 31);
-    {
-        int rank = rincl - nr, off = incl - len;
-        bool in = false;
-        int rs0 = 0;
-#pragma unroll
-        for (int o = 0; o <= 8; o++) {
-            const bool nd_o = o < 8 && ((need >> o) & 1u);
-            if (nd_o && !in) {
-                rs0 = oc[o];
-                in = true;
-            } else if (!nd_o && in) {
-                if (oc[o] > rs0) {
-                    s_rs_w[rank] = rs0;
-                    s_ro_w[rank] = off;
-                    rank++;
-                    off += oc[o] - rs0;
-                }
-                in = false;
-            }
-        }
-    }
-    if (lane == 0) s_ro_w[m] = total;
+    int off;
+    const int total = unit_candidates(t, lane, off);
     // an accumulating splat leaves a slab that no point reaches as it is: no load, no store
-    if (a.accum && total == 0) return;
+    if (a.accum && total == 0) {
+        mid();
+        return;
+    }
+    unit_ranges(t, lane, off, rs);
+    const uint32_t nbmask = __ballot_sync(kFull, t.nl27 >= 0);  // bit r: neighbour r is active
 
     // ---- tile: previous values (accumulate) or zeros, once the bulk store of the warp's last
     // slab has read it (the wait is deferred to here: that read overlaps the ranges above)
     if (BULK) {
         if (lane == 0) bulk_wait_read_all();
-        __syncwarp();
     }
+    __syncwarp();
     if (a.accum) {
         if (BULK) {
             if (lane == 0) {
@@ -687,130 +830,75 @@ __device__ __forceinline__ void splat_unit(const SplatArgs& a, const uint32_t u,
         for (int i = lane; i < n16; i += 32) ((float4*)tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncwarp();
+    mid();
 
-    // ---- candidates, 32 at a time, in sorted order.  Each lane tests one
-    // candidate and sizes the cells of its footprint in the slab (a cell = up
-    // to 4 consecutive x voxels of one (y, z) row).  Most candidates miss the
-    // slab, so the hits are first gathered, in order, into a batch of up to 32
-    // points (lane i holds the i-th); a batch that the next round's hits would
-    // overflow, and the last one, has its cells dealt (deal_cells).  Batches
-    // are dealt in order, so the order of every voxel's sum is the points'
-    // sorted order.
-    float4 bp = make_float4(0.f, 0.f, 0.f, 0.f), buv = make_float4(0.f, 0.f, 0.f, 0.f);
-    uint32_t bb0 = 0u, bb1 = 0u;
-    int bnc = 0, nb = 0;  // this lane's cell count; points in the batch (warp-uniform)
-    // the regions of the padded slab (bit (dx+1)*9 + (dy+1)*3 + (dz+1): below, inside or above
-    // the interior on each axis) that this lane's hits reach
+    // ---- candidates, 32 at a time, in sorted order: those whose footprint box meets the tile join the
+    // hits; hits that the next round's would overflow, and the last ones, are added to the tile
+    int nb = 0;  // hits gathered (warp-uniform)
     uint32_t touched = 0u;
     for (int base = 0;; base += 32) {
-        const bool done = base >= total;  // one more pass deals the last batch
-        const int v = base + lane;
-        int idx = -1;
-        if (v < total) {
-            int lo = 0, hi = m - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (s_ro_w[mid] <= v)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            idx = s_rs_w[lo] + (v - s_ro_w[lo]);
-        }
-        float4 p = make_float4(0.f, 0.f, 0.f, 0.f), uv = make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t box0 = 0u, box1 = 0u;  // footprint in slab-tile coordinates, 8 bits a bound
-        int ncell = 0;
-        if (idx >= 0) {
+        const bool done = base >= total;  // one more pass deals the last hits
+        const int idx = unit_candidate(t, lane, off, base, rs);
+        bool hit = false;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+        if (base + lane < total) {
             p = a.spos[idx];
-            if (HAS_VEL || PPR) uv = a.svel[idx];
+            if (HAS_VEL || PPR) q = a.svel[idx];
             int xl, xh, yl, yh, zl, zh;
             if (!CUBIC) {
-                const int x0 = (int)floorf(p.x) - Ox, y0 = (int)floorf(p.y) - Oy, zb = (int)floorf(p.z) - Zlo;
-                xl = max(x0, 0), xh = min(x0 + 1, P - 1);
-                yl = max(y0, yoff), yh = min(y0 + 1, yoff + TY - 1);
-                zl = max(zb, 0), zh = min(zb + 1, nl - 1);
+                xl = (int)floorf(p.x) - Ox, yl = (int)floorf(p.y) - Oy, zl = (int)floorf(p.z) - Zlo;
+                xh = xl + 1, yh = yl + 1, zh = zl + 1;
             } else {
                 // voxels strictly inside (p - R, p + R) on every axis
-                const float R = PPR ? uv.w : R0;
+                const float R = PPR ? q.w : uni.R;
                 if (PPR && R > a.max_radius) atomicOr(a.err, GVX_DERR_RADIUS);
-                xl = max((int)floorf(p.x - R) + 1 - Ox, 0), xh = min((int)ceilf(p.x + R) - 1 - Ox, P - 1);
-                yl = max((int)floorf(p.y - R) + 1 - Oy, yoff);
-                yh = min((int)ceilf(p.y + R) - 1 - Oy, yoff + TY - 1);
-                zl = max((int)floorf(p.z - R) + 1 - Zlo, 0), zh = min((int)ceilf(p.z + R) - 1 - Zlo, nl - 1);
+                xl = (int)floorf(p.x - R) + 1 - Ox, xh = (int)ceilf(p.x + R) - 1 - Ox;
+                yl = (int)floorf(p.y - R) + 1 - Oy, yh = (int)ceilf(p.y + R) - 1 - Oy;
+                zl = (int)floorf(p.z - R) + 1 - Zlo, zh = (int)ceilf(p.z + R) - 1 - Zlo;
+                if (PPR && !HAS_VEL) {
+                    const CubicRadius c(R);
+                    q = make_float4(c.inv_h, c.norm, c.r2l, R);
+                }
             }
-            if (xl <= xh && yl <= yh && zl <= zh) {
-                const int nch = (xh - xl + 4) >> 2, ny = yh - yl + 1;
-                ncell = nch * ny * (zh - zl + 1);
-                box0 = (uint32_t)xl | ((uint32_t)xh << 8) | ((uint32_t)yl << 16) | ((uint32_t)yh << 24);
-                box1 = (uint32_t)zl | ((uint32_t)zh << 8);
-                // per axis: 1 = reaches below the interior, 2 = the interior, 4 = above it; the
-                // product of the three spread sets has one bit per region reached (no carries)
-                const int zpl = z0 + zl, zph = z0 + zh;
-                const uint32_t tx = (uint32_t)(xl < ap) | (uint32_t)(xl <= P - 1 - ap && xh >= ap) << 1 |
-                                    (uint32_t)(xh > P - 1 - ap) << 2;
-                const uint32_t ty = (uint32_t)(yl < ap) | (uint32_t)(yl <= P - 1 - ap && yh >= ap) << 1 |
-                                    (uint32_t)(yh > P - 1 - ap) << 2;
-                const uint32_t tz = (uint32_t)(zpl < ap) | (uint32_t)(zpl <= P - 1 - ap && zph >= ap) << 1 |
-                                    (uint32_t)(zph > P - 1 - ap) << 2;
-                touched |= ((tx & 1u) | (tx & 2u) << 8 | (tx & 4u) << 16) *
-                           ((ty & 1u) | (ty & 2u) << 2 | (ty & 4u) << 4) * tz;
+            xl = max(xl, 0), xh = min(xh, P - 1);
+            yl = max(yl, yoff), yh = min(yh, yoff + TY - 1);
+            zl = max(zl, 0), zh = min(zh, nl - 1);
+            hit = xl <= xh && yl <= yh && zl <= zh;
+            if (hit && nbmask != 0x7FFFFFFu && ap) touched |= box_regions(xl, xh, yl, yh, z0 + zl, z0 + zh, P, ap);
+        }
+        // the hits that there is room for; when there is no more, all gathered are dealt first
+        uint32_t hm = __ballot_sync(kFull, hit);
+        do {
+            const int at = nb + __popc(hm & lt);
+            if (hit && at < H::most) {
+                sp[at] = p;
+                if (HAS_VEL || PPR) sq[at] = q;
+                hit = false;
             }
-        }
-        const uint32_t hm = __ballot_sync(kFull, ncell > 0);
-        const int h = __popc(hm);
-        if (done ? nb > 0 : nb + h > 32) {
-            deal_cells<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(tile, bp, buv, bb0, bb1, bnc, P, TY, yoff, Ox, Oy, Zlo, R0,
-                                                           h0, inv_h0, norm0, r2h0, r2l0, lane);
-            bnc = 0;
-            nb = 0;
-        }
+            nb = min(nb + __popc(hm), H::most);
+            hm = __ballot_sync(kFull, hit);
+            if (hm || (done && nb > 0)) {
+                __syncwarp();
+                deal_cells<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(tile, sp, sq, nb, P, TY, yoff, nl, Ox, Oy, Zlo, uni, lane);
+                nb = 0;
+            }
+        } while (hm);
         if (done) break;
-        if (h == 0) continue;
-        // lane nb + i takes the i-th hit of this round: the lane of the (i+1)-th set bit of hm
-        const int d = lane - nb;
-        const bool take = d >= 0 && d < h;
-        int src = lane;
-        if (take) {
-            int lo = 0, hi = 31;
-#pragma unroll
-            for (int it = 0; it < 5; it++) {
-                const int mid = (lo + hi) >> 1;
-                if (__popc(hm & (kFull >> (31 - mid))) > d)
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
-            src = lo;
-        }
-        const float4 np = make_float4(__shfl_sync(kFull, p.x, src), __shfl_sync(kFull, p.y, src),
-                                      __shfl_sync(kFull, p.z, src), __shfl_sync(kFull, p.w, src));
-        float4 nuv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (HAS_VEL || PPR)
-            nuv = make_float4(__shfl_sync(kFull, uv.x, src), __shfl_sync(kFull, uv.y, src),
-                              __shfl_sync(kFull, uv.z, src), __shfl_sync(kFull, uv.w, src));
-        const uint32_t n0 = __shfl_sync(kFull, box0, src), n1 = __shfl_sync(kFull, box1, src);
-        const int nn = __shfl_sync(kFull, ncell, src);
-        if (take) {
-            bp = np;
-            buv = nuv;
-            bb0 = n0;
-            bb1 = n1;
-            bnc = nn;
-        }
-        nb += h;
     }
 
-    // ---- apron voxels with no neighbouring brick take the boundary value (0):
-    // the apron region facing each missing neighbour (apron 1), clipped to the slab.  The tile
-    // was zeroed, so with the boundary value 0 only the regions that some hit reached are reset.
+    // ---- apron voxels with no neighbouring brick take the boundary value (0): the apron region facing
+    // each missing neighbour (apron 1), clipped to the slab.  The tile was zeroed, so with the boundary
+    // value 0 only the regions that some hit reached are reset.
     uint32_t reset = ~nbmask & 0x7FFFFFFu & ~(1u << 13);
-    if (a.boundval == 0.0f) reset &= __reduce_or_sync(kFull, touched);
+    if (a.boundval == 0.0f && reset) reset &= __reduce_or_sync(kFull, touched);
     if (push) reset &= (1u << 4) | (1u << 22);  // the tile's only apron voxels: the two x faces
     if (ap && reset && !a.accum) reset_regions<HAS_DEN, HAS_VEL>(a, tile, reset, z0, nl, TY, yoff, lane);
 
     // ---- out to HBM
     if (push) {
-        if (PUSHABLE) push_out<HAS_DEN, HAS_VEL>(a, tile, s, z0, nl, nbs, lane);
+        const int nbs = t.nl27 >= 0 ? a.leaf_slot[t.nl27] : -1;
+        if (PUSHABLE) push_out<HAS_DEN, HAS_VEL>(a, tile, t.s, z0, nl, nbs, lane);
+        __syncwarp();
     } else if (BULK) {
         fence_async_smem();
         __syncwarp();
@@ -832,83 +920,85 @@ __device__ __forceinline__ void splat_unit(const SplatArgs& a, const uint32_t u,
     }
 }
 
-template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks) k_splat_slab(SplatArgs a)
+template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL, class Of, class Args>
+__device__ __forceinline__ void cell_loop(const SplatArgs& a0, uint32_t total, uint32_t* next, unsigned char* smem, Of of,
+                                         Args args)
 {
-    using T = Tile<HAS_DEN, HAS_VEL>;
-    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr bool CUBIC = MODE == GVX_SPLAT_CUBIC;
+    __shared__ __align__(8) uint64_t s_bar[kCellWarps];
+    __shared__ int s_rs[kCellWarps][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned char* tile = smem + (size_t)wid * T::bytes(a.slab_layers * a.tile_rows * a.P);
-    __shared__ __align__(8) uint64_t s_bar[kSlabWarps];
-    __shared__ int s_rs[kSlabWarps][kMaxRanges + 1];
-    __shared__ int s_ro[kSlabWarps][kMaxRanges + 1];
+    const bool push = HAS_DEN && HAS_VEL && a0.push;
+    unsigned char* mem = smem + (size_t)wid * cell_warp_bytes<HAS_DEN, HAS_VEL, MODE, PPR>(a0.slab_layers, a0.tile_rows, a0.P);
     if (lane == 0) {
         mbar_init(&s_bar[wid], 1);
         mbar_fence_init();
     }
-    __syncthreads();
+    __syncwarp();
     uint32_t phase = 0;
-    const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
-    // units one at a time from a counter (zeroed before the launch), the next one claimed while
-    // the current one runs (its atomic's latency hidden: the 4M frame's splat 3.10 -> 3.04 ms):
-    // bricks differ widely in cost and the costly ones cluster (dense regions, the surface of an
-    // accumulating frame), so claims of several units leave warps idle at the end (measured: the
-    // batched clouds' splats 16.7 -> 23.2 ms with claims of 4)
-    uint32_t un = lane == 0 ? atomicAdd(a.next, 1u) : 0u;
-    for (;;) {
-        const uint32_t u = __shfl_sync(kFull, un, 0);
-        if (u >= units) break;
-        if (lane == 0) un = atomicAdd(a.next, 1u);  // the next unit, claimed while this one runs
-        splat_unit<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(a, u, tile, &s_bar[wid], s_rs[wid], s_ro[wid], phase, lane);
-    }
+    const int dx = lane / 9 - 1, dy = lane / 3 % 3 - 1, dz = lane % 3 - 1;
+    unit_loop(
+        total, next, push, lane, of, args,
+        [&](const SplatArgs& a, SplatUnit& t) {
+            // the neighbour's octants whose points, whose footprints reach `reach` voxels from their own,
+            // can touch the tile; with per-point radii the reach is that of the largest radius (ceil R
+            // voxels, at most brick - 1)
+            t.start = t.end = 0;
+            if (t.nl27 < 0) return;
+            const int reach = PPR && a.rmax ? min(a.reach, (int)ceilf(__uint_as_float(*a.rmax))) : a.reach;
+            const int below = CUBIC ? reach : 0, b = a.brick, ap = a.apron, y0 = push ? 0 : -ap, y1 = push ? b - 1 : b - 1 + ap;
+            int lx, hx, ly, hy, lz, hz;
+            const bool nx = unit_halves(dx, b, -ap, b - 1 + ap, below, reach, lx, hx);
+            const bool ny = unit_halves(dy, b, y0, y1, below, reach, ly, hy);
+            const bool nz = unit_halves(dz, b, t.z0 - ap, t.z0 - ap + t.nl - 1, below, reach, lz, hz);
+            if (nx && ny && nz) unit_octants(a, t, 4 * lx + 2 * ly + lz, 4 * hx + 2 * hy + hz);
+        },
+        [&](const SplatArgs& a, const SplatUnit& t, uint32_t, auto mid) {
+            cell_unit<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(a, t, mem, &s_bar[wid], s_rs[wid], phase, lane, mid);
+        });
     if (!(HAS_DEN && HAS_VEL) && lane == 0) bulk_wait_all();
+}
+
+// resident blocks per SM that the registers are budgeted for: with density and velocity the tiles leave
+// room for no more than 5; density alone, per-point radii, 238k bricks: 0.88 ms at 6, 0.86 at 5, 0.98 at 4;
+// uniform R = 3.5, 3k bricks of 16^3: 0.78 / 0.66 / 0.71
+constexpr int kCellMinBlocks = 5;
+
+template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
+__global__ void __launch_bounds__(kCellWarps * 32, kCellMinBlocks) k_splat_cells(SplatArgs a)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
+    cell_loop<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
+        a, units, a.next, smem,
+        [&](uint32_t u, uint32_t& lu) {
+            lu = u;
+            return 0u;
+        },
+        [&](uint32_t) -> const SplatArgs& { return a; });
 }
 
 // The same work over many grids in one persistent launch: the units of grid
 // k are [ustart[k], ustart[k+1]) of one global range, taken by the warps from
-// a counter; every grid has the same brick and tile shape (slab_layers, P).
+// the counter ustart[ngrids + 1] (zeroed before every launch); every grid has
+// the same brick and tile shape (slab_layers, P).
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks)
-    k_splat_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
+__global__ void __launch_bounds__(kCellWarps * 32, kCellMinBlocks)
+    k_splat_cells_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
-    using T = Tile<HAS_DEN, HAS_VEL>;
     extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    unsigned char* tile = smem + (size_t)wid * T::bytes(args[0].slab_layers * args[0].tile_rows * args[0].P);
-    __shared__ __align__(8) uint64_t s_bar[kSlabWarps];
-    __shared__ int s_rs[kSlabWarps][kMaxRanges + 1];
-    __shared__ int s_ro[kSlabWarps][kMaxRanges + 1];
     __shared__ uint32_t s_us[kBatchMaxGrids + 1];
     for (int i = threadIdx.x; i <= ngrids; i += blockDim.x) s_us[i] = ustart[i];
-    if (lane == 0) {
-        mbar_init(&s_bar[wid], 1);
-        mbar_fence_init();
-    }
     __syncthreads();
-    uint32_t phase = 0;
-    const uint32_t total = s_us[ngrids];
-    // units are taken one at a time from a counter (ustart[ngrids + 1], zeroed before every
-    // launch), the next claimed while the current runs: a brick of a dense cloud costs many times
-    // a sparse one, and a fixed stride would leave the warps that drew the dense ones running
-    // alone at the end
-    uint32_t* next = ustart + ngrids + 1;
-    uint32_t un = lane == 0 ? atomicAdd(next, 1u) : 0u;
-    for (;;) {
-        const uint32_t u = __shfl_sync(kFull, un, 0);
-        if (u >= total) break;
-        if (lane == 0) un = atomicAdd(next, 1u);  // the next unit, claimed while this one runs
-        int lo = 0, hi = ngrids - 1;  // the grid k with ustart[k] <= u < ustart[k+1]
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_us[mid] <= u)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        splat_unit<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(args[lo], u - s_us[lo], tile, &s_bar[wid], s_rs[wid],
-                                                       s_ro[wid], phase, lane);
-    }
-    if (!(HAS_DEN && HAS_VEL) && lane == 0) bulk_wait_all();
+    uint32_t k = 0u;  // the last unit's grid: a warp's units come in rising order, so its search starts there
+    cell_loop<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
+        args[0], s_us[ngrids], ustart + ngrids + 1, smem,
+        [&](uint32_t u, uint32_t& lu) {
+            while (s_us[k + 1] <= u) k++;
+            lu = u - s_us[k];
+            return k;
+        },
+        [&](uint32_t g) -> const SplatArgs& { return args[g]; });
 }
 
 // ---------------------------------------------------------------------------
@@ -917,7 +1007,7 @@ __global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks)
 //
 // What bounds it: instruction issue (the general slab kernel spends 2 x 1,080 warp instructions on a
 // brick of two points, 75% of the issue slots) ahead of the HBM writes of the bricks.  So, unlike
-// splat_unit:
+// the cells' kernel:
 //  - a lane's candidates are ONE range per neighbour, from its first needed octant to its last one
 //    (a superset of the needed octants, two loads instead of nine and no list of runs; the footprint
 //    test drops the others), found from a candidate's number with one warp-wide OR of the ranges'
@@ -931,57 +1021,9 @@ __global__ void __launch_bounds__(kSlabWarps * 32, kSlabMinBlocks)
 // 24 batched clouds, 5M points, 2.07M bricks: 7.10 -> 2.37 ms (8.3 GB written: 3.5 TB/s), 100k points
 // in 36k bricks 92 -> 43 us, a fusion frame's splat 108 -> 84 us.
 struct TriLane {
-    int dx, dy, dz;   // the lane's neighbour, lanes 27-31 none
-    int lox, hix, loy, hiy;  // first and last half of the neighbour that can reach the tile, along x and y
-    bool need;        // some half can, along both
+    int lox, hix, loy, hiy;  // first and last half of the lane's neighbour that can reach the tile, along x and y
+    bool need;               // some half can, along both
 };
-
-// halves of a neighbour at offset d (bricks) whose points reach voxels [v0, v1] of the brick: points of
-// floor coordinate f touch f and f + 1
-__device__ __forceinline__ bool tri_halves(int d, int b, int v0, int v1, int& lo, int& hi)
-{
-    const int hb = b >> 1, c = d * b;
-    const bool n0 = c <= v1 && c + hb - 1 >= v0 - 1, n1 = c + hb <= v1 && c + b - 1 >= v0 - 1;
-    lo = n0 ? 0 : 1;
-    hi = n1 ? 1 : 0;
-    return n0 || n1;
-}
-
-// the unit's brick and slab, and what the lane needs of them
-struct TriUnit {
-    uint32_t s;      // atlas slot
-    int z0, nl;      // padded layers of the unit
-    int leaf;
-    int nl27;        // the lane's neighbour (leaf index, -1: none)
-    int4 org;        // the node's first 16 bytes: (lev.., x, y, z)
-    int start, end;  // the lane's candidates in the sorted points
-};
-
-__device__ __forceinline__ void tri_slot(const SplatArgs& a, uint32_t u, TriUnit& t)
-{
-    const uint32_t S = (uint32_t)a.slabs;
-    const uint32_t ui = S == 1u ? u : u / S;
-    t.s = a.unit_slots ? a.unit_slots[ui] : ui;
-    t.z0 = (int)(u - ui * S) * a.slab_layers;
-    t.nl = min(a.slab_layers, a.P - t.z0);
-    t.leaf = a.slot_leaf[t.s];
-}
-__device__ __forceinline__ void tri_neighbour(const SplatArgs& a, TriUnit& t, int nbi)
-{
-    t.nl27 = nbi >= 0 ? a.nbr[(size_t)t.leaf * 27 + nbi] : -1;
-    t.org = *(const int4*)(a.nodes0 + t.leaf);
-}
-__device__ __forceinline__ void tri_range(const SplatArgs& a, TriUnit& t, const TriLane& L)
-{
-    t.start = t.end = 0;
-    int loz, hiz;
-    if (t.nl27 >= 0 && L.need && tri_halves(L.dz, a.brick, t.z0 - a.apron, t.z0 - a.apron + t.nl - 1, loz, hiz)) {
-        const int o0 = 4 * L.lox + 2 * L.loy + loz, o1 = 4 * L.hix + 2 * L.hiy + hiz + 1;
-        const int* oc = a.leaf_oct + (size_t)t.nl27 * 8;
-        t.start = oc[o0];
-        t.end = o1 == 8 ? a.leaf_range[t.nl27].y : oc[o1];
-    }
-}
 
 // A unit with more than kDenseCandidates candidates in dense leaves (the core of a dense cloud:
 // thousands of points a brick) is summed voxel by voxel, a lane each, from the cells around the voxel:
@@ -1007,7 +1049,7 @@ __device__ __forceinline__ float tri_weight(float w, float wx, float wy, float w
 }
 
 // the sums of voxels e0 + lane of the unit
-__device__ __forceinline__ void tri_dense(const SplatArgs& a, const TriUnit& t, int e0, int lane)
+__device__ __forceinline__ void tri_dense(const SplatArgs& a, const SplatUnit& t, int e0, int lane)
 {
     const int P = a.P, P2 = P * P, ap = a.apron;
     const int nvox = t.nl * P2;
@@ -1097,14 +1139,14 @@ __device__ __forceinline__ void tri_dense(const SplatArgs& a, const TriUnit& t, 
 }
 
 struct TriShared {
-    int rs[kSlabWarps][32];      // per range with points: its first sorted index, less its first candidate number
-    float4 hit[kSlabWarps][32];  // the hits of a round of candidates, in order
-    uint64_t bar[kSlabWarps];
+    int rs[kTriWarps][32];      // per range with points: its first sorted index, less its first candidate number
+    float4 hit[kTriWarps][32];  // the hits of a round of candidates, in order
+    uint64_t bar[kTriWarps];
 };
 
 // the sums of one unit into `tile` and out to HBM; mid(): called once, before the candidates
 template <class Mid>
-__device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, float* tile, TriShared& sh, int wid,
+__device__ __forceinline__ void tri_unit(const SplatArgs& a, const SplatUnit& t, float* tile, TriShared& sh, int wid,
                                          int lane, uint32_t& phase, uint32_t grid, Mid mid)
 {
     const int P = a.P, P2 = P * P, ap = a.apron;
@@ -1112,23 +1154,15 @@ __device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, f
     const int nvox = t.nl * P2;
     const size_t gofs = (size_t)t.s * (P2 * P) + (size_t)t.z0 * P2;
     const uint32_t lt = (1u << lane) - 1u;
-    // ---- the lanes' ranges: places among the candidates
-    const int len = t.end - t.start;
-    int off = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kFull, off, o);
-        if (lane >= o) off += v;
-    }
-    const int total = __shfl_sync(kFull, off, 31);
-    off -= len;
+    int off;
+    const int total = unit_candidates(t, lane, off);
     if (a.accum && total == 0) {  // no point reaches the slab: left as it is
         mid();
         return;
     }
     if (a.cell_tab && total > kDenseCandidates) {
-        const bool dn = len > 0 && a.leaf_dense[t.nl27] != 0;
-        if (__reduce_add_sync(kFull, dn ? len : 0) > kDenseCandidates) {
+        const bool dn = t.end > t.start && a.leaf_dense[t.nl27] != 0;
+        if (__reduce_add_sync(kFull, dn ? t.end - t.start : 0) > kDenseCandidates) {
             mid();
             uint32_t at = kDenseCap;
             if (a.dense_units && lane == 0) at = atomicAdd(a.dense_units, 1u);
@@ -1141,10 +1175,9 @@ __device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, f
             return;
         }
     }
-    const uint32_t some = __ballot_sync(kFull, len > 0);
     // (active neighbours: those in the lookup the table was made from, which are those with a slot)
     const uint32_t nbmask = __ballot_sync(kFull, t.nl27 >= 0);
-    if (len > 0) sh.rs[wid][__popc(some & lt)] = t.start - off;
+    unit_ranges(t, lane, off, sh.rs[wid]);
 
     // ---- the tile, once the last unit's bulk store has read it
     if (lane == 0) bulk_wait_read_all();
@@ -1163,31 +1196,17 @@ __device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, f
     uint32_t touched = 0u;
     const int cx = lane & 1, cy = (lane >> 1) & 1, cz = (lane >> 2) & 1, hq = lane >> 3;
     for (int base = 0; base < total; base += 32) {
-        const int v = base + lane;
-        // the range of candidate v: the ranges with points that start at or before it, less one
-        const uint32_t starts = __reduce_or_sync(kFull, len > 0 && off >= base && off < base + 32 ? 1u << (off - base) : 0u);
-        const int before = __popc(__ballot_sync(kFull, len > 0 && off < base));
+        const int idx = unit_candidate(t, lane, off, base, sh.rs[wid]);
         bool hit = false;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v < total) {
-            p = a.spos[sh.rs[wid][before - 1 + __popc(starts & (kFull >> (31 - lane)))] + v];
+        if (base + lane < total) {
+            p = a.spos[idx];
             const int x = (int)floorf(p.x) - Ox, y = (int)floorf(p.y) - Oy, z = (int)floorf(p.z) - Zlo;
             // the footprint is x, x + 1 and so on
             hit = (unsigned)(x + 1) <= (unsigned)P && (unsigned)(y + 1) <= (unsigned)P &&
                   (unsigned)(z + 1) <= (unsigned)t.nl;
-            if (hit && nbmask != 0x7FFFFFFu && ap) {
-                // the regions of the padded brick reached (see splat_unit): per axis 1 below the
-                // interior, 2 inside, 4 above
-                const int zp = t.z0 + z;
-                const uint32_t tx = (uint32_t)(x < ap) | (uint32_t)(x + 1 >= ap && x <= P - 1 - ap) << 1 |
-                                    (uint32_t)(x + 1 > P - 1 - ap) << 2;
-                const uint32_t ty = (uint32_t)(y < ap) | (uint32_t)(y + 1 >= ap && y <= P - 1 - ap) << 1 |
-                                    (uint32_t)(y + 1 > P - 1 - ap) << 2;
-                const uint32_t tz = (uint32_t)(zp < ap) | (uint32_t)(zp + 1 >= ap && zp <= P - 1 - ap) << 1 |
-                                    (uint32_t)(zp + 1 > P - 1 - ap) << 2;
-                touched |= ((tx & 1u) | (tx & 2u) << 8 | (tx & 4u) << 16) *
-                           ((ty & 1u) | (ty & 2u) << 2 | (ty & 4u) << 4) * tz;
-            }
+            if (hit && nbmask != 0x7FFFFFFu && ap)
+                touched |= box_regions(x, x + 1, y, y + 1, t.z0 + z, t.z0 + z + 1, P, ap);
         }
         const uint32_t hm = __ballot_sync(kFull, hit);
         if (hm == 0u) continue;
@@ -1249,13 +1268,6 @@ __device__ __forceinline__ void tri_unit(const SplatArgs& a, const TriUnit& t, f
     }
 }
 
-// Units are claimed two at a time where there are many for every warp: the counter is one address, which
-// takes an atomic every two nanoseconds (24 clouds, 2.07M bricks: 3.24 ms one at a time, 2.37 two, 2.44
-// four, 2.53 eight); costly units do not pile up in a claim, the dense ones being listed elsewhere.
-constexpr uint32_t kTriClaim = 2, kTriClaimUnits = 16;
-
-// Units [0, total) of all grids from the counter `next`; of(u, local) -> the number of u's grid and its
-// unit there, args(k) -> that grid's arguments
 template <class Of, class Args>
 __device__ __forceinline__ void tri_loop(const SplatArgs& a0, uint32_t total, uint32_t* next, unsigned char* smem, Of of,
                                          Args args)
@@ -1270,66 +1282,25 @@ __device__ __forceinline__ void tri_loop(const SplatArgs& a0, uint32_t total, ui
     __syncwarp();
     uint32_t phase = 0;
     TriLane L;
-    L.dx = lane / 9 - 1, L.dy = (lane / 3) % 3 - 1, L.dz = lane % 3 - 1;
-    const bool nx = tri_halves(L.dx, a0.brick, -a0.apron, a0.P - 1 - a0.apron, L.lox, L.hix);
-    const bool ny = tri_halves(L.dy, a0.brick, -a0.apron, a0.P - 1 - a0.apron, L.loy, L.hiy);
-    L.need = lane < 27 && nx && ny;
-    const int nbi = lane < 27 ? (L.dz + 1) * 9 + (L.dy + 1) * 3 + (L.dx + 1) : -1;
-    // Units from the counter, in three steps ahead of each other: while unit t is summed, the neighbours
-    // (asked for as it starts) and then the candidate ranges of t1 arrive, and the brick of t2.
-    const uint32_t claim = total >= kTriClaimUnits * gridDim.x * kSlabWarps ? kTriClaim : 1u;
-    uint32_t cur = 0u, lim = 0u, pre = lane == 0 ? atomicAdd(next, claim) : 0u, lu;
-    auto take = [&]() {  // the next unit's number (total and above: none)
-        if (cur == lim) {
-            cur = __shfl_sync(kFull, pre, 0);
-            lim = cur + claim;
-            if (lane == 0 && cur < total) pre = atomicAdd(next, claim);
-        }
-        return cur++;
-    };
-    uint32_t u = take();
-    if (u < total) {
-        TriUnit t, t1;
-        uint32_t k = of(u, lu), k1;
-        tri_slot(args(k), lu, t);
-        u = take();
-        bool more = u < total;
-        k1 = k;
-        t1 = t;
-        if (more) {
-            k1 = of(u, lu);
-            tri_slot(args(k1), lu, t1);
-        }
-        tri_neighbour(args(k), t, nbi);
-        tri_range(args(k), t, L);
-        for (;;) {
-            TriUnit t2 = t1;
-            uint32_t k2 = k1;
-            bool more2 = false;
-            if (more) {
-                tri_neighbour(args(k1), t1, nbi);
-                u = take();
-                more2 = u < total;
-                if (more2) {
-                    k2 = of(u, lu);
-                    tri_slot(args(k2), lu, t2);
-                }
-            }
-            tri_unit(args(k), t, tile, sh, wid, lane, phase, k, [&]() {
-                if (more) tri_range(args(k1), t1, L);
-            });
-            if (!more) break;
-            k = k1;
-            t = t1;
-            k1 = k2;
-            t1 = t2;
-            more = more2;
-        }
-    }
+    const int dz = lane % 3 - 1;
+    const bool nx = unit_halves(lane / 9 - 1, a0.brick, -a0.apron, a0.P - 1 - a0.apron, 0, 1, L.lox, L.hix);
+    const bool ny = unit_halves(lane / 3 % 3 - 1, a0.brick, -a0.apron, a0.P - 1 - a0.apron, 0, 1, L.loy, L.hiy);
+    L.need = nx && ny;
+    unit_loop(
+        total, next, false, lane, of, args,
+        [&](const SplatArgs& a, SplatUnit& t) {
+            int lz, hz;
+            t.start = t.end = 0;
+            if (t.nl27 >= 0 && L.need && unit_halves(dz, a.brick, t.z0 - a.apron, t.z0 - a.apron + t.nl - 1, 0, 1, lz, hz))
+                unit_octants(a, t, 4 * L.lox + 2 * L.loy + lz, 4 * L.hix + 2 * L.hiy + hz);
+        },
+        [&](const SplatArgs& a, const SplatUnit& t, uint32_t k, auto mid) {
+            tri_unit(a, t, tile, sh, wid, lane, phase, k, mid);
+        });
     if (lane == 0) bulk_wait_all();
 }
 
-__global__ void __launch_bounds__(kSlabWarps * 32, 8) k_splat_tri(SplatArgs a)
+__global__ void __launch_bounds__(kTriWarps * 32, kTriMinBlocks) k_splat_tri(SplatArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
@@ -1343,7 +1314,7 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 8) k_splat_tri(SplatArgs a)
 }
 
 // the same over many grids: ustart as in k_splat_batch, the counters after it
-__global__ void __launch_bounds__(kSlabWarps * 32, 8)
+__global__ void __launch_bounds__(kTriWarps * 32, kTriMinBlocks)
     k_splat_tri_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1362,23 +1333,23 @@ __global__ void __launch_bounds__(kSlabWarps * 32, 8)
 }
 
 // the listed units of k_splat_tri (args: one grid's) or k_splat_tri_batch, 32 voxels a warp
-__global__ void __launch_bounds__(kSlabWarps * 32, 8)
+__global__ void __launch_bounds__(kTriWarps * 32, 8)
     k_tri_dense(const SplatArgs* __restrict__ args, SplatArgs one, const uint32_t* __restrict__ units,
                 const uint4* __restrict__ list, int chunks)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t total = min(*units, kDenseCap) * (uint32_t)chunks, nw = gridDim.x * kSlabWarps;
+    const uint32_t total = min(*units, kDenseCap) * (uint32_t)chunks, nw = gridDim.x * kTriWarps;
     const int dx = lane / 9 - 1, dy = (lane / 3) % 3 - 1, dz = lane % 3 - 1;
     const int nbi = lane < 27 ? (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1) : -1;
-    for (uint32_t u = blockIdx.x * kSlabWarps + (threadIdx.x >> 5); u < total; u += nw) {
+    for (uint32_t u = blockIdx.x * kTriWarps + (threadIdx.x >> 5); u < total; u += nw) {
         const uint4 e = list[u / (uint32_t)chunks];
         const SplatArgs& a = args ? args[e.x] : one;
-        TriUnit t;
+        SplatUnit t;
         t.s = e.y;
         t.z0 = (int)e.z;
         t.nl = (int)e.w;
         t.leaf = a.slot_leaf[t.s];
-        tri_neighbour(a, t, nbi);
+        unit_neighbour(a, t, nbi);
         const int e0 = (int)(u % (uint32_t)chunks) * 32;
         if (e0 < t.nl * a.P * a.P) tri_dense(a, t, e0, lane);
     }
@@ -1612,30 +1583,36 @@ constexpr int kListDensePoints = 32768;
 // the splats of k_splat_tri
 static bool tri_kind(const SplatKind& k) { return k.mode == GVX_SPLAT_TRILINEAR && k.has_d && !k.has_v; }
 
+// the kernel of a kind (single grid, batch), its warps a block and its shared memory a warp
+struct SplatKernel {
+    void *one, *batch;
+    int warps;
+    size_t (*warp_bytes)(int layers, int rows, int P);
+};
+static size_t tri_warp_bytes(int layers, int rows, int P) { return (size_t)layers * rows * P * sizeof(float); }
+
+template <bool D, bool V, int MODE, bool PPR, bool SMALL>
+static SplatKernel cell_kernel()
+{
+    return SplatKernel{(void*)k_splat_cells<D, V, MODE, PPR, SMALL>, (void*)k_splat_cells_batch<D, V, MODE, PPR, SMALL>,
+                       kCellWarps, cell_warp_bytes<D, V, MODE, PPR>};
+}
 template <bool D, bool V>
-static void* pick_kernel(const SplatKind& k, bool batch)
+static SplatKernel pick_kernel(const SplatKind& k)
 {
     if (k.mode == GVX_SPLAT_TRILINEAR) {
         if constexpr (D && !V)
-            return batch ? (void*)k_splat_tri_batch : (void*)k_splat_tri;
+            return SplatKernel{(void*)k_splat_tri, (void*)k_splat_tri_batch, kTriWarps, tri_warp_bytes};
         else
-            return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_TRILINEAR, false, true>
-                         : (void*)k_splat_slab<D, V, GVX_SPLAT_TRILINEAR, false, true>;
+            return cell_kernel<D, V, GVX_SPLAT_TRILINEAR, false, true>();
     }
-    if (k.ppr)
-        return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_CUBIC, true, false>
-                     : (void*)k_splat_slab<D, V, GVX_SPLAT_CUBIC, true, false>;
-    if (k.small)
-        return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_CUBIC, false, true>
-                     : (void*)k_splat_slab<D, V, GVX_SPLAT_CUBIC, false, true>;
-    return batch ? (void*)k_splat_batch<D, V, GVX_SPLAT_CUBIC, false, false>
-                 : (void*)k_splat_slab<D, V, GVX_SPLAT_CUBIC, false, false>;
+    if (k.ppr) return cell_kernel<D, V, GVX_SPLAT_CUBIC, true, false>();
+    return k.small ? cell_kernel<D, V, GVX_SPLAT_CUBIC, false, true>() : cell_kernel<D, V, GVX_SPLAT_CUBIC, false, false>();
 }
 
-static void* splat_kernel(const SplatKind& k, bool batch)
+static SplatKernel splat_kernel(const SplatKind& k)
 {
-    return k.has_d ? (k.has_v ? pick_kernel<true, true>(k, batch) : pick_kernel<true, false>(k, batch))
-                   : pick_kernel<false, true>(k, batch);
+    return k.has_d ? (k.has_v ? pick_kernel<true, true>(k) : pick_kernel<true, false>(k)) : pick_kernel<false, true>(k);
 }
 
 // Tile geometry of a grid's splat: a push tile (apron 1, not accumulating) covers the interior
@@ -1669,12 +1646,22 @@ static int clamp_layers(const SlabShape& sh, int P, size_t eb, int want)
     return std::min(std::min(want, sh.span), fit);
 }
 
-// The trilinear density splat takes a whole padded brick a unit where the launch has a unit for every
-// resident warp (152 SMs x 32) and the tile is small (4 KB for bricks of 8), else half of it: 100k
-// points in 36k bricks 43 us whole, 65 in halves; fusion frames 84 / 88; 24 clouds 2.4 / 3.3 ms; 6k
-// points in 720 bricks 14 / 11 us
-constexpr int kTriWholeP = 10;
-constexpr uint64_t kTriWholeBricks = 152 * 32;
+// The slab height a splat takes by itself: a push tile the brick's whole interior (one unit a brick: the
+// candidate ranges and the z pushes once), others the whole padded brick where its tile is small, else
+// half of it -- and lower slabs where that leaves fewer than kUnitsWanted units, down to two layers:
+// dealing a brick's candidates again for every slab costs less than warps without work.  Measured
+// (bricks, density alone unless said): trilinear 36k of 8^3 whole 43 us, halves 65; 2.07M 2.4 / 3.3 ms;
+// 720 of them 14 us whole, 10.1 halves, 10.9 of four layers, 11.3 of two; cubic of per-point radii 1-3,
+// 238k: 0.86 ms whole, 1.13 halves, 1.67 of three layers; cubic R 3.5, 3k of 16^3: 1.42 ms whole, 0.88
+// halves, 0.77 of five layers, 0.61 of three, 0.66 of two.
+constexpr uint64_t kUnitsWanted = 152 * 24 * 3;
+constexpr size_t kWholeTile = 6 * 1024;
+static int default_layers(const SlabShape& sh, int P, size_t eb, uint64_t bricks)
+{
+    int l = sh.push || (size_t)sh.span * sh.rows * P * eb <= kWholeTile ? sh.span : (sh.span + 1) / 2;
+    while (!sh.push && l > 5 && bricks * (uint64_t)((sh.span + l - 1) / l) < kUnitsWanted) l = (l + 1) / 2;
+    return l;
+}
 
 // validation of one grid's splat and its kernel kind (bricks: how many the launch covers); *layers in:
 // the wanted slab height (<= 0: the default), out: clamped to the tile budget
@@ -1713,10 +1700,7 @@ static gvx_status splat_check(gvx_grid* g, int mode, float radius, int chan_d, i
     }
     const int P = g->P;
     const SlabShape sh = slab_shape(g, accum, dense, has_d && has_v);
-    // a push tile takes the brick's whole interior (one unit a brick: the candidate ranges and the z
-    // pushes once; 4M frame 2.80 -> 2.54 ms against two 4-layer slabs), else half the padded brick
-    const bool whole = sh.push || (mode == GVX_SPLAT_TRILINEAR && !has_v && P <= kTriWholeP && bricks >= kTriWholeBricks);
-    *layers = clamp_layers(sh, P, has_v ? 16 : 4, *layers > 0 ? *layers : (whole ? sh.span : (sh.span + 1) / 2));
+    *layers = clamp_layers(sh, P, has_v ? 16 : 4, *layers > 0 ? *layers : default_layers(sh, P, has_v ? 16 : 4, bricks));
     if (*layers < 1) {
         gvx_set_error("Splat: a %d^2 layer of the padded brick exceeds the shared tile budget", P);
         return GVX_ERR_UNSUPPORTED;
@@ -1757,6 +1741,10 @@ static void splat_fill(gvx_grid* g, const SplatKind& k, float radius, int chan_d
     a.vel = k.has_v ? g->ch[chan_v].data.as<float4>() : nullptr;
     const SlabShape sh = slab_shape(g, accum, dense, k.has_d && k.has_v);
     a.push = sh.push;
+    if (sh.push && layers == sh.span && g->push_tab_P == P) {
+        a.push_tab = g->push_tab.as<uint32_t>();
+        a.push_count = g->push_count;
+    }
     a.tile_rows = sh.rows;
     a.slab_layers = layers;
     a.slabs = (sh.span + layers - 1) / layers;
@@ -1768,6 +1756,36 @@ static void splat_fill(gvx_grid* g, const SplatKind& k, float radius, int chan_d
     a.accum = accum != 0;
     a.boundval = 0.0f;
     a.err = g->d_err.as<uint32_t>();
+}
+
+// The table of push_out for push tiles of one unit a brick: per boundary voxel and neighbour (0, dy, dz)
+// that takes it, its place in the tile, its place in the neighbour's padded brick << 12, the lane that
+// holds the neighbour's slot << 24; filled up to a multiple of 32 with the last entry.
+static gvx_status push_table(gvx_grid* g)
+{
+    const int P = g->P, b = g->brick;
+    if (g->push_tab_P == P) return GVX_OK;
+    std::vector<uint32_t> t;
+    for (int dz = -1; dz <= 1; dz++)
+        for (int dy = -1; dy <= 1; dy++) {
+            if (dy == 0 && dz == 0) continue;
+            for (int lz = 0; lz < b; lz++)
+                for (int ly = 0; ly < b; ly++) {
+                    if ((dy < 0 && ly != 0) || (dy > 0 && ly != b - 1) || (dz < 0 && lz != 0) || (dz > 0 && lz != b - 1))
+                        continue;
+                    const int yr = dy < 0 ? P - 1 : dy > 0 ? 0 : ly + 1, zr = dz < 0 ? P - 1 : dz > 0 ? 0 : lz + 1;
+                    for (int x = 0; x < P; x++)
+                        t.push_back((uint32_t)((lz * b + ly) * P + x) | (uint32_t)((zr * P + yr) * P + x) << 12 |
+                                    (uint32_t)(9 + (dy + 1) * 3 + (dz + 1)) << 24);
+                }
+        }
+    while (t.size() % 32) t.push_back(t.back());
+    GVX_CK(gvx_ensure(g->push_tab, t.size() * sizeof(uint32_t)));
+    GVX_CK(cudaMemcpyAsync(g->push_tab.p, t.data(), t.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, g->stream));
+    GVX_CK(cudaStreamSynchronize(g->stream));
+    g->push_tab_P = P;
+    g->push_count = (int)t.size();
+    return GVX_OK;
 }
 
 // validation, InsertPoints grouping and the kernel arguments of one grid's splat;
@@ -1784,6 +1802,8 @@ static gvx_status splat_prepare(gvx_grid* g, int mode, int n, float radius, cons
     if (rc) return rc;
     rc = gvx_prepare_points(g, n, trans, kind->has_v || kind->ppr);
     if (rc) return rc;
+    // (a tile of the whole interior has at most 4096 places: bricks up to 8)
+    if (slab_shape(g, accum, dn, kind->has_d && kind->has_v).push && g->brick <= 8) GVX_CK_STATUS(push_table(g));
     splat_fill(g, *kind, radius, chan_d, chan_v, accum, dn, layers, out);
     return GVX_OK;
 }
@@ -1810,9 +1830,9 @@ static void splat_finish(gvx_grid* g, int chan_d, int chan_v, int accum)
     }
 }
 
-static size_t splat_smem(const SplatArgs& a, const SplatKind& k)
+static size_t splat_smem(const SplatArgs& a, const SplatKernel& k)
 {
-    return (size_t)a.slab_layers * a.tile_rows * a.P * (k.has_v ? 16 : 4) * kSlabWarps;
+    return k.warp_bytes(a.slab_layers, a.tile_rows, a.P) * (size_t)k.warps;
 }
 
 // The slots whose brick has points of the current grouping in itself or one of its 26 neighbours:
@@ -1846,13 +1866,13 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
     gvx_status rc = splat_prepare(g, mode, n, radius, trans, chan_d, chan_v, accum, 0, -1, 0, &a, &kind);
     if (rc) return rc;
     if (a.nslots) {
-        const size_t smem = splat_smem(a, kind);
-        void* kern = splat_kernel(kind, false);
-        GVX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const SplatKernel kern = splat_kernel(kind);
+        const size_t smem = splat_smem(a, kern);
+        GVX_CK(cudaFuncSetAttribute(kern.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
-        GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSlabWarps * 32, smem));
+        GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern.one, kern.warps * 32, smem));
         const uint64_t units = (uint64_t)a.nslots * a.slabs;
-        const uint64_t ctas_needed = (units + kSlabWarps - 1) / kSlabWarps;
+        const uint64_t ctas_needed = (units + kern.warps - 1) / kern.warps;
         const uint32_t grid =
             (uint32_t)std::min<uint64_t>(ctas_needed, (uint64_t)sm_count(g->device) * std::max(per_sm, 1));
         GVX_CK(gvx_ensure(g->d_next, 3 * sizeof(uint32_t)));  // units taken, slots touched, units listed
@@ -1875,10 +1895,10 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
             g->launches++;
         }
         void* args[] = {&a};
-        GVX_CK(cudaLaunchKernel(kern, dim3(grid), dim3(kSlabWarps * 32), args, smem, g->stream));
+        GVX_CK(cudaLaunchKernel(kern.one, dim3(grid), dim3(kern.warps * 32), args, smem, g->stream));
         g->launches++;
         if (list_dense) {
-            k_tri_dense<<<sm_count(g->device) * 8, kSlabWarps * 32, 0, g->stream>>>(
+            k_tri_dense<<<sm_count(g->device) * 8, kTriWarps * 32, 0, g->stream>>>(
                 nullptr, a, a.dense_units, a.dense_list, (a.slab_layers * a.P * a.P + 31) / 32);
             g->launches++;
             GVX_CK(cudaGetLastError());
@@ -1985,7 +2005,7 @@ static gvx_status batch_dense_units(gvx_batch* b, const SplatKind& k, const Spla
     if (!tri_kind(k)) return GVX_OK;
     SplatArgs none;
     memset(&none, 0, sizeof(none));
-    k_tri_dense<<<sm_count(b->device) * 8, kSlabWarps * 32, 0, b->stream>>>(
+    k_tri_dense<<<sm_count(b->device) * 8, kTriWarps * 32, 0, b->stream>>>(
         dargs, none, units, b->dense_units.as<uint4>(), (a0.slab_layers * a0.P * a0.P + 31) / 32);
     b->launches++;
     GVX_CK(cudaGetLastError());
@@ -2002,13 +2022,13 @@ static void batch_set_dense(gvx_batch* b, SplatArgs& a, DevBuf& ustart, size_t n
 // one launch of the batch kernel over args/ustart already on the device
 static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, int ngrids, int blocks)
 {
-    const size_t smem = splat_smem(a0, k);
-    void* kern = splat_kernel(k, true);
+    const SplatKernel kern = splat_kernel(k);
+    const size_t smem = splat_smem(a0, kern);
     const SplatArgs* dargs = b->d_args.as<SplatArgs>();
     uint32_t* dus = b->d_ustart.as<uint32_t>();
     GVX_CK(cudaMemsetAsync(dus + ngrids + 1, 0, 2 * sizeof(uint32_t), b->stream));  // units taken, units listed
     void* args[] = {(void*)&dargs, (void*)&dus, (void*)&ngrids};
-    GVX_CK(cudaLaunchKernel(kern, dim3(blocks), dim3(kSlabWarps * 32), args, smem, b->stream));
+    GVX_CK(cudaLaunchKernel(kern.batch, dim3(blocks), dim3(kern.warps * 32), args, smem, b->stream));
     b->launches++;
     return batch_dense_units(b, k, a0, dargs, dus + ngrids + 2);
 }
@@ -2064,10 +2084,10 @@ static gvx_status batch_upload(gvx_batch* b, const std::vector<SplatArgs>& args,
 
 static gvx_status batch_max_blocks(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, int* per_sm)
 {
-    void* kern = splat_kernel(k, true);
-    const size_t smem = splat_smem(a0, k);
-    GVX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, kSlabWarps * 32, smem));
+    const SplatKernel kern = splat_kernel(k);
+    const size_t smem = splat_smem(a0, kern);
+    GVX_CK(cudaFuncSetAttribute(kern.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern.batch, kern.warps * 32, smem));
     *per_sm = std::max(*per_sm, 1);
     return GVX_OK;
 }
@@ -2224,13 +2244,13 @@ static gvx_status frame_splat(gvx_batch* b, const SplatKind& kind, const SplatAr
     const int ng = (int)b->grids.size();
     k_batch_ustart<<<1, 32, 0, b->stream>>>(b->f_cnt.as<const uint32_t*>(), b->f_caps.as<uint32_t>(), ng, a0.slabs,
                                             b->f_ustart.as<uint32_t>());
-    const size_t smem = splat_smem(a0, kind);  // (the shared-memory limit set by batch_max_blocks)
-    void* kern = splat_kernel(kind, true);
+    const SplatKernel kern = splat_kernel(kind);
+    const size_t smem = splat_smem(a0, kern);  // (the shared-memory limit set by batch_max_blocks)
     const SplatArgs* dargs = b->f_args.as<SplatArgs>();
     uint32_t* dus = b->f_ustart.as<uint32_t>();
     int n = ng;
     void* kargs[] = {(void*)&dargs, (void*)&dus, (void*)&n};
-    GVX_CK(cudaLaunchKernel(kern, dim3(blocks), dim3(kSlabWarps * 32), kargs, smem, b->stream));
+    GVX_CK(cudaLaunchKernel(kern.batch, dim3(blocks), dim3(kern.warps * 32), kargs, smem, b->stream));
     b->launches += 2;
     GVX_CK_STATUS(batch_dense_units(b, kind, a0, dargs, dus + ng + 2));
     // every grid's device error word (topology and splat) into its plan's record
@@ -2536,7 +2556,8 @@ gvx_status gvx_batch_splat(gvx_batch* b, int mode, float radius, int chan_densit
     rc = batch_max_blocks(b, kind, args[0], &per_sm);
     if (rc) return rc;
     if (bps <= 0 || bps > per_sm) bps = per_sm;
-    const uint64_t ctas_needed = ((uint64_t)us.back() + kSlabWarps - 1) / kSlabWarps;
+    const uint64_t warps = (uint64_t)splat_kernel(kind).warps;
+    const uint64_t ctas_needed = ((uint64_t)us.back() + warps - 1) / warps;
     const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(ctas_needed, (uint64_t)sm_count(b->device) * bps));
     const bool same = b->exec && b->cap_args.size() == args.size() && b->cap_kind == kind &&
                       b->cap_blocks == blocks &&
