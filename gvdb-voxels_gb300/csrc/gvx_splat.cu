@@ -959,13 +959,17 @@ __device__ __forceinline__ void cell_loop(const SplatArgs& a0, uint32_t total, u
     if (!(HAS_DEN && HAS_VEL) && lane == 0) bulk_wait_all();
 }
 
-// resident blocks per SM that the registers are budgeted for: with density and velocity the tiles leave
-// room for no more than 5; density alone, per-point radii, 238k bricks: 0.88 ms at 6, 0.86 at 5, 0.98 at 4;
-// uniform R = 3.5, 3k bricks of 16^3: 0.78 / 0.66 / 0.71
-constexpr int kCellMinBlocks = 5;
+// resident blocks per SM that the registers are budgeted for: 5 with density and velocity, whose tiles
+// leave room for no more (778k points: frames of 865 us, 892 at 6); 6 else (frames of 300k points in 16^3
+// bricks, three in flight: 684 us at 5, 572 at 6, 588 at 7; one at a time 912 / 1042 / 1135)
+template <bool HAS_DEN, bool HAS_VEL>
+constexpr int cell_min_blocks()
+{
+    return HAS_DEN && HAS_VEL ? 5 : 6;
+}
 
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kCellWarps * 32, kCellMinBlocks) k_splat_cells(SplatArgs a)
+__global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_VEL>()) k_splat_cells(SplatArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
@@ -983,7 +987,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, kCellMinBlocks) k_splat_cells
 // the counter ustart[ngrids + 1] (zeroed before every launch); every grid has
 // the same brick and tile shape (slab_layers, P).
 template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
-__global__ void __launch_bounds__(kCellWarps * 32, kCellMinBlocks)
+__global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_VEL>())
     k_splat_cells_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
     extern __shared__ __align__(128) unsigned char smem[];
