@@ -383,6 +383,332 @@ __global__ void k_gather(GatherArgs a)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Lists of subcells that are the octants of their bricks (bricks of 8, subcells of 4), without colours,
+// of the points a full topology build was made from: the build has sorted them by (leaf, octant), so the
+// subcells' own points are runs already, and the points of a list are those of the 27 octants around its
+// subcell whose box touches it.  The entries are not written out: the insert counts them (the caller
+// gets their number), and stores each point once, in sorted order, with a flag per face of its octant
+// that its box crosses; the gather tests the flags as it reads the runs.
+// 6M points, 32M entries: emitting, sorting and copying the entries took 1.6 ms and the insert 2.0 ms in
+// all, storing the points XX.
+struct ScDirectArgs {
+    const uint32_t* skeys;   // sorted keys: leaf << 3 | octant
+    const uint32_t* svals;
+    uint32_t n, invalid_key;
+    const char* pos;
+    int off, stride;
+    float t[3];
+    float rins, inv_b;
+    LeafLookup L;
+    float3 qmin, qrange;
+    uint2* q;                // FP16: 16-bit fractions, flags in the upper half of .y
+    float4* pts;             // FP32: position, flags in .w
+    uint32_t* total;         // entries; total[1]: a point is no longer where the build found it
+};
+
+constexpr float kDirectMaxRadius = 2.0f;  // boxes reach no further than the next subcell of 4 voxels
+
+// the translated position of sorted entry i as 16-bit fractions of the box (see k_sc_copy_q)
+__device__ __forceinline__ uint32_t sc_fraction(float w, float mn, float rg)
+{
+    const float f = __fmul_rn(__fdiv_rn(__fsub_rn(w, mn), rg), 65535.0f);
+    return f > 0.0f ? (f >= 65535.0f ? 65535u : __float2uint_rz(f)) : 0u;  // saturating, NaN -> 0
+}
+
+template <bool FP16>
+__global__ void __launch_bounds__(256) k_sc_direct(ScDirectArgs a)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t entries = 0u;
+    bool moved = false;
+    if (i < a.n) {
+        const uint32_t sk = a.skeys[i];
+        const float* p = (const float*)(a.pos + (size_t)a.svals[i] * (size_t)a.stride + a.off);
+        const float raw[3] = {p[0], p[1], p[2]};
+        float w[3];
+        bool in = raw[2] != GVX_NOHIT;
+        for (int k = 0; k < 3; k++) {
+            w[k] = raw[k] + a.t[k];
+            in = in && w[k] >= 0.f;
+        }
+        int c[3], fl = 0;
+        uint32_t key = a.invalid_key;
+        if (in) {
+            bool inside = true;
+            for (int k = 0; k < 3; k++) {
+                c[k] = (int)(w[k] * a.inv_b) - a.L.ks.lo[k];
+                inside = inside && c[k] >= 0 && c[k] < (1 << a.L.ks.bits[k]);
+            }
+            if (inside)
+                key = ks_pack(a.L.ks, c[0], c[1], c[2], 0) << 3 |
+                      (uint32_t)(((((int)w[0]) >> 2) & 1) << 2 | ((((int)w[1]) >> 2) & 1) << 1 | ((((int)w[2]) >> 2) & 1));
+        }
+        moved = key != sk;
+        if (in && !moved) {
+            // per axis: bit 0 the box reaches the subcell below the point's own, bit 1 the one above
+            int r[3][2];
+            for (int k = 0; k < 3; k++) {
+                const int own = (int)w[k] >> 2;
+                const int lo = (int)(w[k] - a.rins) / 4, hi = (int)((w[k] + 1.0f) + a.rins) / 4;
+                fl |= (lo < own ? 1 : 0) << (2 * k) | (hi > own ? 2 : 0) << (2 * k);
+                r[k][0] = lo - own;
+                r[k][1] = hi - own;
+            }
+            const int oct = (int)(sk & 7u);
+            for (int dx = r[0][0]; dx <= r[0][1]; dx++)
+                for (int dy = r[1][0]; dy <= r[1][1]; dy++)
+                    for (int dz = r[2][0]; dz <= r[2][1]; dz++) {
+                        // the brick of that subcell, and whether it is there
+                        const int bx = (((oct >> 2) & 1) + dx) >> 1, by = (((oct >> 1) & 1) + dy) >> 1,
+                                  bz = ((oct & 1) + dz) >> 1;
+                        entries += (bx | by | bz) == 0 || ll_find(a.L, c[0] + bx, c[1] + by, c[2] + bz) >= 0;
+                    }
+        }
+        if (FP16)
+            a.q[i] = make_uint2(sc_fraction(w[0], a.qmin.x, a.qrange.x) | sc_fraction(w[1], a.qmin.y, a.qrange.y) << 16,
+                                sc_fraction(w[2], a.qmin.z, a.qrange.z) | (uint32_t)fl << 16);
+        else
+            a.pts[i] = make_float4(w[0], w[1], w[2], __uint_as_float((uint32_t)fl));
+    }
+    entries = __reduce_add_sync(0xFFFFFFFFu, entries);
+    __shared__ uint32_t s_sum;
+    if (threadIdx.x == 0) s_sum = 0u;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum, entries);
+    const int any = __syncthreads_or(moved);
+    if (threadIdx.x == 0) {
+        atomicAdd(a.total, s_sum);
+        if (any) a.total[1] = 1u;
+    }
+}
+
+// per leaf and octant: its run of sorted points (the grouping's tables may be remade before the gather)
+__global__ void k_sc_runs(const int2* __restrict__ leaf_range, const int* __restrict__ leaf_oct, uint32_t nleaves,
+                          int2* __restrict__ runs)
+{
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nleaves * 8u) return;
+    const uint32_t leaf = t >> 3, o = t & 7u;
+    runs[t] = make_int2(leaf_oct[t], o == 7u ? leaf_range[leaf].y : leaf_oct[t + 1]);
+}
+
+namespace {
+struct GatherDirectArgs {
+    uint32_t nsub;
+    int P, apron;
+    const int* slot_leaf;
+    const GvxNode* nodes0;
+    const int* nbr;
+    const int2* runs;
+    const uint2* q;
+    const float4* pts;
+    float qmin[3], qrange[3];
+    float radius;
+    int levelset, accum;  // FP32; FP16 is a level set from 3 without accumulation
+    float* out;
+    uint32_t* next;
+};
+constexpr int kDirectWarps = 8;
+}  // namespace
+
+// One warp per subcell of 4^3 voxels, two voxels a lane (z and z + 2).  What bounds it: the distances
+// (eleven float steps a listed point and warp, each rounded on its own as in k_gather_fp16).  The lanes
+// test 32 points of the 27 runs at a time; the listed ones wait, decoded, in shared memory until there
+// are 32.  6M points, 433k subcells, 32M entries: XX us against 1154 for the written lists.
+template <bool FP16>
+__global__ void __launch_bounds__(kDirectWarps * 32) k_gather_direct(GatherDirectArgs a)
+{
+    __shared__ float4 s_ent[kDirectWarps][64];
+    __shared__ int2 s_rs[kDirectWarps][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float4* ent = s_ent[wid];
+    int2* rs = s_rs[wid];
+    const uint32_t lt = (1u << lane) - 1u;
+    const int dx = lane / 9 - 1, dy = lane / 3 % 3 - 1, dz = lane % 3 - 1;  // lane < 27: its octant, from the subcell's
+    // a point there is listed when its box crosses the faces between: the flag "above" of an octant below
+    const uint32_t need = lane < 27 ? (dx < 0 ? 2u : dx > 0 ? 1u : 0u) | (dy < 0 ? 8u : dy > 0 ? 4u : 0u) |
+                                          (dz < 0 ? 32u : dz > 0 ? 16u : 0u)
+                                    : 0u;
+    const int vx = lane & 3, vy = (lane >> 2) & 3, vz = lane >> 4;  // voxels (vx, vy, vz) and (vx, vy, vz + 2)
+    WarpUnits wu(a.next, lane);
+    uint32_t s;
+    while (wu.next(a.next, a.nsub, lane, s)) {
+        const uint32_t slot = s >> 3;
+        const int ox = (int)(s & 1u), oy = (int)(s >> 1 & 1u), oz = (int)(s >> 2 & 1u);  // (subcell x fastest)
+        const int leaf = a.slot_leaf[slot];
+        const int4 org = *(const int4*)(a.nodes0 + leaf);
+        int2 run = make_int2(0, 0);
+        if (lane < 27) {
+            const int hx = ox + dx, hy = oy + dy, hz = oz + dz;  // -1 .. 2: the brick before, its halves, the one after
+            const int nl = a.nbr[(size_t)leaf * 27 + ((hz >> 1) + 1) * 9 + ((hy >> 1) + 1) * 3 + (hx >> 1) + 1];
+            if (nl >= 0) run = a.runs[(size_t)nl * 8 + (hx & 1) * 4 + (hy & 1) * 2 + (hz & 1)];
+        }
+        const int len = run.y - run.x;
+        int off = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xFFFFFFFFu, off, o);
+            if (lane >= o) off += v;
+        }
+        const int total = __shfl_sync(0xFFFFFFFFu, off, 31);
+        off -= len;
+        const uint32_t some = __ballot_sync(0xFFFFFFFFu, len > 0);
+        // per run with points: its first sorted index less its first candidate number, and what it needs
+        if (len > 0) rs[__popc(some & lt)] = make_int2(run.x - off, (int)need);
+        __syncwarp();
+        float m0 = __int_as_float(0x7f800000), m1 = m0;  // the smallest squared distances so far
+        const float wx = (float)(org.y + 4 * ox + vx), wy = (float)(org.z + 4 * oy + vy);
+        const float wz0 = (float)(org.w + 4 * oz + vz), wz1 = wz0 + 2.0f;
+        auto nearest = [&](const float4 p) {
+            if (FP16) {
+                const float dx = __fsub_rn(p.x, wx), dy = __fsub_rn(p.y, wy);
+                const float dxy = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+                const float d0 = __fsub_rn(p.z, wz0), d1 = __fsub_rn(p.z, wz1);
+                m0 = fminf(m0, __fadd_rn(dxy, __fmul_rn(d0, d0)));
+                m1 = fminf(m1, __fadd_rn(dxy, __fmul_rn(d1, d1)));
+            } else {
+                const float dx = p.x - wx, dy = p.y - wy, d0 = p.z - wz0, d1 = p.z - wz1;
+                const float dxy = fmaf(dy, dy, dx * dx);
+                m0 = fminf(m0, fmaf(d0, d0, dxy));
+                m1 = fminf(m1, fmaf(d1, d1, dxy));
+            }
+        };
+        int have = 0;  // listed points waiting
+        for (int base = 0; base < total; base += 32) {
+            // candidate base + lane: its run is the number of runs that start at or before it, less one
+            const uint32_t starts =
+                __reduce_or_sync(0xFFFFFFFFu, len > 0 && off >= base && off < base + 32 ? 1u << (off - base) : 0u);
+            const int before = __popc(__ballot_sync(0xFFFFFFFFu, len > 0 && off < base));
+            bool listed = false;
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (base + lane < total) {
+                const int2 r = rs[before - 1 + __popc(starts & (0xFFFFFFFFu >> (31 - lane)))];
+                if (FP16) {
+                    const uint2 u = a.q[r.x + base + lane];
+                    listed = ((u.y >> 16) & (uint32_t)r.y) == (uint32_t)r.y;
+                    if (listed) {
+                        p.x = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.x & 0xFFFFu), 65535.0f), a.qrange[0]), a.qmin[0]);
+                        p.y = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.x >> 16), 65535.0f), a.qrange[1]), a.qmin[1]);
+                        p.z = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.y & 0xFFFFu), 65535.0f), a.qrange[2]), a.qmin[2]);
+                    }
+                } else {
+                    p = a.pts[r.x + base + lane];
+                    listed = (__float_as_uint(p.w) & (uint32_t)r.y) == (uint32_t)r.y;
+                }
+            }
+            const uint32_t lm = __ballot_sync(0xFFFFFFFFu, listed);
+            if (listed) ent[have + __popc(lm & lt)] = p;
+            have += __popc(lm);
+            __syncwarp();
+            if (have >= 32) {
+#pragma unroll 8
+                for (int e = 0; e < 32; e++) nearest(ent[e]);
+                have -= 32;
+                const float4 rest = ent[32 + (lane < have ? lane : 0)];
+                __syncwarp();
+                if (lane < have) ent[lane] = rest;
+                __syncwarp();
+            }
+        }
+        for (int e = 0; e < have; e++) nearest(ent[e]);
+        __syncwarp();
+        // min_j (sqrt(d2_j) - R) = sqrt(min_j d2_j) - R: rounded sqrt and subtraction are monotone
+        const int P = a.P, z0 = 4 * oz + vz + a.apron;
+        const size_t i0 = (((size_t)slot * P + z0) * P + (4 * oy + vy + a.apron)) * P + (4 * ox + vx + a.apron);
+        const size_t i1 = i0 + 2 * (size_t)P * P;
+        const float c0 = __fsqrt_rn(m0), c1 = __fsqrt_rn(m1);  // +inf without points: the start value stays
+        if (FP16 || a.levelset) {
+            const float v0 = a.accum ? a.out[i0] : 3.0f, v1 = a.accum ? a.out[i1] : 3.0f;
+            a.out[i0] = fminf(v0, __fsub_rn(c0, a.radius));
+            a.out[i1] = fminf(v1, __fsub_rn(c1, a.radius));
+        } else {
+            const float v0 = a.accum ? a.out[i0] : 0.0f, v1 = a.accum ? a.out[i1] : 0.0f;
+            a.out[i0] = fmaxf(v0, __fsub_rn(a.radius, c0));
+            a.out[i1] = fmaxf(v1, __fsub_rn(a.radius, c1));
+        }
+    }
+}
+
+template <bool FP16>
+static gvx_status gather_direct(gvx_grid* g, float radius, int levelset, int accum, float* out)
+{
+    GatherDirectArgs a;
+    memset(&a, 0, sizeof(a));
+    a.nsub = g->sc_nsub;
+    a.P = g->P;
+    a.apron = g->apron;
+    a.slot_leaf = g->slot_leaf.as<int>();
+    a.nodes0 = g->nodes[0].as<GvxNode>();
+    a.nbr = g->nbr.as<int>();
+    a.runs = g->sc_runs.as<int2>();
+    a.q = g->sc_q.as<uint2>();
+    a.pts = g->sc_pts.as<float4>();
+    for (int k = 0; k < 3; k++) {
+        a.qmin[k] = g->sc_qmin[k];
+        a.qrange[k] = g->sc_qrange[k];
+    }
+    a.radius = radius;
+    a.levelset = levelset;
+    a.accum = accum;
+    a.out = out;
+    GVX_CK(gvx_ensure(g->d_next, sizeof(uint32_t)));
+    GVX_CK(cudaMemsetAsync(g->d_next.p, 0, sizeof(uint32_t), g->stream));
+    a.next = g->d_next.as<uint32_t>();
+    const unsigned blocks = std::min<unsigned>(blocks_for((uint64_t)a.nsub * 32u, kDirectWarps * 32), 152u * 8u);
+    k_gather_direct<FP16><<<blocks, kDirectWarps * 32, 0, g->stream>>>(a);
+    g->launches++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
+}
+
+// the direct lists of the points of the last full build; *done false: the points are not where it found
+// them any more (moved in place), and the entries are to be written out
+static gvx_status insert_direct(gvx_grid* g, int n, float radius, const float t[3], const float qmin[3],
+                                const float qrange[3], bool fp16, uint32_t* m, bool* done)
+{
+    cudaStream_t st = g->stream;
+    const uint32_t nleaves = (uint32_t)g->count[0];
+    if (fp16)
+        GVX_CK(gvx_ensure(g->sc_q, (size_t)n * sizeof(uint2)));
+    else
+        GVX_CK(gvx_ensure(g->sc_pts, (size_t)n * sizeof(float4)));
+    GVX_CK(gvx_ensure(g->sc_runs, (size_t)nleaves * 8 * sizeof(int2)));
+    uint32_t* total = g->d_counts.as<uint32_t>() + 60;
+    GVX_CK(cudaMemsetAsync(total, 0, 2 * sizeof(uint32_t), st));
+    ScDirectArgs a;
+    memset(&a, 0, sizeof(a));
+    a.skeys = g->keys[g->sorted_buf].as<uint32_t>();
+    a.svals = g->vals[g->sorted_buf].as<uint32_t>();
+    a.n = (uint32_t)n;
+    a.L = g->lookup;
+    a.invalid_key = 1u << (g->lookup.ks.total_bits + 3);
+    a.pos = g->pts.pos;
+    a.off = g->pts.pos_off;
+    a.stride = g->pts.pos_stride;
+    for (int k = 0; k < 3; k++) a.t[k] = t[k];
+    a.rins = radius;
+    a.inv_b = 1.0f / (float)g->brick;
+    a.qmin = make_float3(qmin[0], qmin[1], qmin[2]);
+    a.qrange = make_float3(qrange[0], qrange[1], qrange[2]);
+    a.q = fp16 ? g->sc_q.as<uint2>() : nullptr;
+    a.pts = fp16 ? nullptr : g->sc_pts.as<float4>();
+    a.total = total;
+    if (fp16)
+        k_sc_direct<true><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    else
+        k_sc_direct<false><<<blocks_for(n, 256), 256, 0, st>>>(a);
+    k_sc_runs<<<blocks_for((uint64_t)nleaves * 8u, 256), 256, 0, st>>>(g->leaf_range.as<int2>(), g->leaf_oct.as<int>(),
+                                                                      nleaves, g->sc_runs.as<int2>());
+    g->launches += 2;
+    uint32_t h[2];
+    GVX_CK(cudaMemcpyAsync(h, total, sizeof(h), cudaMemcpyDeviceToHost, st));
+    GVX_CK(cudaStreamSynchronize(st));
+    *m = h[0];
+    *done = h[1] == 0u;
+    return GVX_OK;
+}
+
 // InsertPointsSubcell and InsertPointsSubcell_FP16: the same lists, FP32
 // translated positions or 16-bit fractions of the bounding box
 static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, const float trans[3], int* sc_len,
@@ -424,12 +750,6 @@ static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, 
     GVX_CK(gvx_ensure(g->d_err, 64));
     GVX_CK(gvx_ensure(g->d_counts, 64 * sizeof(uint32_t)));
     GVX_CK(cudaMemsetAsync(g->d_err.p, 0, 4, st));
-    GVX_CK(gvx_ensure(g->sc_cnt, (size_t)n * 4 + 4));
-    GVX_CK(gvx_ensure(g->sc_off, (size_t)n * 4 + 4));
-    GVX_CK(gvx_ensure(g->sc_beg, (size_t)nsub * 4));
-    GVX_CK(gvx_ensure(g->sc_end, (size_t)nsub * 4));
-    GVX_CK(cudaMemsetAsync(g->sc_beg.p, 0, (size_t)nsub * 4, st));
-    GVX_CK(cudaMemsetAsync(g->sc_end.p, 0, (size_t)nsub * 4, st));
     const float t[3] = {trans ? trans[0] : 0.f, trans ? trans[1] : 0.f, trans ? trans[2] : 0.f};
     // mPosMin / mPosRange of the last GetBoundingBox (VG.cpp:5452-5462), host floats as the reference's
     float qmin[3], qrange[3];
@@ -454,7 +774,14 @@ static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, 
     a.leaf_slot = g->leaf_slot.as<int>();
     a.err = g->d_err.as<uint32_t>();
     uint32_t m = 0;
-    if (n > 0) {
+    bool direct = n > 0 && g->brick == 8 && subcell == 4 && radius <= kDirectMaxRadius && !g->pts.clr &&
+                  g->key_shift == 3 && g->group_valid && g->full_group_gen == g->topo_gen &&
+                  g->group_pos == g->pts.pos && g->group_n == n && t[0] == g->group_trans[0] &&
+                  t[1] == g->group_trans[1] && t[2] == g->group_trans[2];
+    if (direct) GVX_CK_STATUS(insert_direct(g, n, radius, t, qmin, qrange, fp16, &m, &direct));
+    if (n > 0 && !direct) {
+        GVX_CK(gvx_ensure(g->sc_cnt, (size_t)n * 4 + 4));
+        GVX_CK(gvx_ensure(g->sc_off, (size_t)n * 4 + 4));
         a.cnt = g->sc_cnt.as<uint32_t>();
         k_sc_points<false><<<blocks_for(n, 256), 256, 0, st>>>(a);
         g->launches++;
@@ -465,7 +792,13 @@ static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, 
         GVX_CK(cudaMemcpyAsync(&m, total, 4, cudaMemcpyDeviceToHost, st));
         GVX_CK(cudaStreamSynchronize(st));
     }
-    if (m > 0) {
+    if (!direct) {
+        GVX_CK(gvx_ensure(g->sc_beg, (size_t)nsub * 4));
+        GVX_CK(gvx_ensure(g->sc_end, (size_t)nsub * 4));
+        GVX_CK(cudaMemsetAsync(g->sc_beg.p, 0, (size_t)nsub * 4, st));
+        GVX_CK(cudaMemsetAsync(g->sc_end.p, 0, (size_t)nsub * 4, st));
+    }
+    if (m > 0 && !direct) {
         GVX_CK(gvx_ensure(g->sc_keys[0], (size_t)m * 4));
         GVX_CK(gvx_ensure(g->sc_keys[1], (size_t)m * 4));
         GVX_CK(gvx_ensure(g->sc_vals[0], (size_t)m * 4));
@@ -511,6 +844,7 @@ static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, 
     g->sc_nsub = (uint32_t)nsub;
     g->sc_has_clr = g->pts.clr != nullptr;
     g->sc_fp16 = fp16;
+    g->sc_direct = direct;
     for (int k = 0; k < 3; k++) {
         g->sc_qmin[k] = qmin[k];
         g->sc_qrange[k] = qrange[k];
@@ -571,6 +905,11 @@ gvx_status gvx_gather_levelset_fp16(gvx_grid* g, int subcell, int n, float radiu
                       "(call InsertPointsSubcell_FP16 first)", subcell);
         return GVX_ERR_STATE;
     }
+    if (g->sc_direct) {  // (no colours)
+        GVX_CK_STATUS(gather_direct<true>(g, radius, 1, 0, g->ch[cl].data.as<float>()));
+        apron_invalidate(g->ch[cl]);
+        return GVX_OK;
+    }
     GatherQArgs a;
     memset(&a, 0, sizeof(a));
     a.nsub = g->sc_nsub;
@@ -630,6 +969,11 @@ gvx_status gvx_gather_run(gvx_grid* g, int levelset, int subcell, float radius, 
         gvx_set_error("%s: no FP32 subcell lists of size %d for this topology (call InsertPointsSubcell first)",
                       what, subcell);
         return GVX_ERR_STATE;
+    }
+    if (g->sc_direct) {  // (no colours)
+        GVX_CK_STATUS(gather_direct<false>(g, radius, levelset, accum ? 1 : 0, g->ch[chan].data.as<float>()));
+        apron_invalidate(g->ch[chan]);  // the gathers write interior voxels only
+        return GVX_OK;
     }
     GatherArgs a;
     memset(&a, 0, sizeof(a));

@@ -163,6 +163,7 @@ struct gvx_grid {
     float group_trans[3] = {0, 0, 0};
     const void* group_pos = nullptr;
     int group_n = -1;
+    uint64_t full_group_gen = 0;  // topo_gen of the full build the grouping was made by (else another number)
     DevBuf spos, svel;  // sorted float4 (x,y,z,weight) and (vx,vy,vz,radius)
     bool perm_valid = false;  // spos/svel match the grouping and the bound attributes
     bool perm_has_svel = false;
@@ -197,6 +198,8 @@ struct gvx_grid {
     float sc_qmin[3] = {0, 0, 0}, sc_qrange[3] = {0, 0, 0};  // mPosMin / mPosRange they were stored against
     bool sc_fp16 = false;           // the lists are InsertPointsSubcell_FP16's
     bool colavg_seen = false;       // an avgColor ScatterDensity ran (the reference's AUX_COLAVG exists)
+    bool sc_direct = false;         // no entries: the points of the last full build in sorted order, the
+    DevBuf sc_runs;                 // runs of every leaf's octants (gvx_gather.cu)
     int sc_size = 0;
     uint32_t sc_len = 0, sc_nsub = 0;
     bool sc_has_clr = false;

@@ -1311,6 +1311,7 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
                         &g->launches);
     if (rc) return rc;
     g->sorted_buf = res;
+    g->full_group_gen = ~0ull;
     g->key_shift = kshift;
     g->n_sorted = (uint32_t)n;
     for (int a = 0; a < 3; a++) g->sort_trans[a] = t[a];
@@ -1760,6 +1761,7 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     rc = fill_leaf_ranges(g, L0);
     if (rc) return rc;
     g->group_valid = true;
+    g->full_group_gen = g->topo_gen;
     g->group_pos = g->pts.pos;
     g->group_n = n;
     for (int a = 0; a < 3; a++) g->group_trans[a] = o[a];
@@ -2705,6 +2707,7 @@ gvx_status gvx_topo_plan_finish(gvx_grid* g, bool* held, bool frame)
         g->root_pos[a] = P.fb.rootpos[a];
     }
     g->group_valid = true;
+    g->full_group_gen = g->topo_gen;
     g->group_pos = g->pts.pos;
     g->group_n = P.fb.n;
     g->root_level = depth;
