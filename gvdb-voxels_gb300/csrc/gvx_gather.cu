@@ -390,8 +390,8 @@ __global__ void k_gather(GatherArgs a)
 // subcell whose box touches it.  The entries are not written out: the insert counts them (the caller
 // gets their number), and stores each point once, in sorted order, with a flag per face of its octant
 // that its box crosses; the gather tests the flags as it reads the runs.
-// 6M points, 32M entries: emitting, sorting and copying the entries took 1.6 ms and the insert 2.0 ms in
-// all, storing the points XX.
+// 6M points, 32M entries: counting, emitting, sorting and copying the entries took 1.7 ms, the insert
+// that stores the points 0.15 ms.
 struct ScDirectArgs {
     const uint32_t* skeys;   // sorted keys: leaf << 3 | octant
     const uint32_t* svals;
@@ -406,6 +406,16 @@ struct ScDirectArgs {
     float4* pts;             // FP32: position, flags in .w
     uint32_t* total;         // entries; total[1]: a point is no longer where the build found it
 };
+
+// whether a full build's lookup has the leaf
+__device__ __forceinline__ bool leaf_there(const LeafLookup& L, int cx, int cy, int cz)
+{
+    if (cx < 0 || cy < 0 || cz < 0 || cx >= (1 << L.ks.bits[0]) || cy >= (1 << L.ks.bits[1]) ||
+        cz >= (1 << L.ks.bits[2]))
+        return false;
+    const uint32_t key = ks_pack(L.ks, cx, cy, cz, 0);
+    return br_test(L.a, key) || br_test(L.b, key);
+}
 
 constexpr float kDirectMaxRadius = 2.0f;  // boxes reach no further than the next subcell of 4 voxels
 
@@ -462,7 +472,7 @@ __global__ void __launch_bounds__(256) k_sc_direct(ScDirectArgs a)
                         // the brick of that subcell, and whether it is there
                         const int bx = (((oct >> 2) & 1) + dx) >> 1, by = (((oct >> 1) & 1) + dy) >> 1,
                                   bz = ((oct & 1) + dz) >> 1;
-                        entries += (bx | by | bz) == 0 || ll_find(a.L, c[0] + bx, c[1] + by, c[2] + bz) >= 0;
+                        entries += (bx | by | bz) == 0 || leaf_there(a.L, c[0] + bx, c[1] + by, c[2] + bz);
                     }
         }
         if (FP16)
@@ -510,19 +520,31 @@ struct GatherDirectArgs {
     uint32_t* next;
 };
 constexpr int kDirectWarps = 8;
+
+// two squares, each rounded on its own: x x + 0 in one step, which the sum that follows cannot be fused
+// with (a packed product and a packed sum are, whatever their rounding modifiers: one step less than
+// k_gather_fp16 rounds)
+__device__ __forceinline__ float2 square2(float2 x) { return __ffma2_rn(x, x, make_float2(0.f, 0.f)); }
 }  // namespace
 
-// One warp per subcell of 4^3 voxels, two voxels a lane (z and z + 2).  What bounds it: the distances
-// (eleven float steps a listed point and warp, each rounded on its own as in k_gather_fp16).  The lanes
-// test 32 points of the 27 runs at a time; the listed ones wait, decoded, in shared memory until there
-// are 32.  6M points, 433k subcells, 32M entries: XX us against 1154 for the written lists.
+// One warp per subcell of 4^3 voxels; each half of the warp takes every second listed point, a lane the
+// four voxels of a column.  What bounds it: instruction issue, half of it the distances, whose float
+// steps are each rounded on its own as in k_gather_fp16 (packed two to an instruction: 1.00 -> 0.84 ms;
+// with two voxels a lane and the whole warp on every point 1.03).  The lanes test 32 points of the 27 runs at a time; the listed ones, a
+// fifth, wait in shared memory until there are 32, and are decoded together.  The subcells of a claim
+// come from four distant places: dense ones lie side by side, and claims of neighbours left one warp
+// with half of the launch's time (1.32 ms, 1.03 with the claims spread).
+// 6M points, 433k subcells, 32M listed: 0.84 ms; 1.15 from written entries.
 template <bool FP16>
 __global__ void __launch_bounds__(kDirectWarps * 32) k_gather_direct(GatherDirectArgs a)
 {
-    __shared__ float4 s_ent[kDirectWarps][64];
+    // listed points that wait (FP16: as stored), and the 32 being added
+    __shared__ float4 s_ent[kDirectWarps][FP16 ? 32 : 64];
+    __shared__ uint2 s_raw[kDirectWarps][FP16 ? 64 : 1];
     __shared__ int2 s_rs[kDirectWarps][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float4* ent = s_ent[wid];
+    uint2* raw = s_raw[wid];
     int2* rs = s_rs[wid];
     const uint32_t lt = (1u << lane) - 1u;
     const int dx = lane / 9 - 1, dy = lane / 3 % 3 - 1, dz = lane % 3 - 1;  // lane < 27: its octant, from the subcell's
@@ -530,10 +552,12 @@ __global__ void __launch_bounds__(kDirectWarps * 32) k_gather_direct(GatherDirec
     const uint32_t need = lane < 27 ? (dx < 0 ? 2u : dx > 0 ? 1u : 0u) | (dy < 0 ? 8u : dy > 0 ? 4u : 0u) |
                                           (dz < 0 ? 32u : dz > 0 ? 16u : 0u)
                                     : 0u;
-    const int vx = lane & 3, vy = (lane >> 2) & 3, vz = lane >> 4;  // voxels (vx, vy, vz) and (vx, vy, vz + 2)
+    const int vx = lane & 3, vy = (lane >> 2) & 3, half = lane >> 4;
+    const uint32_t quarter = a.nsub / kUnitClaim;
     WarpUnits wu(a.next, lane);
-    uint32_t s;
-    while (wu.next(a.next, a.nsub, lane, s)) {
+    uint32_t u;
+    while (wu.next(a.next, a.nsub, lane, u)) {
+        const uint32_t s = u < quarter * kUnitClaim ? (u % kUnitClaim) * quarter + u / kUnitClaim : u;
         const uint32_t slot = s >> 3;
         const int ox = (int)(s & 1u), oy = (int)(s >> 1 & 1u), oz = (int)(s >> 2 & 1u);  // (subcell x fastest)
         const int leaf = a.slot_leaf[slot];
@@ -557,75 +581,110 @@ __global__ void __launch_bounds__(kDirectWarps * 32) k_gather_direct(GatherDirec
         // per run with points: its first sorted index less its first candidate number, and what it needs
         if (len > 0) rs[__popc(some & lt)] = make_int2(run.x - off, (int)need);
         __syncwarp();
-        float m0 = __int_as_float(0x7f800000), m1 = m0;  // the smallest squared distances so far
-        const float wx = (float)(org.y + 4 * ox + vx), wy = (float)(org.z + 4 * oy + vy);
-        const float wz0 = (float)(org.w + 4 * oz + vz), wz1 = wz0 + 2.0f;
+        float m2[4];  // the smallest squared distances so far
+        const float2 nxy = make_float2(-(float)(org.y + 4 * ox + vx), -(float)(org.z + 4 * oy + vy));
+        float2 nz[2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) m2[k] = __int_as_float(0x7f800000);
+        nz[0] = make_float2(-(float)(org.w + 4 * oz), -(float)(org.w + 4 * oz + 1));
+        nz[1] = make_float2(-(float)(org.w + 4 * oz + 2), -(float)(org.w + 4 * oz + 3));
+        // (two floats an instruction; adding the negated voxel is subtracting it)
         auto nearest = [&](const float4 p) {
-            if (FP16) {
-                const float dx = __fsub_rn(p.x, wx), dy = __fsub_rn(p.y, wy);
-                const float dxy = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-                const float d0 = __fsub_rn(p.z, wz0), d1 = __fsub_rn(p.z, wz1);
-                m0 = fminf(m0, __fadd_rn(dxy, __fmul_rn(d0, d0)));
-                m1 = fminf(m1, __fadd_rn(dxy, __fmul_rn(d1, d1)));
-            } else {
-                const float dx = p.x - wx, dy = p.y - wy, d0 = p.z - wz0, d1 = p.z - wz1;
-                const float dxy = fmaf(dy, dy, dx * dx);
-                m0 = fminf(m0, fmaf(d0, d0, dxy));
-                m1 = fminf(m1, fmaf(d1, d1, dxy));
+            const float2 e = __fadd2_rn(make_float2(p.x, p.y), nxy), e2 = square2(e);
+            const float exy = FP16 ? __fadd_rn(e2.x, e2.y) : fmaf(e.y, e.y, e2.x);
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const float2 ez = __fadd2_rn(make_float2(p.z, p.z), nz[k]), xy = make_float2(exy, exy);
+                const float2 d2 = FP16 ? __fadd2_rn(xy, square2(ez)) : __ffma2_rn(ez, ez, xy);
+                m2[2 * k] = fminf(m2[2 * k], d2.x);
+                m2[2 * k + 1] = fminf(m2[2 * k + 1], d2.y);
             }
         };
         int have = 0;  // listed points waiting
-        for (int base = 0; base < total; base += 32) {
+        // the first n of them (at most 32)
+        auto add_listed = [&](int n) {
+            if (FP16) {
+                const uint2 q = raw[lane];
+                float4 p;
+                p.x = __fadd_rn(__fmul_rn(__fdiv_rn((float)(q.x & 0xFFFFu), 65535.0f), a.qrange[0]), a.qmin[0]);
+                p.y = __fadd_rn(__fmul_rn(__fdiv_rn((float)(q.x >> 16), 65535.0f), a.qrange[1]), a.qmin[1]);
+                p.z = __fadd_rn(__fmul_rn(__fdiv_rn((float)(q.y & 0xFFFFu), 65535.0f), a.qrange[2]), a.qmin[2]);
+                p.w = 0.f;
+                ent[lane] = p;
+                __syncwarp();
+            }
+            if (n == 32) {
+#pragma unroll
+                for (int e = 0; e < 32; e += 2) nearest(ent[e + half]);
+            } else {
+                for (int e = half; e < n; e += 2) nearest(ent[e]);
+            }
+            __syncwarp();
+        };
+        for (int base = 0;; base += 32) {
+            const bool last = base >= total;  // one more pass adds the last listed ones
             // candidate base + lane: its run is the number of runs that start at or before it, less one
             const uint32_t starts =
                 __reduce_or_sync(0xFFFFFFFFu, len > 0 && off >= base && off < base + 32 ? 1u << (off - base) : 0u);
             const int before = __popc(__ballot_sync(0xFFFFFFFFu, len > 0 && off < base));
             bool listed = false;
+            uint2 q = make_uint2(0u, 0u);
             float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
             if (base + lane < total) {
                 const int2 r = rs[before - 1 + __popc(starts & (0xFFFFFFFFu >> (31 - lane)))];
-                if (FP16) {
-                    const uint2 u = a.q[r.x + base + lane];
-                    listed = ((u.y >> 16) & (uint32_t)r.y) == (uint32_t)r.y;
-                    if (listed) {
-                        p.x = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.x & 0xFFFFu), 65535.0f), a.qrange[0]), a.qmin[0]);
-                        p.y = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.x >> 16), 65535.0f), a.qrange[1]), a.qmin[1]);
-                        p.z = __fadd_rn(__fmul_rn(__fdiv_rn((float)(u.y & 0xFFFFu), 65535.0f), a.qrange[2]), a.qmin[2]);
-                    }
-                } else {
+                if (FP16)
+                    q = a.q[r.x + base + lane];
+                else
                     p = a.pts[r.x + base + lane];
-                    listed = (__float_as_uint(p.w) & (uint32_t)r.y) == (uint32_t)r.y;
-                }
+                const uint32_t flags = FP16 ? q.y >> 16 : __float_as_uint(p.w);
+                listed = (flags & (uint32_t)r.y) == (uint32_t)r.y;
             }
             const uint32_t lm = __ballot_sync(0xFFFFFFFFu, listed);
-            if (listed) ent[have + __popc(lm & lt)] = p;
+            if (listed) {
+                if (FP16)
+                    raw[have + __popc(lm & lt)] = q;
+                else
+                    ent[have + __popc(lm & lt)] = p;
+            }
             have += __popc(lm);
+            if (have < 32 && !last) continue;
             __syncwarp();
-            if (have >= 32) {
-#pragma unroll 8
-                for (int e = 0; e < 32; e++) nearest(ent[e]);
-                have -= 32;
-                const float4 rest = ent[32 + (lane < have ? lane : 0)];
-                __syncwarp();
-                if (lane < have) ent[lane] = rest;
-                __syncwarp();
+            const int n = min(have, 32);
+            if (n > 0) add_listed(n);
+            if (last) break;
+            have -= 32;
+            uint2 q1 = q;
+            float4 p1 = p;
+            if (lane < have) {
+                if (FP16)
+                    q1 = raw[32 + lane];
+                else
+                    p1 = ent[32 + lane];
+            }
+            __syncwarp();
+            if (lane < have) {
+                if (FP16)
+                    raw[lane] = q1;
+                else
+                    ent[lane] = p1;
             }
         }
-        for (int e = 0; e < have; e++) nearest(ent[e]);
         __syncwarp();
+        // the halves' results; then lane half h stores the voxels 2h and 2h + 1 of the column
+#pragma unroll
+        for (int k = 0; k < 4; k++) m2[k] = fminf(m2[k], __shfl_xor_sync(0xFFFFFFFFu, m2[k], 16));
         // min_j (sqrt(d2_j) - R) = sqrt(min_j d2_j) - R: rounded sqrt and subtraction are monotone
-        const int P = a.P, z0 = 4 * oz + vz + a.apron;
-        const size_t i0 = (((size_t)slot * P + z0) * P + (4 * oy + vy + a.apron)) * P + (4 * ox + vx + a.apron);
-        const size_t i1 = i0 + 2 * (size_t)P * P;
-        const float c0 = __fsqrt_rn(m0), c1 = __fsqrt_rn(m1);  // +inf without points: the start value stays
-        if (FP16 || a.levelset) {
-            const float v0 = a.accum ? a.out[i0] : 3.0f, v1 = a.accum ? a.out[i1] : 3.0f;
-            a.out[i0] = fminf(v0, __fsub_rn(c0, a.radius));
-            a.out[i1] = fminf(v1, __fsub_rn(c1, a.radius));
-        } else {
-            const float v0 = a.accum ? a.out[i0] : 0.0f, v1 = a.accum ? a.out[i1] : 0.0f;
-            a.out[i0] = fmaxf(v0, __fsub_rn(a.radius, c0));
-            a.out[i1] = fmaxf(v1, __fsub_rn(a.radius, c1));
+        const int P = a.P;
+        const size_t i0 = (((size_t)slot * P + (4 * oz + 2 * half + a.apron)) * P + (4 * oy + vy + a.apron)) * P +
+                          (4 * ox + vx + a.apron);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const size_t i = i0 + (size_t)k * P * P;
+            const float c = __fsqrt_rn(half ? m2[2 + k] : m2[k]);  // +inf without points: the start value stays
+            if (FP16 || a.levelset)
+                a.out[i] = fminf(a.accum ? a.out[i] : 3.0f, __fsub_rn(c, a.radius));
+            else
+                a.out[i] = fmaxf(a.accum ? a.out[i] : 0.0f, __fsub_rn(a.radius, c));
         }
     }
 }
