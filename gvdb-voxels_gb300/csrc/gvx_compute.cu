@@ -17,6 +17,7 @@
 //    (Jacobi, the ordering in which every read comes first) and 0 outside
 //    the atlas.  The channel's device pointer never moves.
 #include "gvx_grid.cuh"
+#include "gvx_ptx.cuh"
 
 namespace {
 constexpr int kComputeThreads = 256;
@@ -116,6 +117,73 @@ __global__ void k_smooth_slots(float* data, int P, int apron, size_t nslots, flo
     }
 }
 
+// The same for bricks of 8 (padded 10^3, 4000 bytes), the blocks two slots ahead of their stencils: a
+// slot comes in one bulk copy while the two before it are worked on, and leaves whole in another (the
+// apron as it came), so that no sector is written in part.  The block per slot above waits for its own
+// load and writes rows of 32 bytes across sectors: 54k slots 130 us, 78 here; both ways at the copy rate 67.
+constexpr int kSmoothThreads = 128, kSmoothStages = 3;
+__global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_t nslots, float p1, float p2, uint32_t* err)
+{
+    constexpr int P = 10, P2 = P * P, P3 = P2 * P;
+    __shared__ __align__(128) float s_in[kSmoothStages][P3 + 24], s_out[P3 + 24];
+    __shared__ __align__(8) uint64_t s_bar[kSmoothStages];
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        for (int k = 0; k < kSmoothStages; k++) mbar_init(&s_bar[k], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    auto fetch = [&](uint32_t s, int k) {  // (one thread)
+        mbar_expect_tx(&s_bar[k], P3 * 4);
+        bulk_g2s(s_in[k], data + (size_t)s * P3, P3 * 4, &s_bar[k]);
+    };
+    if (tid == 0)
+        for (int k = 0; k < kSmoothStages - 1; k++)
+            if (blockIdx.x + (uint64_t)k * gridDim.x < nslots) fetch(blockIdx.x + (uint32_t)k * gridDim.x, k);
+    // the thread's four voxels: a half row
+    const int x0 = 1 + (tid & 1) * 4, y = 1 + (tid >> 1 & 7), z = 1 + (tid >> 4);
+    const int c = (z * P + y) * P + x0;
+    uint32_t phase = 0u;  // bit k: the parity stage k's next copy completes
+    int k = 0;
+    for (uint64_t s = blockIdx.x; s < nslots; s += gridDim.x) {
+        // (the stage fetched into was read by every thread before the barrier at the end of the last turn)
+        const uint64_t ahead = s + (uint64_t)(kSmoothStages - 1) * gridDim.x;
+        if (tid == 0 && ahead < nslots) fetch((uint32_t)ahead, (k + kSmoothStages - 1) % kSmoothStages);
+        if (!mbar_wait_bounded(&s_bar[k], (phase >> k) & 1u)) atomicOr(err, GVX_DERR_TIMEOUT);
+        phase ^= 1u << k;
+        const float* in = s_in[k];
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            v[q] = p1 * in[c + q];
+            v[q] += in[c + q - 1];
+            v[q] += in[c + q + 1];
+            v[q] += in[c + q - P];
+            v[q] += in[c + q + P];
+            v[q] += in[c + q - P2];
+            v[q] += in[c + q + P2];
+            v[q] = smooth_value(v[q], p1, p2);
+        }
+        if (tid == 0) bulk_wait_read_all();  // the last slot has left the output buffer
+        __syncthreads();
+        for (int i = tid; i < P3 / 4; i += kSmoothThreads) {
+            // the apron of the four voxels i 4 .. i 4 + 3 (their interior ones are written below)
+            ((float4*)s_out)[i] = ((const float4*)in)[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; q++) s_out[c + q] = v[q];
+        fence_async_smem();
+        __syncthreads();
+        if (tid == 0) {
+            bulk_s2g(data + s * P3, s_out, P3 * 4);
+            bulk_commit();
+        }
+        k = (k + 1) % kSmoothStages;
+    }
+    if (tid == 0) bulk_wait_all();
+}
+
 // FUNC_SMOOTH without an apron: every voxel from its atlas neighbours in the
 // snapshot `src` (0 outside the atlas) into `dst`
 __global__ void k_smooth_atlas(const float* __restrict__ src, float* __restrict__ dst, AtlasShape s, float p1,
@@ -172,7 +240,12 @@ extern "C" gvx_status gvx_compute(gvx_grid* g, int effect, int chan, int iterati
     cudaStream_t st = g->stream;
     const unsigned flat_grid = std::min(blocks_for(nvox, kComputeThreads), 152u * 64u);
     for (int it = 0; it < iterations; it++) {
-        if (effect == GVX_FUNC_SMOOTH && g->apron > 0) {
+        if (effect == GVX_FUNC_SMOOTH && P == 10 && g->apron == 1 && nslots < (1u << 31)) {
+            GVX_CK(gvx_ensure(g->d_err, 64));
+            const unsigned grid = (unsigned)std::min<size_t>(nslots, 152u * 13u);
+            k_smooth8<<<grid, kSmoothThreads, 0, st>>>(ch.data.as<float>(), (uint32_t)nslots, params[0], params[1],
+                                                       g->d_err.as<uint32_t>());
+        } else if (effect == GVX_FUNC_SMOOTH && g->apron > 0) {
             const size_t smem = (size_t)P * P * P * sizeof(float);
             if (smem > 48 * 1024)
                 GVX_CK(cudaFuncSetAttribute(k_smooth_slots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
