@@ -34,6 +34,11 @@ struct ApronArgs {
     const unsigned char* only;  // optional per-slot mark: bricks whose aprons are copied (others kept)
 };
 
+// What bounds it: the lines of the bricks, nearly every sector of which an apron row's end touches (read
+// and written once: 57k bricks of 4 KB in 70 us at the copy rate), and the chain of loads before a
+// brick's first copy.  The brick of a warp's next turn has its neighbours' slots looked up while the
+// current one is copied (57k bricks: 105 us before, 101 with it).  4-byte voxels of any type are copied as words (uchar4
+// voxels, moved byte by byte, took 249 us).
 template <class T>
 __global__ void __launch_bounds__(kApronWarps * 32) k_apron(ApronArgs a, T boundval)
 {
@@ -43,13 +48,18 @@ __global__ void __launch_bounds__(kApronWarps * 32) k_apron(ApronArgs a, T bound
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const int P3 = a.P * a.P * a.P;
     T* data = (T*)a.data;
+    // the lane's neighbour of the brick in slot s (-1: none, or a brick that keeps its apron)
+    auto neighbour = [&](uint32_t s) {
+        if (s >= a.nslots || lane >= 27 || (a.only && !a.only[s])) return -1;
+        const int nl = a.nbr[(size_t)a.slot_leaf[s] * 27 + lane];
+        return nl >= 0 ? a.leaf_slot[nl] : -1;
+    };
+    int ns_next = neighbour(wglobal);
     for (uint32_t s = wglobal; s < a.nslots; s += nwarps) {
+        const int ns_here = ns_next;
+        ns_next = neighbour(s + nwarps);
         if (a.only && !a.only[s]) continue;  // warp-uniform: one brick per warp
-        const int leaf = a.slot_leaf[s];
-        if (lane < 27) {
-            const int nl = a.nbr[(size_t)leaf * 27 + lane];
-            s_ns[wid][lane] = nl >= 0 ? a.leaf_slot[nl] : -1;
-        }
+        if (lane < 27) s_ns[wid][lane] = ns_here;
         __syncwarp();
         T* dst = data + (size_t)s * P3;
         // U values per lane are loaded before any is stored: the sources (neighbours' interiors)
@@ -258,9 +268,12 @@ static gvx_status apron_launch(gvx_grid* g, int chan, float boundval, const unsi
     const uint64_t warps_needed = a.nslots;
     unsigned blocks = (unsigned)std::min<uint64_t>((warps_needed + kApronWarps - 1) / kApronWarps, 152ull * 16ull);
     switch (g->ch[chan].type) {
-    case GVX_T_FLOAT:
-        k_apron<float><<<blocks, threads, 0, g->stream>>>(a, boundval);
+    case GVX_T_FLOAT: {
+        uint32_t bits;
+        memcpy(&bits, &boundval, 4);
+        k_apron<uint32_t><<<blocks, threads, 0, g->stream>>>(a, bits);
         break;
+    }
     case GVX_T_FLOAT3:
     case GVX_T_FLOAT4:
         k_apron<float4><<<blocks, threads, 0, g->stream>>>(a, make_float4(boundval, boundval, boundval, boundval));
@@ -272,7 +285,7 @@ static gvx_status apron_launch(gvx_grid* g, int chan, float boundval, const unsi
     }
     case GVX_T_UCHAR4: {
         const unsigned char bv = (unsigned char)boundval;
-        k_apron<uchar4><<<blocks, threads, 0, g->stream>>>(a, make_uchar4(bv, bv, bv, bv));
+        k_apron<uint32_t><<<blocks, threads, 0, g->stream>>>(a, bv * 0x01010101u);
         break;
     }
     default:
