@@ -199,12 +199,18 @@ gvx_status gvx_create(int device, gvx_grid** out)
         return gvx_cuda_fail(e, "cudaStreamCreate");
     }
     g->own_stream = true;
-    // the device error word starts clear; from then on it is cleared when it is read
-    e = gvx_ensure(g->d_err, 64);
-    if (e == cudaSuccess) e = cudaMemset(g->d_err.p, 0, 64);
+    // what builds read back, in one buffer, so that one copy brings it: the counts, the bounding box, the
+    // error word.  That starts clear; from then on it is cleared when it is read
+    e = gvx_ensure(g->d_counts, kReadWords * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(g->d_counts.p, 0, kReadWords * sizeof(uint32_t));
+    if (e == cudaSuccess) {
+        g->d_bbox.p = g->d_counts.as<uint32_t>() + kReadBbox;
+        g->d_err.p = g->d_counts.as<uint32_t>() + kReadErr;
+        g->d_bbox.cap = g->d_err.cap = 64;
+    }
     if (e != cudaSuccess) {
         cudaStreamDestroy(g->stream);
-        gvx_free(g->d_err);
+        gvx_free(g->d_counts);
         delete g;
         return gvx_cuda_fail(e, "gvx_create: error word");
     }
@@ -225,7 +231,7 @@ gvx_status gvx_destroy(gvx_grid* g)
                       &g->keys[0], &g->keys[1], &g->vals[0], &g->vals[1], &g->spos, &g->svel,
                       &g->sort.buf, &g->d0_bits,
                       &g->d0_prefix, &g->x0_bits, &g->x0_prefix, &g->masks, &g->upper, &g->lists, &g->tmp_scan,
-                      &g->d_counts, &g->d_err, &g->d_bbox, &g->d_rmax, &g->d_next, &g->push_tab, &g->touched, &g->dense_units, &g->cell_tab, &g->host_stage,
+                      &g->d_counts, &g->d_rmax, &g->d_next, &g->push_tab, &g->touched, &g->dense_units, &g->cell_tab, &g->host_stage,
                       &g->api_keys[0], &g->api_keys[1], &g->api_vals[0], &g->api_vals[1], &g->lk_bits, &g->lk_prefix,
                       &g->inc0, &g->inc_remap, &g->sc_cnt, &g->sc_off, &g->sc_keys[0], &g->sc_keys[1],
                       &g->sc_vals[0], &g->sc_vals[1], &g->sc_pts, &g->sc_beg, &g->sc_end, &g->atlas_tmp,

@@ -67,6 +67,9 @@ __device__ inline int ll_find(const LeafLookup& L, int cx, int cy, int cz)
     return (L.cap && r >= L.cap) ? -1 : (int)r;
 }
 
+// words of d_counts: 64 counts, the bounding boxes (16), the error word (16)
+enum { kReadBbox = 64, kReadErr = 80, kReadWords = 96 };
+
 struct gvx_grid {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -175,7 +178,7 @@ struct gvx_grid {
     // scratch of the topology build
     DevBuf d0_bits, d0_prefix, x0_bits, x0_prefix, masks, upper, lists, tmp_scan, d_counts;
     DevBuf inc0, inc_remap;  // incremental build: linked + new level-0 bitmaps, linked rank -> pool index
-    DevBuf d_err, d_bbox;
+    DevBuf d_err, d_bbox;  // (inside d_counts)
     DevBuf d_rmax;  // float bits of the largest per-point radius of the last point permute
     DevBuf d_next;  // work-unit counters of the splat launch
     DevBuf push_tab;  // places of the push tiles' boundary voxels, for bricks of padded side push_tab_P

@@ -195,8 +195,9 @@ gvx_status gvx_onesweep_pass(uint32_t tile, uint32_t tiles, const uint32_t* kin,
                              uint32_t* vout, uint32_t n, int shift, const uint32_t* hist, uint32_t* lookback,
                              uint32_t* counter, uint32_t* err, cudaStream_t st);
 int gvx_sort_passes(int bits);
-// the scratch of a sort of n keys, zeroed, before its key producer counts digits into the histograms
-gvx_status gvx_sort_prepare(SortScratch& s, uint32_t n, int bits, cudaStream_t st);
+// the scratch of a sort of n keys: its ranges to be zeroed, before its key producer counts digits into the
+// histograms
+gvx_status gvx_sort_prepare(SortScratch& s, uint32_t n, int bits, struct ClearList& clear);
 uint32_t* gvx_sort_hist_ptr(SortScratch& s);
 
 // device helper used by key producers: accumulate digit histograms of a key
@@ -205,6 +206,30 @@ __device__ inline void gvx_sort_count_key(uint32_t* sh, uint32_t key, int passes
 {
     for (int p = 0; p < passes; p++) atomicAdd(&sh[p * 256 + ((key >> (8 * p)) & 255u)], 1u);
 }
+
+// ---- ranges set to a word, in one launch (gvx_topology.cu) -----------------
+// A build clears a dozen buffers, most of them small: a launch each, 2 to 4 us of the stream's time, was a
+// fifth of a small frame (6k points, planned: 15 of 50 launches).
+struct ClearList {
+    static constexpr int kMax = 24;
+    int n = 0;
+    uint32_t* p[kMax];
+    uint64_t words[kMax];
+    uint32_t value[kMax];
+    gvx_status full = GVX_OK;
+    void add(void* ptr, uint64_t nwords, uint32_t v)
+    {
+        if (nwords == 0) return;
+        if (n == kMax) {
+            full = GVX_ERR_CAPACITY;
+            return;
+        }
+        p[n] = (uint32_t*)ptr;
+        words[n] = nwords;
+        value[n++] = v;
+    }
+};
+gvx_status gvx_clear(const ClearList& c, cudaStream_t st, int64_t* launches);
 
 // ---- generic exclusive scan of popcounts of a bitmap (gvx_topology.cu) -----
 gvx_status gvx_bitmap_prefix(const uint32_t* bits, uint32_t* prefix, uint32_t words, uint32_t* total,

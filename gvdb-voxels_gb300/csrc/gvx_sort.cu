@@ -278,12 +278,12 @@ constexpr size_t kHistWords = 4 * 256, kCounterWords = 64;
 
 uint32_t* gvx_sort_hist_ptr(SortScratch& s) { return s.buf.as<uint32_t>(); }
 
-gvx_status gvx_sort_prepare(SortScratch& s, uint32_t n, int bits, cudaStream_t st)
+gvx_status gvx_sort_prepare(SortScratch& s, uint32_t n, int bits, ClearList& clear)
 {
     const uint32_t tile = sort_tile(n), tiles = (n + tile - 1) / tile;
     const size_t words = kHistWords + kCounterWords + (size_t)gvx_sort_passes(bits) * tiles * 256;
     GVX_CK(gvx_ensure(s.buf, words * sizeof(uint32_t)));
-    GVX_CK(cudaMemsetAsync(s.buf.p, 0, words * sizeof(uint32_t), st));
+    clear.add(s.buf.p, words, 0u);
     return GVX_OK;
 }
 
@@ -326,7 +326,9 @@ static gvx_status sort_run(const uint32_t* kin, const uint32_t* vin, uint32_t* c
 static gvx_status sort_histograms(const uint32_t* keys, uint32_t n, int bits, SortScratch& s, cudaStream_t st,
                                   int64_t* launches)
 {
-    GVX_CK_STATUS(gvx_sort_prepare(s, n, bits, st));
+    ClearList clear;
+    GVX_CK_STATUS(gvx_sort_prepare(s, n, bits, clear));
+    GVX_CK(cudaMemsetAsync(clear.p[0], 0, clear.words[0] * sizeof(uint32_t), st));
     const uint32_t blocks = std::min<uint32_t>((n + 4095u) / 4096u, 1024u);
     k_sort_hist<<<blocks, 256, 0, st>>>(keys, n, gvx_sort_passes(bits), gvx_sort_hist_ptr(s));
     (*launches)++;

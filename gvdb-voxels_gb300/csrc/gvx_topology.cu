@@ -382,6 +382,61 @@ __global__ void k_prefix_upper(UpperDesc ud, uint32_t* upper, uint32_t* counts)
 }
 
 // ---------------------------------------------------------------------------
+// The ranges of a ClearList: a block sets 4096 words of one of them, by 16 bytes where the range is aligned
+struct ClearArgs {
+    ClearList c;
+    uint32_t chunk[ClearList::kMax];  // the first chunk of each range
+};
+constexpr uint32_t kClearChunk = 4096;
+__global__ void __launch_bounds__(256) k_clear(ClearArgs a)
+{
+    int r = 0;
+    while (r + 1 < a.c.n && a.chunk[r + 1] <= blockIdx.x) r++;
+    const uint64_t w0 = (uint64_t)(blockIdx.x - a.chunk[r]) * kClearChunk;
+    const uint64_t left = a.c.words[r] - w0;
+    const uint32_t m = left < kClearChunk ? (uint32_t)left : kClearChunk;
+    uint32_t* p = a.c.p[r] + w0;
+    const uint32_t v = a.c.value[r];
+    const uint32_t m4 = ((uintptr_t)p & 15u) ? 0u : m / 4u;
+    const uint4 q = make_uint4(v, v, v, v);
+    for (uint32_t i = threadIdx.x; i < m4; i += 256u) ((uint4*)p)[i] = q;
+    for (uint32_t i = m4 * 4u + threadIdx.x; i < m; i += 256u) p[i] = v;
+}
+
+gvx_status gvx_clear(const ClearList& c, cudaStream_t st, int64_t* launches)
+{
+    if (c.full) {
+        gvx_set_error("clear: more than %d ranges", ClearList::kMax);
+        return c.full;
+    }
+    if (c.n == 0) return GVX_OK;
+    ClearArgs a;
+    a.c = c;
+    uint64_t chunks = 0;
+    for (int r = 0; r < c.n; r++) {
+        a.chunk[r] = (uint32_t)chunks;
+        chunks += (c.words[r] + kClearChunk - 1) / kClearChunk;
+    }
+    if (chunks > 0x7FFFFFFFull) {
+        gvx_set_error("clear: %llu chunks", (unsigned long long)chunks);
+        return GVX_ERR_CAPACITY;
+    }
+    k_clear<<<(unsigned)chunks, 256, 0, st>>>(a);
+    (*launches)++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
+}
+
+// the accumulators of GetBoundingBox and of the active leaves' box (k_bbox, k_leaf_bounds) before them
+static void clear_bboxes(gvx_grid* g, ClearList& c)
+{
+    uint32_t* b = g->d_bbox.as<uint32_t>();
+    c.add(b, 3, 0xFFFFFFFFu);  // min = all ones, max = 0 (order-preserving bits)
+    c.add(b + 3, 3, 0u);
+    c.add(b + 8, 3, 0x7FFFFFFFu);
+    c.add(b + 11, 3, 0x80000000u);
+}
+
 // generic exclusive prefix of popcounts over a bitmap (reduce, scan, apply)
 namespace {
 constexpr int kPfxThreads = 256;
@@ -899,17 +954,10 @@ __global__ void k_flag_bits(const GvxNode* __restrict__ nodes, DevCount nc, uint
 
 // UpdateAtlas: active leaf k (pool order) -> atlas slot k, mValue, atlas map
 // (VG.cpp:2650-2690, AL.cpp:692-715)
-__global__ void k_atlas_assign(GvxNode* nodes, DevCount nc, const uint32_t* __restrict__ fbits,
-                               const uint32_t* __restrict__ fprefix, int sx, int sy, int P, int apron,
-                               int* leaf_slot, int* slot_leaf, int4* amap)
+// the atlas position of slot s, and its leaf i there
+__device__ __forceinline__ void atlas_place(GvxNode* nodes, uint32_t i, uint32_t s, int sx, int sy, int P, int apron,
+                                            int* leaf_slot, int* slot_leaf, int4* amap)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nc.get()) return;
-    if (!((fbits[i >> 5] >> (i & 31)) & 1u)) {
-        leaf_slot[i] = -1;
-        return;
-    }
-    const uint32_t s = fprefix[i >> 5] + __popc(fbits[i >> 5] & ((1u << (i & 31)) - 1u));
     const int a2 = sx * sy;
     const int z = (int)s / a2, rem = (int)s - z * a2;
     const int y = rem / sx, x = rem - y * sx;
@@ -922,20 +970,36 @@ __global__ void k_atlas_assign(GvxNode* nodes, DevCount nc, const uint32_t* __re
     amap[s] = make_int4(nd->pos[0], nd->pos[1], nd->pos[2], (int)i);
 }
 
-// GetBoundingBox's accumulators before k_bbox: min = all ones, max = 0 (order-preserving bits)
-__global__ void k_bbox_reset(uint32_t* out)
+// a thread per slot; the flags, their prefix and two clears of the general case below took five launches
+// more, 4 us each
+__global__ void k_atlas_all(GvxNode* nodes, DevCount nc, uint32_t slots, int sx, int sy, int P, int apron,
+                            int* leaf_slot, int* slot_leaf, int4* amap, uint32_t* nslots)
 {
-    if (threadIdx.x < 6) out[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t n = nc.get();
+    if (i == 0 && nslots) *nslots = n;
+    if (i < n)
+        atlas_place(nodes, i, i, sx, sy, P, apron, leaf_slot, slot_leaf, amap);
+    else if (i < slots)
+        amap[i] = make_int4(-1, -1, -1, -1);
 }
 
-__global__ void k_bounds_init(int* out)
+__global__ void k_atlas_assign(GvxNode* nodes, DevCount nc, const uint32_t* __restrict__ fbits,
+                               const uint32_t* __restrict__ fprefix, int sx, int sy, int P, int apron,
+                               int* leaf_slot, int* slot_leaf, int4* amap)
 {
-    if (threadIdx.x < 3) out[threadIdx.x] = 0x7FFFFFFF;
-    else if (threadIdx.x < 6) out[threadIdx.x] = (int)0x80000000;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nc.get()) return;
+    if (!((fbits[i >> 5] >> (i & 31)) & 1u)) {
+        leaf_slot[i] = -1;
+        return;
+    }
+    const uint32_t s = fprefix[i >> 5] + __popc(fbits[i >> 5] & ((1u << (i & 31)) - 1u));
+    atlas_place(nodes, i, s, sx, sy, P, apron, leaf_slot, slot_leaf, amap);
 }
 
-// ComputeBounds (VG.cpp:1792-1816): bbox of active leaves
-__global__ void k_leaf_bounds(const GvxNode* __restrict__ nodes, uint32_t n, int range, int* out)
+// ComputeBounds (VG.cpp:1792-1816): bbox of active leaves (threads 0-5 of a block hold its atomics)
+__device__ __forceinline__ void leaf_bounds(const GvxNode* __restrict__ nodes, uint32_t n, int range, int* out)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;  // whole warps: the grid is a multiple of 32
     int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
@@ -970,6 +1034,11 @@ __global__ void k_leaf_bounds(const GvxNode* __restrict__ nodes, uint32_t n, int
             atomicMax(&out[threadIdx.x], v);
         }
     }
+}
+
+__global__ void k_leaf_bounds(const GvxNode* __restrict__ nodes, uint32_t n, int range, int* out)
+{
+    leaf_bounds(nodes, n, range, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -1242,62 +1311,60 @@ gvx_status gvx_check_device_error(gvx_grid* g, const char* stage)
     return report_device_error(g, e, stage);
 }
 
-// `bytes` (at most 256) of device memory and the device error word in one round
-// trip through pinned staging, then the error word reported as above
-// (queued: the copies into the staging; then, once the stream has passed them,
-// readback_finish takes the bytes and reports the error word)
-static gvx_status readback_start(gvx_grid* g, const void* src, size_t bytes, const char* stage)
+// The counts, the bounding boxes and the device error word in one copy through pinned staging
+// (queued: the copy; then, once the stream has passed it, readback_finish takes
+// `bytes` from word `first` of d_counts and reports the error word as above)
+static gvx_status readback_start(gvx_grid* g)
 {
-    if (bytes > 256) {
-        gvx_set_error("%s: readback of %zu bytes", stage, bytes);
-        return GVX_ERR_INVALID_ARG;
-    }
     if (!g->h_pin) GVX_CK(cudaMallocHost(&g->h_pin, 512));
-    GVX_CK(cudaMemcpyAsync(g->h_pin, src, bytes, cudaMemcpyDeviceToHost, g->stream));
-    GVX_CK(cudaMemcpyAsync((char*)g->h_pin + 256, g->d_err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
+    GVX_CK(cudaMemcpyAsync(g->h_pin, g->d_counts.p, kReadWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream));
     return GVX_OK;
 }
 
-static gvx_status readback_finish(gvx_grid* g, void* dst, size_t bytes, const char* stage)
+static gvx_status readback_finish(gvx_grid* g, void* dst, int first, size_t bytes, const char* stage)
 {
     GVX_CK(cudaStreamSynchronize(g->stream));
-    memcpy(dst, g->h_pin, bytes);
-    uint32_t e = 0;
-    memcpy(&e, (const char*)g->h_pin + 256, sizeof(e));
-    return report_device_error(g, e, stage);
+    const uint32_t* h = (const uint32_t*)g->h_pin;
+    memcpy(dst, h + first, bytes);
+    return report_device_error(g, h[kReadErr], stage);
 }
 
-static gvx_status readback_checked(gvx_grid* g, void* dst, const void* src, size_t bytes, const char* stage)
+static gvx_status readback_checked(gvx_grid* g, void* dst, int first, size_t bytes, const char* stage)
 {
-    gvx_status rc = readback_start(g, src, bytes, stage);
-    return rc ? rc : readback_finish(g, dst, bytes, stage);
+    gvx_status rc = readback_start(g);
+    return rc ? rc : readback_finish(g, dst, first, bytes, stage);
 }
 
 static gvx_status ensure_grid_scratch(gvx_grid* g)
 {
-    GVX_CK(gvx_ensure(g->d_err, 64));
-    GVX_CK(gvx_ensure(g->d_bbox, 64));
-    GVX_CK(gvx_ensure(g->d_counts, 64 * sizeof(uint32_t)));
-    return GVX_OK;
+    if (g->d_err.p) return GVX_OK;  // (made with the grid)
+    gvx_set_error("grid without its readback buffer");
+    return GVX_ERR_STATE;
 }
 
 // sort the points by compact key in key space `ks` (positions + t), fill
 // leaf_range for the leaves of `L` (whose key space must be ks)
-static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpace& ks, bool fuse_hist)
+// (octants below the leaf key when the key space leaves room for it: 28 bits of leaves)
+static int sort_shift(const KeySpace& ks) { return ks.total_bits <= 28 ? 3 : 0; }
+
+// the scratch of sort_points, its ranges to be zeroed before it
+static gvx_status sort_points_scratch(gvx_grid* g, int n, const KeySpace& ks, ClearList& clear)
+{
+    return gvx_sort_prepare(g->sort, (uint32_t)n, ks.total_bits + sort_shift(ks) + 1, clear);
+}
+
+static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpace& ks)
 {
     GVX_CK(gvx_ensure(g->keys[0], (size_t)n * 4));
     GVX_CK(gvx_ensure(g->keys[1], (size_t)n * 4));
     GVX_CK(gvx_ensure(g->vals[0], (size_t)n * 4));
     GVX_CK(gvx_ensure(g->vals[1], (size_t)n * 4));
-    // the octant below the leaf key when the key space leaves room for it (28 bits of leaves)
-    const int kshift = ks.total_bits <= 28 ? 3 : 0;
+    const int kshift = sort_shift(ks);
     int lb = 0;
     while ((1 << lb) < g->brick) lb++;
     const uint32_t invalid_key = 1u << (ks.total_bits + kshift);
     const int bits = ks.total_bits + kshift + 1;
     const int passes = gvx_sort_passes(bits);
-    gvx_status rc = gvx_sort_prepare(g->sort, (uint32_t)n, bits, g->stream);
-    if (rc) return rc;
     const unsigned kb = std::min(blocks_for(n, 256), 152u * 8u);
     k_keys<<<kb, 256, 0, g->stream>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, t[0], t[1], t[2],
                                       ks, 1.0f / (float)g->brick, kshift, lb, passes, invalid_key,
@@ -1307,8 +1374,8 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
     uint32_t* kk[2] = {g->keys[0].as<uint32_t>(), g->keys[1].as<uint32_t>()};
     uint32_t* vv[2] = {g->vals[0].as<uint32_t>(), g->vals[1].as<uint32_t>()};
     int res = 0;
-    rc = gvx_sort_pairs(kk, vv, (uint32_t)n, bits, g->sort, fuse_hist, g->stream, g->d_err.as<uint32_t>(), &res,
-                        &g->launches);
+    gvx_status rc = gvx_sort_pairs(kk, vv, (uint32_t)n, bits, g->sort, true, g->stream, g->d_err.as<uint32_t>(), &res,
+                                   &g->launches);
     if (rc) return rc;
     g->sorted_buf = res;
     g->full_group_gen = ~0ull;
@@ -1320,14 +1387,20 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
     return GVX_OK;
 }
 
-static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves)
+// the tables fill_leaf_ranges writes, their ranges to be zeroed before it
+static gvx_status leaf_range_scratch(gvx_grid* g, uint32_t nleaves, ClearList& clear)
 {
     GVX_CK(gvx_ensure(g->leaf_range, (size_t)(nleaves + 1) * sizeof(int2)));
     // (after the octants, and cleared with them: the dense numbers of the leaves, the dense leaves' count)
     const size_t oct_words = (size_t)(nleaves + 1) * 9 + 1;
     GVX_CK(gvx_ensure(g->leaf_oct, oct_words * sizeof(int)));
-    GVX_CK(cudaMemsetAsync(g->leaf_range.p, 0, (size_t)(nleaves + 1) * sizeof(int2), g->stream));
-    GVX_CK(cudaMemsetAsync(g->leaf_oct.p, 0, oct_words * sizeof(int), g->stream));
+    clear.add(g->leaf_range.p, (uint64_t)(nleaves + 1) * 2, 0u);
+    clear.add(g->leaf_oct.p, oct_words, 0u);
+    return GVX_OK;
+}
+
+static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves)
+{
     const bool dense = g->key_shift && g->brick == 8;
     uint32_t* dense_list = nullptr;
     g->leaf_dense = dense ? g->leaf_oct.as<int>() + (size_t)(nleaves + 1) * 8 : nullptr;
@@ -1449,6 +1522,13 @@ static gvx_status grow_nodes(gvx_grid* g, int lev, int64_t cnt)
     return GVX_OK;
 }
 
+// the child lists of levels 1..depth, cnt[l] nodes each, start empty
+static void clear_clists(gvx_grid* g, int depth, const int64_t* cnt, ClearList& clear)
+{
+    for (int l = 1; l <= depth; l++)
+        clear.add(g->clist[l].p, (uint64_t)cnt[l] * g->res[l] * g->res[l] * g->res[l] * 2u, 0xFFFFFFFFu);
+}
+
 // FULL rebuild: ActivateBricksGPU + ActivateExtraBricksGPU semantics
 // A full build between its counts readback being queued and being read: what
 // topo_full_complete needs of topo_full_launch.
@@ -1476,6 +1556,7 @@ struct gvx_topo_staged {
     uint64_t last_gen;  // topo_gen after it
 };
 
+static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpace& ks, FullBuild& fb, ClearList& clear);
 static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
                                       const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback);
 
@@ -1536,31 +1617,22 @@ static gvx_status topo_full_launch(gvx_grid* g, int n, float radius, const float
         fb.mn[a] = mn[a];
         fb.mx[a] = mx[a];
     }
+    ClearList clear;
+    GVX_CK_STATUS(topo_full_scratch(g, n, depth, ks, fb, clear));
+    GVX_CK_STATUS(gvx_clear(clear, g->stream, &g->launches));
     return topo_full_launch_ks(g, n, radius, o, depth, rootpos, ks, fb, true);
 }
 
-// a full build in key space `ks` up to its node counts (d_counts), which are queued for the
-// host when queue_readback
-static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
-                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback)
+// the scratch of a full build in key space `ks` (fb.words0, fb.ud: its sizes), its ranges to be cleared
+static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpace& ks, FullBuild& fb, ClearList& clear)
 {
-    cudaStream_t st = g->stream;
-    const int b = g->brick;
-    const bool extra = radius >= 1.0f;
     const uint32_t words0 = std::max<uint32_t>(1u, (uint32_t)((1ull << ks.total_bits) / 32ull));
-    const uint32_t invalid_key = 1u << ks.total_bits;
-
-    // ---- scratch
     GVX_CK(gvx_ensure(g->d0_bits, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->d0_prefix, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->x0_bits, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->x0_prefix, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->masks, (size_t)std::max(n, 1) * 4));
     GVX_CK(gvx_ensure(g->leaf_key, (size_t)std::max(n, 1) * 4));
-    GVX_CK(cudaMemsetAsync(g->d0_bits.p, 0, (size_t)words0 * 4, st));
-    GVX_CK(cudaMemsetAsync(g->x0_bits.p, 0, (size_t)words0 * 4, st));
-    GVX_CK(cudaMemsetAsync(g->d_counts.p, 0, 64 * sizeof(uint32_t), st));
-
     UpperDesc ud;
     memset(&ud, 0, sizeof(ud));
     ud.nlev = depth - 1;
@@ -1573,10 +1645,29 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
         upper_words += 4u * ud.words[l];
     }
     GVX_CK(gvx_ensure(g->upper, (size_t)std::max<uint32_t>(upper_words, 1u) * 4));
-    if (upper_words) GVX_CK(cudaMemsetAsync(g->upper.p, 0, (size_t)upper_words * 4, st));
+    clear.add(g->d0_bits.p, words0, 0u);
+    clear.add(g->x0_bits.p, words0, 0u);
+    clear.add(g->d_counts.p, 64, 0u);
+    clear.add(g->upper.p, upper_words, 0u);
+    fb.words0 = words0;
+    fb.ud = ud;
+    return sort_points_scratch(g, n, ks, clear);
+}
+
+// a full build in key space `ks` up to its node counts (d_counts), which are queued for the
+// host when queue_readback; its scratch (topo_full_scratch) is cleared
+static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
+                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback)
+{
+    cudaStream_t st = g->stream;
+    const int b = g->brick;
+    const bool extra = radius >= 1.0f;
+    const uint32_t words0 = fb.words0;
+    const uint32_t invalid_key = 1u << ks.total_bits;
+    const UpperDesc& ud = fb.ud;
 
     // ---- one sort of the compact level-0 keys
-    gvx_status rc = sort_points(g, n, o, ks, true);
+    gvx_status rc = sort_points(g, n, o, ks);
     if (rc) return rc;
     const uint32_t* skeys = g->keys[g->sorted_buf].as<uint32_t>();
     const uint32_t* svals = g->vals[g->sorted_buf].as<uint32_t>();
@@ -1627,9 +1718,7 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
         fb.rootpos[a] = rootpos[a];
     }
     fb.ks = ks;
-    fb.words0 = words0;
-    fb.ud = ud;
-    return queue_readback ? readback_start(g, counts, 64 * sizeof(uint32_t), "RebuildTopology") : GVX_OK;
+    return queue_readback ? readback_start(g) : GVX_OK;
 }
 
 static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
@@ -1646,7 +1735,7 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
     const BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
     uint32_t hc[64];
-    gvx_status rc = readback_finish(g, hc, sizeof(hc), "RebuildTopology");
+    gvx_status rc = readback_finish(g, hc, 0, sizeof(hc), "RebuildTopology");
     if (rc) return rc;
     const uint32_t U0 = hc[0], X0 = hc[1];
     uint32_t Ul[GVX_MAXLEV] = {}, Xl[GVX_MAXLEV] = {};
@@ -1667,10 +1756,11 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     rc = grow_nodes(g, depth, 1);
     if (rc) return rc;
     g->count[depth] = 1;
-    for (int l = 1; l <= depth; l++) {
-        const size_t vc = (size_t)g->res[l] * g->res[l] * g->res[l];
-        GVX_CK(cudaMemsetAsync(g->clist[l].p, 0xFF, (size_t)g->count[l] * vc * sizeof(uint64_t), st));
-    }
+    const uint32_t L0 = U0 + X0;
+    ClearList clear;
+    clear_clists(g, depth, g->count, clear);
+    GVX_CK_STATUS(leaf_range_scratch(g, L0, clear));
+    GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
     size_t list_words = (size_t)X0 + 1;
     for (int l = 1; l < depth; l++) list_words += (size_t)Ul[l] + Xl[l];
     GVX_CK(gvx_ensure(g->lists, list_words * 4));
@@ -1750,7 +1840,6 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     g->lookup.b_offset_p = nullptr;
     g->lookup.cap = 0;
     g->lookup_valid = true;
-    const uint32_t L0 = U0 + X0;
     GVX_CK(gvx_ensure(g->nbr, (size_t)std::max<uint32_t>(L0, 1u) * 27 * sizeof(int)));
     if (L0) {
         k_neighbors<<<blocks_for((uint64_t)L0 * 27, 256), 256, 0, st>>>(g->leaf_key.as<uint32_t>(), dc_host(L0), g->lookup,
@@ -1825,7 +1914,10 @@ static gvx_status build_active_lookup(gvx_grid* g, const KeySpace& ks, uint32_t 
     GVX_CK(gvx_ensure(g->lk_prefix, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->remap, (size_t)L0 * 4 + 4));
     GVX_CK(gvx_ensure(g->leaf_key, (size_t)L0 * 4 + 4));
-    GVX_CK(cudaMemsetAsync(g->lk_bits.p, 0, (size_t)words0 * 4, st));
+    ClearList clear;
+    clear.add(g->lk_bits.p, words0, 0u);
+    GVX_CK_STATUS(leaf_range_scratch(g, L0, clear));
+    GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
     uint32_t* counts = g->d_counts.as<uint32_t>();
     if (L0) {
         k_node_bits<<<blocks_for(L0, 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(), L0, ks, 0, g->range[0],
@@ -1862,7 +1954,7 @@ static gvx_status build_active_lookup(gvx_grid* g, const KeySpace& ks, uint32_t 
     if (rc) return rc;
     if (readback == kReadUsed) {
         uint32_t used = 0;
-        gvx_status rc = readback_checked(g, &used, counts + kCntActive, 4, "RebuildTopology");
+        gvx_status rc = readback_checked(g, &used, kCntActive, 4, "RebuildTopology");
         if (rc) return rc;
         g->used_leaves = used;
         return GVX_OK;
@@ -1935,10 +2027,11 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
     GVX_CK(gvx_ensure(g->inc0, (size_t)words0 * 16));
     GVX_CK(gvx_ensure(g->masks, (size_t)std::max(n, 1) * 4));
     GVX_CK(gvx_ensure(g->lists, (size_t)std::max(n, 1) * 4));
-    GVX_CK(cudaMemsetAsync(g->d0_bits.p, 0, (size_t)words0 * 4, st));
-    GVX_CK(cudaMemsetAsync(g->x0_bits.p, 0, (size_t)words0 * 4, st));
-    GVX_CK(cudaMemsetAsync(g->inc0.p, 0, (size_t)words0 * 16, st));
-    GVX_CK(cudaMemsetAsync(g->d_counts.p, 0, 64 * sizeof(uint32_t), st));
+    ClearList clear;
+    clear.add(g->d0_bits.p, words0, 0u);
+    clear.add(g->x0_bits.p, words0, 0u);
+    clear.add(g->inc0.p, (uint64_t)words0 * 4u, 0u);
+    clear.add(g->d_counts.p, 64, 0u);
     // per upper level: D (touched via direct leaves), A (via box leaves), L bits, L prefix, N bits, N prefix
     UpperDesc ud;
     memset(&ud, 0, sizeof(ud));
@@ -1951,13 +2044,15 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
         upper_words += 6u * ud.words[l];
     }
     GVX_CK(gvx_ensure(g->upper, (size_t)std::max<uint32_t>(upper_words, 1u) * 4));
-    if (upper_words) GVX_CK(cudaMemsetAsync(g->upper.p, 0, (size_t)upper_words * 4, st));
+    clear.add(g->upper.p, upper_words, 0u);
+    GVX_CK_STATUS(sort_points_scratch(g, n, ks, clear));
+    GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
     uint32_t* upper = g->upper.as<uint32_t>();
     uint32_t* counts = g->d_counts.as<uint32_t>();
     uint32_t* err = g->d_err.as<uint32_t>();
 
     // ---- touched cells: the points' leaves (D0) and their boxes [int(p)-r, int(p)+r] (X0), PT.cuh:420-465
-    gvx_status rc = sort_points(g, n, o, ks, true);
+    gvx_status rc = sort_points(g, n, o, ks);
     if (rc) return rc;
     const uint32_t* skeys = g->keys[g->sorted_buf].as<uint32_t>();
     const uint32_t* svals = g->vals[g->sorted_buf].as<uint32_t>();
@@ -2029,7 +2124,7 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
 
     // ---- new-node counts to the host
     uint32_t hc[64];
-    rc = readback_checked(g, hc, counts, sizeof(hc), "RebuildTopology");
+    rc = readback_checked(g, hc, 0, sizeof(hc), "RebuildTopology");
     if (rc) return rc;
     uint32_t nnew[GVX_MAXLEV] = {};
     uint64_t total_new = 0;
@@ -2048,6 +2143,7 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
                                                                  d0.bits, g->x0_bits.as<uint32_t>(), accum ? 1 : 0);
         g->launches++;
         // ---- pools grow, keeping their nodes and child lists; new lists start empty
+        ClearList grown;
         for (int l = 0; l < depth; l++) {
             if (!nnew[l]) continue;
             const size_t cnt = (size_t)old[l] + nnew[l];
@@ -2057,9 +2153,10 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
                 const size_t vb = (size_t)g->res[l] * g->res[l] * g->res[l] * sizeof(uint64_t);
                 rc = grow_keep(g, g->clist[l], cnt * vb, (size_t)old[l] * vb);
                 if (rc) return rc;
-                GVX_CK(cudaMemsetAsync((char*)g->clist[l].p + (size_t)old[l] * vb, 0xFF, (size_t)nnew[l] * vb, st));
+                grown.add((char*)g->clist[l].p + (size_t)old[l] * vb, (uint64_t)nnew[l] * (vb / 4), 0xFFFFFFFFu);
             }
         }
+        GVX_CK_STATUS(gvx_clear(grown, st, &g->launches));
         // ---- sorted keys of the new nodes
         GVX_CK(gvx_ensure(g->lists, (size_t)(total_new + 1) * 4));
         const uint32_t* nl[GVX_MAXLEV] = {};
@@ -2214,8 +2311,9 @@ static gvx_status rebuild_begin(gvx_grid* g, int n, float radius, const float or
     // accumulating build is reported by this build's first readback)
 
     // ---- GetBoundingBox: one reduction, 24 bytes to the host
-    uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
-    GVX_CK(cudaMemcpyAsync(g->d_bbox.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
+    ClearList clear;
+    clear_bboxes(g, clear);
+    GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
     // a multiple of 3 blocks (of 256 threads): the packed path needs the thread count divisible by 3
     const unsigned bb = (std::min(blocks_for(n, 256), 152u * 8u) + 2u) / 3u * 3u;
     k_bbox<<<bb, 256, 0, st>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, o[0], o[1], o[2],
@@ -2224,14 +2322,12 @@ static gvx_status rebuild_begin(gvx_grid* g, int n, float radius, const float or
     // an incremental build also needs the box of the active leaves: same readback
     const bool maybe_incremental = g->root_level >= 0 && !g->rebuild_topo && mode != GVX_TOPO_FULL;
     int* act_dev = g->d_bbox.as<int>() + 8;
-    k_bounds_init<<<1, 32, 0, st>>>(act_dev);
-    g->launches++;
     if (maybe_incremental && g->count[0] > 0) {
         k_leaf_bounds<<<blocks_for(g->count[0], 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(),
                                                                      (uint32_t)g->count[0], g->range[0], act_dev);
         g->launches++;
     }
-    return readback_start(g, g->d_bbox.p, 14 * sizeof(uint32_t), "GetBoundingBox");
+    return readback_start(g);
 }
 
 // the rest of RebuildTopology, from the bounding box (and active-leaf box) read
@@ -2314,7 +2410,7 @@ gvx_status gvx_topo_stage2(gvx_grid* g)
 {
     gvx_topo_staged& S = *g->staged;
     uint32_t hb[14];
-    gvx_status rc = readback_finish(g, hb, sizeof(hb), "GetBoundingBox");
+    gvx_status rc = readback_finish(g, hb, kReadBbox, sizeof(hb), "GetBoundingBox");
     if (rc) return rc;
     return rebuild_after_bbox(g, S.n, S.radius, nullptr, S.mode, S.min_depth, hb, &S.fb, &S.pending);
 }
@@ -2357,7 +2453,7 @@ void gvx_topo_staged_free(gvx_grid* g)
 // unplanned build sets it.  Otherwise the planned build is void and the caller
 // builds the grid again without a plan.
 
-enum { kRecCounts = 0, kRecBbox = 64, kRecErr = 80, kRecWords = 96 };
+enum { kRecCounts = 0, kRecBbox = kReadBbox, kRecErr = kReadErr, kRecWords = kReadWords };
 enum { kCntSlots = 56 };  // d_counts slot of a planned UpdateAtlas's slot count
 
 struct gvx_topo_plan {
@@ -2441,13 +2537,6 @@ static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuil
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
     const BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
 
-    for (int l = 0; l < depth; l++) GVX_CK_STATUS(grow_nodes(g, l, P.cap[l]));
-    GVX_CK_STATUS(grow_nodes(g, depth, 1));
-    for (int l = 1; l <= depth; l++) {
-        const size_t vc = (size_t)g->res[l] * g->res[l] * g->res[l];
-        const size_t cnt = l < depth ? P.cap[l] : 1;
-        GVX_CK(cudaMemsetAsync(g->clist[l].p, 0xFF, cnt * vc * sizeof(uint64_t), st));
-    }
     // lists: X0 (cap0), then D_l and X_l (cap_l each) per upper level
     size_t list_words = cap0;
     for (int l = 1; l < depth; l++) list_words += 2 * (size_t)P.cap[l];
@@ -2529,6 +2618,17 @@ static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuil
     return fill_leaf_ranges(g, cap0);
 }
 
+// UpdateAtlas where every leaf of the pool is active: leaf i in slot i, the other slots free (atlas map -1)
+static gvx_status atlas_all(gvx_grid* g, DevCount nl, int64_t slots, uint32_t* nslots)
+{
+    k_atlas_all<<<blocks_for((uint64_t)std::max<int64_t>(slots, 1), 256), 256, 0, g->stream>>>(
+        g->nodes[0].as<GvxNode>(), nl, (uint32_t)slots, g->sub[0], g->sub[1], g->P, g->apron, g->leaf_slot.as<int>(),
+        g->slot_leaf.as<int>(), g->amap.as<int4>(), nslots);
+    g->launches++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
+}
+
 // UpdateAtlas of a planned build: slots in pool order over the leaf capacity, the slot count
 // to d_counts[kCntSlots]
 static gvx_status plan_atlas(gvx_grid* g, const gvx_topo_plan& P)
@@ -2538,23 +2638,10 @@ static gvx_status plan_atlas(gvx_grid* g, const gvx_topo_plan& P)
     const DevCount nl = dc_dev(g->d_counts.as<uint32_t>(), 0, 1, cap0);
     GVX_CK_STATUS(gvx_grow_atlas(g, cap0));
     const int64_t slots = (int64_t)g->sub[0] * g->sub[1] * g->sub[2];
-    const uint32_t fw = cap0 / 32u + 1u;
     GVX_CK(gvx_ensure(g->amap, (size_t)slots * sizeof(int4)));
-    GVX_CK(cudaMemsetAsync(g->amap.p, 0xFF, (size_t)slots * sizeof(int4), st));
     GVX_CK(gvx_ensure(g->leaf_slot, (size_t)cap0 * 4));
     GVX_CK(gvx_ensure(g->slot_leaf, (size_t)std::max<int64_t>(slots, 1) * 4));
-    GVX_CK(gvx_ensure(g->bm_a, (size_t)fw * 4));
-    GVX_CK(gvx_ensure(g->bm_a_prefix, (size_t)fw * 4));
-    GVX_CK(cudaMemsetAsync(g->bm_a.p, 0, (size_t)fw * 4, st));
-    k_flag_bits<<<blocks_for(cap0, 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(), nl, g->bm_a.as<uint32_t>());
-    g->launches++;
-    GVX_CK_STATUS(gvx_bitmap_prefix(g->bm_a.as<uint32_t>(), g->bm_a_prefix.as<uint32_t>(), fw,
-                                    g->d_counts.as<uint32_t>() + kCntSlots, g->tmp_scan, st, &g->launches));
-    k_atlas_assign<<<blocks_for(cap0, 256), 256, 0, st>>>(
-        g->nodes[0].as<GvxNode>(), nl, g->bm_a.as<uint32_t>(), g->bm_a_prefix.as<uint32_t>(), g->sub[0], g->sub[1],
-        g->P, g->apron, g->leaf_slot.as<int>(), g->slot_leaf.as<int>(), g->amap.as<int4>());
-    g->launches++;
-    return GVX_OK;
+    return atlas_all(g, nl, slots, g->d_counts.as<uint32_t>() + kCntSlots);  // a full build: every leaf is active
 }
 
 gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool frame)
@@ -2571,16 +2658,28 @@ gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool fr
     GVX_CK_STATUS(ensure_grid_scratch(g));
     P.enqueued = false;
 
+    // ---- everything the build clears, sized by the capacities
+    GVX_CK(gvx_ensure(g->leaf_key, ((size_t)std::max<uint32_t>(cap0, (uint32_t)n) + 1) * 4));
+    FullBuild fb{};
+    ClearList clear;
+    clear_bboxes(g, clear);
+    GVX_CK_STATUS(topo_full_scratch(g, n, depth, P.fb.ks, fb, clear));
+    int64_t cap[GVX_MAXLEV] = {};
+    for (int l = 0; l <= depth; l++) {
+        cap[l] = l < depth ? P.cap[l] : 1;
+        GVX_CK_STATUS(grow_nodes(g, l, cap[l]));
+    }
+    clear_clists(g, depth, cap, clear);
+    GVX_CK_STATUS(leaf_range_scratch(g, cap0, clear));
+    GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
+
     // ---- GetBoundingBox (read by gvx_topo_plan_finish)
-    k_bbox_reset<<<1, 32, 0, st>>>(g->d_bbox.as<uint32_t>());
     const unsigned bb = (std::min(blocks_for(n, 256), 152u * 8u) + 2u) / 3u * 3u;
     k_bbox<<<bb, 256, 0, st>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, 0.f, 0.f, 0.f,
                                g->d_bbox.as<uint32_t>(), g->d_err.as<uint32_t>());
-    g->launches += 2;
+    g->launches++;
 
     // ---- the full build in the plan's key space, sized by the capacities
-    GVX_CK(gvx_ensure(g->leaf_key, ((size_t)std::max<uint32_t>(cap0, (uint32_t)n) + 1) * 4));
-    FullBuild fb{};
     GVX_CK_STATUS(topo_full_launch_ks(g, n, P.fb.radius, o, depth, P.fb.rootpos, P.fb.ks, fb, false));
     P.fb.words0 = fb.words0;
     P.fb.ud = fb.ud;
@@ -2598,9 +2697,8 @@ gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool fr
     g->lookup.cap = 0;
     g->lookup_valid = false;
     if (rc) return rc;
-    GVX_CK(cudaMemcpyAsync(P.rec + kRecCounts, g->d_counts.p, 64 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    GVX_CK(cudaMemcpyAsync(P.rec + kRecBbox, g->d_bbox.p, 6 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    if (!frame) GVX_CK_STATUS(gvx_topo_plan_record_error(g, st));  // (a frame records it after its splat)
+    // (with the error word; a frame records that again after its splat)
+    GVX_CK(cudaMemcpyAsync(P.rec, g->d_counts.p, kReadWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GVX_CK(cudaGetLastError());
     P.sorted_buf = g->sorted_buf;
     P.enqueued = true;
@@ -2770,7 +2868,7 @@ gvx_status gvx_topo_rebuild(gvx_grid* g, int n, float radius, const float orig[3
     rc = rebuild_begin(g, n, radius, orig, mode);
     if (rc) return rc;
     uint32_t hb[14];
-    rc = readback_finish(g, hb, sizeof(hb), "GetBoundingBox");
+    rc = readback_finish(g, hb, kReadBbox, sizeof(hb), "GetBoundingBox");
     if (rc) return rc;
     rc = rebuild_after_bbox(g, n, radius, orig, mode, min_depth, hb, nullptr, nullptr);
     // a full build plans the next ones (any points of the same count and radius)
@@ -2884,13 +2982,19 @@ gvx_status gvx_topo_update_atlas(gvx_grid* g)
     const uint32_t L0 = (uint32_t)g->count[0];
     const uint32_t fw = std::max<uint32_t>(1u, (L0 + 31u) / 32u);
     GVX_CK(gvx_ensure(g->amap, (size_t)slots * sizeof(int4)));
-    GVX_CK(cudaMemsetAsync(g->amap.p, 0xFF, (size_t)slots * sizeof(int4), st));
     GVX_CK(gvx_ensure(g->leaf_slot, (size_t)std::max<uint32_t>(L0, 1u) * 4));
     GVX_CK(gvx_ensure(g->slot_leaf, (size_t)std::max<int64_t>(slots, 1) * 4));
-    GVX_CK(gvx_ensure(g->bm_a, (size_t)fw * 4));
-    GVX_CK(gvx_ensure(g->bm_a_prefix, (size_t)fw * 4));
-    GVX_CK(cudaMemsetAsync(g->bm_a.p, 0, (size_t)fw * 4, st));
-    if (L0) {
+    if (used == g->count[0]) {
+        GVX_CK_STATUS(atlas_all(g, dc_host(L0), slots, nullptr));
+    } else {
+        GVX_CK(gvx_ensure(g->bm_a, (size_t)fw * 4));
+        GVX_CK(gvx_ensure(g->bm_a_prefix, (size_t)fw * 4));
+        ClearList clear;
+        clear.add(g->amap.p, (uint64_t)slots * 4u, 0xFFFFFFFFu);
+        clear.add(g->bm_a.p, fw, 0u);
+        GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
+    }
+    if (L0 && used != g->count[0]) {
         k_flag_bits<<<blocks_for(L0, 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(), dc_host(L0), g->bm_a.as<uint32_t>());
         g->launches++;
         rc = gvx_bitmap_prefix(g->bm_a.as<uint32_t>(), g->bm_a_prefix.as<uint32_t>(), fw, nullptr, g->tmp_scan, st,
@@ -2927,20 +3031,30 @@ gvx_status gvx_topo_update_atlas(gvx_grid* g)
 // them.  The result is read when the host asks for it (gvx_get_info), so
 // FinishTopology adds no synchronisation.  host_stage: ints [0..2] min,
 // [3..5] max, [6..8] res max.
-__global__ void k_bounds_seed(const GvxNode* __restrict__ nodes, uint32_t n, int* out, int reset_res_max)
+// One launch: the blocks lower and raise the accumulators (ints [10..15]), and the last of them to get there
+// (counter [9]) writes the result and leaves accumulators and counter as it found them.
+__global__ void k_compute_bounds(const GvxNode* __restrict__ nodes, uint32_t n, int range, int* out, int reset_res_max)
 {
+    leaf_bounds(nodes, n, range, out + 10);
+    __shared__ bool s_last;
+    if (threadIdx.x < 6) __threadfence();  // (the threads that hold the block's atomics)
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd((unsigned int*)out + 9, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (!s_last || threadIdx.x >= 3) return;
+    __threadfence();
     const int a = threadIdx.x;
-    if (a < 3) {
-        out[a] = n ? nodes[0].pos[a] : 0x7FFFFFFF;
-        out[3 + a] = n ? nodes[0].pos[a] : (int)0x80000000;
-        if (reset_res_max) out[6 + a] = 0;
-    }
-}
-
-__global__ void k_bounds_res_max(int* out, uint32_t n)
-{
-    const int a = threadIdx.x;
-    if (a < 3 && n) out[6 + a] = max(out[6 + a], out[3 + a] - out[a]);
+    volatile int* acc = out + 10;
+    int mn = n ? nodes[0].pos[a] : 0x7FFFFFFF, mx = n ? nodes[0].pos[a] : (int)0x80000000;
+    mn = min(mn, acc[a]);
+    mx = max(mx, acc[3 + a]);
+    out[a] = mn;
+    out[3 + a] = mx;
+    const int rm = reset_res_max ? 0 : out[6 + a];
+    out[6 + a] = n ? max(rm, mx - mn) : rm;
+    acc[a] = 0x7FFFFFFF;
+    acc[3 + a] = (int)0x80000000;
+    if (a == 0) out[9] = 0;
 }
 
 gvx_status gvx_topo_compute_bounds(gvx_grid* g)
@@ -2949,17 +3063,18 @@ gvx_status gvx_topo_compute_bounds(gvx_grid* g)
     gvx_status rc = ensure_grid_scratch(g);
     if (rc) return rc;
     const uint32_t L0 = (uint32_t)g->count[0];
-    GVX_CK(gvx_ensure(g->host_stage, 64));
-    k_bounds_seed<<<1, 32, 0, g->stream>>>(g->nodes[0].as<GvxNode>(), L0, g->host_stage.as<int>(),
-                                          g->vox_res_max_reset ? 1 : 0);
+    if (!g->host_stage.p) {
+        GVX_CK(gvx_ensure(g->host_stage, 64));
+        ClearList clear;
+        clear.add(g->host_stage.p, 10, 0u);
+        clear.add(g->host_stage.as<int>() + 10, 3, 0x7FFFFFFFu);
+        clear.add(g->host_stage.as<int>() + 13, 3, 0x80000000u);
+        GVX_CK_STATUS(gvx_clear(clear, g->stream, &g->launches));
+    }
+    k_compute_bounds<<<blocks_for(std::max(L0, 1u), 256), 256, 0, g->stream>>>(
+        g->nodes[0].as<GvxNode>(), L0, g->range[0], g->host_stage.as<int>(), g->vox_res_max_reset ? 1 : 0);
     g->launches++;
     g->vox_res_max_reset = false;
-    if (L0) {
-        k_leaf_bounds<<<blocks_for(L0, 256), 256, 0, g->stream>>>(g->nodes[0].as<GvxNode>(), L0, g->range[0],
-                                                                   g->host_stage.as<int>());
-        k_bounds_res_max<<<1, 32, 0, g->stream>>>(g->host_stage.as<int>(), L0);
-        g->launches += 2;
-    }
     GVX_CK(cudaGetLastError());
     g->bounds_pending = true;
     return GVX_OK;
@@ -2999,7 +3114,11 @@ gvx_status gvx_topo_group_points(gvx_grid* g, int n, const float trans[3])
         return GVX_OK;
     gvx_status rc = ensure_grid_scratch(g);
     if (rc) return rc;
-    rc = sort_points(g, n, t, g->lookup.ks, true);
+    ClearList clear;
+    GVX_CK_STATUS(sort_points_scratch(g, n, g->lookup.ks, clear));
+    GVX_CK_STATUS(leaf_range_scratch(g, (uint32_t)g->count[0], clear));
+    GVX_CK_STATUS(gvx_clear(clear, g->stream, &g->launches));
+    rc = sort_points(g, n, t, g->lookup.ks);
     if (rc) return rc;
     rc = fill_leaf_ranges(g, (uint32_t)g->count[0]);
     if (rc) return rc;
