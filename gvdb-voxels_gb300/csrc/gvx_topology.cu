@@ -291,94 +291,42 @@ struct UpperDesc {
     int tshift[GVX_MAXLEV];
 };
 
-// parents of direct leaves -> D_l bitmaps
-__global__ void k_upper_direct(const uint32_t* __restrict__ dlist, const uint32_t* __restrict__ count, KeySpace ks,
-                               UpperDesc ud, uint32_t* upper)
+// parents of the cells of a word of a level-0 bitmap -> a bitmap per upper level.  Neighbouring cells share
+// their parents: a parent met again ends the walk up, and one whose bit is set is not set again (atomics on
+// the few words of the top levels, one after the other, took most of 13 us in a frame of a fused scene).
+__device__ __forceinline__ void upper_word(uint32_t bits, uint32_t w, const KeySpace& ks, const UpperDesc& ud,
+                                           uint32_t* upper, int which)
 {
-    // grid-stride over the leaves in whole warps (the match_any below takes every lane)
-    const uint32_t cnt = *count, stride = gridDim.x * blockDim.x;
-    for (uint32_t j0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); j0 < cnt; j0 += stride) {
-        const uint32_t j = j0 + (threadIdx.x & 31u);
-        const bool valid = j < cnt;
-        int c[3] = {0, 0, 0};
-        if (valid) ks_unpack(ks, dlist[j], 0, c);
-        for (int l = 1; l <= ud.nlev; l++) {
-            const int t = ud.tshift[l];
-            const uint32_t k = valid ? ks_pack(ks, c[0] >> t, c[1] >> t, c[2] >> t, t) : 0xFFFFFFFFu;
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, k);
-            if (valid && (threadIdx.x & 31) == __ffs(peers) - 1)
-                atomicOr(&upper[ud.off[l] + (k >> 5)], 1u << (k & 31));
-        }
-    }
-}
-
-// parents of extra leaves -> A_l bitmaps (X_l = A_l & ~D_l later)
-__global__ void k_upper_extra(const uint32_t* __restrict__ x0bits, uint32_t words, KeySpace ks, UpperDesc ud,
-                              uint32_t* upper)
-{
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= words) return;
-    uint32_t bits = x0bits[w];
     uint32_t last[GVX_MAXLEV];
+#pragma unroll
     for (int l = 0; l < GVX_MAXLEV; l++) last[l] = 0xFFFFFFFFu;
     while (bits) {
         const int b = __ffs(bits) - 1;
         bits &= bits - 1u;
         int c[3];
         ks_unpack(ks, w * 32u + (uint32_t)b, 0, c);
-        for (int l = 1; l <= ud.nlev; l++) {
+#pragma unroll
+        for (int l = 1; l < GVX_MAXLEV; l++) {
+            if (l > ud.nlev) break;
             const int t = ud.tshift[l];
             const uint32_t k = ks_pack(ks, c[0] >> t, c[1] >> t, c[2] >> t, t);
-            if (k == last[l]) continue;
+            if (k == last[l]) break;  // (and its parents)
             last[l] = k;
-            atomicOr(&upper[ud.off[l] + ud.words[l] + (k >> 5)], 1u << (k & 31));
+            uint32_t* p = &upper[ud.off[l] + (which ? ud.words[l] : 0u) + (k >> 5)];
+            if (!((*(volatile uint32_t*)p >> (k & 31)) & 1u)) atomicOr(p, 1u << (k & 31));
         }
     }
 }
 
-// small bitmaps: one block per (level, D|X); X = A & ~D first; exclusive
-// prefix popcounts, total -> counts[2 + 2*(l-1) + which]
-__global__ void k_prefix_upper(UpperDesc ud, uint32_t* upper, uint32_t* counts)
+// D_l: parents of the leaves with points; A_l: of the box leaves (x0bits, where there are any)
+__global__ void k_upper_bits(const uint32_t* __restrict__ d0bits, const uint32_t* __restrict__ x0bits, uint32_t words,
+                             KeySpace ks, UpperDesc ud, uint32_t* upper)
 {
-    const int l = 1 + blockIdx.x / 2, which = blockIdx.x & 1;
-    if (l > ud.nlev) return;
-    const uint32_t words = ud.words[l];
-    uint32_t* D = upper + ud.off[l];
-    uint32_t* B = upper + ud.off[l] + (which ? words : 0u);
-    uint32_t* pre = upper + ud.off[l] + 2u * words + (which ? words : 0u);
-    __shared__ uint32_t s_w[32];
-    __shared__ uint32_t s_carry;
-    if (threadIdx.x == 0) s_carry = 0u;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (uint32_t base = 0; base < words; base += blockDim.x) {
-        const uint32_t w = base + threadIdx.x;
-        uint32_t v = 0u;
-        if (w < words) {
-            uint32_t bits = B[w];
-            if (which) {
-                bits &= ~D[w];
-                B[w] = bits;
-            }
-            v = __popc(bits);
-        }
-        uint32_t x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) s_w[warp] = x;
-        __syncthreads();
-        uint32_t wp = 0u;
-        for (int i = 0; i < warp; i++) wp += s_w[i];
-        uint32_t tot = 0u;
-        for (int i = 0; i < nw; i++) tot += s_w[i];
-        if (w < words) pre[w] = s_carry + wp + x - v;
-        __syncthreads();
-        if (threadIdx.x == 0) s_carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) counts[2 + 2 * (l - 1) + which] = s_carry;
+    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= words) return;
+    const uint32_t d = d0bits[w], x = x0bits ? x0bits[w] : 0u;
+    upper_word(d, w, ks, ud, upper, 0);
+    upper_word(x, w, ks, ud, upper, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -437,12 +385,51 @@ static void clear_bboxes(gvx_grid* g, ClearList& c)
     c.add(b + 11, 3, 0x80000000u);
 }
 
-// generic exclusive prefix of popcounts over a bitmap (reduce, scan, apply)
+// ---------------------------------------------------------------------------
+// Exclusive prefix sums of several arrays in one go (of the popcounts of bitmap words, or of the words): a
+// job each.  A job's word may be put together from bitmaps, (src | plus) & ~minus, and is stored then (store
+// may be src: the value is the same again).  With `list` the set bits' keys, in order, go there (cap at
+// most), and zero[0 .. keys) is cleared.
+//
+// Up to 32 blocks of 1024 words a job (a key space of 2^20 leaves), one launch does it: a block sums the
+// words before its own by itself, 31 loads a thread at most, which takes less than the launch that would
+// have summed them (4 us of the stream's time; with the list's, a third launch: 12 us -> 4 for 2^16 leaves).
+// Above, a launch sums the blocks first: those sums would be read 32 times and more.
 namespace {
-constexpr int kPfxThreads = 256;
-constexpr int kPfxPerThread = 16;
-constexpr uint32_t kPfxChunk = kPfxThreads * kPfxPerThread;
+struct PfxJob {
+    const uint32_t *src, *plus, *minus;
+    uint32_t* store;
+    uint32_t* prefix;
+    uint32_t words;
+    uint32_t* total;
+    uint32_t* list;
+    uint32_t cap;
+    uint32_t* zero;
+    uint32_t sums;  // where its block sums start (two launches)
+};
+struct PfxJobs {
+    static constexpr int kMax = 2 * GVX_MAXLEV + 1;
+    int n = 0;
+    PfxJob j[kMax];
+    PfxJob& add(const uint32_t* src, uint32_t* prefix, uint32_t words, uint32_t* total)
+    {
+        PfxJob& q = j[n++];
+        q = PfxJob{src, nullptr, nullptr, nullptr, prefix, words, total, nullptr, 0xFFFFFFFFu, nullptr, 0u};
+        return q;
+    }
+};
+constexpr uint32_t kPfxSelf = 32;
+constexpr int kPfxThreads = 256, kPfxPer = 16, kPfxSelfThreads = 1024;
+constexpr uint32_t kPfxChunk = kPfxThreads * kPfxPer;
 }  // namespace
+
+__device__ __forceinline__ uint32_t pfx_word(const PfxJob& q, uint32_t w)
+{
+    uint32_t v = q.src[w];
+    if (q.plus) v |= q.plus[w];
+    if (q.minus) v &= ~q.minus[w];
+    return v;
+}
 
 // POPC: the scanned values are the popcounts of bitmap words, else the words themselves
 template <bool POPC>
@@ -451,71 +438,78 @@ __device__ __forceinline__ uint32_t pfx_value(uint32_t v)
     return POPC ? (uint32_t)__popc(v) : v;
 }
 
-// per block of kPfxChunk words: the sum (all loads issued before any add: the block's chunk is
-// one round trip, not kPfxPerThread)
-template <bool POPC>
-__global__ void __launch_bounds__(kPfxThreads) k_pfx_reduce(const uint32_t* __restrict__ bits, uint32_t words,
-                                                            uint32_t* block_sums)
+// the sum of v over the block, in every thread
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_w)
 {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = v;
+    __syncthreads();
+    uint32_t t = 0u;
+    for (int i = 0; i < THREADS / 32; i++) t += s_w[i];
+    return t;
+}
+
+// per block of kPfxChunk words: the sum (all loads issued before any add: the block's chunk is
+// one round trip, not kPfxPer)
+template <bool POPC>
+__global__ void __launch_bounds__(kPfxThreads) k_pfx_reduce(PfxJobs jobs, uint32_t* sums)
+{
+    const PfxJob& q = jobs.j[blockIdx.y];
     const uint32_t base = blockIdx.x * kPfxChunk + threadIdx.x;
-    uint32_t v[kPfxPerThread];
+    if (blockIdx.x * kPfxChunk >= q.words) return;
+    uint32_t v[kPfxPer];
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) {
+    for (int k = 0; k < kPfxPer; k++) {
         const uint32_t w = base + (uint32_t)k * kPfxThreads;
-        v[k] = w < words ? bits[w] : 0u;
+        v[k] = w < q.words ? pfx_word(q, w) : 0u;
     }
     uint32_t s = 0u;
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) s += pfx_value<POPC>(v[k]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    __shared__ uint32_t ws[kPfxThreads / 32];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0u;
-        for (int i = 0; i < kPfxThreads / 32; i++) t += ws[i];
-        block_sums[blockIdx.x] = t;
-    }
+    for (int k = 0; k < kPfxPer; k++) s += pfx_value<POPC>(v[k]);
+    __shared__ uint32_t s_w[kPfxThreads / 32];
+    s = block_sum<kPfxThreads>(s, s_w);
+    if (threadIdx.x == 0) sums[q.sums + blockIdx.x] = s;
 }
 
 // the block's chunk in and out through shared memory (coalesced global loads and stores; index i
-// of the chunk at i + i/32, so that a thread's kPfxPerThread consecutive values and the warps'
-// strided rows are both free of bank conflicts), each thread scanning kPfxPerThread consecutive
-// values after the block offset from the earlier blocks' sums
-template <bool POPC>
-__global__ void __launch_bounds__(kPfxThreads) k_pfx_apply(const uint32_t* __restrict__ bits, uint32_t words,
-                                                           const uint32_t* __restrict__ block_sums, uint32_t* prefix,
-                                                           uint32_t* total)
+// of the chunk at i + i/32, so that a thread's PER consecutive values and the warps'
+// strided rows are both free of bank conflicts), each thread scanning PER consecutive
+// values after what comes before the block: SELF sums the words, else the earlier blocks' sums are added up
+template <bool POPC, int THREADS, int PER, bool SELF>
+__global__ void __launch_bounds__(THREADS) k_pfx_apply(PfxJobs jobs, const uint32_t* __restrict__ sums)
 {
-    __shared__ uint32_t s_v[kPfxChunk + kPfxChunk / 32];
-    __shared__ uint32_t s_w[kPfxThreads / 32];
-    __shared__ uint32_t s_off;
-    const uint32_t cbase = blockIdx.x * kPfxChunk;
+    constexpr uint32_t CHUNK = THREADS * PER;
+    __shared__ uint32_t s_v[CHUNK + CHUNK / 32];
+    __shared__ uint32_t s_w[THREADS / 32];
+    const PfxJob& q = jobs.j[blockIdx.y];
+    const uint32_t cbase = blockIdx.x * CHUNK;
+    if (cbase >= q.words) return;
+    uint32_t v[PER];
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) {
-        const uint32_t i = (uint32_t)k * kPfxThreads + threadIdx.x, w = cbase + i;
-        s_v[i + (i >> 5)] = w < words ? pfx_value<POPC>(bits[w]) : 0u;
+    for (int k = 0; k < PER; k++) {
+        const uint32_t w = cbase + (uint32_t)k * THREADS + threadIdx.x;
+        v[k] = w < q.words ? pfx_word(q, w) : 0u;
     }
-    {
-        uint32_t o = 0u;
-        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += kPfxThreads) o += block_sums[i];
-        for (int k = 16; k > 0; k >>= 1) o += __shfl_xor_sync(0xFFFFFFFFu, o, k);
-        if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = o;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t t = 0u;
-            for (int k = 0; k < kPfxThreads / 32; k++) t += s_w[k];
-            s_off = t;
-            if (total && blockIdx.x + 1 == gridDim.x) *total = t + block_sums[blockIdx.x];
-        }
-        __syncthreads();
+    uint32_t before = 0u;
+    if (SELF) {
+#pragma unroll 8
+        for (uint32_t w = threadIdx.x; w < cbase; w += THREADS) before += pfx_value<POPC>(pfx_word(q, w));
+    } else {
+        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += THREADS) before += sums[q.sums + i];
     }
-    const uint32_t block_off = s_off;
-    uint32_t cnt[kPfxPerThread];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = (uint32_t)k * THREADS + threadIdx.x;
+        s_v[i + (i >> 5)] = pfx_value<POPC>(v[k]);
+    }
+    before = block_sum<THREADS>(before, s_w);
+    uint32_t cnt[PER];
     uint32_t s = 0u;
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) {
-        const uint32_t i = threadIdx.x * kPfxPerThread + k;
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = threadIdx.x * PER + k;
         cnt[k] = s_v[i + (i >> 5)];
         s += cnt[k];
     }
@@ -528,31 +522,57 @@ __global__ void __launch_bounds__(kPfxThreads) k_pfx_apply(const uint32_t* __res
     __syncthreads();  // s_w is reused
     if (lane == 31) s_w[warp] = x;
     __syncthreads();
-    uint32_t run = block_off + x - s;
+    uint32_t run = before + x - s;
     for (int k = 0; k < warp; k++) run += s_w[k];
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) {
-        const uint32_t i = threadIdx.x * kPfxPerThread + k;
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = threadIdx.x * PER + k;
         s_v[i + (i >> 5)] = run;
         run += cnt[k];
     }
+    // (the last thread of the last block: the words past the end count nothing)
+    if (q.total && threadIdx.x == THREADS - 1 && q.words - cbase <= CHUNK) *q.total = run;
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kPfxPerThread; k++) {
-        const uint32_t i = (uint32_t)k * kPfxThreads + threadIdx.x, w = cbase + i;
-        if (w < words) prefix[w] = s_v[i + (i >> 5)];
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = (uint32_t)k * THREADS + threadIdx.x, w = cbase + i;
+        if (w >= q.words) break;
+        uint32_t o = s_v[i + (i >> 5)];
+        q.prefix[w] = o;
+        if (q.store) q.store[w] = v[k];
+        if (q.list) {
+            uint32_t b = v[k];
+            while (b && o < q.cap) {  // cap: the list's capacity
+                const int bit = __ffs(b) - 1;
+                b &= b - 1u;
+                if (q.zero) q.zero[o] = 0u;
+                q.list[o++] = w * 32u + (uint32_t)bit;
+            }
+        }
     }
 }
 
 template <bool POPC>
-static gvx_status pfx_run(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total, DevBuf& tmp, cudaStream_t st,
-                          int64_t* launches)
+static gvx_status pfx_run(PfxJobs& jobs, DevBuf& tmp, cudaStream_t st, int64_t* launches)
 {
-    const uint32_t nb = std::max<uint32_t>(1u, (n + kPfxChunk - 1) / kPfxChunk);
-    GVX_CK(gvx_ensure(tmp, (size_t)(nb + 1) * sizeof(uint32_t)));
-    k_pfx_reduce<POPC><<<nb, kPfxThreads, 0, st>>>(in, n, tmp.as<uint32_t>());
-    k_pfx_apply<POPC><<<nb, kPfxThreads, 0, st>>>(in, n, tmp.as<uint32_t>(), out, total);
-    *launches += 2;
+    if (jobs.n == 0) return GVX_OK;
+    uint32_t most = 1u, sums = 0u;
+    for (int i = 0; i < jobs.n; i++) {
+        jobs.j[i].sums = sums;
+        sums += (jobs.j[i].words + kPfxChunk - 1) / kPfxChunk;
+        most = std::max(most, jobs.j[i].words);
+    }
+    if (most <= kPfxSelf * kPfxSelfThreads) {
+        const dim3 grid((most + kPfxSelfThreads - 1) / kPfxSelfThreads, (unsigned)jobs.n);
+        k_pfx_apply<POPC, kPfxSelfThreads, 1, true><<<grid, kPfxSelfThreads, 0, st>>>(jobs, nullptr);
+        (*launches)++;
+    } else {
+        GVX_CK(gvx_ensure(tmp, (size_t)(sums + 1) * sizeof(uint32_t)));
+        const dim3 grid((most + kPfxChunk - 1) / kPfxChunk, (unsigned)jobs.n);
+        k_pfx_reduce<POPC><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
+        k_pfx_apply<POPC, kPfxThreads, kPfxPer, false><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
+        *launches += 2;
+    }
     GVX_CK(cudaGetLastError());
     return GVX_OK;
 }
@@ -560,28 +580,43 @@ static gvx_status pfx_run(const uint32_t* in, uint32_t* out, uint32_t n, uint32_
 gvx_status gvx_bitmap_prefix(const uint32_t* bits, uint32_t* prefix, uint32_t words, uint32_t* total, DevBuf& tmp,
                              cudaStream_t st, int64_t* launches)
 {
-    return pfx_run<true>(bits, prefix, words, total, tmp, st, launches);
+    PfxJobs jobs;
+    jobs.add(bits, prefix, words, total);
+    return pfx_run<true>(jobs, tmp, st, launches);
 }
 
 gvx_status gvx_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total, DevBuf& tmp, cudaStream_t st,
                         int64_t* launches)
 {
-    return pfx_run<false>(in, out, n, total, tmp, st, launches);
+    PfxJobs jobs;
+    jobs.add(in, out, n, total);
+    return pfx_run<false>(jobs, tmp, st, launches);
 }
 
-// set bits -> sorted key list (select)
-__global__ void k_select(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix, uint32_t words,
-                         uint32_t* out, uint32_t cap)
+// set bits -> sorted key lists, where the lists are sized after the prefixes (a thread a word)
+__global__ void k_select(PfxJobs jobs)
 {
+    const PfxJob& q = jobs.j[blockIdx.y];
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= words) return;
-    uint32_t b = bits[w];
-    uint32_t o = prefix[w];
-    while (b && o < cap) {  // cap: the list's capacity
+    if (w >= q.words) return;
+    uint32_t b = q.src[w];
+    uint32_t o = q.prefix[w];
+    while (b && o < q.cap) {
         const int k = __ffs(b) - 1;
         b &= b - 1u;
-        out[o++] = w * 32u + (uint32_t)k;
+        q.list[o++] = w * 32u + (uint32_t)k;
     }
+}
+
+static gvx_status select_run(const PfxJobs& jobs, cudaStream_t st, int64_t* launches)
+{
+    if (jobs.n == 0) return GVX_OK;
+    uint32_t most = 1u;
+    for (int i = 0; i < jobs.n; i++) most = std::max(most, jobs.j[i].words);
+    k_select<<<dim3((most + 255u) / 256u, (unsigned)jobs.n), 256, 0, st>>>(jobs);
+    (*launches)++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
 }
 
 struct NodeLevelArgs {
@@ -606,10 +641,39 @@ struct NodeLevelArgs {
     uint32_t cap, pcap;
 };
 
-// one node per thread: Node record, parent reference, and the parent's child-list slot
-// (SetupNode VG.cpp:2512-2524, gvdbLinkBricks cuda_gvdb_nodes.cuh:470-505)
-__global__ void k_write_nodes(NodeLevelArgs a)
+// the levels of a tree below its root, and the root
+struct TreeArgs {
+    int depth;
+    int rootpos[3];
+    GvxNode* root;
+    NodeLevelArgs a[GVX_MAXLEV];
+};
+
+__device__ void write_root(const TreeArgs& t)
 {
+    GvxNode nd;
+    nd.lev = (uint8_t)t.depth;
+    nd.flags = 1;
+    nd.prio = 0;
+    nd.pad = 0;
+    for (int k = 0; k < 3; k++) {
+        nd.pos[k] = t.rootpos[k];
+        nd.value[k] = -1;
+        nd.vrange[k] = 0.f;
+    }
+    nd.parent = ID_UNDEFL_U64;
+    nd.childlist = 1ull | ((uint64_t)t.depth << 8);
+    nd.mask = 0ull;
+    *t.root = nd;
+}
+
+// one node per thread, a level per blockIdx.y: Node record, parent reference, and the parent's child-list
+// slot (SetupNode VG.cpp:2512-2524, gvdbLinkBricks cuda_gvdb_nodes.cuh:470-505).  A node's parent is found
+// by rank, so no level waits for another.
+__global__ void k_write_nodes(TreeArgs t)
+{
+    const NodeLevelArgs& a = t.a[blockIdx.y];
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) write_root(t);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t ucount = a.ucount, xcount = a.xcount, pucount = a.pucount;
     if (a.dc) {
@@ -658,26 +722,6 @@ __global__ void k_write_nodes(NodeLevelArgs a)
         a.pclist[(size_t)pidx * res * res * res + bit] = ((uint64_t)i << 16) | ((uint64_t)a.lev << 8);
     a.nodes[i] = nd;
     if (a.leaf_key) a.leaf_key[i] = key;
-}
-
-__global__ void k_write_root(GvxNode* root, int lev, int px, int py, int pz)
-{
-    GvxNode nd;
-    nd.lev = (uint8_t)lev;
-    nd.flags = 1;
-    nd.prio = 0;
-    nd.pad = 0;
-    nd.pos[0] = px;
-    nd.pos[1] = py;
-    nd.pos[2] = pz;
-    for (int k = 0; k < 3; k++) {
-        nd.value[k] = -1;
-        nd.vrange[k] = 0.f;
-    }
-    nd.parent = ID_UNDEFL_U64;
-    nd.childlist = 1ull | ((uint64_t)lev << 8);
-    nd.mask = 0ull;
-    *root = nd;
 }
 
 // run of equal leaf keys in sorted order -> [start, end) of its leaf.  With octants in the keys
@@ -1073,44 +1117,58 @@ __device__ __forceinline__ bool in_node_set(const GvxNode& nd, int set)
     return set == kSetActive ? nd.flags != 0 : nd.parent != ID_UNDEF64_U64;
 }
 
+// the nodes of a level, their set's bitmap and the table k_node_remap fills; a level per blockIdx.y
+struct NodeSet {
+    const GvxNode* nodes;
+    uint32_t n;
+    int t, range;
+    BitRank br;
+    int* remap;
+    uint32_t* leaf_key;
+};
+struct NodeSets {
+    int n = 0;
+    uint32_t most = 0u;
+    NodeSet s[GVX_MAXLEV];
+    void add(const GvxNode* nodes, uint32_t cnt, int t, int range, const BitRank& br, int* remap, uint32_t* leaf_key)
+    {
+        if (cnt == 0) return;
+        s[n++] = NodeSet{nodes, cnt, t, range, br, remap, leaf_key};
+        most = most < cnt ? cnt : most;
+    }
+    dim3 grid() const { return dim3((most + 255u) / 256u, (unsigned)n); }
+};
+
 // bitmap of a level's linked (or active) nodes; linked nodes outside the key
 // space cannot be touched and are left out, an active leaf outside it is an error
-__global__ void k_node_bits(const GvxNode* __restrict__ nodes, uint32_t n, KeySpace ks, int t, int range, int set,
-                            uint32_t* bits, uint32_t* err)
+__global__ void k_node_bits(NodeSets a, KeySpace ks, int set, uint32_t* err)
 {
+    const NodeSet& q = a.s[blockIdx.y];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const GvxNode nd = nodes[i];
+    if (i >= q.n) return;
+    const GvxNode nd = q.nodes[i];
     if (!in_node_set(nd, set)) return;
     uint32_t key;
-    if (node_key(nd, ks, t, range, &key))
-        atomicOr(&bits[key >> 5], 1u << (key & 31));
+    if (node_key(nd, ks, q.t, q.range, &key))
+        atomicOr(&q.br.bits[key >> 5], 1u << (key & 31));
     else if (set == kSetActive)
         atomicOr(err, GVX_DERR_DEGENERATE);
 }
 
 // rank in the set's bitmap -> pool index; with `leaf_key`, also the compact key
 // of every leaf (kNoKey where the leaf is not in the set)
-__global__ void k_node_remap(const GvxNode* __restrict__ nodes, uint32_t n, KeySpace ks, int t, int range, int set,
-                             BitRank br, int* remap, uint32_t* leaf_key)
+__global__ void k_node_remap(NodeSets a, KeySpace ks, int set)
 {
+    const NodeSet& q = a.s[blockIdx.y];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const GvxNode nd = nodes[i];
+    if (i >= q.n) return;
+    const GvxNode nd = q.nodes[i];
     uint32_t key = kNoKey;
-    if (in_node_set(nd, set) && node_key(nd, ks, t, range, &key))
-        remap[br_rank(br, key)] = (int)i;
+    if (in_node_set(nd, set) && node_key(nd, ks, q.t, q.range, &key))
+        q.remap[br_rank(q.br, key)] = (int)i;
     else
         key = kNoKey;
-    if (leaf_key) leaf_key[i] = key;
-}
-
-// N = (D | A) & ~L: touched (by a point, or by a point's box) and not linked
-__global__ void k_new_bits(const uint32_t* __restrict__ D, const uint32_t* __restrict__ A,
-                           const uint32_t* __restrict__ L, uint32_t* N, uint32_t words)
-{
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < words) N[w] = (D[w] | A[w]) & ~L[w];
+    if (q.leaf_key) q.leaf_key[i] = key;
 }
 
 // markers of the existing leaves (VG.cpp:1028-1043, 1078-1085): a linked leaf
@@ -1150,10 +1208,15 @@ struct IncNodeArgs {
     uint32_t* err;
 };
 
-// one new node per thread: SetupNode (VG.cpp:2512-2524) and its link
-// (gvdbLinkBricks); the parent is a linked node or a new one of this build
-__global__ void k_inc_write_nodes(IncNodeArgs a)
+struct IncTreeArgs {
+    IncNodeArgs a[GVX_MAXLEV];
+};
+
+// one new node per thread, a level per blockIdx.y: SetupNode (VG.cpp:2512-2524) and its link
+// (gvdbLinkBricks); the parent is a linked node or a new one of this build, found by rank
+__global__ void k_inc_write_nodes(IncTreeArgs t)
 {
+    const IncNodeArgs& a = t.a[blockIdx.y];
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= a.count) return;
     const uint32_t i = a.base + j;
@@ -1558,7 +1621,8 @@ struct gvx_topo_staged {
 
 static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpace& ks, FullBuild& fb, ClearList& clear);
 static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
-                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback);
+                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback,
+                                      uint32_t* lists = nullptr, const uint32_t* list_cap = nullptr);
 
 // the compact level-0 key space of a full build over the points' bounding box
 // (+ dilation margin), inside the root
@@ -1655,9 +1719,11 @@ static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpac
 }
 
 // a full build in key space `ks` up to its node counts (d_counts), which are queued for the
-// host when queue_readback; its scratch (topo_full_scratch) is cleared
+// host when queue_readback; its scratch (topo_full_scratch) is cleared.  lists (optional): room for the keys of
+// X0 (list_cap[0]), then of D_l and X_l (list_cap[l] each) per upper level
 static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
-                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback)
+                                      const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback,
+                                      uint32_t* lists, const uint32_t* list_cap)
 {
     cudaStream_t st = g->stream;
     const int b = g->brick;
@@ -1677,17 +1743,17 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
     k_mark_runs<<<blocks_for(n, 256), 256, 0, st>>>(skeys, (uint32_t)n, g->key_shift, invalid_key,
                                                     g->d0_bits.as<uint32_t>());
     g->launches++;
-    rc = gvx_bitmap_prefix(g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0, counts + 0, g->tmp_scan,
-                           st, &g->launches);
-    if (rc) return rc;
     BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
-    k_select<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, d0.prefix, words0, g->leaf_key.as<uint32_t>(), 0xFFFFFFFFu);
-    g->launches++;
+    PfxJobs direct;
+    PfxJob& dj = direct.add(d0.bits, d0.prefix, words0, counts + 0);
+    dj.list = g->leaf_key.as<uint32_t>();
+    dj.zero = g->masks.as<uint32_t>();
+    rc = pfx_run<true>(direct, g->tmp_scan, st, &g->launches);
+    if (rc) return rc;
 
     // ---- X0: dilation leaves (radius >= 1, VG.cpp:1207-1208)
     BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
     if (extra) {
-        GVX_CK(cudaMemsetAsync(g->masks.p, 0, (size_t)n * 4, st));
         k_point_masks<<<blocks_for(n, 256), 256, 0, st>>>(skeys, svals, (uint32_t)n, g->key_shift, invalid_key, d0, g->pts.pos,
                                                           g->pts.pos_off, g->pts.pos_stride, o[0], o[1], o[2],
                                                           radius, 2.0f, b, g->masks.as<uint32_t>());
@@ -1696,17 +1762,33 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
             g->masks.as<uint32_t>(), d0, x0.bits, g->d_err.as<uint32_t>());
         g->launches += 2;
     }
-    rc = gvx_bitmap_prefix(x0.bits, x0.prefix, words0, counts + 1, g->tmp_scan, st, &g->launches);
-    if (rc) return rc;
-
     // ---- upper levels: parents of D0 (direct) and of X0 (extra)
     if (ud.nlev > 0) {
-        k_upper_direct<<<std::min(blocks_for(n, 256), 152u * 8u), 256, 0, st>>>(g->leaf_key.as<uint32_t>(), counts + 0, ks, ud,
-                                                           g->upper.as<uint32_t>());
-        k_upper_extra<<<blocks_for(words0, 256), 256, 0, st>>>(x0.bits, words0, ks, ud, g->upper.as<uint32_t>());
-        k_prefix_upper<<<2 * ud.nlev, 256, 0, st>>>(ud, g->upper.as<uint32_t>(), counts);
-        g->launches += 3;
+        k_upper_bits<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, extra ? x0.bits : nullptr, words0, ks, ud,
+                                                              g->upper.as<uint32_t>());
+        g->launches++;
     }
+    // ---- ranks of X0, D_l and X_l = A_l & ~D_l, and their counts; the keys too where the lists have their room
+    PfxJobs ranks;
+    uint32_t* lp = lists;
+    auto listed = [&](PfxJob& q, uint32_t cap) {
+        if (!lists) return;
+        q.list = lp;
+        q.cap = cap;
+        lp += cap;
+    };
+    listed(ranks.add(x0.bits, x0.prefix, words0, counts + 1), list_cap ? list_cap[0] : 0u);
+    for (int l = 1; l <= ud.nlev; l++) {
+        uint32_t* base = g->upper.as<uint32_t>() + ud.off[l];
+        const uint32_t w = ud.words[l];
+        listed(ranks.add(base, base + 2u * w, w, counts + 2 + 2 * (l - 1)), list_cap ? list_cap[l] : 0u);
+        PfxJob& x = ranks.add(base + w, base + 3u * w, w, counts + 3 + 2 * (l - 1));
+        x.minus = base;
+        x.store = base + w;
+        listed(x, list_cap ? list_cap[l] : 0u);
+    }
+    rc = pfx_run<true>(ranks, g->tmp_scan, st, &g->launches);
+    if (rc) return rc;
     GVX_CK(cudaGetLastError());
 
     // ---- counts to the host (the one mid-build synchronisation)
@@ -1719,6 +1801,43 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
     }
     fb.ks = ks;
     return queue_readback ? readback_start(g) : GVX_OK;
+}
+
+// what a full build's level has from its key space
+static void level_args(const gvx_grid* g, const FullBuild& fb, int l, NodeLevelArgs& a)
+{
+    memset(&a, 0, sizeof(a));
+    a.lev = l;
+    a.depth = fb.depth;
+    a.ks = fb.ks;
+    a.tshift = g->tshift[l];
+    a.tshift_parent = g->tshift[l + 1];
+    a.logdim_parent = g->logdim[l + 1];
+    a.res_parent = g->res[l + 1];
+    for (int k = 0; k < 3; k++) {
+        a.lo[k] = fb.ks.lo[k] >> g->tshift[l];
+        a.root_rel[k] = fb.rootpos[k] / g->range[l];
+    }
+    a.range = g->range[l];
+    if (l + 1 < fb.depth) {
+        uint32_t* base = g->upper.as<uint32_t>() + fb.ud.off[l + 1];
+        const uint32_t w = fb.ud.words[l + 1];
+        a.pd = BitRank{base, base + 2 * w, w};
+        a.px = BitRank{base + w, base + 3 * w, w};
+    }
+    a.nodes = g->nodes[l].as<GvxNode>();
+    a.pclist = g->clist[l + 1].as<uint64_t>();
+    a.leaf_key = l == 0 ? g->leaf_key.as<uint32_t>() : nullptr;
+}
+
+// the nodes of all levels (most nodes a level) and the root
+static void write_tree(gvx_grid* g, const FullBuild& fb, TreeArgs& t, uint32_t most)
+{
+    t.depth = fb.depth;
+    for (int a = 0; a < 3; a++) t.rootpos[a] = fb.rootpos[a];
+    t.root = g->nodes[fb.depth].as<GvxNode>();
+    k_write_nodes<<<dim3(blocks_for(most, 256), (unsigned)fb.depth), 256, 0, g->stream>>>(t);
+    g->launches++;
 }
 
 static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
@@ -1765,71 +1884,43 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     for (int l = 1; l < depth; l++) list_words += (size_t)Ul[l] + Xl[l];
     GVX_CK(gvx_ensure(g->lists, list_words * 4));
     uint32_t* x0list = g->lists.as<uint32_t>();
-    k_select<<<blocks_for(words0, 256), 256, 0, st>>>(x0.bits, x0.prefix, words0, x0list, 0xFFFFFFFFu);
-    g->launches++;
+    PfxJobs sel;
+    sel.add(x0.bits, x0.prefix, words0, nullptr).list = x0list;
     uint32_t* lp = x0list + X0 + 1;
     const uint32_t* dl[GVX_MAXLEV] = {};
     const uint32_t* xl[GVX_MAXLEV] = {};
-    dl[0] = g->leaf_key.as<uint32_t>();  // D0 list (overwritten in place by k_write_nodes with the same keys)
     xl[0] = x0list;
     for (int l = 1; l < depth; l++) {
         uint32_t* base = g->upper.as<uint32_t>() + ud.off[l];
         const uint32_t w = ud.words[l];
-        k_select<<<blocks_for(w, 256), 256, 0, st>>>(base, base + 2 * w, w, lp, 0xFFFFFFFFu);
+        sel.add(base, base + 2 * w, w, nullptr).list = lp;
         dl[l] = lp;
         lp += Ul[l];
-        k_select<<<blocks_for(w, 256), 256, 0, st>>>(base + w, base + 3 * w, w, lp, 0xFFFFFFFFu);
+        sel.add(base + w, base + 3 * w, w, nullptr).list = lp;
         xl[l] = lp;
         lp += Xl[l];
-        g->launches += 2;
     }
-    // leaf keys in pool order: D0 (already there) then X0
+    // leaf keys in pool order: the D0 list of the first half, again (the buffer may have been replaced),
+    // and X0's, which level 0's nodes append
     GVX_CK(gvx_ensure(g->leaf_key, (size_t)std::max<uint64_t>((uint64_t)U0 + X0, (uint64_t)n) * 4 + 4));
-    // (ensure may have reallocated: D0 list must be rebuilt in that case)
-    k_select<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, d0.prefix, words0, g->leaf_key.as<uint32_t>(), 0xFFFFFFFFu);
+    sel.add(d0.bits, d0.prefix, words0, nullptr).list = g->leaf_key.as<uint32_t>();
     dl[0] = g->leaf_key.as<uint32_t>();
-    if (X0)
-        GVX_CK(cudaMemcpyAsync(g->leaf_key.as<uint32_t>() + U0, x0list, (size_t)X0 * 4, cudaMemcpyDeviceToDevice, st));
-    g->launches++;
+    GVX_CK_STATUS(select_run(sel, st, &g->launches));
 
-    // ---- nodes, parents and child lists, top-down
-    k_write_root<<<1, 1, 0, st>>>(g->nodes[depth].as<GvxNode>(), depth, rootpos[0], rootpos[1], rootpos[2]);
-    g->launches++;
+    // ---- nodes, parents and child lists
+    TreeArgs t;
+    uint32_t most = 1u;
     for (int l = depth - 1; l >= 0; l--) {
-        NodeLevelArgs a;
-        memset(&a, 0, sizeof(a));
-        a.lev = l;
-        a.depth = depth;
+        NodeLevelArgs& a = t.a[l];
+        level_args(g, fb, l, a);
         a.ucount = Ul[l];
         a.xcount = Xl[l];
         a.dlist = dl[l];
         a.xlist = xl[l];
-        a.ks = ks;
-        a.tshift = g->tshift[l];
-        a.tshift_parent = g->tshift[l + 1];
-        a.logdim_parent = g->logdim[l + 1];
-        a.res_parent = g->res[l + 1];
-        for (int k = 0; k < 3; k++) {
-            a.lo[k] = ks.lo[k] >> g->tshift[l];
-            a.root_rel[k] = rootpos[k] / g->range[l];
-        }
-        a.range = g->range[l];
-        if (l + 1 < depth) {
-            uint32_t* base = g->upper.as<uint32_t>() + ud.off[l + 1];
-            const uint32_t w = ud.words[l + 1];
-            a.pd = BitRank{base, base + 2 * w, w};
-            a.px = BitRank{base + w, base + 3 * w, w};
-            a.pucount = Ul[l + 1];
-        }
-        a.nodes = g->nodes[l].as<GvxNode>();
-        a.pclist = g->clist[l + 1].as<uint64_t>();
-        a.leaf_key = nullptr;
-        const uint32_t cnt = Ul[l] + Xl[l];
-        if (cnt) {
-            k_write_nodes<<<blocks_for(cnt, 256), 256, 0, st>>>(a);
-            g->launches++;
-        }
+        a.pucount = l + 1 < depth ? Ul[l + 1] : 0u;
+        most = std::max(most, Ul[l] + Xl[l]);
     }
+    write_tree(g, fb, t, most);
 
     // ---- leaf lookup, neighbours, point ranges
     g->lookup.ks = ks;
@@ -1919,20 +2010,18 @@ static gvx_status build_active_lookup(gvx_grid* g, const KeySpace& ks, uint32_t 
     GVX_CK_STATUS(leaf_range_scratch(g, L0, clear));
     GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
     uint32_t* counts = g->d_counts.as<uint32_t>();
+    const BitRank lk{g->lk_bits.as<uint32_t>(), g->lk_prefix.as<uint32_t>(), words0};
+    NodeSets act;
+    act.add(g->nodes[0].as<GvxNode>(), L0, 0, g->range[0], lk, g->remap.as<int>(), g->leaf_key.as<uint32_t>());
     if (L0) {
-        k_node_bits<<<blocks_for(L0, 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(), L0, ks, 0, g->range[0],
-                                                         kSetActive, g->lk_bits.as<uint32_t>(),
-                                                         g->d_err.as<uint32_t>());
+        k_node_bits<<<act.grid(), 256, 0, st>>>(act, ks, kSetActive, g->d_err.as<uint32_t>());
         g->launches++;
     }
     gvx_status rc = gvx_bitmap_prefix(g->lk_bits.as<uint32_t>(), g->lk_prefix.as<uint32_t>(), words0,
                                       counts + kCntActive, g->tmp_scan, st, &g->launches);
     if (rc) return rc;
-    const BitRank lk{g->lk_bits.as<uint32_t>(), g->lk_prefix.as<uint32_t>(), words0};
     if (L0) {
-        k_node_remap<<<blocks_for(L0, 256), 256, 0, st>>>(g->nodes[0].as<GvxNode>(), L0, ks, 0, g->range[0],
-                                                          kSetActive, lk, g->remap.as<int>(),
-                                                          g->leaf_key.as<uint32_t>());
+        k_node_remap<<<act.grid(), 256, 0, st>>>(act, ks, kSetActive);
         g->launches++;
     }
     g->lookup.ks = ks;
@@ -2059,15 +2148,15 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
     k_mark_runs<<<blocks_for(n, 256), 256, 0, st>>>(skeys, (uint32_t)n, g->key_shift, invalid_key,
                                                     g->d0_bits.as<uint32_t>());
     g->launches++;
-    rc = gvx_bitmap_prefix(g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0, counts + kCntD0,
-                           g->tmp_scan, st, &g->launches);
-    if (rc) return rc;
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
     uint32_t* dlist = g->lists.as<uint32_t>();
-    k_select<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, d0.prefix, words0, dlist, 0xFFFFFFFFu);
-    g->launches++;
+    PfxJobs direct;
+    PfxJob& dj = direct.add(d0.bits, d0.prefix, words0, counts + kCntD0);
+    dj.list = dlist;
+    dj.zero = g->masks.as<uint32_t>();
+    rc = pfx_run<true>(direct, g->tmp_scan, st, &g->launches);
+    if (rc) return rc;
     if (radius > 0.f) {
-        GVX_CK(cudaMemsetAsync(g->masks.p, 0, (size_t)n * 4, st));
         k_point_masks<<<blocks_for(n, 256), 256, 0, st>>>(skeys, svals, (uint32_t)n, g->key_shift, invalid_key, d0, g->pts.pos,
                                                           g->pts.pos_off, g->pts.pos_stride, o[0], o[1], o[2],
                                                           radius, 1.0f, b, g->masks.as<uint32_t>());
@@ -2077,9 +2166,9 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
         g->launches += 2;
     }
     if (ud.nlev > 0) {
-        k_upper_direct<<<std::min(blocks_for(n, 256), 152u * 8u), 256, 0, st>>>(dlist, counts + kCntD0, ks, ud, upper);
-        k_upper_extra<<<blocks_for(words0, 256), 256, 0, st>>>(g->x0_bits.as<uint32_t>(), words0, ks, ud, upper);
-        g->launches += 2;
+        k_upper_bits<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, radius > 0.f ? g->x0_bits.as<uint32_t>() : nullptr,
+                                                              words0, ks, ud, upper);
+        g->launches++;
     }
 
     // ---- linked sets L_l with rank -> pool index, levels 0..top
@@ -2090,36 +2179,38 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
     }
     GVX_CK(gvx_ensure(g->inc_remap, rtotal * 4 + 4));
     BitRank Lb[GVX_MAXLEV] = {}, Nb[GVX_MAXLEV] = {};
+    NodeSets linked;
+    PfxJobs lranks;
     for (int l = 0; l <= top; l++) {
         uint32_t* base = l == 0 ? g->inc0.as<uint32_t>() : upper + ud.off[l] + 2u * ud.words[l];
         const uint32_t w = l == 0 ? words0 : ud.words[l];
         Lb[l] = BitRank{base, base + w, w};
         Nb[l] = BitRank{base + 2u * w, base + 3u * w, w};
-        if (old[l]) {
-            k_node_bits<<<blocks_for(old[l], 256), 256, 0, st>>>(g->nodes[l].as<GvxNode>(), old[l], ks,
-                                                                 g->tshift[l], g->range[l], kSetLinked, Lb[l].bits,
-                                                                 err);
-            g->launches++;
-        }
-        rc = gvx_bitmap_prefix(Lb[l].bits, Lb[l].prefix, w, nullptr, g->tmp_scan, st, &g->launches);
-        if (rc) return rc;
-        if (old[l]) {
-            k_node_remap<<<blocks_for(old[l], 256), 256, 0, st>>>(g->nodes[l].as<GvxNode>(), old[l], ks,
-                                                                  g->tshift[l], g->range[l], kSetLinked, Lb[l],
-                                                                  g->inc_remap.as<int>() + roff[l], nullptr);
-            g->launches++;
-        }
+        linked.add(g->nodes[l].as<GvxNode>(), old[l], g->tshift[l], g->range[l], Lb[l],
+                   g->inc_remap.as<int>() + roff[l], nullptr);
+        lranks.add(Lb[l].bits, Lb[l].prefix, w, nullptr);
     }
-    // ---- new nodes N_l = T_l & ~L_l, levels 0..depth-1
-    for (int l = 0; l < depth; l++) {
-        const uint32_t* D = l == 0 ? d0.bits : upper + ud.off[l];
-        const uint32_t* A = l == 0 ? g->x0_bits.as<uint32_t>() : upper + ud.off[l] + ud.words[l];
-        k_new_bits<<<blocks_for(Nb[l].words, 256), 256, 0, st>>>(D, A, Lb[l].bits, Nb[l].bits, Nb[l].words);
+    if (linked.n) {
+        k_node_bits<<<linked.grid(), 256, 0, st>>>(linked, ks, kSetLinked, err);
         g->launches++;
-        rc = gvx_bitmap_prefix(Nb[l].bits, Nb[l].prefix, Nb[l].words, counts + kCntNew + l, g->tmp_scan, st,
-                               &g->launches);
-        if (rc) return rc;
     }
+    rc = pfx_run<true>(lranks, g->tmp_scan, st, &g->launches);
+    if (rc) return rc;
+    if (linked.n) {
+        k_node_remap<<<linked.grid(), 256, 0, st>>>(linked, ks, kSetLinked);
+        g->launches++;
+    }
+    // ---- new nodes N_l = T_l & ~L_l = (D_l | A_l) & ~L_l (touched by a point or by a point's box, and not
+    // linked), levels 0..depth-1
+    PfxJobs nranks;
+    for (int l = 0; l < depth; l++) {
+        PfxJob& q = nranks.add(l == 0 ? d0.bits : upper + ud.off[l], Nb[l].prefix, Nb[l].words, counts + kCntNew + l);
+        q.plus = l == 0 ? g->x0_bits.as<uint32_t>() : upper + ud.off[l] + ud.words[l];
+        q.minus = Lb[l].bits;
+        q.store = Nb[l].bits;
+    }
+    rc = pfx_run<true>(nranks, g->tmp_scan, st, &g->launches);
+    if (rc) return rc;
     GVX_CK(cudaGetLastError());
 
     // ---- new-node counts to the host
@@ -2161,18 +2252,23 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
         GVX_CK(gvx_ensure(g->lists, (size_t)(total_new + 1) * 4));
         const uint32_t* nl[GVX_MAXLEV] = {};
         uint32_t* lp = g->lists.as<uint32_t>();
+        PfxJobs sel;
         for (int l = 0; l < depth; l++) {
             if (!nnew[l]) continue;
-            k_select<<<blocks_for(Nb[l].words, 256), 256, 0, st>>>(Nb[l].bits, Nb[l].prefix, Nb[l].words, lp, 0xFFFFFFFFu);
-            g->launches++;
+            sel.add(Nb[l].bits, Nb[l].prefix, Nb[l].words, nullptr).list = lp;
             nl[l] = lp;
             lp += nnew[l];
         }
-        // ---- new nodes and their links (gvdbLinkBricks top-down, VG.cpp:1121-1129)
+        GVX_CK_STATUS(select_run(sel, st, &g->launches));
+        // ---- new nodes and their links (gvdbLinkBricks, VG.cpp:1121-1129)
+        IncTreeArgs tree;
+        unsigned nlev = 0;
+        uint32_t most = 0u;
         for (int l = depth - 1; l >= 0; l--) {
             if (!nnew[l]) continue;
-            IncNodeArgs a;
+            IncNodeArgs& a = tree.a[nlev++];
             memset(&a, 0, sizeof(a));
+            most = std::max(most, nnew[l]);
             a.lev = l;
             a.count = nnew[l];
             a.base = old[l];
@@ -2197,9 +2293,9 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
             a.tshift_parent = g->tshift[l + 1];
             a.pclist = g->clist[l + 1].as<uint64_t>();
             a.err = err;
-            k_inc_write_nodes<<<blocks_for(nnew[l], 256), 256, 0, st>>>(a);
-            g->launches++;
         }
+        k_inc_write_nodes<<<dim3(blocks_for(most, 256), nlev), 256, 0, st>>>(tree);
+        g->launches++;
         for (int l = 0; l < depth; l++) g->count[l] = (int64_t)old[l] + nnew[l];
         // ---- delink, bottom-up (VG.cpp:1131-1140)
         const uint32_t L0 = (uint32_t)g->count[0];
@@ -2537,70 +2633,30 @@ static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuil
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
     const BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
 
-    // lists: X0 (cap0), then D_l and X_l (cap_l each) per upper level
-    size_t list_words = cap0;
-    for (int l = 1; l < depth; l++) list_words += 2 * (size_t)P.cap[l];
-    GVX_CK(gvx_ensure(g->lists, list_words * 4 + 4));
-    uint32_t* x0list = g->lists.as<uint32_t>();
-    k_select<<<blocks_for(words0, 256), 256, 0, st>>>(x0.bits, x0.prefix, words0, x0list, cap0);
-    g->launches++;
-    uint32_t* lp = x0list + cap0;
-    const uint32_t* dl[GVX_MAXLEV] = {};
-    const uint32_t* xl[GVX_MAXLEV] = {};
-    dl[0] = g->leaf_key.as<uint32_t>();  // the D0 list of the first half; level 0's nodes append X0 to it
-    xl[0] = x0list;
-    for (int l = 1; l < depth; l++) {
-        uint32_t* base = g->upper.as<uint32_t>() + ud.off[l];
-        const uint32_t w = ud.words[l];
-        k_select<<<blocks_for(w, 256), 256, 0, st>>>(base, base + 2 * w, w, lp, P.cap[l]);
-        dl[l] = lp;
-        lp += P.cap[l];
-        k_select<<<blocks_for(w, 256), 256, 0, st>>>(base + w, base + 3 * w, w, lp, P.cap[l]);
-        xl[l] = lp;
-        lp += P.cap[l];
-        g->launches += 2;
-    }
-
-    // ---- nodes, parents and child lists, top-down, counts from d_counts
-    k_write_root<<<1, 1, 0, st>>>(g->nodes[depth].as<GvxNode>(), depth, fb.rootpos[0], fb.rootpos[1],
-                                  fb.rootpos[2]);
-    g->launches++;
-    for (int l = depth - 1; l >= 0; l--) {
-        NodeLevelArgs a;
-        memset(&a, 0, sizeof(a));
-        a.lev = l;
-        a.depth = depth;
-        a.dlist = dl[l];
-        a.xlist = xl[l];
-        a.ks = ks;
-        a.tshift = g->tshift[l];
-        a.tshift_parent = g->tshift[l + 1];
-        a.logdim_parent = g->logdim[l + 1];
-        a.res_parent = g->res[l + 1];
-        for (int k = 0; k < 3; k++) {
-            a.lo[k] = ks.lo[k] >> g->tshift[l];
-            a.root_rel[k] = fb.rootpos[k] / g->range[l];
+    // ---- nodes, parents and child lists, counts from d_counts; the lists as topo_full_launch_ks wrote them
+    TreeArgs t;
+    uint32_t most = 1u;
+    const uint32_t* lp = g->lists.as<uint32_t>();
+    for (int l = 0; l < depth; l++) {
+        NodeLevelArgs& a = t.a[l];
+        level_args(g, fb, l, a);
+        if (l > 0) {
+            a.dlist = lp;
+            lp += P.cap[l];
+        } else {
+            a.dlist = g->leaf_key.as<uint32_t>();  // the D0 list; level 0's nodes append X0 to it
         }
-        a.range = g->range[l];
-        a.ci_pu = -1;
-        if (l + 1 < depth) {
-            uint32_t* base = g->upper.as<uint32_t>() + ud.off[l + 1];
-            const uint32_t w = ud.words[l + 1];
-            a.pd = BitRank{base, base + 2 * w, w};
-            a.px = BitRank{base + w, base + 3 * w, w};
-            a.ci_pu = 2 + 2 * l;
-            a.pcap = P.cap[l + 1];
-        }
-        a.nodes = g->nodes[l].as<GvxNode>();
-        a.pclist = g->clist[l + 1].as<uint64_t>();
-        a.leaf_key = l == 0 ? g->leaf_key.as<uint32_t>() : nullptr;
+        a.xlist = lp;
+        lp += P.cap[l];
+        a.ci_pu = l + 1 < depth ? 2 + 2 * l : -1;
+        a.pcap = l + 1 < depth ? P.cap[l + 1] : 0u;
         a.dc = dcnt;
         a.ci_u = l == 0 ? 0 : 2 + 2 * (l - 1);
         a.ci_x = a.ci_u + 1;
         a.cap = P.cap[l];
-        k_write_nodes<<<blocks_for(P.cap[l], 256), 256, 0, st>>>(a);
-        g->launches++;
+        most = std::max(most, P.cap[l]);
     }
+    write_tree(g, fb, t, most);
 
     // ---- leaf lookup (X0 offset U0 from d_counts), neighbours, point ranges
     g->lookup.ks = ks;
@@ -2680,7 +2736,11 @@ gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool fr
     g->launches++;
 
     // ---- the full build in the plan's key space, sized by the capacities
-    GVX_CK_STATUS(topo_full_launch_ks(g, n, P.fb.radius, o, depth, P.fb.rootpos, P.fb.ks, fb, false));
+    size_t list_words = cap0;  // X0's keys, then those of D_l and X_l per upper level
+    for (int l = 1; l < depth; l++) list_words += 2 * (size_t)P.cap[l];
+    GVX_CK(gvx_ensure(g->lists, list_words * 4 + 4));
+    GVX_CK_STATUS(topo_full_launch_ks(g, n, P.fb.radius, o, depth, P.fb.rootpos, P.fb.ks, fb, false,
+                                      g->lists.as<uint32_t>(), P.cap));
     P.fb.words0 = fb.words0;
     P.fb.ud = fb.ud;
     gvx_status rc = plan_pools(g, P, fb);
