@@ -292,17 +292,21 @@ struct UpperDesc {
 };
 
 // parents of the cells of a word of a level-0 bitmap -> a bitmap per upper level.  Neighbouring cells share
-// their parents: a parent met again ends the walk up, and one whose bit is set is not set again (atomics on
-// the few words of the top levels, one after the other, took most of 13 us in a frame of a fused scene).
+// their parents: a parent met again ends the walk up, and above level 1 one whose bit is set is not set again
+// (atomics on the few words of the top levels, one after the other, took most of 13 us in a frame of a fused
+// scene; at level 1, where there are many words, waiting for the look would cost more than it saves).
 __device__ __forceinline__ void upper_word(uint32_t bits, uint32_t w, const KeySpace& ks, const UpperDesc& ud,
                                            uint32_t* upper, int which)
 {
     uint32_t last[GVX_MAXLEV];
 #pragma unroll
     for (int l = 0; l < GVX_MAXLEV; l++) last[l] = 0xFFFFFFFFu;
+    // runs of cells along z that share their level-1 parent: one of each is taken
+    const int lz = min(min(ud.tshift[1], ks.bits[2]), 5);
+    const uint32_t run = 0xFFFFFFFFu >> (32 - (1 << lz));
     while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1u;
+        const int b = (__ffs(bits) - 1) >> lz << lz;
+        bits &= ~(run << b);
         int c[3];
         ks_unpack(ks, w * 32u + (uint32_t)b, 0, c);
 #pragma unroll
@@ -313,20 +317,19 @@ __device__ __forceinline__ void upper_word(uint32_t bits, uint32_t w, const KeyS
             if (k == last[l]) break;  // (and its parents)
             last[l] = k;
             uint32_t* p = &upper[ud.off[l] + (which ? ud.words[l] : 0u) + (k >> 5)];
-            if (!((*(volatile uint32_t*)p >> (k & 31)) & 1u)) atomicOr(p, 1u << (k & 31));
+            if (l == 1 || !((*(volatile uint32_t*)p >> (k & 31)) & 1u)) atomicOr(p, 1u << (k & 31));
         }
     }
 }
 
-// D_l: parents of the leaves with points; A_l: of the box leaves (x0bits, where there are any)
+// D_l: parents of the leaves with points; A_l: of the box leaves (x0bits: blockIdx.y 1, where there are any)
 __global__ void k_upper_bits(const uint32_t* __restrict__ d0bits, const uint32_t* __restrict__ x0bits, uint32_t words,
                              KeySpace ks, UpperDesc ud, uint32_t* upper)
 {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= words) return;
-    const uint32_t d = d0bits[w], x = x0bits ? x0bits[w] : 0u;
-    upper_word(d, w, ks, ud, upper, 0);
-    upper_word(x, w, ks, ud, upper, 1);
+    const uint32_t* bits = blockIdx.y ? x0bits : d0bits;
+    upper_word(bits[w], w, ks, ud, upper, (int)blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -419,16 +422,33 @@ struct PfxJobs {
     }
 };
 constexpr uint32_t kPfxSelf = 32;
-constexpr int kPfxThreads = 256, kPfxPer = 16, kPfxSelfThreads = 1024;
-constexpr uint32_t kPfxChunk = kPfxThreads * kPfxPer;
+constexpr int kPfxThreads = 256, kPfxSelfThreads = 1024;
 }  // namespace
 
-__device__ __forceinline__ uint32_t pfx_word(const PfxJob& q, uint32_t w)
+// words base + k STEP, k < N, of a job, 0 from `end` on: all loads of an array before the next one's (a
+// choice between arrays at each word would make every load wait for the last)
+template <int N>
+__device__ __forceinline__ void pfx_words(const PfxJob& q, uint32_t base, uint32_t step, uint32_t end, uint32_t (&v)[N])
 {
-    uint32_t v = q.src[w];
-    if (q.plus) v |= q.plus[w];
-    if (q.minus) v &= ~q.minus[w];
-    return v;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const uint32_t w = base + (uint32_t)k * step;
+        v[k] = w < end ? q.src[w] : 0u;
+    }
+    if (q.plus) {
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const uint32_t w = base + (uint32_t)k * step;
+            v[k] |= w < end ? q.plus[w] : 0u;
+        }
+    }
+    if (q.minus) {
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            const uint32_t w = base + (uint32_t)k * step;
+            v[k] &= w < end ? ~q.minus[w] : 0u;
+        }
+    }
 }
 
 // POPC: the scanned values are the popcounts of bitmap words, else the words themselves
@@ -451,23 +471,18 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* s_w)
     return t;
 }
 
-// per block of kPfxChunk words: the sum (all loads issued before any add: the block's chunk is
-// one round trip, not kPfxPer)
-template <bool POPC>
+// per block of PER words a thread: the sum
+template <bool POPC, int PER>
 __global__ void __launch_bounds__(kPfxThreads) k_pfx_reduce(PfxJobs jobs, uint32_t* sums)
 {
     const PfxJob& q = jobs.j[blockIdx.y];
-    const uint32_t base = blockIdx.x * kPfxChunk + threadIdx.x;
-    if (blockIdx.x * kPfxChunk >= q.words) return;
-    uint32_t v[kPfxPer];
-#pragma unroll
-    for (int k = 0; k < kPfxPer; k++) {
-        const uint32_t w = base + (uint32_t)k * kPfxThreads;
-        v[k] = w < q.words ? pfx_word(q, w) : 0u;
-    }
+    const uint32_t cbase = blockIdx.x * (kPfxThreads * PER);
+    if (cbase >= q.words) return;
+    uint32_t v[PER];
+    pfx_words<PER>(q, cbase + threadIdx.x, kPfxThreads, q.words, v);
     uint32_t s = 0u;
 #pragma unroll
-    for (int k = 0; k < kPfxPer; k++) s += pfx_value<POPC>(v[k]);
+    for (int k = 0; k < PER; k++) s += pfx_value<POPC>(v[k]);
     __shared__ uint32_t s_w[kPfxThreads / 32];
     s = block_sum<kPfxThreads>(s, s_w);
     if (threadIdx.x == 0) sums[q.sums + blockIdx.x] = s;
@@ -487,15 +502,15 @@ __global__ void __launch_bounds__(THREADS) k_pfx_apply(PfxJobs jobs, const uint3
     const uint32_t cbase = blockIdx.x * CHUNK;
     if (cbase >= q.words) return;
     uint32_t v[PER];
-#pragma unroll
-    for (int k = 0; k < PER; k++) {
-        const uint32_t w = cbase + (uint32_t)k * THREADS + threadIdx.x;
-        v[k] = w < q.words ? pfx_word(q, w) : 0u;
-    }
+    pfx_words<PER>(q, cbase + threadIdx.x, THREADS, q.words, v);
     uint32_t before = 0u;
     if (SELF) {
-#pragma unroll 8
-        for (uint32_t w = threadIdx.x; w < cbase; w += THREADS) before += pfx_value<POPC>(pfx_word(q, w));
+        for (uint32_t w = threadIdx.x; w < cbase; w += 8u * THREADS) {
+            uint32_t u[8];
+            pfx_words<8>(q, w, THREADS, cbase, u);
+#pragma unroll
+            for (int k = 0; k < 8; k++) before += pfx_value<POPC>(u[k]);
+        }
     } else {
         for (uint32_t i = threadIdx.x; i < blockIdx.x; i += THREADS) before += sums[q.sums + i];
     }
@@ -552,26 +567,39 @@ __global__ void __launch_bounds__(THREADS) k_pfx_apply(PfxJobs jobs, const uint3
     }
 }
 
+template <bool POPC, int PER>
+static gvx_status pfx_two(PfxJobs& jobs, uint32_t most, DevBuf& tmp, cudaStream_t st, int64_t* launches)
+{
+    constexpr uint32_t chunk = kPfxThreads * PER;
+    uint32_t sums = 0u;
+    for (int i = 0; i < jobs.n; i++) {
+        jobs.j[i].sums = sums;
+        sums += (jobs.j[i].words + chunk - 1) / chunk;
+    }
+    GVX_CK(gvx_ensure(tmp, (size_t)(sums + 1) * sizeof(uint32_t)));
+    const dim3 grid((most + chunk - 1) / chunk, (unsigned)jobs.n);
+    k_pfx_reduce<POPC, PER><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
+    k_pfx_apply<POPC, kPfxThreads, PER, false><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
+    *launches += 2;
+    return GVX_OK;
+}
+
+// (two launches: blocks of 1024 words, so that the key lists have the threads, until there are 1024 sums to
+// add up in a block; then of 4096.  2^16 words with their list: 17 us by 4096, 6 by 1024)
 template <bool POPC>
 static gvx_status pfx_run(PfxJobs& jobs, DevBuf& tmp, cudaStream_t st, int64_t* launches)
 {
     if (jobs.n == 0) return GVX_OK;
-    uint32_t most = 1u, sums = 0u;
-    for (int i = 0; i < jobs.n; i++) {
-        jobs.j[i].sums = sums;
-        sums += (jobs.j[i].words + kPfxChunk - 1) / kPfxChunk;
-        most = std::max(most, jobs.j[i].words);
-    }
+    uint32_t most = 1u;
+    for (int i = 0; i < jobs.n; i++) most = std::max(most, jobs.j[i].words);
     if (most <= kPfxSelf * kPfxSelfThreads) {
         const dim3 grid((most + kPfxSelfThreads - 1) / kPfxSelfThreads, (unsigned)jobs.n);
         k_pfx_apply<POPC, kPfxSelfThreads, 1, true><<<grid, kPfxSelfThreads, 0, st>>>(jobs, nullptr);
         (*launches)++;
+    } else if (most <= (1u << 20)) {
+        GVX_CK_STATUS((pfx_two<POPC, 4>(jobs, most, tmp, st, launches)));
     } else {
-        GVX_CK(gvx_ensure(tmp, (size_t)(sums + 1) * sizeof(uint32_t)));
-        const dim3 grid((most + kPfxChunk - 1) / kPfxChunk, (unsigned)jobs.n);
-        k_pfx_reduce<POPC><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
-        k_pfx_apply<POPC, kPfxThreads, kPfxPer, false><<<grid, kPfxThreads, 0, st>>>(jobs, tmp.as<uint32_t>());
-        *launches += 2;
+        GVX_CK_STATUS((pfx_two<POPC, 16>(jobs, most, tmp, st, launches)));
     }
     GVX_CK(cudaGetLastError());
     return GVX_OK;
@@ -1321,9 +1349,15 @@ __global__ void k_delink_upper(GvxNode* nodes, uint32_t n, const uint64_t* __res
     }
     const uint64_t* cl = clist + (size_t)i * vc;
     bool any = false;
-    for (uint32_t s0 = 0; s0 < vc; s0 += 32u) {
-        const uint32_t s = s0 + (uint32_t)lane;
-        if (__any_sync(0xFFFFFFFFu, s < vc && cl[s] != ID_UNDEF64_U64)) {
+    // eight loads a turn: one at a time, 600 ns each, a node whose children come late took 8 us
+    for (uint32_t s0 = (uint32_t)lane; s0 - (uint32_t)lane < vc; s0 += 256u) {
+        uint64_t c[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) c[k] = s0 + 32u * k < vc ? cl[s0 + 32u * k] : ID_UNDEF64_U64;
+        bool here = false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) here = here || c[k] != ID_UNDEF64_U64;
+        if (__any_sync(0xFFFFFFFFu, here)) {
             any = true;
             break;
         }
@@ -1764,8 +1798,8 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
     }
     // ---- upper levels: parents of D0 (direct) and of X0 (extra)
     if (ud.nlev > 0) {
-        k_upper_bits<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, extra ? x0.bits : nullptr, words0, ks, ud,
-                                                              g->upper.as<uint32_t>());
+        k_upper_bits<<<dim3(blocks_for(words0, 256), extra ? 2 : 1), 256, 0, st>>>(d0.bits, x0.bits, words0, ks, ud,
+                                                                                   g->upper.as<uint32_t>());
         g->launches++;
     }
     // ---- ranks of X0, D_l and X_l = A_l & ~D_l, and their counts; the keys too where the lists have their room
@@ -2166,8 +2200,8 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
         g->launches += 2;
     }
     if (ud.nlev > 0) {
-        k_upper_bits<<<blocks_for(words0, 256), 256, 0, st>>>(d0.bits, radius > 0.f ? g->x0_bits.as<uint32_t>() : nullptr,
-                                                              words0, ks, ud, upper);
+        k_upper_bits<<<dim3(blocks_for(words0, 256), radius > 0.f ? 2 : 1), 256, 0, st>>>(
+            d0.bits, g->x0_bits.as<uint32_t>(), words0, ks, ud, upper);
         g->launches++;
     }
 
