@@ -1462,7 +1462,10 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
     const uint32_t invalid_key = 1u << (ks.total_bits + kshift);
     const int bits = ks.total_bits + kshift + 1;
     const int passes = gvx_sort_passes(bits);
-    const unsigned kb = std::min(blocks_for(n, 256), 152u * 8u);
+    // a block adds its digit counts up in L2: with a point or two a thread that cost as much as the keys
+    // (400k points of a surface in 1216 blocks 13.6 us, in 390 6; 777k 12.8, in 759 8; 4M in 1216 23, in 304 33)
+    const unsigned kb =
+        std::min(blocks_for(n, 256), std::max(152u * 2u, std::min(blocks_for(n, 1024), 152u * 8u)));
     k_keys<<<kb, 256, 0, g->stream>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, t[0], t[1], t[2],
                                       ks, 1.0f / (float)g->brick, kshift, lb, passes, invalid_key,
                                       g->keys[0].as<uint32_t>(), g->vals[0].as<uint32_t>(),
@@ -2416,6 +2419,11 @@ static void bbox_depth(gvx_grid* g, const uint32_t* hb, float mn[3], float mx[3]
     }
 }
 
+// the blocks of k_bbox (256 threads): a multiple of 3, since the packed path needs the thread count divisible
+// by 3; four an SM, as their atomics on six words come one after the other (400k points: eight an SM 7.9 us,
+// four 5.8; 4M: 20 and 19, two 28)
+static unsigned bbox_blocks(int n) { return (std::min(blocks_for(n, 256), 152u * 4u) + 2u) / 3u * 3u; }
+
 // RebuildTopology up to GetBoundingBox's readback, which is queued
 static gvx_status rebuild_begin(gvx_grid* g, int n, float radius, const float orig[3], int mode)
 {
@@ -2444,8 +2452,7 @@ static gvx_status rebuild_begin(gvx_grid* g, int n, float radius, const float or
     ClearList clear;
     clear_bboxes(g, clear);
     GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
-    // a multiple of 3 blocks (of 256 threads): the packed path needs the thread count divisible by 3
-    const unsigned bb = (std::min(blocks_for(n, 256), 152u * 8u) + 2u) / 3u * 3u;
+    const unsigned bb = bbox_blocks(n);
     k_bbox<<<bb, 256, 0, st>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, o[0], o[1], o[2],
                                g->d_bbox.as<uint32_t>(), g->d_err.as<uint32_t>());
     g->launches++;
@@ -2661,7 +2668,6 @@ static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuil
     const int depth = fb.depth;
     const KeySpace ks = fb.ks;
     const uint32_t words0 = fb.words0;
-    const UpperDesc& ud = fb.ud;
     const uint32_t* dcnt = g->d_counts.as<uint32_t>();
     const uint32_t cap0 = P.cap[0];
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
@@ -2723,7 +2729,6 @@ static gvx_status atlas_all(gvx_grid* g, DevCount nl, int64_t slots, uint32_t* n
 // to d_counts[kCntSlots]
 static gvx_status plan_atlas(gvx_grid* g, const gvx_topo_plan& P)
 {
-    cudaStream_t st = g->stream;
     const uint32_t cap0 = P.cap[0];
     const DevCount nl = dc_dev(g->d_counts.as<uint32_t>(), 0, 1, cap0);
     GVX_CK_STATUS(gvx_grow_atlas(g, cap0));
@@ -2764,7 +2769,7 @@ gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool fr
     GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
 
     // ---- GetBoundingBox (read by gvx_topo_plan_finish)
-    const unsigned bb = (std::min(blocks_for(n, 256), 152u * 8u) + 2u) / 3u * 3u;
+    const unsigned bb = bbox_blocks(n);
     k_bbox<<<bb, 256, 0, st>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, 0.f, 0.f, 0.f,
                                g->d_bbox.as<uint32_t>(), g->d_err.as<uint32_t>());
     g->launches++;
