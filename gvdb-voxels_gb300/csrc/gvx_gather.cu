@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(kDirectWarps * 32) k_gather_direct(GatherDirec
         // (two floats an instruction; adding the negated voxel is subtracting it)
         auto nearest = [&](const float4 p) {
             const float2 e = __fadd2_rn(make_float2(p.x, p.y), nxy), e2 = square2(e);
-            const float exy = FP16 ? __fadd_rn(e2.x, e2.y) : fmaf(e.y, e.y, e2.x);
+            const float exy = FP16 ? __fadd_rn(e2.x, e2.y) : fmaf(e.x, e.x, e2.y);  // (as k_gather rounds)
 #pragma unroll
             for (int k = 0; k < 2; k++) {
                 const float2 ez = __fadd2_rn(make_float2(p.z, p.z), nz[k]), xy = make_float2(exy, exy);
