@@ -6,7 +6,7 @@
 // voxel at the same index-space position in whichever brick holds it, or the
 // boundary value when no brick does.  The reference finds that brick with a
 // full root-to-leaf descent per apron voxel; here the 26 neighbours of every
-// leaf are resolved once per topology (gvx_topology.cu, k_neighbors) and one
+// leaf are resolved once per topology (gvx_topology.cu, k_leaf_tables) and one
 // warp copies a brick's 6P^2-12P+8 apron voxels with loads/stores of the
 // channel's native element (float4 for FLOAT3/FLOAT4 channels).  The warp
 // first resolves the brick's 26 neighbour slots into shared memory; the

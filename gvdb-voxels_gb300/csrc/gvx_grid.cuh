@@ -125,6 +125,7 @@ struct gvx_grid {
     // leaves of many points (kDenseLeaf), bricks of 8: their points in cell order inside every octant
     int* leaf_dense = nullptr;      // per leaf 0, or 1 + its number among them (in leaf_oct's buffer); null: none are made
     uint32_t* dense_count = nullptr;
+    int64_t dense_leaves = -1;  // their number where a build has read it back (-1: not known)
     DevBuf cell_tab;                // per dense leaf the first sorted index of its 512 cells; the list of the dense leaves
     DevBuf leaf_slot;    // atlas slot per leaf, -1 if inactive
     DevBuf slot_leaf;    // leaf per atlas slot (active slots only)

@@ -60,6 +60,36 @@ inline int ceil_log2(int64_t v)
 
 }  // namespace
 
+// the threads' bounds (order-preserving bits) into out: warp, then block, then one atomic per block and bound
+// (6 addresses take every atomic)
+__device__ __forceinline__ void bbox_reduce(uint32_t mn[3], uint32_t mx[3], bool nan, uint32_t* out, uint32_t* err)
+{
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        for (int s = 16; s > 0; s >>= 1) {
+            mn[a] = min(mn[a], __shfl_xor_sync(0xFFFFFFFFu, mn[a], s));
+            mx[a] = max(mx[a], __shfl_xor_sync(0xFFFFFFFFu, mx[a], s));
+        }
+    }
+    __shared__ uint32_t s_b[32][6];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    if (lane == 0)
+        for (int a = 0; a < 3; a++) {
+            s_b[wid][a] = mn[a];
+            s_b[wid][3 + a] = mx[a];
+        }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        uint32_t v = s_b[0][threadIdx.x];
+        for (int w = 1; w < nw; w++) v = threadIdx.x < 3 ? min(v, s_b[w][threadIdx.x]) : max(v, s_b[w][threadIdx.x]);
+        if (threadIdx.x < 3)
+            atomicMin(&out[threadIdx.x], v);
+        else
+            atomicMax(&out[threadIdx.x], v);
+    }
+    if (nan) atomicOr(err, GVX_DERR_BADPOINT);
+}
+
 // ---------------------------------------------------------------------------
 // bounding box of pos + orig over ALL points (GetBoundingBox includes points
 // that the key kernel later drops)
@@ -123,31 +153,7 @@ __global__ void k_bbox(const char* pos, int off, int stride, uint32_t n, float o
             }
         }
     }
-    // warp, then block, then one atomic per block and bound (6 addresses take every atomic)
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        for (int s = 16; s > 0; s >>= 1) {
-            mn[a] = min(mn[a], __shfl_xor_sync(0xFFFFFFFFu, mn[a], s));
-            mx[a] = max(mx[a], __shfl_xor_sync(0xFFFFFFFFu, mx[a], s));
-        }
-    }
-    __shared__ uint32_t s_b[32][6];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    if (lane == 0)
-        for (int a = 0; a < 3; a++) {
-            s_b[wid][a] = mn[a];
-            s_b[wid][3 + a] = mx[a];
-        }
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        uint32_t v = s_b[0][threadIdx.x];
-        for (int w = 1; w < nw; w++) v = threadIdx.x < 3 ? min(v, s_b[w][threadIdx.x]) : max(v, s_b[w][threadIdx.x]);
-        if (threadIdx.x < 3)
-            atomicMin(&out[threadIdx.x], v);
-        else
-            atomicMax(&out[threadIdx.x], v);
-    }
-    if (nan) atomicOr(err, GVX_DERR_BADPOINT);
+    bbox_reduce(mn, mx, nan, out, err);
 }
 
 // compact level-0 key of every point (invalid points -> invalid_key, sorted
@@ -155,11 +161,15 @@ __global__ void k_bbox(const char* pos, int off, int stride, uint32_t n, float o
 // key is (leaf key << 3) | octant, octant = 4 hx + 2 hy + hz the half of the
 // brick (2^lb voxels) that the point's voxel lies in on every axis, so the
 // stable sort leaves every leaf's points in (octant, index) order; invalid_key
-// is the shifted one then
+// is the shifted one then.  BBOX: the bounding box too, as k_bbox (a planned build does not wait for it: one
+// launch and one pass over the positions less)
+template <bool BBOX>
 __global__ void k_keys(const char* pos, int off, int stride, uint32_t n, float ox, float oy, float oz,
                        KeySpace ks, float inv_b, int kshift, int lb, int passes, uint32_t invalid_key,
-                       uint32_t* keys, uint32_t* vals, uint32_t* hist, uint32_t* err)
+                       uint32_t* keys, uint32_t* vals, uint32_t* hist, uint32_t* bbox, uint32_t* err)
 {
+    uint32_t mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
+    bool nan = false;
     __shared__ uint32_t sh[4 * 256];
     for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) sh[i] = 0u;
     __syncthreads();
@@ -170,6 +180,14 @@ __global__ void k_keys(const char* pos, int off, int stride, uint32_t n, float o
         w[0] += ox;
         w[1] += oy;
         w[2] += oz;
+        if (BBOX) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                if (w[a] != w[a]) nan = true;
+                mn[a] = min(mn[a], f2ord(w[a]));
+                mx[a] = max(mx[a], f2ord(w[a]));
+            }
+        }
         uint32_t key = invalid_key;
         if (w[0] >= 0.f && w[1] >= 0.f && w[2] >= 0.f) {
             int c[3];
@@ -201,6 +219,7 @@ __global__ void k_keys(const char* pos, int off, int stride, uint32_t n, float o
     for (int i = threadIdx.x; i < passes * 256; i += blockDim.x)
         if (sh[i]) atomicAdd(&hist[i], sh[i]);
     if (degen) atomicOr(err, GVX_DERR_DEGENERATE);
+    if (BBOX) bbox_reduce(mn, mx, nan, bbox, err);
 }
 
 // first point of every run of equal valid leaf keys (sorted keys >> kshift) sets the key's bit
@@ -333,6 +352,9 @@ __global__ void k_upper_bits(const uint32_t* __restrict__ d0bits, const uint32_t
 }
 
 // ---------------------------------------------------------------------------
+// slots of d_counts: a planned UpdateAtlas's slot count, the dense leaves of the grouping
+enum { kCntSlots = 56, kCntDense = 57 };
+
 // The ranges of a ClearList: a block sets 4096 words of one of them, by 16 bytes where the range is aligned
 struct ClearArgs {
     ClearList c;
@@ -758,11 +780,10 @@ __global__ void k_write_nodes(TreeArgs t)
 // dense_list (optional): the leaves of kDenseLeaf points and more, in no order -- the keys are sorted, so
 // such a run reaches kDenseLeaf - 1 entries back from its last one
 constexpr int kDenseLeaf = 128;
-__global__ void k_group_runs(const uint32_t* __restrict__ skeys, uint32_t n, int kshift, uint32_t invalid_key,
-                             LeafLookup L, int2* leaf_range, int* leaf_oct, uint32_t* dense_list, uint32_t* dense_count)
+__device__ __forceinline__ void group_run(uint32_t i, const uint32_t* __restrict__ skeys, uint32_t n, int kshift,
+                                          uint32_t invalid_key, const LeafLookup& L, int2* leaf_range, int* leaf_oct,
+                                          uint32_t* dense_list, uint32_t* dense_count)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     const uint32_t sk = skeys[i], k = sk >> kshift;
     if (k >= invalid_key) return;
     const uint32_t prev = i == 0 ? 0xFFFFFFFFu : skeys[i - 1];
@@ -998,9 +1019,9 @@ __global__ void k_octant_partition(const int2* __restrict__ leaf_range, DevCount
 // 27-neighbourhood of every leaf (leaf pool indices, -1 where no leaf; all -1
 // for an inactive leaf, whose key is kNoKey)
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;
-__global__ void k_neighbors(const uint32_t* __restrict__ leaf_key, DevCount nl, LeafLookup L, int* nbr)
+__device__ __forceinline__ void leaf_neighbour(uint32_t t, const uint32_t* __restrict__ leaf_key, const DevCount& nl,
+                                               const LeafLookup& L, int* nbr)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t nleaves = nl.get();
     if (t >= nleaves * 27u) return;
     const uint32_t leaf = t / 27u, d = t % 27u;
@@ -1012,6 +1033,21 @@ __global__ void k_neighbors(const uint32_t* __restrict__ leaf_key, DevCount nl, 
     int c[3];
     ks_unpack(L.ks, key, 0, c);
     nbr[t] = ll_find(L, c[0] + (int)(d % 3u) - 1, c[1] + (int)((d / 3u) % 3u) - 1, c[2] + (int)(d / 9u) - 1);
+}
+
+// the neighbours of the leaves (the first nb blocks) and the runs of their points, which need no more of each
+// other than the lookup: one launch
+__global__ void k_leaf_tables(uint32_t nb, const uint32_t* __restrict__ leaf_key, DevCount nl, int* nbr,
+                              const uint32_t* __restrict__ skeys, uint32_t n, int kshift, uint32_t invalid_key,
+                              LeafLookup L, int2* leaf_range, int* leaf_oct, uint32_t* dense_list,
+                              uint32_t* dense_count)
+{
+    if (blockIdx.x < nb) {
+        leaf_neighbour(blockIdx.x * blockDim.x + threadIdx.x, leaf_key, nl, L, nbr);
+        return;
+    }
+    const uint32_t i = (blockIdx.x - nb) * blockDim.x + threadIdx.x;
+    if (i < n) group_run(i, skeys, n, kshift, invalid_key, L, leaf_range, leaf_oct, dense_list, dense_count);
 }
 
 // active leaves (mFlags) -> bitmap over pool indices
@@ -1450,7 +1486,7 @@ static gvx_status sort_points_scratch(gvx_grid* g, int n, const KeySpace& ks, Cl
     return gvx_sort_prepare(g->sort, (uint32_t)n, ks.total_bits + sort_shift(ks) + 1, clear);
 }
 
-static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpace& ks)
+static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpace& ks, bool bbox = false)
 {
     GVX_CK(gvx_ensure(g->keys[0], (size_t)n * 4));
     GVX_CK(gvx_ensure(g->keys[1], (size_t)n * 4));
@@ -1466,10 +1502,10 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
     // (400k points of a surface in 1216 blocks 13.6 us, in 390 6; 777k 12.8, in 759 8; 4M in 1216 23, in 304 33)
     const unsigned kb =
         std::min(blocks_for(n, 256), std::max(152u * 2u, std::min(blocks_for(n, 1024), 152u * 8u)));
-    k_keys<<<kb, 256, 0, g->stream>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, t[0], t[1], t[2],
-                                      ks, 1.0f / (float)g->brick, kshift, lb, passes, invalid_key,
-                                      g->keys[0].as<uint32_t>(), g->vals[0].as<uint32_t>(),
-                                      gvx_sort_hist_ptr(g->sort), g->d_err.as<uint32_t>());
+    (bbox ? k_keys<true> : k_keys<false>)<<<kb, 256, 0, g->stream>>>(
+        g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, t[0], t[1], t[2], ks, 1.0f / (float)g->brick,
+        kshift, lb, passes, invalid_key, g->keys[0].as<uint32_t>(), g->vals[0].as<uint32_t>(),
+        gvx_sort_hist_ptr(g->sort), g->d_bbox.as<uint32_t>(), g->d_err.as<uint32_t>());
     g->launches++;
     uint32_t* kk[2] = {g->keys[0].as<uint32_t>(), g->keys[1].as<uint32_t>()};
     uint32_t* vv[2] = {g->vals[0].as<uint32_t>(), g->vals[1].as<uint32_t>()};
@@ -1491,27 +1527,32 @@ static gvx_status sort_points(gvx_grid* g, int n, const float t[3], const KeySpa
 static gvx_status leaf_range_scratch(gvx_grid* g, uint32_t nleaves, ClearList& clear)
 {
     GVX_CK(gvx_ensure(g->leaf_range, (size_t)(nleaves + 1) * sizeof(int2)));
-    // (after the octants, and cleared with them: the dense numbers of the leaves, the dense leaves' count)
-    const size_t oct_words = (size_t)(nleaves + 1) * 9 + 1;
+    // (after the octants, and cleared with them: the dense numbers of the leaves)
+    const size_t oct_words = (size_t)(nleaves + 1) * 9;
     GVX_CK(gvx_ensure(g->leaf_oct, oct_words * sizeof(int)));
     clear.add(g->leaf_range.p, (uint64_t)(nleaves + 1) * 2, 0u);
     clear.add(g->leaf_oct.p, oct_words, 0u);
+    clear.add(g->d_counts.as<uint32_t>() + kCntDense, 1, 0u);
     return GVX_OK;
 }
 
-static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves)
+// (nl: the leaves' neighbours too, of that many)
+static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves, const DevCount* nl = nullptr)
 {
     const bool dense = g->key_shift && g->brick == 8;
     uint32_t* dense_list = nullptr;
     g->leaf_dense = dense ? g->leaf_oct.as<int>() + (size_t)(nleaves + 1) * 8 : nullptr;
-    g->dense_count = dense ? (uint32_t*)(g->leaf_dense + nleaves + 1) : nullptr;
+    g->dense_count = dense ? g->d_counts.as<uint32_t>() + kCntDense : nullptr;
+    g->dense_leaves = -1;
     if (dense) {
         const size_t most = g->n_sorted / kDenseLeaf + 1;
         GVX_CK(gvx_ensure(g->cell_tab, most * 513 * sizeof(int)));  // 512 cells a leaf, then the list of the leaves
         dense_list = g->cell_tab.as<uint32_t>() + most * 512;
     }
-    if (g->n_sorted) {
-        k_group_runs<<<blocks_for(g->n_sorted, 256), 256, 0, g->stream>>>(
+    const unsigned nb = nl ? blocks_for((uint64_t)nleaves * 27, 256) : 0u;
+    if (g->n_sorted || nb) {
+        k_leaf_tables<<<nb + blocks_for(g->n_sorted, 256), 256, 0, g->stream>>>(
+            nb, g->leaf_key.as<uint32_t>(), nl ? *nl : dc_host(0), g->nbr.as<int>(),
             g->keys[g->sorted_buf].as<uint32_t>(), g->n_sorted, g->key_shift, 1u << g->lookup.ks.total_bits,
             g->lookup, g->leaf_range.as<int2>(), g->leaf_oct.as<int>(),
             dense_list, g->dense_count);
@@ -1567,7 +1608,7 @@ gvx_status gvx_topo_octants(gvx_grid* g, const GvxSortedAttr* attr)
     memset(&none, 0, sizeof(none));
     const uint32_t nleaves = g->oct_leaves;
     if (g->key_shift) {
-        if (g->leaf_dense && g->n_sorted >= (uint32_t)kDenseLeaf) {
+        if (g->leaf_dense && g->n_sorted >= (uint32_t)kDenseLeaf && g->dense_leaves != 0) {
             k_cell_sort<<<std::min(g->n_sorted / kDenseLeaf, 152u * 4u), kCellThreads, 0, g->stream>>>(
                 g->cell_tab.as<uint32_t>() + ((size_t)g->n_sorted / kDenseLeaf + 1) * 512, g->dense_count, g->leaf_range.as<int2>(), g->pts.pos, g->pts.pos_off,
                 g->pts.pos_stride, g->sort_trans[0], g->sort_trans[1], g->sort_trans[2],
@@ -1756,7 +1797,7 @@ static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpac
 }
 
 // a full build in key space `ks` up to its node counts (d_counts), which are queued for the
-// host when queue_readback; its scratch (topo_full_scratch) is cleared.  lists (optional): room for the keys of
+// host when queue_readback (otherwise the bounding box is made too); its scratch (topo_full_scratch) is cleared.  lists (optional): room for the keys of
 // X0 (list_cap[0]), then of D_l and X_l (list_cap[l] each) per upper level
 static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const float o[3], int depth,
                                       const int rootpos[3], const KeySpace& ks, FullBuild& fb, bool queue_readback,
@@ -1770,7 +1811,7 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
     const UpperDesc& ud = fb.ud;
 
     // ---- one sort of the compact level-0 keys
-    gvx_status rc = sort_points(g, n, o, ks);
+    gvx_status rc = sort_points(g, n, o, ks, !queue_readback);
     if (rc) return rc;
     const uint32_t* skeys = g->keys[g->sorted_buf].as<uint32_t>();
     const uint32_t* svals = g->vals[g->sorted_buf].as<uint32_t>();
@@ -1969,13 +2010,9 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     g->lookup.cap = 0;
     g->lookup_valid = true;
     GVX_CK(gvx_ensure(g->nbr, (size_t)std::max<uint32_t>(L0, 1u) * 27 * sizeof(int)));
-    if (L0) {
-        k_neighbors<<<blocks_for((uint64_t)L0 * 27, 256), 256, 0, st>>>(g->leaf_key.as<uint32_t>(), dc_host(L0), g->lookup,
-                                                                        g->nbr.as<int>());
-        g->launches++;
-    }
     g->nbr_valid = true;
-    rc = fill_leaf_ranges(g, L0);
+    const DevCount nl = dc_host(L0);
+    rc = fill_leaf_ranges(g, L0, &nl);
     if (rc) return rc;
     g->group_valid = true;
     g->full_group_gen = g->topo_gen;
@@ -2070,13 +2107,9 @@ static gvx_status build_active_lookup(gvx_grid* g, const KeySpace& ks, uint32_t 
     g->lookup.cap = 0;
     g->lookup_valid = true;
     GVX_CK(gvx_ensure(g->nbr, (size_t)std::max<uint32_t>(L0, 1u) * 27 * sizeof(int)));
-    if (L0) {
-        k_neighbors<<<blocks_for((uint64_t)L0 * 27, 256), 256, 0, st>>>(g->leaf_key.as<uint32_t>(), dc_host(L0), g->lookup,
-                                                                        g->nbr.as<int>());
-        g->launches++;
-    }
     g->nbr_valid = true;
-    rc = fill_leaf_ranges(g, L0);
+    const DevCount nl = dc_host(L0);
+    rc = fill_leaf_ranges(g, L0, &nl);
     if (rc) return rc;
     if (readback == kReadUsed) {
         uint32_t used = 0;
@@ -2591,7 +2624,6 @@ void gvx_topo_staged_free(gvx_grid* g)
 // builds the grid again without a plan.
 
 enum { kRecCounts = 0, kRecBbox = kReadBbox, kRecErr = kReadErr, kRecWords = kReadWords };
-enum { kCntSlots = 56 };  // d_counts slot of a planned UpdateAtlas's slot count
 
 struct gvx_topo_plan {
     FullBuild fb;                      // key space, depth, root, points, radius (words0, ud after enqueue)
@@ -2707,11 +2739,8 @@ static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuil
     g->lookup.b_offset_p = dcnt;
     g->lookup.cap = cap0;
     GVX_CK(gvx_ensure(g->nbr, (size_t)cap0 * 27 * sizeof(int)));
-    k_neighbors<<<blocks_for((uint64_t)cap0 * 27, 256), 256, 0, st>>>(g->leaf_key.as<uint32_t>(),
-                                                                      dc_dev(dcnt, 0, 1, cap0), g->lookup,
-                                                                      g->nbr.as<int>());
-    g->launches++;
-    return fill_leaf_ranges(g, cap0);
+    const DevCount nl = dc_dev(dcnt, 0, 1, cap0);
+    return fill_leaf_ranges(g, cap0, &nl);
 }
 
 // UpdateAtlas where every leaf of the pool is active: leaf i in slot i, the other slots free (atlas map -1)
@@ -2768,13 +2797,8 @@ gvx_status gvx_topo_plan_enqueue(gvx_grid* g, const GvxSortedAttr* attr, bool fr
     GVX_CK_STATUS(leaf_range_scratch(g, cap0, clear));
     GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
 
-    // ---- GetBoundingBox (read by gvx_topo_plan_finish)
-    const unsigned bb = bbox_blocks(n);
-    k_bbox<<<bb, 256, 0, st>>>(g->pts.pos, g->pts.pos_off, g->pts.pos_stride, (uint32_t)n, 0.f, 0.f, 0.f,
-                               g->d_bbox.as<uint32_t>(), g->d_err.as<uint32_t>());
-    g->launches++;
-
-    // ---- the full build in the plan's key space, sized by the capacities
+    // ---- GetBoundingBox (read by gvx_topo_plan_finish) and the full build in the plan's key space, sized by
+    // the capacities
     size_t list_words = cap0;  // X0's keys, then those of D_l and X_l per upper level
     for (int l = 1; l < depth; l++) list_words += 2 * (size_t)P.cap[l];
     GVX_CK(gvx_ensure(g->lists, list_words * 4 + 4));
@@ -2913,6 +2937,7 @@ gvx_status gvx_topo_plan_finish(gvx_grid* g, bool* held, bool frame)
     g->last_rebuild = 1;
     g->oct_leaves = (uint32_t)cnt[0];
     g->perm_valid = false;
+    g->dense_leaves = (int64_t)rec[kRecCounts + kCntDense];
     if (!frame) {  // the topology alone: UpdateAtlas and the octant pass are the caller's next calls
         g->atlas_valid = false;
         g->atlas_prefix = -1;
