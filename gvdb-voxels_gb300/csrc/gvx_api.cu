@@ -230,7 +230,7 @@ gvx_status gvx_destroy(gvx_grid* g)
                       &g->own_w[0], &g->own_r[0], &g->own_pos[1], &g->own_vel[1], &g->own_w[1], &g->own_r[1],
                       &g->keys[0], &g->keys[1], &g->vals[0], &g->vals[1], &g->spos, &g->svel,
                       &g->sort.buf, &g->d0_bits,
-                      &g->d0_prefix, &g->x0_bits, &g->x0_prefix, &g->masks, &g->upper, &g->lists, &g->tmp_scan,
+                      &g->d0_prefix, &g->x0_bits, &g->x0_prefix, &g->upper, &g->lists, &g->tmp_scan,
                       &g->d_counts, &g->d_rmax, &g->d_next, &g->push_tab, &g->touched, &g->dense_units, &g->cell_tab, &g->host_stage,
                       &g->api_keys[0], &g->api_keys[1], &g->api_vals[0], &g->api_vals[1], &g->lk_bits, &g->lk_prefix,
                       &g->inc0, &g->inc_remap, &g->sc_cnt, &g->sc_off, &g->sc_keys[0], &g->sc_keys[1],

@@ -177,7 +177,7 @@ struct gvx_grid {
     SortScratch sort;
 
     // scratch of the topology build
-    DevBuf d0_bits, d0_prefix, x0_bits, x0_prefix, masks, upper, lists, tmp_scan, d_counts;
+    DevBuf d0_bits, d0_prefix, x0_bits, x0_prefix, upper, lists, tmp_scan, d_counts;
     DevBuf inc0, inc_remap;  // incremental build: linked + new level-0 bitmaps, linked rank -> pool index
     DevBuf d_err, d_bbox;  // (inside d_counts)
     DevBuf d_rmax;  // float bits of the largest per-point radius of the last point permute

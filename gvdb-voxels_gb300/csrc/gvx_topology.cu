@@ -222,83 +222,148 @@ __global__ void k_keys(const char* pos, int off, int stride, uint32_t n, float o
     if (BBOX) bbox_reduce(mn, mx, nan, bbox, err);
 }
 
-// first point of every run of equal valid leaf keys (sorted keys >> kshift) sets the key's bit
-__global__ void k_mark_runs(const uint32_t* __restrict__ skeys, uint32_t n, int kshift, uint32_t invalid_key,
-                            uint32_t* bits)
+// The cells of a build, from the sorted keys (>> kshift: leaf keys): the first point of every run of equal
+// valid ones sets its bit in d0bits.  BOX: also the leaves touched by the points' boxes
+// [int(p)-r, int(p)+2r] (cuda_gvdb_particles.cuh:481-482; hi_mul = 2 for the full rebuild's box, 1 for the
+// incremental box [int(p)-r, int(p)+r], PT.cuh:433-434) in x0bits, the points' own leaves among them (the
+// ranks leave those out).  A point's leaves are 27 bits (dz+1)*9 + (dy+1)*3 + (dx+1); a warp's points of one
+// leaf join theirs, and nine lanes a leaf set them, a lane the three along z, which are neighbours in a word;
+// leaves of one word, side by side in the sorted order, are joined first where a warp has two of them and more
+// a word: a word's nine rows cost 110 instructions, a leaf's a third of 40 and nine atomics of L2 (4M points
+// in 777k leaves: 130 us leaf by leaf, 100 so; 300k points of a depth frame 7.4 and 8.5, always by words 13).
+// lim: per axis, the first key-space coordinate past the root (a key space rounded up to powers of two may
+// reach past it).
+// The marks used to wait for the ranks of d0bits, which numbered a mask per leaf: three launches more, and
+// two passes over the ranks (6k points a frame 96 us, 81 so; 6M points: 111 us of kernels, 90 so).
+template <bool BOX>
+__global__ void __launch_bounds__(256)
+    k_mark_cells(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals, uint32_t n, int kshift,
+                 uint32_t invalid_key, const char* pos, int off, int stride, float ox, float oy, float oz,
+                 float radius, float hi_mul, int lb, KeySpace ks, int3 lim, uint32_t* d0bits, uint32_t* x0bits,
+                 uint32_t* err)
 {
+    constexpr uint32_t kFull = 0xFFFFFFFFu;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t k = skeys[i] >> kshift;
-    if (k >= invalid_key) return;
-    if (i == 0 || (skeys[i - 1] >> kshift) != k) atomicOr(&bits[k >> 5], 1u << (k & 31));
-}
-
-// dilation mask of every direct leaf: OR over its points of the leaves touched
-// by the box [int(p)-r, int(p)+2r] (cuda_gvdb_particles.cuh:481-482), encoded
-// as 27 bits (dz+1)*9 + (dy+1)*3 + (dx+1)
-// (hi_mul = 2 for the full rebuild's box, 1 for the incremental box [int(p)-r, int(p)+r], PT.cuh:433-434)
-__global__ void k_point_masks(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals, uint32_t n,
-                              int kshift, uint32_t invalid_key, BitRank d0, const char* pos, int off, int stride,
-                              float ox, float oy, float oz, float radius, float hi_mul, int brick, uint32_t* masks)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < n;
-    uint32_t key = live ? skeys[i] >> kshift : invalid_key;
+    const int lane = threadIdx.x & 31;
+    const uint32_t key = i < n ? skeys[i] >> kshift : invalid_key;
     const bool valid = key < invalid_key;
+    uint32_t prev = __shfl_up_sync(kFull, key, 1);
+    if (lane == 0) prev = valid && i > 0 ? skeys[i - 1] >> kshift : invalid_key;
+    if (valid && prev != key) atomicOr(&d0bits[key >> 5], 1u << (key & 31));
+    if (!BOX) return;
     uint32_t m = 0u;
-    int leaf = -1;
     if (valid) {
-        leaf = (int)br_rank(d0, key);
         float w[3];
         load_pos(pos, off, stride, svals[i], w);
         w[0] += ox;
         w[1] += oy;
         w[2] += oz;
-        int lo[3], hi[3];
+        uint32_t ax[3];  // per axis, bits 0 to 2: the leaf below, the own one, the one above
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const int ip = (int)w[a];
             const int bmin = (int)((float)ip - radius);
             const int bmax = (int)((float)ip + hi_mul * radius);
-            const int cl = ip / brick;
-            lo[a] = bmin / brick - cl;  // C truncation, as bmin/rres*rres
-            hi[a] = bmax / brick - cl;
-            lo[a] = max(lo[a], -1);
-            hi[a] = min(hi[a], 1);
+            // C truncation of x / brick, as bmin/rres*rres
+            auto cell = [&](int x) { return (x + ((x >> 31) & ((1 << lb) - 1))) >> lb; };
+            const int cl = cell(ip);
+            const int lo = max(cell(bmin) - cl, -1), hi = min(cell(bmax) - cl, 1);
+            ax[a] = lo > hi ? 0u : (7u << (lo + 1)) & (7u >> (1 - hi));
         }
-        for (int dz = lo[2]; dz <= hi[2]; dz++)
-            for (int dy = lo[1]; dy <= hi[1]; dy++)
-                for (int dx = lo[0]; dx <= hi[0]; dx++) m |= 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
+        const uint32_t y = (ax[1] & 1u) | (ax[1] & 2u) << 2 | (ax[1] & 4u) << 4;
+        const uint32_t zz = (ax[2] & 1u) | (ax[2] & 2u) << 8 | (ax[2] & 4u) << 16;
+        m = ax[0] * y * zz;  // (copies side by side: no carries)
     }
-    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, valid ? (uint32_t)leaf : 0xFFFFFFFFu);
-    const uint32_t agg = __reduce_or_sync(peers, m);
-    const int lane = threadIdx.x & 31;
-    if (valid && lane == __ffs(peers) - 1) atomicOr(&masks[leaf], agg);
-}
-
-// leaves of the dilation boxes that hold no point -> X0 bitmap; lim: per axis, the first key-space
-// coordinate past the root (a key space rounded up to powers of two may reach past it)
-__global__ void k_dilate(const uint32_t* __restrict__ dlist, const uint32_t* __restrict__ count, KeySpace ks,
-                         int3 lim, const uint32_t* __restrict__ masks, BitRank d0, uint32_t* x0bits, uint32_t* err)
-{
-    // grid-stride over the leaves (their count is on the device; the grid is sized for the points)
-    const uint32_t cnt = *count, stride = gridDim.x * blockDim.x;
-    bool degen = false;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < cnt; j += stride) {
-        const uint32_t m = masks[j] & ~(1u << 13);
-        if (!m) continue;
-        int c[3];
-        ks_unpack(ks, dlist[j], 0, c);
-        for (int b = 0; b < 27; b++) {
-            if (!((m >> b) & 1u)) continue;
-            const int nx = c[0] + (b % 3) - 1, ny = c[1] + (b / 3) % 3 - 1, nz = c[2] + b / 9 - 1;
-            if (nx < 0 || ny < 0 || nz < 0 || nx >= lim.x || ny >= lim.y || nz >= lim.z) {
-                degen = true;  // the reference descends outside the root here
-                continue;
+    const bool first = valid && (lane == 0 || prev != key);
+    uint32_t runs = __ballot_sync(kFull, first);
+    // equal keys are side by side: a run's first lane gets the masks of the lanes after it
+    const uint32_t after = runs & ~((2u << lane) - 1u);
+    const int end = after ? __ffs(after) - 1 : 32;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t m2 = __shfl_down_sync(kFull, m, o);
+        if (lane + o < end) m |= m2;
+    }
+    bool degen = false;  // a leaf outside the root: the reference descends there
+    m &= ~(1u << 13);    // (the point's own leaf)
+    int c[3];
+    ks_unpack(ks, key, 0, c);
+    const uint32_t layers = (c[2] > 0 && c[2] - 1 < lim.z ? 0x1FFu : 0u) | (c[2] < lim.z ? 0x1FFu << 9 : 0u) |
+                            (c[2] + 1 < lim.z ? 0x1FFu << 18 : 0u);
+    if (m & ~layers) degen = true;
+    m &= layers;
+    uint32_t words = __ballot_sync(kFull, first && (lane == 0 || (prev ^ key) >> 5));
+    if (ks.bits[2] >= 5 && 2 * __popc(words) < __popc(runs)) {
+        // several leaves of one word (of one x and y): their nine rows, joined over the warp
+        const int b = (int)(key & 31u);
+        uint32_t rows = __reduce_or_sync(kFull, first ? m : 0u);
+        rows |= rows >> 9 | rows >> 18;
+        while (words) {
+            const int src = __ffs(words) - 1;
+            words &= words - 1u;
+            const uint32_t W = __shfl_sync(kFull, key, src) >> 5;
+            const bool mine = first && key >> 5 == W;
+            int wc[3];
+            ks_unpack(ks, W << 5, 0, wc);
+            uint32_t row = 0u;  // lane r < 9: the bits of row r
+#pragma unroll
+            for (int r = 0; r < 9; r++) {
+                if (!((rows >> r) & 1u)) continue;
+                uint32_t z = mine ? m >> r : 0u;
+                z = (z & 1u) | (z >> 8 & 2u) | (z >> 16 & 4u);
+                const uint32_t bits = b == 0 ? z >> 1 : (b == 31 ? (z & 3u) << 30 : z << (b - 1));
+                const uint32_t all = __reduce_or_sync(kFull, bits);
+                if (lane == r) row = all;
+                // past the word's ends
+                if (z && (b == 0 || b == 31)) {
+                    const int nx = wc[0] + r % 3 - 1, ny = wc[1] + r / 3 - 1;
+                    if (nx < 0 || ny < 0 || nx >= lim.x || ny >= lim.y) {
+                        degen = true;
+                    } else {
+                        const uint32_t k = ks_pack(ks, nx, ny, c[2], 0);
+                        if (b == 0 && (z & 1u)) atomicOr(&x0bits[(k >> 5) - 1u], 0x80000000u);
+                        if (b == 31 && (z & 4u)) atomicOr(&x0bits[(k >> 5) + 1u], 1u);
+                    }
+                }
             }
-            const uint32_t nk = ks_pack(ks, nx, ny, nz, 0);
-            if (!br_test(d0, nk)) atomicOr(&x0bits[nk >> 5], 1u << (nk & 31));
+            if (row) {
+                const int nx = wc[0] + lane % 3 - 1, ny = wc[1] + lane / 3 - 1;
+                if (nx < 0 || ny < 0 || nx >= lim.x || ny >= lim.y)
+                    degen = true;
+                else
+                    atomicOr(&x0bits[ks_pack(ks, nx, ny, wc[2], 0) >> 5], row);
+            }
         }
+        runs = 0u;
+    }
+    const int dx = lane % 3 - 1, dy = lane / 3 % 3 - 1;
+    while (runs) {
+        // three runs a turn, nine lanes each
+        const int l0 = __ffs(runs) - 1;
+        runs &= runs - 1u;
+        const int l1 = __ffs(runs) - 1;
+        runs &= runs - 1u;  // (0 stays 0)
+        const int l2 = __ffs(runs) - 1;
+        runs &= runs - 1u;
+        const int src = lane < 9 ? l0 : lane < 18 ? l1 : lane < 27 ? l2 : -1;
+        const uint32_t gm = __shfl_sync(kFull, m, max(src, 0)), gk = __shfl_sync(kFull, key, max(src, 0));
+        // bits 0, 1, 2: the leaves below, beside and above
+        uint32_t z = gm >> ((dy + 1) * 3 + dx + 1);
+        z = (z & 1u) | (z >> 8 & 2u) | (z >> 16 & 4u);
+        if (src < 0 || z == 0u) continue;
+        int gc[3];
+        ks_unpack(ks, gk, 0, gc);
+        const int nx = gc[0] + dx, ny = gc[1] + dy;
+        if (nx < 0 || ny < 0 || nx >= lim.x || ny >= lim.y) {
+            degen = true;
+            continue;
+        }
+        const uint32_t k = ks_pack(ks, nx, ny, gc[2], 0);
+        const int b = (int)(k & 31u);
+        const uint32_t here = b == 0 ? z >> 1 : (b == 31 ? (z & 3u) << 30 : z << (b - 1));
+        if (here) atomicOr(&x0bits[k >> 5], here);
+        if (b == 0 && (z & 1u)) atomicOr(&x0bits[(k >> 5) - 1u], 0x80000000u);
+        if (b == 31 && (z & 4u)) atomicOr(&x0bits[(k >> 5) + 1u], 1u);
     }
     if (degen) atomicOr(err, GVX_DERR_DEGENERATE);
 }
@@ -347,8 +412,9 @@ __global__ void k_upper_bits(const uint32_t* __restrict__ d0bits, const uint32_t
 {
     const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= words) return;
-    const uint32_t* bits = blockIdx.y ? x0bits : d0bits;
-    upper_word(bits[w], w, ks, ud, upper, (int)blockIdx.y);
+    uint32_t bits = d0bits[w];
+    if (blockIdx.y) bits = x0bits[w] & ~bits;
+    upper_word(bits, w, ks, ud, upper, (int)blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -414,7 +480,7 @@ static void clear_bboxes(gvx_grid* g, ClearList& c)
 // Exclusive prefix sums of several arrays in one go (of the popcounts of bitmap words, or of the words): a
 // job each.  A job's word may be put together from bitmaps, (src | plus) & ~minus, and is stored then (store
 // may be src: the value is the same again).  With `list` the set bits' keys, in order, go there (cap at
-// most), and zero[0 .. keys) is cleared.
+// most).
 //
 // Up to 32 blocks of 1024 words a job (a key space of 2^20 leaves), one launch does it: a block sums the
 // words before its own by itself, 31 loads a thread at most, which takes less than the launch that would
@@ -429,7 +495,6 @@ struct PfxJob {
     uint32_t* total;
     uint32_t* list;
     uint32_t cap;
-    uint32_t* zero;
     uint32_t sums;  // where its block sums start (two launches)
 };
 struct PfxJobs {
@@ -439,7 +504,7 @@ struct PfxJobs {
     PfxJob& add(const uint32_t* src, uint32_t* prefix, uint32_t words, uint32_t* total)
     {
         PfxJob& q = j[n++];
-        q = PfxJob{src, nullptr, nullptr, nullptr, prefix, words, total, nullptr, 0xFFFFFFFFu, nullptr, 0u};
+        q = PfxJob{src, nullptr, nullptr, nullptr, prefix, words, total, nullptr, 0xFFFFFFFFu, 0u};
         return q;
     }
 };
@@ -582,7 +647,6 @@ __global__ void __launch_bounds__(THREADS) k_pfx_apply(PfxJobs jobs, const uint3
             while (b && o < q.cap) {  // cap: the list's capacity
                 const int bit = __ffs(b) - 1;
                 b &= b - 1u;
-                if (q.zero) q.zero[o] = 0u;
                 q.list[o++] = w * 32u + (uint32_t)bit;
             }
         }
@@ -1643,7 +1707,7 @@ gvx_status gvx_topo_octants(gvx_grid* g, const GvxSortedAttr* attr)
     return GVX_OK;
 }
 
-// k_dilate's per-axis limit: the key space's end or the root's (rootpos in voxels, the root's
+// k_mark_cells' per-axis limit: the key space's end or the root's (rootpos in voxels, the root's
 // side in leaves), whichever comes first
 static int3 dilate_limit(const KeySpace& ks, const int rootpos[3], int brick, int root_leaves)
 {
@@ -1651,6 +1715,16 @@ static int3 dilate_limit(const KeySpace& ks, const int rootpos[3], int brick, in
     for (int a = 0; a < 3; a++)
         l[a] = (int)std::min<int64_t>(int64_t(1) << ks.bits[a], (int64_t)rootpos[a] / brick + root_leaves - ks.lo[a]);
     return make_int3(l[0], l[1], l[2]);
+}
+
+// k_mark_cells over the sorted points (hi_mul 0: no boxes)
+static void mark_cells(gvx_grid* g, int n, const float o[3], const KeySpace& ks, float radius, float hi_mul, int3 lim)
+{
+    (hi_mul > 0.f ? k_mark_cells<true> : k_mark_cells<false>)<<<blocks_for(n, 256), 256, 0, g->stream>>>(
+        g->keys[g->sorted_buf].as<uint32_t>(), g->vals[g->sorted_buf].as<uint32_t>(), (uint32_t)n, g->key_shift,
+        1u << ks.total_bits, g->pts.pos, g->pts.pos_off, g->pts.pos_stride, o[0], o[1], o[2], radius, hi_mul,
+        g->logdim[0], ks, lim, g->d0_bits.as<uint32_t>(), g->x0_bits.as<uint32_t>(), g->d_err.as<uint32_t>());
+    g->launches++;
 }
 
 static gvx_status grow_nodes(gvx_grid* g, int lev, int64_t cnt)
@@ -1773,7 +1847,6 @@ static gvx_status topo_full_scratch(gvx_grid* g, int n, int depth, const KeySpac
     GVX_CK(gvx_ensure(g->d0_prefix, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->x0_bits, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->x0_prefix, (size_t)words0 * 4));
-    GVX_CK(gvx_ensure(g->masks, (size_t)std::max(n, 1) * 4));
     GVX_CK(gvx_ensure(g->leaf_key, (size_t)std::max(n, 1) * 4));
     UpperDesc ud;
     memset(&ud, 0, sizeof(ud));
@@ -1807,47 +1880,27 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
     const int b = g->brick;
     const bool extra = radius >= 1.0f;
     const uint32_t words0 = fb.words0;
-    const uint32_t invalid_key = 1u << ks.total_bits;
     const UpperDesc& ud = fb.ud;
 
     // ---- one sort of the compact level-0 keys
     gvx_status rc = sort_points(g, n, o, ks, !queue_readback);
     if (rc) return rc;
-    const uint32_t* skeys = g->keys[g->sorted_buf].as<uint32_t>();
-    const uint32_t* svals = g->vals[g->sorted_buf].as<uint32_t>();
     uint32_t* counts = g->d_counts.as<uint32_t>();
 
-    // ---- D0: leaves holding points
-    k_mark_runs<<<blocks_for(n, 256), 256, 0, st>>>(skeys, (uint32_t)n, g->key_shift, invalid_key,
-                                                    g->d0_bits.as<uint32_t>());
-    g->launches++;
+    // ---- D0: leaves holding points; A0: the dilation leaves with them (radius >= 1, VG.cpp:1207-1208)
     BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
-    PfxJobs direct;
-    PfxJob& dj = direct.add(d0.bits, d0.prefix, words0, counts + 0);
-    dj.list = g->leaf_key.as<uint32_t>();
-    dj.zero = g->masks.as<uint32_t>();
-    rc = pfx_run<true>(direct, g->tmp_scan, st, &g->launches);
-    if (rc) return rc;
-
-    // ---- X0: dilation leaves (radius >= 1, VG.cpp:1207-1208)
     BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
-    if (extra) {
-        k_point_masks<<<blocks_for(n, 256), 256, 0, st>>>(skeys, svals, (uint32_t)n, g->key_shift, invalid_key, d0, g->pts.pos,
-                                                          g->pts.pos_off, g->pts.pos_stride, o[0], o[1], o[2],
-                                                          radius, 2.0f, b, g->masks.as<uint32_t>());
-        k_dilate<<<std::min(blocks_for(n, 256), 152u * 8u), 256, 0, st>>>(
-            g->leaf_key.as<uint32_t>(), counts + 0, ks, dilate_limit(ks, rootpos, b, g->range[depth] / b),
-            g->masks.as<uint32_t>(), d0, x0.bits, g->d_err.as<uint32_t>());
-        g->launches += 2;
-    }
+    mark_cells(g, n, o, ks, radius, extra ? 2.0f : 0.0f, dilate_limit(ks, rootpos, b, g->range[depth] / b));
+
     // ---- upper levels: parents of D0 (direct) and of X0 (extra)
     if (ud.nlev > 0) {
         k_upper_bits<<<dim3(blocks_for(words0, 256), extra ? 2 : 1), 256, 0, st>>>(d0.bits, x0.bits, words0, ks, ud,
                                                                                    g->upper.as<uint32_t>());
         g->launches++;
     }
-    // ---- ranks of X0, D_l and X_l = A_l & ~D_l, and their counts; the keys too where the lists have their room
+    // ---- ranks of D_l and X_l = A_l & ~D_l, and their counts; the keys too where the lists have their room
     PfxJobs ranks;
+    ranks.add(d0.bits, d0.prefix, words0, counts + 0).list = g->leaf_key.as<uint32_t>();
     uint32_t* lp = lists;
     auto listed = [&](PfxJob& q, uint32_t cap) {
         if (!lists) return;
@@ -1855,7 +1908,10 @@ static gvx_status topo_full_launch_ks(gvx_grid* g, int n, float radius, const fl
         q.cap = cap;
         lp += cap;
     };
-    listed(ranks.add(x0.bits, x0.prefix, words0, counts + 1), list_cap ? list_cap[0] : 0u);
+    PfxJob& xj = ranks.add(x0.bits, x0.prefix, words0, counts + 1);
+    xj.minus = d0.bits;
+    xj.store = x0.bits;
+    listed(xj, list_cap ? list_cap[0] : 0u);
     for (int l = 1; l <= ud.nlev; l++) {
         uint32_t* base = g->upper.as<uint32_t>() + ud.off[l];
         const uint32_t w = ud.words[l];
@@ -2043,7 +2099,7 @@ static gvx_status topo_full(gvx_grid* g, int n, float radius, const float o[3], 
 }
 
 // slots of d_counts read back by the incremental build
-enum { kCntNew = 0, kCntD0 = 20, kCntActive = 48 };
+enum { kCntNew = 0, kCntActive = 48 };
 
 // grows a pool buffer keeping its first `keep` bytes (PoolAlloc "preserve
 // existing on expand", VG.cpp:1096)
@@ -2177,15 +2233,12 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
     }
     ks.total_bits = (int)total_bits;
     const uint32_t words0 = std::max<uint32_t>(1u, (uint32_t)((1ull << total_bits) / 32ull));
-    const uint32_t invalid_key = 1u << ks.total_bits;
 
     // ---- scratch: D0 / X0 (touched level-0 cells), L0 / N0 (linked / new), upper levels
     GVX_CK(gvx_ensure(g->d0_bits, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->d0_prefix, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->x0_bits, (size_t)words0 * 4));
     GVX_CK(gvx_ensure(g->inc0, (size_t)words0 * 16));
-    GVX_CK(gvx_ensure(g->masks, (size_t)std::max(n, 1) * 4));
-    GVX_CK(gvx_ensure(g->lists, (size_t)std::max(n, 1) * 4));
     ClearList clear;
     clear.add(g->d0_bits.p, words0, 0u);
     clear.add(g->x0_bits.p, words0, 0u);
@@ -2213,28 +2266,8 @@ static gvx_status topo_incremental(gvx_grid* g, int n, float radius, const float
     // ---- touched cells: the points' leaves (D0) and their boxes [int(p)-r, int(p)+r] (X0), PT.cuh:420-465
     gvx_status rc = sort_points(g, n, o, ks);
     if (rc) return rc;
-    const uint32_t* skeys = g->keys[g->sorted_buf].as<uint32_t>();
-    const uint32_t* svals = g->vals[g->sorted_buf].as<uint32_t>();
-    k_mark_runs<<<blocks_for(n, 256), 256, 0, st>>>(skeys, (uint32_t)n, g->key_shift, invalid_key,
-                                                    g->d0_bits.as<uint32_t>());
-    g->launches++;
-    const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
-    uint32_t* dlist = g->lists.as<uint32_t>();
-    PfxJobs direct;
-    PfxJob& dj = direct.add(d0.bits, d0.prefix, words0, counts + kCntD0);
-    dj.list = dlist;
-    dj.zero = g->masks.as<uint32_t>();
-    rc = pfx_run<true>(direct, g->tmp_scan, st, &g->launches);
-    if (rc) return rc;
-    if (radius > 0.f) {
-        k_point_masks<<<blocks_for(n, 256), 256, 0, st>>>(skeys, svals, (uint32_t)n, g->key_shift, invalid_key, d0, g->pts.pos,
-                                                          g->pts.pos_off, g->pts.pos_stride, o[0], o[1], o[2],
-                                                          radius, 1.0f, b, g->masks.as<uint32_t>());
-        k_dilate<<<std::min(blocks_for(n, 256), 152u * 8u), 256, 0, st>>>(
-            dlist, counts + kCntD0, ks, dilate_limit(ks, g->root_pos, b, g->range[R] / b), g->masks.as<uint32_t>(), d0,
-            g->x0_bits.as<uint32_t>(), err);
-        g->launches += 2;
-    }
+    const BitRank d0{g->d0_bits.as<uint32_t>(), nullptr, words0};
+    mark_cells(g, n, o, ks, radius, radius > 0.f ? 1.0f : 0.0f, dilate_limit(ks, g->root_pos, b, g->range[R] / b));
     if (ud.nlev > 0) {
         k_upper_bits<<<dim3(blocks_for(words0, 256), radius > 0.f ? 2 : 1), 256, 0, st>>>(
             d0.bits, g->x0_bits.as<uint32_t>(), words0, ks, ud, upper);
