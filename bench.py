@@ -426,7 +426,7 @@ def run_ours(args, rank, world, pool):
         "hbm_gbs_step": (b_topo + b_pts + b_atlas + b_apron) / (ms * 1e-3) / 1e9,
         "active_bricks": nb,
         "active_bricks_per_frame": nb_frames,
-        "roofline": {"kernel": "k_splat_slab (cubic, density+velocity)", "bound": "hbm", "achieved": achieved,
+        "roofline": {"kernel": "k_splat_cells (cubic, density+velocity)", "bound": "hbm", "achieved": achieved,
                      "peak": peak, "peak_source": peak_src, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "algorithmic_bytes": splat_bytes, "launch_ms": splat_avg,
                      "bytes_model": "24 B per point (position, velocity) + P^3 * 20 B per active brick (density "

@@ -1,8 +1,8 @@
 // gvx_splat.cu -- point -> brick-atlas splats.
 //
 // Modes
-//   TRILINEAR, CUBIC (no reference counterpart): one warp per z-slab of an
-//     active PADDED brick PULLS the points of the brick's 27-neighbourhood
+//   TRILINEAR, CUBIC (no reference counterpart): one warp per unit, a z-slab of an
+//     active PADDED brick or the whole brick, PULLS the points of the brick's 27-neighbourhood
 //     (points are grouped by brick by the topology sort), keeps those whose
 //     footprint reaches its slab, and adds them into a shared-memory copy of
 //     the slab in their global sorted order, one point at a time across the
@@ -15,7 +15,8 @@
 //   REF_SCATTER: ScatterDensity semantics (gvdb_volume_gvdb.cpp:5624-5660,
 //     cuda_gvdb_particles.cuh:516-573): (1 - d^2/r^2)^3 at the point's voxel
 //     and its 6 face neighbours, inside the point's own padded brick, summed
-//     in shared memory instead of the reference's racy surface read-modify-write.
+//     by reductions in L2 (bricks of few points) or in shared memory instead of the reference's racy surface
+//     read-modify-write.
 //
 // Sample convention of all modes: voxel v of the index space is sampled at the
 // integer coordinate v (as gvdbGatherDensity, cuda_gvdb_particles.cuh:705).
@@ -1317,7 +1318,7 @@ __global__ void __launch_bounds__(kTriWarps * 32, kTriMinBlocks) k_splat_tri(Spl
         [&](uint32_t) -> const SplatArgs& { return a; });
 }
 
-// the same over many grids: ustart as in k_splat_batch, the counters after it
+// the same over many grids: ustart as in k_splat_cells_batch, the counters after it
 __global__ void __launch_bounds__(kTriWarps * 32, kTriMinBlocks)
     k_splat_tri_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
