@@ -1,5 +1,5 @@
-"""GPU test of the ranks and key lists of a build on both sides of the size (2^20 leaf cells) from which their
-sums take a launch of their own: a first build, a planned one, and appended frames, against the oracle."""
+"""GPU test of the ranks and key lists of a build on both sides of the sizes (2^20, 2^25 leaf cells) from which their
+sums take a launch of their own, and larger blocks: a first build, a planned one, and appended frames, against the oracle."""
 import numpy as np
 import pytest
 
@@ -19,7 +19,8 @@ def _points(n, box, seed):
 
 @pytest.mark.parametrize("radius", [0.0, 2.0])
 @pytest.mark.parametrize("box,n", [((100, 100, 100), 40), ((240, 500, 500), 3000), ((1000, 1000, 500), 3000),
-                                   ((1000, 1000, 1000), 3000), ((2000, 1000, 1000), 60_000)])
+                                   ((1000, 1000, 1000), 3000), ((2000, 1000, 1000), 60_000),
+                                   ((4000, 4000, 2000), 3000)])
 def test_builds_against_the_oracle(gvx_mod, orc, box, n, radius):
     g = gvx_mod.Grid(0)
     g.configure(LOGDIM)
