@@ -37,8 +37,8 @@ struct ApronArgs {
 // What bounds it: the lines of the bricks, nearly every sector of which an apron row's end touches (read
 // and written once: 57k bricks of 4 KB in 70 us at the copy rate), and the chain of loads before a
 // brick's first copy.  The brick of a warp's next turn has its neighbours' slots looked up while the
-// current one is copied (57k bricks: 105 us before, 101 with it).  4-byte voxels of any type are copied as words (uchar4
-// voxels, moved byte by byte, took 249 us).
+// current one is copied (57k bricks: 105 us before, 101 with it).  4-byte voxels of any type are copied as
+// words (uchar4 voxels, moved byte by byte, took 249 us).
 template <class T>
 __global__ void __launch_bounds__(kApronWarps * 32) k_apron(ApronArgs a, T boundval)
 {
