@@ -466,7 +466,8 @@ __device__ __forceinline__ void unit_ranges(const SplatUnit& t, int lane, int of
     if (t.end > t.start) rs[__popc(some & ((1u << lane) - 1u))] = t.start - off;
 }
 // sorted index of candidate base + lane: its range is the number of ranges with points that start at or
-// before it, less one
+// before it, less one.  base is below the candidates' count: the first range with points then starts at or
+// before every candidate asked for (without candidates there is none, and rs is not to be read)
 __device__ __forceinline__ int unit_candidate(const SplatUnit& t, int lane, int off, int base, const int* rs)
 {
     const bool some = t.end > t.start;
@@ -839,7 +840,7 @@ __device__ __forceinline__ void cell_unit(const SplatArgs& a, const SplatUnit& t
     uint32_t touched = 0u;
     for (int base = 0;; base += 32) {
         const bool done = base >= total;  // one more pass deals the last hits
-        const int idx = unit_candidate(t, lane, off, base, rs);
+        const int idx = done ? 0 : unit_candidate(t, lane, off, base, rs);
         bool hit = false;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
         if (base + lane < total) {
