@@ -264,6 +264,8 @@ void gvx_topo_plan_replayed(gvx_grid* g);  // its captured build was launched ag
 gvx_status gvx_topo_plan_finish(gvx_grid* g, bool* held, bool frame);
 void gvx_topo_plan_free(gvx_grid* g);
 uint64_t gvx_topo_plan_id(const gvx_grid* g);  // changes whenever the plan is made again
+// where a planned build puts the dense numbers of its leaves (gvx_grid::leaf_dense), while no buffer moves
+int* gvx_topo_plan_dense(const gvx_grid* g);
 // device count of the atlas slots a planned build assigns (clamped to *cap by the reader)
 const uint32_t* gvx_topo_plan_slots(const gvx_grid* g, uint32_t* cap);
 // InsertPoints: grouping + sorted attribute arrays

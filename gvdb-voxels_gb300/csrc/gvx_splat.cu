@@ -2393,6 +2393,9 @@ static gvx_status frame_upload(gvx_batch* b, const SplatKind& kind, float radius
     std::vector<uint32_t> caps(ng);
     for (size_t i = 0; i < ng; i++) {
         splat_fill(b->grids[i], kind, radius, chan_d, chan_v, 0, batch_dense(b), layers, &args[i]);
+        // (the tables of the build the splat follows, not those of the grid's present grouping)
+        args[i].leaf_dense = gvx_topo_plan_dense(b->grids[i]);
+        args[i].cell_tab = args[i].leaf_dense ? b->grids[i]->cell_tab.as<int>() : nullptr;
         if (tri_kind(kind)) batch_set_dense(b, args[i], b->f_ustart, ng);
         cnt[i] = gvx_topo_plan_slots(b->grids[i], &caps[i]);
     }

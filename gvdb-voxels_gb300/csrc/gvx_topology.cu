@@ -1600,15 +1600,26 @@ static gvx_status leaf_range_scratch(gvx_grid* g, uint32_t nleaves, ClearList& c
     return GVX_OK;
 }
 
+// the dense numbers of the leaves: in leaf_oct's buffer, after the octants of the nleaves its build made room
+// for (null: that build orders no cells)
+static int* dense_table(const gvx_grid* g, int kshift, uint32_t nleaves)
+{
+    return kshift && g->brick == 8 ? g->leaf_oct.as<int>() + (size_t)(nleaves + 1) * 8 : nullptr;
+}
+
+static void set_dense_table(gvx_grid* g, int* table)
+{
+    g->leaf_dense = table;
+    g->dense_count = table ? g->d_counts.as<uint32_t>() + kCntDense : nullptr;
+}
+
 // (nl: the leaves' neighbours too, of that many)
 static gvx_status fill_leaf_ranges(gvx_grid* g, uint32_t nleaves, const DevCount* nl = nullptr)
 {
-    const bool dense = g->key_shift && g->brick == 8;
     uint32_t* dense_list = nullptr;
-    g->leaf_dense = dense ? g->leaf_oct.as<int>() + (size_t)(nleaves + 1) * 8 : nullptr;
-    g->dense_count = dense ? g->d_counts.as<uint32_t>() + kCntDense : nullptr;
+    set_dense_table(g, dense_table(g, g->key_shift, nleaves));
     g->dense_leaves = -1;
-    if (dense) {
+    if (g->leaf_dense) {
         const size_t most = g->n_sorted / kDenseLeaf + 1;
         GVX_CK(gvx_ensure(g->cell_tab, most * 513 * sizeof(int)));  // 512 cells a leaf, then the list of the leaves
         dense_list = g->cell_tab.as<uint32_t>() + most * 512;
@@ -2685,6 +2696,11 @@ bool gvx_topo_plan_ready(const gvx_grid* g)
 
 uint64_t gvx_topo_plan_id(const gvx_grid* g) { return g->plan ? g->plan->id : 0; }
 
+int* gvx_topo_plan_dense(const gvx_grid* g)
+{
+    return g->plan ? dense_table(g, sort_shift(g->plan->fb.ks), g->plan->cap[0]) : nullptr;
+}
+
 const uint32_t* gvx_topo_plan_slots(const gvx_grid* g, uint32_t* cap)
 {
     *cap = g->plan ? g->plan->cap[0] : 0u;
@@ -2955,6 +2971,9 @@ gvx_status gvx_topo_plan_finish(gvx_grid* g, bool* held, bool frame)
     g->nbr_valid = true;
     g->sorted_buf = P.sorted_buf;
     g->n_sorted = (uint32_t)P.fb.n;
+    // (a replayed graph ran none of the host code that sets these, and another grouping may have set them since)
+    g->key_shift = sort_shift(P.fb.ks);
+    set_dense_table(g, gvx_topo_plan_dense(g));
     for (int a = 0; a < 3; a++) {
         g->sort_trans[a] = 0.f;
         g->group_trans[a] = 0.f;
