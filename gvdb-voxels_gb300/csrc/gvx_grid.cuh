@@ -67,6 +67,15 @@ __device__ inline int ll_find(const LeafLookup& L, int cx, int cy, int cz)
     return (L.cap && r >= L.cap) ? -1 : (int)r;
 }
 
+// A brick of 8's cell (voxel) that translated position w lies in: octant, then (x, y, z) inside it; org: the
+// node's first 16 bytes (lev.., x, y, z); in: whether w lies in the brick at all
+__device__ __forceinline__ int brick8_cell(const float w[3], const int4& org, bool& in)
+{
+    const int x = (int)w[0], y = (int)w[1], z = (int)w[2];
+    in = w[0] >= 0.f && w[1] >= 0.f && w[2] >= 0.f && ((x ^ org.y) | (y ^ org.z) | (z ^ org.w)) >> 3 == 0;
+    return ((x >> 2) & 1) << 8 | ((y >> 2) & 1) << 7 | ((z >> 2) & 1) << 6 | (x & 3) << 4 | (y & 3) << 2 | (z & 3);
+}
+
 // words of d_counts: 64 counts, the bounding boxes (16), the error word (16)
 enum { kReadBbox = 64, kReadErr = 80, kReadWords = 96 };
 

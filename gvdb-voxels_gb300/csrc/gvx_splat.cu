@@ -46,12 +46,26 @@ constexpr float kInvPi = 0.318309886183790671538f;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 }  // namespace
 
+// the cell order of the dense leaves (k_cell_sort), for positions read again under the same grouping; leaf_dense
+// null: there is none
+struct CellOrder {
+    const uint32_t* skeys;  // leaf key << 3 | octant
+    uint32_t invalid_key;
+    LeafLookup L;
+    const GvxNode* nodes0;
+    const int2* leaf_range;
+    const int* cell_tab;
+    int* leaf_dense;
+};
+
 // sorted point attributes: (x, y, z, weight) and (vx, vy, vz, radius); with
-// per-point radii also the largest radius (float bits, NaN counted as huge)
+// per-point radii also the largest radius (float bits, NaN counted as huge).  A leaf with a point that is not
+// in the cell it was sorted into (its position was written in place since) loses its dense number: k_tri_dense
+// takes a point to be in its cell
 __global__ void k_permute(const uint32_t* __restrict__ svals, uint32_t n, const char* pos, int poff, int pstride,
                           const char* vel, int voff, int vstride, const float* __restrict__ weight,
                           const float* __restrict__ radius, float tx, float ty, float tz, float4* spos,
-                          float4* svel, unsigned int* rmax)
+                          float4* svel, unsigned int* rmax, CellOrder co)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (radius && rmax) {
@@ -63,7 +77,8 @@ __global__ void k_permute(const uint32_t* __restrict__ svals, uint32_t n, const 
     if (i >= n) return;
     const uint32_t j = svals[i];
     const float* p = (const float*)(pos + (size_t)j * pstride + poff);
-    spos[i] = make_float4(p[0] + tx, p[1] + ty, p[2] + tz, weight ? weight[j] : 1.0f);
+    const float w[3] = {p[0] + tx, p[1] + ty, p[2] + tz};
+    spos[i] = make_float4(w[0], w[1], w[2], weight ? weight[j] : 1.0f);
     if (svel) {
         float4 v = make_float4(0.f, 0.f, 0.f, radius ? radius[j] : 0.f);
         if (vel) {
@@ -74,6 +89,19 @@ __global__ void k_permute(const uint32_t* __restrict__ svals, uint32_t n, const 
         }
         svel[i] = v;
     }
+    if (!co.leaf_dense) return;
+    const uint32_t key = co.skeys[i] >> 3;
+    if (key >= co.invalid_key) return;
+    int c[3];
+    ks_unpack(co.L.ks, key, 0, c);
+    const int leaf = ll_find(co.L, c[0], c[1], c[2]);
+    const int dense = leaf >= 0 ? co.leaf_dense[leaf] : 0;
+    if (!dense) return;
+    bool in;
+    const int cell = brick8_cell(w, *(const int4*)(co.nodes0 + leaf), in);
+    const int* ct = co.cell_tab + (size_t)(dense - 1) * 512 + cell;
+    const int end = cell == 511 ? co.leaf_range[leaf].y : ct[1];
+    if (!in || (int)i < ct[0] || (int)i >= end) co.leaf_dense[leaf] = 0;
 }
 
 struct SplatArgs {
@@ -1676,10 +1704,21 @@ gvx_status gvx_prepare_points(gvx_grid* g, int n, const float trans[3], bool nee
     rc = attr_buffers(&rmax);
     if (rc) return rc;
     if (m) {
+        CellOrder co;
+        memset(&co, 0, sizeof(co));
+        if (g->leaf_dense && g->dense_leaves != 0) {
+            co.skeys = g->keys[g->sorted_buf].as<uint32_t>();
+            co.invalid_key = 1u << g->lookup.ks.total_bits;
+            co.L = g->lookup;
+            co.nodes0 = g->nodes[0].as<GvxNode>();
+            co.leaf_range = g->leaf_range.as<int2>();
+            co.cell_tab = g->cell_tab.as<int>();
+            co.leaf_dense = g->leaf_dense;
+        }
         k_permute<<<blocks_for(m, 256), 256, 0, g->stream>>>(
             g->vals[g->sorted_buf].as<uint32_t>(), m, g->pts.pos, g->pts.pos_off, g->pts.pos_stride, g->pts.vel,
             g->pts.vel_off, g->pts.vel_stride, g->pts.weight, g->pts.radius, t[0], t[1], t[2], g->spos.as<float4>(),
-            want_svel ? g->svel.as<float4>() : nullptr, rmax);
+            want_svel ? g->svel.as<float4>() : nullptr, rmax, co);
         g->launches++;
     }
     GVX_CK(cudaGetLastError());

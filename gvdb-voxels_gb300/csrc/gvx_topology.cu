@@ -879,40 +879,54 @@ __device__ __forceinline__ void group_run(uint32_t i, const uint32_t* __restrict
 // sort of each leaf's range of sorted point indices by the cell of the point's voxel, octant first (the
 // order the keys already give), then (x, y, z) inside the octant; cell_tab gets the first sorted index
 // of every cell.  One block a leaf, every warp a contiguous part of its points, so that equal cells keep
-// their order; the leaves differ in size by factors of a hundred, the blocks take them in turn.
+// their order; the leaves differ in size by factors of a hundred, the blocks take them in turn.  A leaf
+// with a point that is no longer where its key was made (written in place since) keeps its order and gets
+// no dense number.
 constexpr int kCellThreads = 512, kCellWarps = kCellThreads / 32;
 __global__ void __launch_bounds__(kCellThreads)
     k_cell_sort(const uint32_t* __restrict__ dense_list, const uint32_t* __restrict__ dense_count,
-                const int2* __restrict__ leaf_range, const char* pos, int off, int stride, float ox, float oy, float oz,
+                const int2* __restrict__ leaf_range, const GvxNode* __restrict__ nodes0,
+                const uint32_t* __restrict__ skeys, const char* pos, int off, int stride, float ox, float oy, float oz,
                 uint32_t* vals, uint32_t* vtmp, int* __restrict__ cell_tab, int* __restrict__ leaf_dense)
 {
     __shared__ int s_cnt[kCellWarps][512];
     __shared__ int s_sum[kCellWarps];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    auto cell_of = [&](uint32_t v) {
+    auto cell_of = [&](uint32_t v, const int4& org, bool& in) {
         float w[3];
         load_pos(pos, off, stride, v, w);
-        const int x = (int)(w[0] + ox), y = (int)(w[1] + oy), z = (int)(w[2] + oz);
-        return ((x >> 2) & 1) << 8 | ((y >> 2) & 1) << 7 | ((z >> 2) & 1) << 6 | (x & 3) << 4 | (y & 3) << 2 | (z & 3);
+        w[0] += ox;
+        w[1] += oy;
+        w[2] += oz;
+        return brick8_cell(w, org, in);
     };
     const uint32_t count = *dense_count;
     for (uint32_t d = blockIdx.x; d < count; d += gridDim.x) {
         const uint32_t leaf = dense_list[d];
         const int2 r = leaf_range[leaf];
+        const int4 org = *(const int4*)(nodes0 + leaf);  // (lev.., x, y, z)
         const int per = (r.y - r.x + kCellThreads - 1) / kCellThreads * 32;  // points a warp
         const int b0 = min(r.x + warp * per, r.y), b1 = min(b0 + per, r.y);
 #pragma unroll
         for (int w = 0; w < kCellWarps; w++) s_cnt[w][tid] = 0;
         __syncthreads();
+        bool moved = false;
         for (int i0 = b0 + lane; i0 < b1; i0 += 128) {
             int c[4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) c[q] = i0 + 32 * q < b1 ? cell_of(vals[i0 + 32 * q]) : -1;
+            for (int q = 0; q < 4; q++) {
+                c[q] = -1;
+                if (i0 + 32 * q < b1) {
+                    bool in;
+                    c[q] = cell_of(vals[i0 + 32 * q], org, in);
+                    moved = moved || !in || (uint32_t)(c[q] >> 6) != (skeys[i0 + 32 * q] & 7u);
+                }
+            }
 #pragma unroll
             for (int q = 0; q < 4; q++)
                 if (c[q] >= 0) atomicAdd(&s_cnt[warp][c[q]], 1);
         }
-        __syncthreads();
+        if (__syncthreads_or(moved)) continue;
         int run = 0;  // thread c: the places of cell c's points, warp after warp
 #pragma unroll
         for (int w = 0; w < kCellWarps; w++) {
@@ -941,8 +955,9 @@ __global__ void __launch_bounds__(kCellThreads)
 #pragma unroll
             for (int q = 0; q < 4; q++) {
                 const int i = i0 + 32 * q + lane;
+                bool in;
                 v[q] = i < b1 ? vals[i] : 0u;
-                c[q] = i < b1 ? cell_of(v[q]) : -1 - lane;
+                c[q] = i < b1 ? cell_of(v[q], org, in) : -1 - lane;
             }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
@@ -1685,7 +1700,8 @@ gvx_status gvx_topo_octants(gvx_grid* g, const GvxSortedAttr* attr)
     if (g->key_shift) {
         if (g->leaf_dense && g->n_sorted >= (uint32_t)kDenseLeaf && g->dense_leaves != 0) {
             k_cell_sort<<<std::min(g->n_sorted / kDenseLeaf, 152u * 4u), kCellThreads, 0, g->stream>>>(
-                g->cell_tab.as<uint32_t>() + ((size_t)g->n_sorted / kDenseLeaf + 1) * 512, g->dense_count, g->leaf_range.as<int2>(), g->pts.pos, g->pts.pos_off,
+                g->cell_tab.as<uint32_t>() + ((size_t)g->n_sorted / kDenseLeaf + 1) * 512, g->dense_count, g->leaf_range.as<int2>(),
+                g->nodes[0].as<GvxNode>(), g->keys[g->sorted_buf].as<uint32_t>(), g->pts.pos, g->pts.pos_off,
                 g->pts.pos_stride, g->sort_trans[0], g->sort_trans[1], g->sort_trans[2],
                 g->vals[g->sorted_buf].as<uint32_t>(), g->vals[1 - g->sorted_buf].as<uint32_t>(),
                 g->cell_tab.as<int>(), g->leaf_dense);
