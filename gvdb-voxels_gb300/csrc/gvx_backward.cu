@@ -115,6 +115,19 @@ __global__ void __launch_bounds__(kBackThreads) k_splat_backward(BackArgs a)
             if (MODE == GVX_SPLAT_CUBIC && R > (float)(b - 1)) {
                 if (lane == 0) atomicOr(a.err, GVX_DERR_RADIUS);
             }
+            // a point that has left the brick of its key (written in place since the grouping): the bricks
+            // around where it is, found one by one, for this point alone
+            const int qx = (int)floorf(p.x) >> lb, qy = (int)floorf(p.y) >> lb, qz = (int)floorf(p.z) >> lb;
+            if (((qx ^ bx) | (qy ^ by) | (qz ^ bz)) != 0) {
+                bx = qx;
+                by = qy;
+                bz = qz;
+                const int leaf = lane < 27 ? ll_find(a.L, bx + lane % 3 - 1 - a.L.ks.lo[0],
+                                                     by + lane / 3 % 3 - 1 - a.L.ks.lo[1], bz + lane / 9 - 1 - a.L.ks.lo[2])
+                                           : -1;
+                myslot = leaf >= 0 ? a.leaf_slot[leaf] : -1;
+                brick_key = 0xFFFFFFFFu;
+            }
             // support box (world voxels), in the point's brick and its neighbours
             int lo[3], hi[3];
             const float pc[3] = {p.x, p.y, p.z};
