@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 #include <vector>
 
 #include "gvx_grid.cuh"
@@ -26,6 +27,17 @@ gvx_status gvx_cuda_fail(cudaError_t e, const char* what)
     // leaves the context usable (an allocation) is not reported again by a later call's launch check
     (void)cudaGetLastError();
     return GVX_ERR_DEVICE;
+}
+
+gvx_status gvx_allow_smem(const void* kernel, size_t bytes)
+{
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes a;
+    GVX_CK(cudaFuncGetAttributes(&a, kernel));
+    if ((size_t)a.maxDynamicSharedSizeBytes >= bytes) return GVX_OK;
+    GVX_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return GVX_OK;
 }
 
 static std::atomic<uint64_t> g_alloc_epoch{0};

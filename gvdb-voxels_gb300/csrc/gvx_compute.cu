@@ -248,7 +248,7 @@ extern "C" gvx_status gvx_compute(gvx_grid* g, int effect, int chan, int iterati
         } else if (effect == GVX_FUNC_SMOOTH && g->apron > 0) {
             const size_t smem = (size_t)P * P * P * sizeof(float);
             if (smem > 48 * 1024)
-                GVX_CK(cudaFuncSetAttribute(k_smooth_slots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                GVX_CK_STATUS(gvx_allow_smem((const void*)k_smooth_slots, smem));
             const unsigned grid = (unsigned)std::min<size_t>(nslots, 152u * 32u);
             k_smooth_slots<<<grid, kComputeThreads, smem, st>>>(ch.data.as<float>(), P, g->apron, nslots, params[0],
                                                                 params[1]);

@@ -156,6 +156,10 @@ gvx_status gvx_cuda_fail(cudaError_t e, const char* what);
         if (_s != GVX_OK) return _s;    \
     } while (0)
 
+// lets `kernel` be launched with `bytes` of dynamic shared memory.  The limit is the process's, and is only ever
+// raised: the launches of other threads, whose grids may need more of it, stay within it
+gvx_status gvx_allow_smem(const void* kernel, size_t bytes);
+
 cudaError_t gvx_ensure(DevBuf& b, size_t bytes);
 void gvx_free(DevBuf& b);
 // Device allocations and frees made by gvx_ensure / gvx_free in this process (a

@@ -2071,7 +2071,7 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
     if (a.nslots) {
         const SplatKernel kern = splat_kernel(kind);
         const size_t smem = splat_smem(a, kern);
-        GVX_CK(cudaFuncSetAttribute(kern.one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        GVX_CK_STATUS(gvx_allow_smem(kern.one, smem));
         int per_sm = 0;
         GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern.one, kern.warps * 32, smem));
         const uint64_t units = (uint64_t)a.nslots * a.slabs;
@@ -2289,7 +2289,7 @@ static gvx_status batch_max_blocks(gvx_batch* b, const SplatKind& k, const Splat
 {
     const SplatKernel kern = splat_kernel(k);
     const size_t smem = splat_smem(a0, kern);
-    GVX_CK(cudaFuncSetAttribute(kern.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GVX_CK_STATUS(gvx_allow_smem(kern.batch, smem));
     GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern.batch, kern.warps * 32, smem));
     *per_sm = std::max(*per_sm, 1);
     return GVX_OK;
@@ -3080,7 +3080,7 @@ gvx_status gvx_scatter_ref(gvx_grid* g, int n, float radius, const float trans[3
     a.block_points = g->brick <= 8 ? kScatterBlock : 1;
     if (g->brick <= 8) {
         const size_t tab = (size_t)kScatterWarps * (clr_mode == 1 ? 16 : clr_mode == 2 ? 4 : 0) * b3;
-        GVX_CK(cudaFuncSetAttribute(k_scatter_points, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab));
+        GVX_CK_STATUS(gvx_allow_smem((const void*)k_scatter_points, tab));
         int blocks = 0;
         GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_scatter_points, kScatterWarps * 32, tab));
         const uint32_t all = (a.nslots + kScatterWarps - 1) / kScatterWarps;
@@ -3092,7 +3092,7 @@ gvx_status gvx_scatter_ref(gvx_grid* g, int n, float radius, const float trans[3
             return GVX_OK;
         }
     }
-    GVX_CK(cudaFuncSetAttribute(k_scatter_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GVX_CK_STATUS(gvx_allow_smem((const void*)k_scatter_ref, smem));
     int per_sm = 0;
     GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scatter_ref, kSplatThreads, smem));
     const uint32_t grid = std::min<uint32_t>(a.nslots, (uint32_t)(sm_count(g->device) * std::max(per_sm, 1)));
