@@ -121,8 +121,12 @@ __global__ void k_smooth_slots(float* data, int P, int apron, size_t nslots, flo
 // slot comes in one bulk copy while the two before it are worked on, and leaves whole in another (the
 // apron as it came), so that no sector is written in part.  The block per slot above waits for its own
 // load and writes rows of 32 bytes across sectors: 54k slots 130 us, 78 here; both ways at the copy rate 67.
+// A slot whose copy does not come (the bounded wait runs out) stays as it is, with those the block had still to
+// do; the block leaves once the copies it has asked for are in, or the same limit has passed for them too.
+// withheld: a slot that is never asked for (a test's; none otherwise).
 constexpr int kSmoothThreads = 128, kSmoothStages = 3;
-__global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_t nslots, float p1, float p2, uint32_t* err)
+__global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_t nslots, float p1, float p2, uint32_t* err,
+                                                             uint32_t withheld)
 {
     constexpr int P = 10, P2 = P * P, P3 = P2 * P;
     __shared__ __align__(128) float s_in[kSmoothStages][P3 + 24], s_out[P3 + 24];
@@ -134,6 +138,7 @@ __global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_
     }
     __syncthreads();
     auto fetch = [&](uint32_t s, int k) {  // (one thread)
+        if (s == withheld) return;
         mbar_expect_tx(&s_bar[k], P3 * 4);
         bulk_g2s(s_in[k], data + (size_t)s * P3, P3 * 4, &s_bar[k]);
     };
@@ -145,12 +150,14 @@ __global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_
     const int c = (z * P + y) * P + x0;
     uint32_t phase = 0u;  // bit k: the parity stage k's next copy completes
     int k = 0;
-    for (uint64_t s = blockIdx.x; s < nslots; s += gridDim.x) {
+    uint64_t s = blockIdx.x;
+    bool late = false;
+    for (; s < nslots; s += gridDim.x) {
         // (the stage fetched into was read by every thread before the barrier at the end of the last turn)
         const uint64_t ahead = s + (uint64_t)(kSmoothStages - 1) * gridDim.x;
         if (tid == 0 && ahead < nslots) fetch((uint32_t)ahead, (k + kSmoothStages - 1) % kSmoothStages);
-        if (!mbar_wait_bounded(&s_bar[k], (phase >> k) & 1u)) atomicOr(err, GVX_DERR_TIMEOUT);
-        phase ^= 1u << k;
+        const bool came = mbar_wait_bounded(&s_bar[k], (phase >> k) & 1u);
+        if (!came) atomicOr(err, GVX_DERR_TIMEOUT);
         const float* in = s_in[k];
         float v[4];
 #pragma unroll
@@ -165,7 +172,9 @@ __global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_
             v[q] = smooth_value(v[q], p1, p2);
         }
         if (tid == 0) bulk_wait_read_all();  // the last slot has left the output buffer
-        __syncthreads();
+        late = __syncthreads_or(!came);
+        if (late) break;
+        phase ^= 1u << k;
         for (int i = tid; i < P3 / 4; i += kSmoothThreads) {
             // the apron of the four voxels i 4 .. i 4 + 3 (their interior ones are written below)
             ((float4*)s_out)[i] = ((const float4*)in)[i];
@@ -181,7 +190,19 @@ __global__ void __launch_bounds__(kSmoothThreads) k_smooth8(float* data, uint32_
         }
         k = (k + 1) % kSmoothStages;
     }
-    if (tid == 0) bulk_wait_all();
+    if (tid != 0) return;
+    for (int j = 0; late && j < kSmoothStages; j++) {
+        const int i = (k + j) % kSmoothStages;
+        if (s + (uint64_t)j * gridDim.x < nslots) (void)mbar_wait_bounded(&s_bar[i], (phase >> i) & 1u);
+    }
+    bulk_wait_all();
+}
+
+static void smooth8(gvx_grid* g, const GvxChannel& ch, float p1, float p2, uint32_t withheld)
+{
+    const unsigned grid = (unsigned)std::min<int64_t>(ch.slots, 152 * 13);
+    k_smooth8<<<grid, kSmoothThreads, 0, g->stream>>>(ch.data.as<float>(), (uint32_t)ch.slots, p1, p2,
+                                                      g->d_err.as<uint32_t>(), withheld);
 }
 
 // FUNC_SMOOTH without an apron: every voxel from its atlas neighbours in the
@@ -241,10 +262,7 @@ extern "C" gvx_status gvx_compute(gvx_grid* g, int effect, int chan, int iterati
     const unsigned flat_grid = std::min(blocks_for(nvox, kComputeThreads), 152u * 64u);
     for (int it = 0; it < iterations; it++) {
         if (effect == GVX_FUNC_SMOOTH && P == 10 && g->apron == 1 && nslots < (1u << 31)) {
-            GVX_CK(gvx_ensure(g->d_err, 64));
-            const unsigned grid = (unsigned)std::min<size_t>(nslots, 152u * 13u);
-            k_smooth8<<<grid, kSmoothThreads, 0, st>>>(ch.data.as<float>(), (uint32_t)nslots, params[0], params[1],
-                                                       g->d_err.as<uint32_t>());
+            smooth8(g, ch, params[0], params[1], 0xFFFFFFFFu);
         } else if (effect == GVX_FUNC_SMOOTH && g->apron > 0) {
             const size_t smem = (size_t)P * P * P * sizeof(float);
             if (smem > 48 * 1024)
@@ -270,5 +288,26 @@ extern "C" gvx_status gvx_compute(gvx_grid* g, int effect, int chan, int iterati
             if (rc) return rc;
         }
     }
+    return GVX_OK;
+}
+
+// test hook: one smoothing of a T_FLOAT channel of padded 10^3 bricks in which slot `slot` is never loaded (bounded
+// wait, error status at the next check, usable context)
+extern "C" gvx_status gvx_test_smooth_withheld_slot(gvx_grid* g, int chan, int64_t slot)
+{
+    if (!g) {
+        gvx_set_error("null grid handle");
+        return GVX_ERR_INVALID_ARG;
+    }
+    GVX_CK(cudaSetDevice(g->device));
+    if (chan < 0 || chan >= GVX_MAXCH || !g->ch[chan].used || g->ch[chan].type != GVX_T_FLOAT || g->P != 10 ||
+        g->apron != 1 || slot < 0 || slot >= g->ch[chan].slots || g->ch[chan].slots >= (int64_t(1) << 31)) {
+        gvx_set_error("test_smooth_withheld_slot: no such slot");
+        return GVX_ERR_INVALID_ARG;
+    }
+    apron_invalidate(g->ch[chan]);
+    smooth8(g, g->ch[chan], 4.0f, 0.1f, (uint32_t)slot);
+    g->launches++;
+    GVX_CK(cudaGetLastError());
     return GVX_OK;
 }

@@ -114,6 +114,7 @@ def load(path=None):
         "gvx_batch_frame": ([vp, f, i, f, i, i, i], i),
         "gvx_batch_frame_path": ([vp, ip, ip], i),
         "gvx_test_sort_withheld_tile": ([vp, vp, vp, vp, vp, ctypes.c_uint32], i),
+        "gvx_test_smooth_withheld_slot": ([vp, i, i64], i),
         "gvx_batch_kernel_launches": ([vp, ctypes.POINTER(i64)], i),
     }
     for name, (args, res) in sig.items():

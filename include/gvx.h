@@ -450,6 +450,12 @@ gvx_status gvx_test_sort_withheld_tile(gvx_grid* g, const uint32_t* keys_in, con
  * GVX_ERR_TIMEOUT. */
 gvx_status gvx_test_sort_noalloc_withheld_tile(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_out,
                                                uint32_t* vals_out, uint32_t n, void* stream);
+/* Test hook (no reference counterpart): one smoothing (FUNC_SMOOTH with parameters
+ * 4, 0.1, no apron update) of a T_FLOAT channel of bricks of 8 with apron 1 in
+ * which atlas slot `slot` is never loaded.  The wait for it gives up after about
+ * two seconds: the slot, and those its block had still to do, stay as they are,
+ * and the next check (gvx_sync) reports GVX_ERR_TIMEOUT. */
+gvx_status gvx_test_smooth_withheld_slot(gvx_grid* g, int chan, int64_t slot);
 gvx_status gvx_batch_kernel_launches(gvx_batch* b, int64_t* count);
 
 #ifdef __cplusplus
