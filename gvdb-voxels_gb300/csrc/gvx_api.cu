@@ -735,8 +735,7 @@ gvx_status gvx_radix_sort(gvx_grid* g, const uint32_t* keys_in, const uint32_t* 
         return GVX_ERR_INVALID_ARG;
     }
     if (n == 0) return GVX_OK;
-    GVX_CK(gvx_ensure(g->d_err, 64));
-    GVX_CK(cudaMemsetAsync(g->d_err.p, 0, 4, g->stream));
+    GVX_CK_STATUS(gvx_begin_errors(g));
     // The first pass reads the caller's input and the last one writes the caller's output (3M pairs:
     // the four copies around the passes took 30 of 238 us); buffers that overlap, and a single pair,
     // go through the grid's own

@@ -259,7 +259,7 @@ extern "C" gvx_status gvx_splat_backward_ex(gvx_grid* g, int mode, int n, float 
         gvx_set_error("SplatBackward: cubic radius %g outside (0, brick-1]", radius);
         return GVX_ERR_INVALID_ARG;
     }
-    GVX_CK(cudaMemsetAsync(g->d_err.p, 0, 4, g->stream));
+    GVX_CK_STATUS(gvx_begin_errors(g));
     // the grouping of the forward: reused when valid, else re-keyed and re-sorted.
     // GVX_BWD_RECOMPUTE drops it first, so the permutation is recomputed from the
     // positions (keys with their octants, radix sort, the sorted attributes)

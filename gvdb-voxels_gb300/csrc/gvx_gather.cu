@@ -891,9 +891,7 @@ static gvx_status insert_subcell(gvx_grid* g, int subcell, int n, float radius, 
         return GVX_ERR_CAPACITY;
     }
     cudaStream_t st = g->stream;
-    GVX_CK(gvx_ensure(g->d_err, 64));
-    GVX_CK(gvx_ensure(g->d_counts, 64 * sizeof(uint32_t)));
-    GVX_CK(cudaMemsetAsync(g->d_err.p, 0, 4, st));
+    GVX_CK_STATUS(gvx_begin_errors(g));
     const float t[3] = {trans ? trans[0] : 0.f, trans ? trans[1] : 0.f, trans ? trans[2] : 0.f};
     // mPosMin / mPosRange of the last GetBoundingBox (VG.cpp:5452-5462), host floats as the reference's
     float qmin[3], qrange[3];

@@ -1523,6 +1523,16 @@ gvx_status gvx_check_device_error(gvx_grid* g, const char* stage)
     return report_device_error(g, e, stage);
 }
 
+__global__ void k_begin_errors(uint32_t* err) { *err &= GVX_DERR_TIMEOUT; }
+
+gvx_status gvx_begin_errors(gvx_grid* g)
+{
+    k_begin_errors<<<1, 1, 0, g->stream>>>(g->d_err.as<uint32_t>());
+    g->launches++;
+    GVX_CK(cudaGetLastError());
+    return GVX_OK;
+}
+
 // The counts, the bounding boxes and the device error word in one copy through pinned staging
 // (queued: the copy; then, once the stream has passed it, readback_finish takes
 // `bytes` from word `first` of d_counts and reports the error word as above)
@@ -3143,7 +3153,7 @@ gvx_status gvx_topo_import(gvx_grid* g, int root_level, const int64_t* counts, c
     g->perm_valid = false;
     g->sc_valid = false;
     g->atlas_valid = false;
-    GVX_CK(cudaMemsetAsync(g->d_err.p, 0, 4, st));
+    GVX_CK_STATUS(gvx_begin_errors(g));
     const uint32_t words0 = std::max<uint32_t>(1u, (uint32_t)((1ull << total_bits) / 32ull));
     return build_active_lookup(g, ks, words0, kReadUsed);
 }
