@@ -2137,6 +2137,7 @@ struct gvx_batch {
     int cap_blocks = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    int64_t exec_launches = 0;  // of one replay
     cudaEvent_t ev = nullptr;
     BatchTuning tuning;
     int64_t launches = 0;
@@ -2775,8 +2776,11 @@ gvx_status gvx_batch_splat(gvx_batch* b, int mode, float radius, int chan_densit
                 batch_drop_graph(b);
                 rc = batch_upload(b, args, us);
                 if (rc) return rc;
+                const int64_t b0 = b->launches;
                 GVX_CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
                 rc = batch_launch(b, kind, args[0], (int)args.size(), blocks);
+                b->exec_launches = b->launches - b0;
+                b->launches = b0;  // counted when the graph runs
                 cudaGraph_t graph = nullptr;
                 cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
                 if (rc) {
@@ -2794,10 +2798,9 @@ gvx_status gvx_batch_splat(gvx_batch* b, int mode, float radius, int chan_densit
                 b->cap_ustart = us;
                 b->cap_kind = kind;
                 b->cap_blocks = blocks;
-                b->launches--;  // the captured launch runs with the graph below
             }
             GVX_CK(cudaGraphLaunch(b->exec, b->stream));
-            b->launches++;
+            b->launches += b->exec_launches;
         } else {
             rc = batch_upload(b, args, us);
             if (rc) return rc;
