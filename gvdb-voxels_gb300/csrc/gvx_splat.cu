@@ -132,6 +132,7 @@ struct SplatArgs {
     const unsigned int* rmax;  // per-point radii: float bits of the largest (bounds `reach` on the device)
     float max_radius;    // per-point radii above this reach past the 26 neighbours
     bool accum;
+    bool light;          // few points a unit (see kAheadUnits)
     float boundval;
     uint32_t* err;
     uint32_t* next;  // work-unit counter of the single-grid launch
@@ -414,22 +415,44 @@ __device__ __forceinline__ void unit_octants(const SplatArgs& a, SplatUnit& t, i
 // claims cost: one at a time.
 constexpr uint32_t kClaim = 2, kClaimUnits = 16;
 
+// A warp that looks ahead (below) holds up to four units, taken while others have none: with few units a warp,
+// and dense ones among them, the last ones wait in the queue of a warp that is busy while the chip runs empty.
+// So the splats of the cells' kernel look ahead where there are kAheadUnits a warp, or kAheadLight of units that
+// hold few points (SplatArgs::light), whose lookups would not be hidden otherwise.  Cubic splats of R 3.5, us
+// looking ahead / not / as it was with one unit held: 100k points in 4k bricks of 8^3 534 / 330 / 418, in 9k
+// bricks 338 / 286 / 324, in 2.7k of 16^3 326 / 210 / 283; density and velocity of R 2, 20k points in 17k
+// bricks, 11 units a warp, 78 / 92 / 87, of R 3.5, 300k points in 3.4k bricks of 16^3, 11 a warp, 1714 / 1505 /
+// 1601.
+constexpr uint32_t kAheadUnits = 16, kAheadLight = 4, kLightPoints = 1;
+
+// Blocks an SM of a launch with fewer than kFewUnits units a warp, where registers would hold more: other
+// streams' launches find room beside them.  (Frames of 300k points in 16^3 bricks, five units a warp, three in
+// flight: 584 us with the SMs full, 519 with four blocks; one at a time 686 and 796, where looking ahead took 542
+// and 940.  100k points in 8k bricks of 8^3, seven units a warp: 82 us and 99.)
+constexpr int kFewBlocks = 4;
+constexpr uint32_t kFewUnits = 6;
+
 // Units [0, total) of all grids from the counter `next`: of(u, local) -> the number of u's grid and its
 // unit there, args(k) -> that grid's arguments, range(a, t): the lane's candidates, run(a, t, k, mid): the
-// unit, which calls mid() once.  Three steps ahead of each other: while unit t is summed, the neighbours
-// (asked for as it starts) and then the candidate ranges of t1 arrive, and the brick of t2.
-template <class Of, class Args, class Range, class Run>
-__device__ __forceinline__ void unit_loop(uint32_t total, uint32_t* next, bool push, int lane, Of of, Args args,
-                                          Range range, Run run)
+// unit, which calls mid() once.  Looking ahead there are three steps at a time: while unit t is summed, the
+// neighbours (asked for as it starts) and then the candidate ranges of t1 arrive, and the brick of t2.
+// Not looking ahead, a unit is taken when the last one is done.  AHEAD: which of the two, or, where the host does
+// not know the units, as `ahead` says.
+enum { kAheadNever, kAheadAlways, kAheadAsked };
+template <int AHEAD, class Of, class Args, class Range, class Run>
+__device__ __forceinline__ void unit_loop(uint32_t total, uint32_t* next, bool push, bool ahead, int lane, Of of,
+                                          Args args, Range range, Run run)
 {
+    if (AHEAD != kAheadAsked) ahead = AHEAD == kAheadAlways;
     const int nbi = lane < 27 ? (lane % 3) * 9 + (lane / 3 % 3) * 3 + lane / 9 : -1;
     const uint32_t claim = total >= kClaimUnits * gridDim.x * (blockDim.x >> 5) ? kClaim : 1u;
-    uint32_t cur = 0u, lim = 0u, pre = lane == 0 ? atomicAdd(next, claim) : 0u, lu;
+    uint32_t cur = 0u, lim = 0u, pre = ahead && lane == 0 ? atomicAdd(next, claim) : 0u, lu;
     auto take = [&]() {  // the next unit's number (total and above: none)
         if (cur == lim) {
+            if (!ahead && lane == 0) pre = atomicAdd(next, claim);
             cur = __shfl_sync(kFull, pre, 0);
             lim = cur + claim;
-            if (lane == 0 && cur < total) pre = atomicAdd(next, claim);
+            if (ahead && lane == 0 && cur < total) pre = atomicAdd(next, claim);
         }
         return cur++;
     };
@@ -438,8 +461,11 @@ __device__ __forceinline__ void unit_loop(uint32_t total, uint32_t* next, bool p
     SplatUnit t, t1;
     uint32_t k = of(u, lu), k1;
     unit_slot(args(k), lu, push, t);
-    u = take();
-    bool more = u < total;
+    bool more = false;
+    if (ahead) {
+        u = take();
+        more = u < total;
+    }
     k1 = k;
     t1 = t;
     if (more) {
@@ -464,6 +490,16 @@ __device__ __forceinline__ void unit_loop(uint32_t total, uint32_t* next, bool p
         run(args(k), t, k, [&]() {
             if (more) range(args(k1), t1);
         });
+        if (!ahead) {
+            u = take();
+            more = u < total;
+            if (more) {
+                k1 = of(u, lu);
+                unit_slot(args(k1), lu, push, t1);
+                unit_neighbour(args(k1), t1, nbi);
+                range(args(k1), t1);
+            }
+        }
         if (!more) break;
         k = k1;
         t = t1;
@@ -950,7 +986,7 @@ __device__ __forceinline__ void cell_unit(const SplatArgs& a, const SplatUnit& t
     }
 }
 
-template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL, class Of, class Args>
+template <int AHEAD, bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL, class Of, class Args>
 __device__ __forceinline__ void cell_loop(const SplatArgs& a0, uint32_t total, uint32_t* next, unsigned char* smem, Of of,
                                          Args args)
 {
@@ -967,8 +1003,9 @@ __device__ __forceinline__ void cell_loop(const SplatArgs& a0, uint32_t total, u
     __syncwarp();
     uint32_t phase = 0;
     const int dx = lane / 9 - 1, dy = lane / 3 % 3 - 1, dz = lane % 3 - 1;
-    unit_loop(
-        total, next, push, lane, of, args,
+    const bool ahead = total >= (a0.light ? kAheadLight : kAheadUnits) * gridDim.x * kCellWarps;
+    unit_loop<AHEAD>(
+        total, next, push, ahead, lane, of, args,
         [&](const SplatArgs& a, SplatUnit& t) {
             // the neighbour's octants whose points, whose footprints reach `reach` voxels from their own,
             // can touch the tile; with per-point radii the reach is that of the largest radius (ceil R
@@ -1003,7 +1040,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t units = (a.unit_count ? min(*a.unit_count, a.nslots) : a.nslots) * (uint32_t)a.slabs;
-    cell_loop<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
+    cell_loop<kAheadAsked, HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
         a, units, a.next, smem,
         [&](uint32_t u, uint32_t& lu) {
             lu = u;
@@ -1015,8 +1052,9 @@ __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_
 // The same work over many grids in one persistent launch: the units of grid
 // k are [ustart[k], ustart[k+1]) of one global range, taken by the warps from
 // the counter ustart[ngrids + 1] (zeroed before every launch); every grid has
-// the same brick and tile shape (slab_layers, P).
-template <bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
+// the same brick and tile shape (slab_layers, P).  AHEAD: the host knows the units, or the last frame's; with both
+// ways compiled in one kernel its registers spill (24 clouds, 400k bricks, density 1.02 -> 1.12 ms).
+template <int AHEAD, bool HAS_DEN, bool HAS_VEL, int MODE, bool PPR, bool SMALL>
 __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_VEL>())
     k_splat_cells_batch(const SplatArgs* __restrict__ args, uint32_t* __restrict__ ustart, int ngrids)
 {
@@ -1025,7 +1063,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_
     for (int i = threadIdx.x; i <= ngrids; i += blockDim.x) s_us[i] = ustart[i];
     __syncthreads();
     uint32_t k = 0u;  // the last unit's grid: a warp's units come in rising order, so its search starts there
-    cell_loop<HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
+    cell_loop<AHEAD, HAS_DEN, HAS_VEL, MODE, PPR, SMALL>(
         args[0], s_us[ngrids], ustart + ngrids + 1, smem,
         [&](uint32_t u, uint32_t& lu) {
             while (s_us[k + 1] <= u) k++;
@@ -1320,8 +1358,8 @@ __device__ __forceinline__ void tri_loop(const SplatArgs& a0, uint32_t total, ui
     const bool nx = unit_halves(lane / 9 - 1, a0.brick, -a0.apron, a0.P - 1 - a0.apron, 0, 1, L.lox, L.hix);
     const bool ny = unit_halves(lane / 3 % 3 - 1, a0.brick, -a0.apron, a0.P - 1 - a0.apron, 0, 1, L.loy, L.hiy);
     L.need = nx && ny;
-    unit_loop(
-        total, next, false, lane, of, args,
+    unit_loop<kAheadAlways>(
+        total, next, false, true, lane, of, args,
         [&](const SplatArgs& a, SplatUnit& t) {
             int lz, hz;
             t.start = t.end = 0;
@@ -1764,9 +1802,9 @@ constexpr int kListDensePoints = 32768;
 // the splats of k_splat_tri
 static bool tri_kind(const SplatKind& k) { return k.mode == GVX_SPLAT_TRILINEAR && k.has_d && !k.has_v; }
 
-// the kernel of a kind (single grid, batch), its warps a block and its shared memory a warp
+// the kernel of a kind (single grid, batch, batch of few units), its warps a block and its shared memory a warp
 struct SplatKernel {
-    void *one, *batch;
+    void *one, *batch, *batch_few;
     int warps;
     size_t (*warp_bytes)(int layers, int rows, int P);
 };
@@ -1775,20 +1813,28 @@ static size_t tri_warp_bytes(int layers, int rows, int P) { return (size_t)layer
 template <bool D, bool V, int MODE, bool PPR, bool SMALL>
 static SplatKernel cell_kernel()
 {
-    return SplatKernel{(void*)k_splat_cells<D, V, MODE, PPR, SMALL>, (void*)k_splat_cells_batch<D, V, MODE, PPR, SMALL>,
-                       kCellWarps, cell_warp_bytes<D, V, MODE, PPR>};
+    return SplatKernel{(void*)k_splat_cells<D, V, MODE, PPR, SMALL>,
+                       (void*)k_splat_cells_batch<kAheadAlways, D, V, MODE, PPR, SMALL>,
+                       (void*)k_splat_cells_batch<kAheadNever, D, V, MODE, PPR, SMALL>, kCellWarps, cell_warp_bytes<D, V, MODE, PPR>};
 }
 template <bool D, bool V>
 static SplatKernel pick_kernel(const SplatKind& k)
 {
     if (k.mode == GVX_SPLAT_TRILINEAR) {
         if constexpr (D && !V)
-            return SplatKernel{(void*)k_splat_tri, (void*)k_splat_tri_batch, kTriWarps, tri_warp_bytes};
+            return SplatKernel{(void*)k_splat_tri, (void*)k_splat_tri_batch, (void*)k_splat_tri_batch, kTriWarps,
+                               tri_warp_bytes};
         else
             return cell_kernel<D, V, GVX_SPLAT_TRILINEAR, false, true>();
     }
     if (k.ppr) return cell_kernel<D, V, GVX_SPLAT_CUBIC, true, false>();
     return k.small ? cell_kernel<D, V, GVX_SPLAT_CUBIC, false, true>() : cell_kernel<D, V, GVX_SPLAT_CUBIC, false, false>();
+}
+
+// whether a launch of `warps` warps over so many units has few of them
+static bool few_units(uint64_t units, uint64_t warps, bool light)
+{
+    return units < (light ? kAheadLight : kAheadUnits) * warps;
 }
 
 static SplatKernel splat_kernel(const SplatKind& k)
@@ -1969,6 +2015,9 @@ static gvx_status push_table(gvx_grid* g)
     return GVX_OK;
 }
 
+// (an accumulating splat's units are the bricks that points reach, which the host does not know)
+static bool light_units(uint64_t points, uint64_t units, int accum) { return !accum && points < kLightPoints * units; }
+
 // validation, InsertPoints grouping and the kernel arguments of one grid's splat;
 // layers <= 0 picks the default slab height (see splat_check); dense < 0: the tile shape from the
 // grid's own points per brick, else as given (a batch decides for all its grids)
@@ -1986,6 +2035,7 @@ static gvx_status splat_prepare(gvx_grid* g, int mode, int n, float radius, cons
     // (a tile of the whole interior has at most 4096 places: bricks up to 8)
     if (slab_shape(g, accum, dn, kind->has_d && kind->has_v).push && g->brick <= 8) GVX_CK_STATUS(push_table(g));
     splat_fill(g, *kind, radius, chan_d, chan_v, accum, dn, layers, out);
+    out->light = light_units((uint64_t)n, (uint64_t)out->nslots * out->slabs, accum);
     return GVX_OK;
 }
 
@@ -2076,8 +2126,10 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
         GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern.one, kern.warps * 32, smem));
         const uint64_t units = (uint64_t)a.nslots * a.slabs;
         const uint64_t ctas_needed = (units + kern.warps - 1) / kern.warps;
-        const uint32_t grid =
-            (uint32_t)std::min<uint64_t>(ctas_needed, (uint64_t)sm_count(g->device) * std::max(per_sm, 1));
+        const uint64_t sms = (uint64_t)sm_count(g->device);
+        if (!tri_kind(kind) && !accum && units < kFewUnits * sms * kFewBlocks * kern.warps)
+            per_sm = std::min(per_sm, kFewBlocks);
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(ctas_needed, sms * std::max(per_sm, 1));
         GVX_CK(gvx_ensure(g->d_next, 3 * sizeof(uint32_t)));  // units taken, slots touched, units listed
         GVX_CK(cudaMemsetAsync(g->d_next.p, 0, 3 * sizeof(uint32_t), g->stream));
         a.next = g->d_next.as<uint32_t>();
@@ -2156,14 +2208,11 @@ struct gvx_batch {
     int f_path = 0, f_void = 0;          // how the last frame ran, its grids built again without a plan
 };
 
-static bool batch_dense(const gvx_batch* b)
+static uint64_t batch_points(const gvx_batch* b)
 {
-    uint64_t pts = 0, bricks = 0;
-    for (const gvx_grid* g : b->grids) {
-        pts += (uint64_t)(g->group_valid ? g->group_n : g->pts.n);
-        bricks += (uint64_t)g->atlas_used;
-    }
-    return dense_cloud(pts, bricks);
+    uint64_t pts = 0;
+    for (const gvx_grid* g : b->grids) pts += (uint64_t)(g->group_valid ? g->group_n : g->pts.n);
+    return pts;
 }
 
 static uint64_t batch_bricks(const gvx_batch* b)
@@ -2172,6 +2221,8 @@ static uint64_t batch_bricks(const gvx_batch* b)
     for (const gvx_grid* g : b->grids) bricks += (uint64_t)g->atlas_used;
     return bricks;
 }
+
+static bool batch_dense(const gvx_batch* b) { return dense_cloud(batch_points(b), batch_bricks(b)); }
 
 static void frame_drop_graph(gvx_batch* b)
 {
@@ -2223,8 +2274,15 @@ static void batch_set_dense(gvx_batch* b, SplatArgs& a, DevBuf& ustart, size_t n
     a.dense_list = b->dense_units.as<uint4>();
 }
 
+// the kernel of a batch's launch over `units` (a frame's: those of the last one)
+static void* batch_kernel(const SplatKernel& kern, const SplatArgs& a0, uint64_t units, int blocks)
+{
+    return few_units(units, (uint64_t)blocks * kern.warps, a0.light) ? kern.batch_few : kern.batch;
+}
+
 // one launch of the batch kernel over args/ustart already on the device
-static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, int ngrids, int blocks)
+static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs& a0, int ngrids, int blocks,
+                               uint64_t units)
 {
     const SplatKernel kern = splat_kernel(k);
     const size_t smem = splat_smem(a0, kern);
@@ -2232,7 +2290,8 @@ static gvx_status batch_launch(gvx_batch* b, const SplatKind& k, const SplatArgs
     uint32_t* dus = b->d_ustart.as<uint32_t>();
     GVX_CK(cudaMemsetAsync(dus + ngrids + 1, 0, 2 * sizeof(uint32_t), b->stream));  // units taken, units listed
     void* args[] = {(void*)&dargs, (void*)&dus, (void*)&ngrids};
-    GVX_CK(cudaLaunchKernel(kern.batch, dim3(blocks), dim3(kern.warps * 32), args, smem, b->stream));
+    GVX_CK(cudaLaunchKernel(batch_kernel(kern, a0, units, blocks), dim3(blocks), dim3(kern.warps * 32), args, smem,
+                            b->stream));
     b->launches++;
     return batch_dense_units(b, k, a0, dargs, dus + ngrids + 2);
 }
@@ -2273,6 +2332,7 @@ static gvx_status batch_tables(gvx_batch* b, int mode, float radius, int chan_d,
         }
     }
     ustart[b->grids.size()] = (uint32_t)tot;
+    for (SplatArgs& a : args) a.light = light_units(batch_points(b), tot, accum);
     return GVX_OK;
 }
 
@@ -2291,6 +2351,7 @@ static gvx_status batch_max_blocks(gvx_batch* b, const SplatKind& k, const Splat
     const SplatKernel kern = splat_kernel(k);
     const size_t smem = splat_smem(a0, kern);
     GVX_CK_STATUS(gvx_allow_smem(kern.batch, smem));
+    GVX_CK_STATUS(gvx_allow_smem(kern.batch_few, smem));
     GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern.batch, kern.warps * 32, smem));
     *per_sm = std::max(*per_sm, 1);
     return GVX_OK;
@@ -2326,7 +2387,7 @@ static gvx_status batch_tune(gvx_batch* b, int mode, float radius, int chan_d, i
             float ms = 0.f;
             for (int it = 0; it < 3 && rc == GVX_OK; it++) {
                 if (it == 1) cudaEventRecord(e0, b->stream);
-                rc = batch_launch(b, k, args[0], (int)args.size(), blocks);
+                rc = batch_launch(b, k, args[0], (int)args.size(), blocks, us.back());
             }
             if (rc) break;
             cudaEventRecord(e1, b->stream);
@@ -2436,6 +2497,8 @@ static gvx_status frame_upload(gvx_batch* b, const SplatKind& kind, float radius
         // (the tables of the build the splat follows, not those of the grid's present grouping)
         args[i].leaf_dense = gvx_topo_plan_dense(b->grids[i]);
         args[i].cell_tab = args[i].leaf_dense ? b->grids[i]->cell_tab.as<int>() : nullptr;
+        // (the bricks of the last frame)
+        args[i].light = light_units(batch_points(b), batch_bricks(b) * (uint64_t)args[i].slabs, 0);
         if (tri_kind(kind)) batch_set_dense(b, args[i], b->f_ustart, ng);
         cnt[i] = gvx_topo_plan_slots(b->grids[i], &caps[i]);
     }
@@ -2457,7 +2520,8 @@ static gvx_status frame_splat(gvx_batch* b, const SplatKind& kind, const SplatAr
     uint32_t* dus = b->f_ustart.as<uint32_t>();
     int n = ng;
     void* kargs[] = {(void*)&dargs, (void*)&dus, (void*)&n};
-    GVX_CK(cudaLaunchKernel(kern.batch, dim3(blocks), dim3(kern.warps * 32), kargs, smem, b->stream));
+    GVX_CK(cudaLaunchKernel(batch_kernel(kern, a0, batch_bricks(b) * (uint64_t)a0.slabs, blocks), dim3(blocks),
+                            dim3(kern.warps * 32), kargs, smem, b->stream));
     b->launches += 2;
     GVX_CK_STATUS(batch_dense_units(b, kind, a0, dargs, dus + ng + 2));
     // every grid's device error word (topology and splat) into its plan's record
@@ -2778,7 +2842,7 @@ gvx_status gvx_batch_splat(gvx_batch* b, int mode, float radius, int chan_densit
                 if (rc) return rc;
                 const int64_t b0 = b->launches;
                 GVX_CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-                rc = batch_launch(b, kind, args[0], (int)args.size(), blocks);
+                rc = batch_launch(b, kind, args[0], (int)args.size(), blocks, us.back());
                 b->exec_launches = b->launches - b0;
                 b->launches = b0;  // counted when the graph runs
                 cudaGraph_t graph = nullptr;
@@ -2804,7 +2868,7 @@ gvx_status gvx_batch_splat(gvx_batch* b, int mode, float radius, int chan_densit
         } else {
             rc = batch_upload(b, args, us);
             if (rc) return rc;
-            rc = batch_launch(b, kind, args[0], (int)args.size(), blocks);
+            rc = batch_launch(b, kind, args[0], (int)args.size(), blocks, us.back());
             if (rc) return rc;
         }
     }
@@ -2887,6 +2951,7 @@ gvx_status gvx_batch_frame(gvx_batch* b, float topo_radius, int mode, float radi
     a0.tile_rows = sh0.rows;
     a0.slab_layers = layers;
     a0.slabs = (sh0.span + layers - 1) / layers;
+    a0.light = light_units(batch_points(b), batch_bricks(b) * (uint64_t)a0.slabs, 0);
     uint64_t units = 0;
     for (gvx_grid* g : b->grids) {
         uint32_t cap = 0;
