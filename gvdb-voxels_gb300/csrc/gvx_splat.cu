@@ -1795,10 +1795,6 @@ struct SplatKind {
     }
 };
 
-// points from which a splat lists its dense units for a launch of their own: below, the launch would
-// cost more than one warp's half a millisecond on the densest brick that so few points can make
-constexpr int kListDensePoints = 32768;
-
 // the splats of k_splat_tri
 static bool tri_kind(const SplatKind& k) { return k.mode == GVX_SPLAT_TRILINEAR && k.has_d && !k.has_v; }
 
@@ -2133,7 +2129,10 @@ gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float
         GVX_CK(gvx_ensure(g->d_next, 3 * sizeof(uint32_t)));  // units taken, slots touched, units listed
         GVX_CK(cudaMemsetAsync(g->d_next.p, 0, 3 * sizeof(uint32_t), g->stream));
         a.next = g->d_next.as<uint32_t>();
-        const bool list_dense = tri_kind(kind) && a.cell_tab && n >= kListDensePoints;
+        // (fewer points make no dense unit, and without dense leaves, where a build has counted them, there is
+        // none: the launch that sums the listed ones takes 2 us, a warp that sums a unit of 1,500 points where it
+        // met it 140, of 30,000 4 ms)
+        const bool list_dense = tri_kind(kind) && a.cell_tab && n > kDenseCandidates && g->dense_leaves != 0;
         if (list_dense) {
             GVX_CK(gvx_ensure(g->dense_units, kDenseCap * sizeof(uint4)));
             a.dense_units = g->d_next.as<uint32_t>() + 2;
