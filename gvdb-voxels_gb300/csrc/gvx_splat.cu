@@ -1871,19 +1871,26 @@ static int clamp_layers(const SlabShape& sh, int P, size_t eb, int want)
 
 // The slab height a splat takes by itself: a push tile the brick's whole interior (one unit a brick: the
 // candidate ranges and the z pushes once), others the whole padded brick where its tile is small, else
-// half of it -- and lower slabs where that leaves fewer than kUnitsWanted units, down to two layers:
-// dealing a brick's candidates again for every slab costs less than warps without work.  Measured
+// half of it -- and lower slabs where that leaves fewer than kUnitsWanted units, down to five layers, and, but for
+// the trilinear density splat, whose units are light, to two (push tiles too) where it leaves fewer than
+// kUnitsLeast: dealing a brick's candidates again for every slab costs less than warps without work.  Measured
 // (bricks, density alone unless said): trilinear 36k of 8^3 whole 43 us, halves 65; 2.07M 2.4 / 3.3 ms;
 // 720 of them 14 us whole, 10.1 halves, 10.9 of four layers, 11.3 of two; cubic of per-point radii 1-3,
-// 238k: 0.86 ms whole, 1.13 halves, 1.67 of three layers; cubic R 3.5, 3k of 16^3: 1.42 ms whole, 0.88
-// halves, 0.77 of five layers, 0.61 of three, 0.66 of two.
-constexpr uint64_t kUnitsWanted = 152 * 24 * 3;
+// 238k: 0.86 ms whole, 1.13 halves, 1.67 of three layers; cubic of 8k points around one brick, 47 in all: R 2
+// 1.89 ms halves, 1.64 of three layers, 1.25 of two, R 6.5 22.6 / 14.5 / 9.5, with velocity 2.57 ms whole
+// interiors, 1.25 of two layers; 100k points in 729: R 3.5 0.86 ms halves, 0.48 of two layers, in 3.4k: R 2 101 us
+// halves, 109 of three layers.
+constexpr uint64_t kUnitsWanted = 152 * 24 * 3, kUnitsLeast = 152 * 24;
 constexpr size_t kWholeTile = 6 * 1024;
-static int default_layers(const SlabShape& sh, int P, size_t eb, uint64_t bricks)
+static int default_layers(const SlabShape& sh, int P, size_t eb, uint64_t bricks, bool tri)
 {
     int l = sh.push || (size_t)sh.span * sh.rows * P * eb <= kWholeTile ? sh.span : (sh.span + 1) / 2;
-    while (!sh.push && l > 5 && bricks * (uint64_t)((sh.span + l - 1) / l) < kUnitsWanted) l = (l + 1) / 2;
-    return l;
+    for (;;) {
+        const uint64_t units = bricks * (uint64_t)((sh.span + l - 1) / l);
+        const bool few = units < kUnitsWanted && !sh.push && l > 5, very_few = units < kUnitsLeast && !tri && l > 2;
+        if (!few && !very_few) return l;
+        l = (l + 1) / 2;
+    }
 }
 
 // validation of one grid's splat and its kernel kind (bricks: how many the launch covers); *layers in:
@@ -1923,7 +1930,9 @@ static gvx_status splat_check(gvx_grid* g, int mode, float radius, int chan_d, i
     }
     const int P = g->P;
     const SlabShape sh = slab_shape(g, accum, dense, has_d && has_v);
-    *layers = clamp_layers(sh, P, has_v ? 16 : 4, *layers > 0 ? *layers : default_layers(sh, P, has_v ? 16 : 4, bricks));
+    const size_t eb = has_v ? 16 : 4;
+    const bool tri = mode == GVX_SPLAT_TRILINEAR && has_d && !has_v;
+    *layers = clamp_layers(sh, P, eb, *layers > 0 ? *layers : default_layers(sh, P, eb, bricks, tri));
     if (*layers < 1) {
         gvx_set_error("Splat: a %d^2 layer of the padded brick exceeds the shared tile budget", P);
         return GVX_ERR_UNSUPPORTED;
