@@ -422,8 +422,9 @@ constexpr uint32_t kClaim = 2, kClaimUnits = 16;
 // looking ahead / not / as it was with one unit held: 100k points in 4k bricks of 8^3 534 / 330 / 418, in 9k
 // bricks 338 / 286 / 324, in 2.7k of 16^3 326 / 210 / 283; density and velocity of R 2, 20k points in 17k
 // bricks, 11 units a warp, 78 / 92 / 87, of R 3.5, 300k points in 3.4k bricks of 16^3, 11 a warp, 1714 / 1505 /
-// 1601.
-constexpr uint32_t kAheadUnits = 16, kAheadLight = 4, kLightPoints = 1;
+// 1601.  2M points of R 3 in 85k bricks, 24 a warp, 3283 / 3170 us; 24 clouds of 100k, 32 a warp, 4127 / 3486; a
+// million points of radii 1-3, 80 a warp, the same.
+constexpr uint32_t kAheadUnits = 64, kAheadLight = 4, kLightPoints = 1;
 
 // Blocks an SM of a launch with fewer than kFewUnits units a warp, where registers would hold more: other
 // streams' launches find room beside them.  (Frames of 300k points in 16^3 bricks, five units a warp, three in
