@@ -1542,6 +1542,11 @@ __global__ void __launch_bounds__(kScatterWarps * 32) k_scatter_points(ScatterAr
     }
 }
 
+// A brick a block, staged in shared memory.  RUNS: for bricks of many points, whose neighbours in the order share
+// voxels: a thread sums a run of points (see below), in 60 registers; without, in 40, two blocks more an SM (300k
+// points in 2.2k bricks 15 us with runs, 12 without; 27 bricks of thousands, in cell order, 207 us with, 1590
+// without).
+template <bool RUNS>
 __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1560,22 +1565,28 @@ __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
     __syncthreads();
     uint32_t phase = 0;
     const float r2 = a.radius * a.radius;
-    // the block's slots, a thread each: those with points enough are listed
-    for (uint64_t r = blockIdx.x; r < a.nslots; r += (uint64_t)kSplatThreads * gridDim.x) {
-        if (tid == 0) s_n = 0;
-        __syncthreads();
-        const uint64_t mine = r + (uint64_t)tid * gridDim.x;
-        if (mine < a.nslots) {
-            const int2 q = a.leaf_range[a.slot_leaf[mine]];
-            if (q.y - q.x >= a.block_points) s_list[atomicAdd(&s_n, 1)] = (uint32_t)mine;
+    // the block's slots, a thread each: those with points enough are listed (with block_points 1 the blocks are few
+    // turns long, and take their slots as they come)
+    const bool direct = a.block_points <= 1;
+    for (uint64_t r = blockIdx.x; r < a.nslots; r += (direct ? 1u : (uint64_t)kSplatThreads) * gridDim.x) {
+        int listed = 1;
+        if (!direct) {
+            if (tid == 0) s_n = 0;
+            __syncthreads();
+            const uint64_t mine = r + (uint64_t)tid * gridDim.x;
+            if (mine < a.nslots) {
+                const int2 q = a.leaf_range[a.slot_leaf[mine]];
+                if (q.y - q.x >= a.block_points) s_list[atomicAdd(&s_n, 1)] = (uint32_t)mine;
+            }
+            __syncthreads();
+            listed = s_n;
         }
-        __syncthreads();
-        const int listed = s_n;
         for (int l = 0; l < listed; l++) {
-            const uint32_t s = s_list[l];
+            const uint32_t s = direct ? (uint32_t)r : s_list[l];
             const int leaf = a.slot_leaf[s];
             const GvxNode& nd = a.nodes0[leaf];
             const int2 rg = a.leaf_range[leaf];
+            if (rg.y <= rg.x) break;  // no point: the brick is left as it is
             if (tid == 0) {
                 mbar_expect_tx(&s_bar, bytes);
                 bulk_g2s(tden, a.den + (size_t)s * P3, bytes, &s_bar);
@@ -1590,8 +1601,8 @@ __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
             if (a.clr_mode) __syncthreads();
             const float vx = (float)nd.pos[0], vy = (float)nd.pos[1], vz = (float)nd.pos[2];
             const int cnt = a.expand ? 7 : 1;
-            // a run of points a thread: those of one voxel, neighbours in a dense brick's order, are summed in
-            // registers and added to the tile once (lanes side by side in that order would add to one word)
+            // a run of points a thread (lanes side by side in a dense brick's order would add to one word): those
+            // of one voxel, neighbours in that order, are summed in registers and added to the tile once with RUNS
             const int chunk = (rg.y - rg.x + kSplatThreads - 1) / kSplatThreads;
             const int e1 = min(rg.x + (tid + 1) * chunk, rg.y);
             float sum[7];
@@ -1622,6 +1633,31 @@ __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
                 const float pix = (float)(int)px, piy = (float)(int)py, piz = (float)(int)pz;
                 if (pix < 0 || piy < 0 || piz < 0 || pix >= b || piy >= b || piz >= b) continue;
                 const int v = ((int)piz * b + (int)piy) * b + (int)pix;
+                if (!RUNS) {
+                    if (a.clr_mode) {
+                        const uint32_t pt = a.perm[e];
+                        if (a.clr_mode == 1) {
+                            const uint32_t c = *(const uint32_t*)(a.clr + (size_t)pt * (size_t)a.clr_stride + a.clr_off);
+                            atomicAdd(&tclr[v], 1u);
+                            atomicAdd(&tclr[b3 + v], c & 255u);
+                            atomicAdd(&tclr[2 * b3 + v], (c >> 8) & 255u);
+                            atomicAdd(&tclr[3 * b3 + v], (c >> 16) & 255u);
+                        } else {
+                            atomicMax((int*)&tclr[v], (int)pt);
+                        }
+                    }
+                    for (int k = 0; k < cnt; k++) {
+                        const int ox = (k == 1) ? -1 : (k == 2) ? 1 : 0;
+                        const int oy = (k == 3) ? -1 : (k == 4) ? 1 : 0;
+                        const int oz = (k == 5) ? -1 : (k == 6) ? 1 : 0;
+                        const float bx = pix + ox - px, by = piy + oy - py, bz = piz + oz - pz;
+                        const float c = (bx * bx + by * by + bz * bz) / r2;
+                        const int lx = (int)pix + ox + ap, ly = (int)piy + oy + ap, lz = (int)piz + oz + ap;
+                        if (lx < 0 || ly < 0 || lz < 0 || lx >= P || ly >= P || lz >= P) continue;
+                        atomicAdd(&tden[(lz * P + ly) * P + lx], 1.0f + c * (-3.0f + c * (3.0f - c)));
+                    }
+                    continue;
+                }
                 if (v != cur) {
                     flush();
                     cur = v, qx = (int)pix, qy = (int)piy, qz = (int)piz;
@@ -1652,7 +1688,7 @@ __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
                     sum[k] += 1.0f + c * (-3.0f + c * (3.0f - c));
                 }
             }
-            flush();
+            if (RUNS) flush();
             fence_async_smem();
             __syncthreads();
             if (tid == 0) {
@@ -1678,7 +1714,7 @@ __global__ void __launch_bounds__(kSplatThreads) k_scatter_ref(ScatterArgs a)
             if (tid == 0) bulk_wait_read_all();
             __syncthreads();
         }
-        __syncthreads();  // (the list is read before its count is cleared)
+        if (!direct) __syncthreads();  // (the list is read before its count is cleared)
     }
     if (tid == 0) bulk_wait_all();
 }
@@ -3156,8 +3192,21 @@ gvx_status gvx_scatter_ref(gvx_grid* g, int n, float radius, const float trans[3
     apron_invalidate(g->ch[0]);
     if (clr_mode) apron_invalidate(g->ch[clr_chan]);
     if (a.nslots == 0) return GVX_OK;
-    a.block_points = g->brick <= 8 ? kScatterBlock : 1;
-    if (g->brick <= 8) {
+    // (cells are in order in leaves of 128 points and more of bricks of 8)
+    const bool few = g->n_sorted < 192ull * a.nslots;
+    const void* single = few ? (const void*)k_scatter_ref<false> : (const void*)k_scatter_ref<true>;
+    int per_sm = 0;
+    GVX_CK_STATUS(gvx_allow_smem(single, smem));
+    GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, single, kSplatThreads, smem));
+    const uint32_t wave = (uint32_t)(sm_count(g->device) * std::max(per_sm, 1));
+    // The blocks' kernel alone where there is a block for every brick (8k points in 330 bricks 7 us, by the two 15),
+    // or six turns of the blocks do bricks of 16 points (300k points in 2.2k bricks 12 us, by the two 19; of 4.5,
+    // 10k points, 10 and 8), or all are its own on average.  The warps' kernel alone for so few points that a warp
+    // has them all in a few turns: nothing is gained by the other's launch (2 us).
+    const uint64_t each = a.nslots <= 6u * wave ? 16 : kScatterBlock;
+    const bool warps = g->brick <= 8 && a.nslots > wave && g->n_sorted < each * a.nslots;
+    a.block_points = !warps ? 1 : g->n_sorted < 1024u ? 1024 : kScatterBlock;
+    if (warps) {
         const size_t tab = (size_t)kScatterWarps * (clr_mode == 1 ? 16 : clr_mode == 2 ? 4 : 0) * b3;
         GVX_CK_STATUS(gvx_allow_smem((const void*)k_scatter_points, tab));
         int blocks = 0;
@@ -3171,11 +3220,12 @@ gvx_status gvx_scatter_ref(gvx_grid* g, int n, float radius, const float trans[3
             return GVX_OK;
         }
     }
-    GVX_CK_STATUS(gvx_allow_smem((const void*)k_scatter_ref, smem));
-    int per_sm = 0;
-    GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scatter_ref, kSplatThreads, smem));
+    const void* kern = warps ? (const void*)k_scatter_ref<true> : single;
+    GVX_CK_STATUS(gvx_allow_smem(kern, smem));
+    GVX_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSplatThreads, smem));
     const uint32_t grid = std::min<uint32_t>(a.nslots, (uint32_t)(sm_count(g->device) * std::max(per_sm, 1)));
-    k_scatter_ref<<<grid, kSplatThreads, smem, g->stream>>>(a);
+    void* args[] = {&a};
+    GVX_CK(cudaLaunchKernel(kern, dim3(grid), dim3(kSplatThreads), args, smem, g->stream));
     g->launches++;
     GVX_CK(cudaGetLastError());
     return GVX_OK;
