@@ -281,8 +281,9 @@ const uint32_t* gvx_topo_plan_slots(const gvx_grid* g, uint32_t* cap);
 gvx_status gvx_prepare_points(gvx_grid* g, int n, const float trans[3], bool need_svel);
 gvx_status gvx_check_device_error(gvx_grid* g, const char* stage);
 // the device error word before a call whose own errors the next check reports: a timeout that no check has
-// reported yet stays in it (what that wait was for is not in its output), other bits are dropped
-gvx_status gvx_begin_errors(gvx_grid* g);
+// reported yet stays in it (what that wait was for is not in its output), other bits are dropped.  counter
+// (optional): a device word to be zeroed by the same launch
+gvx_status gvx_begin_errors(gvx_grid* g, uint32_t* counter = nullptr);
 
 // splats (gvx_splat.cu) and gathers (gvx_gather.cu)
 gvx_status gvx_splat_run(gvx_grid* g, int mode, int n, float radius, const float trans[3], int chan_d,

@@ -1523,11 +1523,15 @@ gvx_status gvx_check_device_error(gvx_grid* g, const char* stage)
     return report_device_error(g, e, stage);
 }
 
-__global__ void k_begin_errors(uint32_t* err) { *err &= GVX_DERR_TIMEOUT; }
-
-gvx_status gvx_begin_errors(gvx_grid* g)
+__global__ void k_begin_errors(uint32_t* err, uint32_t* counter)
 {
-    k_begin_errors<<<1, 1, 0, g->stream>>>(g->d_err.as<uint32_t>());
+    *err &= GVX_DERR_TIMEOUT;
+    if (counter) *counter = 0u;
+}
+
+gvx_status gvx_begin_errors(gvx_grid* g, uint32_t* counter)
+{
+    k_begin_errors<<<1, 1, 0, g->stream>>>(g->d_err.as<uint32_t>(), counter);
     g->launches++;
     GVX_CK(cudaGetLastError());
     return GVX_OK;
