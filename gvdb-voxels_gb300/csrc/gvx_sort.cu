@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 {
     constexpr uint32_t TILE = (uint32_t)THREADS * ITEMS;
     constexpr int WARPS = THREADS / 32;
-    extern __shared__ uint32_t s_dyn[];
+    extern __shared__ __align__(16) uint32_t s_dyn[];  // (s_whist is cleared 16 bytes at a time)
     uint32_t* s_keys = s_dyn;                     // TILE
     uint32_t* s_vals = s_dyn + TILE;              // TILE
     uint32_t(*s_whist)[256] = (uint32_t(*)[256])(s_dyn + 2 * TILE);  // per warp: digit counts, then offsets
