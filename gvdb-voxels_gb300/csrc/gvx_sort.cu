@@ -5,7 +5,7 @@
 // Only the significant bits of the compact brick key are sorted (8 bits per
 // pass), the digit histograms of all passes come from one upfront count (fused
 // into the key producer when it can), and every pass is a single kernel: tile
-// ranking with warp match_any, decoupled look-back across tiles for the digit
+// ranking by warp ballots, decoupled look-back across tiles for the digit
 // offsets, then a scatter staged through shared memory so that global writes
 // of one digit bucket are contiguous.  Stable: equal keys keep input order.
 //

@@ -1090,7 +1090,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_
 //  - the hits of a round of candidates go to shared memory in order, and four of them are added at a
 //    time, eight lanes (the corners of the footprint) each; lanes that meet on a voxel add one after
 //    another in the points' order.  Every voxel's sum is that of the slab kernel, term by term;
-//  - one unit is the whole padded brick where that leaves enough units for the chip (kTriWholeBricks);
+//  - one unit is the whole padded brick where that leaves enough units for the chip (default_layers);
 //  - the next unit's brick is known, and its neighbour list, ranges and origin are asked for, while
 //    the current one is summed.
 // 24 batched clouds, 5M points, 2.07M bricks: 7.10 -> 2.37 ms (8.3 GB written: 3.5 TB/s), 100k points

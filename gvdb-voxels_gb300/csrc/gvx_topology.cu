@@ -19,7 +19,8 @@
 // each set held as a bitmap with per-word prefix popcounts, so pool order
 // (sorted direct nodes, then sorted extra nodes: the order of the reference's
 // two passes), parent indices and child-list slots are all O(1) rank lookups.
-// The host reads back 24 bytes (bounding box) and the per-level counts.
+// The host reads back the bounding box and the per-level counts, each with the
+// error word, in one copy of 384 bytes (a planned build: once, at its end).
 #include <limits.h>
 #include <math.h>
 #include <string.h>
@@ -234,7 +235,8 @@ __global__ void k_keys(const char* pos, int off, int stride, uint32_t n, float o
 // lim: per axis, the first key-space coordinate past the root (a key space rounded up to powers of two may
 // reach past it).
 // The marks used to wait for the ranks of d0bits, which numbered a mask per leaf: three launches more, and
-// two passes over the ranks (6k points a frame 96 us, 81 so; 6M points: 111 us of kernels, 90 so).
+// two passes over the ranks (6k points a frame 96 us, 81 so; 6M points: 111 us of kernels, 90 so, although
+// whole frames of them in flight went from 1.65 to 1.71 ms: the next build overlaps the last gather less).
 template <bool BOX>
 __global__ void __launch_bounds__(256)
     k_mark_cells(const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals, uint32_t n, int kshift,
@@ -2024,8 +2026,6 @@ static gvx_status topo_full_complete(gvx_grid* g, const FullBuild& fb)
     const KeySpace ks = fb.ks;
     const uint32_t words0 = fb.words0;
     const UpperDesc& ud = fb.ud;
-    const uint32_t* counts = g->d_counts.as<uint32_t>();
-    (void)counts;
     const BitRank d0{g->d0_bits.as<uint32_t>(), g->d0_prefix.as<uint32_t>(), words0};
     const BitRank x0{g->x0_bits.as<uint32_t>(), g->x0_prefix.as<uint32_t>(), words0};
     uint32_t hc[64];
@@ -2555,7 +2555,7 @@ static gvx_status rebuild_begin(gvx_grid* g, int n, float radius, const float or
     // (the device error word is not cleared here: an error left by the unchecked tail of an
     // accumulating build is reported by this build's first readback)
 
-    // ---- GetBoundingBox: one reduction, 24 bytes to the host
+    // ---- GetBoundingBox: one reduction
     ClearList clear;
     clear_bboxes(g, clear);
     GVX_CK_STATUS(gvx_clear(clear, st, &g->launches));
@@ -2775,7 +2775,6 @@ gvx_status gvx_topo_plan_make(gvx_grid* g)
 // part of topo_full_complete after the counts), every launch over the capacities
 static gvx_status plan_pools(gvx_grid* g, const gvx_topo_plan& P, const FullBuild& fb)
 {
-    cudaStream_t st = g->stream;
     const int depth = fb.depth;
     const KeySpace ks = fb.ks;
     const uint32_t words0 = fb.words0;
