@@ -61,7 +61,7 @@ __device__ __forceinline__ float sum4(float a, float b, float c, float d, int la
 }
 
 // One warp per point.  What bounds it: instruction issue (650 warp instructions a point of radius 1-3,
-// 67% of the issue slots), and, one point a claim, the counter, whose one address takes an atomic every
+// 77% of the issue slots), and, one point a claim, the counter, whose one address takes an atomic every
 // one to two nanoseconds.  So points are claimed kBackClaim at a time; they are neighbours in the sorted
 // order, and most lie in the brick of the last one, whose 27 neighbours' slots the lanes keep; a cell's
 // place in the support needs no division; dL/drho is asked for before the distances are formed.

@@ -56,7 +56,7 @@ __global__ void k_sort_hist(const uint32_t* __restrict__ keys, uint32_t n, int p
 
 // One pass over a tile of THREADS * ITEMS pairs per block.
 //
-// What bounds it: instruction issue and the chain of tiles, not HBM (16 bytes a pair and pass).
+// What bounds it: the chain of tiles and instruction issue (half of the slots), not HBM (16 bytes a pair and pass).
 // Every tile needs the digit counts of all tiles before it; the resident tiles start together, so
 // the look-back of a late tile walks over many predecessors before it meets a finished prefix.
 //  - A thread (one digit) loads kWindow predecessors at a time, independent loads in flight, and

@@ -558,8 +558,8 @@ __device__ __forceinline__ uint32_t box_regions(int xl, int xh, int yl, int yh, 
 // box meets the tile -- are gathered, in the points' order, in shared memory, and their footprints' rows
 // are dealt to the lanes.
 //
-// What bounds it: instruction issue (4M SPH frame, a launch of the same density: 63% of the issue slots,
-// 5,700 warp instructions a brick, 25.7 lanes active; of the 7,000 that a unit of the kernel before took,
+// What bounds it: instruction issue (1M points of the 4M SPH frame's density: 65% of the issue slots,
+// 6,400 warp instructions a brick, 25.7 lanes active; by ablations of the kernel before, of its 7,900,
 // 3,000 were the voxels' weights and their first turn at the tile, 1,490 the pushes, 1,090 candidates and
 // zeroing, 760 the lookups of a cell's point, 670 the further turns of lanes that share a row).  So:
 //  - candidates come as one range per neighbour and are located without a search (unit_candidate);
@@ -568,7 +568,7 @@ __device__ __forceinline__ uint32_t box_regions(int xl, int xh, int yl, int yh, 
 //  - deal_cells is in the code once: a second copy for the last hits cost more in instruction fetches
 //    (1.3 of 8 stalled cycles) than the loop around it;
 //  - a push tile's boundary voxels find their places in a table (push_table).
-// 4M points 2.53 -> 2.22 ms, 778k 461 -> 417 us, a million points of radii 1-3 without velocity 1.35 ->
+// 4M points 2.53 -> 2.19 ms, 778k 461 -> 405 us, a million points of radii 1-3 without velocity 1.35 ->
 // 0.86 ms (with whole bricks a unit).  Tried and dropped: lanes that own rows of the tile and take their
 // hits from a mask per row (3.41 ms: half the lanes idle), cells queued row by row so that lanes rarely
 // share one (3.95 ms: the queue costs more than the turns it saves), predicated stores instead of
@@ -1080,9 +1080,9 @@ __global__ void __launch_bounds__(kCellWarps * 32, cell_min_blocks<HAS_DEN, HAS_
 // TRILINEAR density alone: the splat of sparse clouds (batches of point clouds, depth frames, small
 // live clouds), 1-10 points a brick, where a brick's fixed work is most of it.
 //
-// What bounds it: instruction issue (the general slab kernel spends 2 x 1,080 warp instructions on a
-// brick of two points, 75% of the issue slots) ahead of the HBM writes of the bricks.  So, unlike
-// the cells' kernel:
+// What bounds it: the chain of a brick's lookups and candidates (about half of the issue slots are empty, with
+// 17 to 23 of 24 warps resident), ahead of the HBM writes of the bricks; the general slab kernel was bound by
+// issue (2 x 1,080 warp instructions on a brick of two points, 75% of the slots).  So, unlike the cells' kernel:
 //  - a lane's candidates are ONE range per neighbour, from its first needed octant to its last one
 //    (a superset of the needed octants, two loads instead of nine and no list of runs; the footprint
 //    test drops the others), found from a candidate's number with one warp-wide OR of the ranges'
