@@ -112,7 +112,11 @@ gvx_status gvx_fill_channel(gvx_grid* g, int chan, const float value[4]);
 /* SetPoints (VG.h:541, VG.cpp:4900-4908) + SetDataGPU (VG.cpp:4872-4880):
  * borrowed device pointers, byte offset and byte stride per point.
  * vel and clr may be NULL; clr holds 4 bytes (uchar4) per point.  All
- * pointers, offsets and strides 4-byte aligned. */
+ * pointers, offsets and strides 4-byte aligned.
+ * Positions written in place are grouped by brick again after this call (or a
+ * rebuild).  Until then a grouping made before them stands: a splat or adjoint
+ * that reads them again (after gvx_set_point_attribs) takes every point where
+ * it is now, but a splat looks for it only where its old place could reach. */
 gvx_status gvx_set_points(gvx_grid* g, int n, const void* pos, int pos_offset, int pos_stride,
                           const void* vel, int vel_offset, int vel_stride,
                           const void* clr, int clr_offset, int clr_stride);
